@@ -288,16 +288,16 @@ __device__ __forceinline__ float row_norm(const RowVec<D, GL>& r) {
   return sqrtf(group_sum<GL>(s));
 }
 
-// x[i] / n for one shared divisor: one refined reciprocal, then per element a product and one residual
-// correction (the textbook correctly-rounded division with the reciprocal shared across the row).
+// x[i] / n for one shared divisor, by Markstein's theorem (P. W. Markstein, IBM J. Res. Dev. 34(1), 1990): with y the
+// correctly rounded reciprocal of n and q = rn(x y), rn(q + rn(x - q n) y) is the correctly rounded quotient.  The
+// reciprocal is taken once for the row; two multiply-adds and a product per element.
 template <int N>
 __device__ __forceinline__ void divide_by(float (&x)[N], float n) {
-  const float r0 = __frcp_rn(n);
-  const float r = fmaf(fmaf(-n, r0, 1.0f), r0, r0);
+  const float y = __frcp_rn(n);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const float q = x[i] * r;
-    x[i] = fmaf(fmaf(-q, n, x[i]), r, q);
+    const float q = x[i] * y;
+    x[i] = fmaf(fmaf(-q, n, x[i]), y, q);
   }
 }
 
