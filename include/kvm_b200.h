@@ -258,6 +258,29 @@ int kvm_decode_step(const kvm_layer* layer, int32_t batch, kvm_decode_cache cach
                     void* out, int32_t* route_dev, void* workspace, size_t workspace_bytes,
                     void* stream);
 
+/* kvm_decode_step with its arguments in one structure that a caller fills once and keeps (between tokens only the input
+ * addresses and the launch flags change), so that a token costs the host as little as possible.  `n_append_host`, if not
+ * NULL, is the step's schedule in host memory ([batch], read before the call returns); n_append_dev is then needed only
+ * for steps at which more than 64 sequences update, and any_update only says whether there are any.  total_len_host and
+ * state_len_host, if not NULL, are the lengths the step will leave ([batch], host): with them the launch prepares itself
+ * while the previous token's kernel is still running.  (A call under stream capture reads the device's lengths.) */
+typedef struct kvm_decode_call {
+  const kvm_layer* layer;
+  int32_t batch;
+  kvm_decode_cache cache;
+  kvm_tensor4 q, k, v, gate;
+  const int32_t* n_append_dev;
+  const int32_t* n_append_host;
+  const int64_t* total_len_host;
+  const int64_t* state_len_host;
+  int32_t any_update, max_rows;
+  void* out;
+  int32_t* route_dev;
+  void* workspace;
+  size_t workspace_bytes;
+} kvm_decode_call;
+int kvm_decode_step_call(const kvm_decode_call* call, void* stream);
+
 /* Waits for `stream` and returns what the decode kernels that used `workspace` have reported since the last
  * call: KVM_OK or KVM_ERR_DEVICE_TIMEOUT (a bounded wait of the attention kernel's copy pipeline expired; the
  * kernel drained and returned, that token's output is undefined).  `layer` and `batch` as given to

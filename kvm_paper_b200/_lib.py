@@ -61,13 +61,22 @@ class KvmDecodeCache(C.Structure):
                 ("ring_gate", C.c_void_p), ("total_len", C.c_void_p), ("state_len", C.c_void_p)]
 
 
+class KvmDecodeCall(C.Structure):
+    _fields_ = [("layer", C.c_void_p), ("batch", C.c_int32), ("cache", KvmDecodeCache),
+                ("q", KvmTensor4), ("k", KvmTensor4), ("v", KvmTensor4), ("gate", KvmTensor4),
+                ("n_append_dev", C.c_void_p), ("n_append_host", C.c_void_p),
+                ("total_len_host", C.c_void_p), ("state_len_host", C.c_void_p), ("any_update", C.c_int32), ("max_rows", C.c_int32),
+                ("out", C.c_void_p), ("route_dev", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)]
+
+
 EXPORTS = [
     "kvm_prefill_workspace_bytes", "kvm_prefill_forward", "kvm_decode_workspace_bytes", "kvm_decode_step",
     "kvm_memory_refresh", "kvm_last_error_string", "kvm_abi_version", "kvm_decode_step_static", "kvm_prefill_status", "kvm_decode_run",
     "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward",
-    "kvm_prefill_forward_gathered",
+    "kvm_prefill_forward_gathered", "kvm_decode_step_call",
 ]
 STATIC_SCRATCH_BYTES = 32 << 20
+UPDATE_LIST_MAX = 64  # updating sequences that a decode launch can list by itself
 
 _lib = None
 
@@ -107,6 +116,8 @@ def load():
     lib.kvm_decode_step.argtypes = [
         LP(KvmLayer), C.c_int32, KvmDecodeCache, KvmTensor4, KvmTensor4, KvmTensor4, KvmTensor4,
         C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.kvm_decode_step_call.restype = C.c_int
+    lib.kvm_decode_step_call.argtypes = [C.c_void_p, C.c_void_p]  # (a kept kvm_decode_call, by its address)
     lib.kvm_decode_run.restype = C.c_int
     lib.kvm_decode_run.argtypes = [
         LP(KvmLayer), C.c_int32, KvmDecodeCache, C.c_int32, KvmTensor4, KvmTensor4, KvmTensor4, KvmTensor4,

@@ -15,7 +15,7 @@ cudaError_t prefill_dispatch(int D, const LayerDev& L, int batch, long long T, T
                              int s_final, int* status, unsigned phases, cudaStream_t stream, const kvm::GatherDst* gd);
 size_t update_smem_bytes(int D, int C, int capacity);
 cudaError_t decode_dispatch(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q, Tensor4 k,
-                            Tensor4 v, Tensor4 gate, const int* n_append, int any_update, int max_rows, bf16* out,
+                            Tensor4 v, Tensor4 gate, const UpdateSet& upd, const LengthSet& lens, int any_update, int max_rows, bf16* out,
                             int* route, bf16* pk_scr, float* partial, int* counters, int nslots, int overlap,
                             cudaStream_t stream);
 cudaError_t refresh_dispatch(int D, const LayerDev& L, int batch, MemoryDev mem, const int* state_len,
@@ -92,6 +92,14 @@ MemoryDev to_dev(const kvm_memory& m) {
   r.k_sum = static_cast<bf16*>(m.k_sum); r.v_sum = static_cast<bf16*>(m.v_sum); r.vlen = m.vlen;
   r.k_attn = static_cast<bf16*>(m.k_attn); r.v_attn = static_cast<bf16*>(m.v_attn); r.capacity = m.capacity;
   return r;
+}
+
+DecodeCacheDev to_dev(const kvm_decode_cache& cache) {
+  DecodeCacheDev c;
+  c.mem = to_dev(cache.memory);
+  c.ring_k = static_cast<bf16*>(cache.ring_k); c.ring_v = static_cast<bf16*>(cache.ring_v);
+  c.ring_g = static_cast<bf16*>(cache.ring_gate); c.total_len = cache.total_len; c.state_len = cache.state_len;
+  return c;
 }
 
 int check_memory(const kvm_memory& m, const kvm_layer* l) {
@@ -400,7 +408,8 @@ size_t kvm_decode_workspace_bytes(const kvm_layer* layer, int32_t batch, int32_t
 static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_decode_cache& cache, kvm_tensor4 q, kvm_tensor4 k,
                             kvm_tensor4 v, kvm_tensor4 gate, const int32_t* n_append_dev, int32_t any_update, int32_t max_rows,
                             void* out, int32_t* route_dev, void* workspace, size_t workspace_bytes, void* stream,
-                            int overlap, const char* who, bool clear_counters = false) {
+                            int overlap, const char* who, bool clear_counters = false, const int32_t* n_append_host = nullptr,
+                            const int64_t* total_host = nullptr, const int64_t* rows_host = nullptr) {
   if (int rc = check_layer(layer)) return rc;
   if (batch <= 0) return fail(KVM_ERR_BAD_ARGUMENT, "batch %d must be positive", batch);
   const int D = layer->head_dim;
@@ -413,7 +422,42 @@ static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_dec
   if (int rc = check_memory(cache.memory, layer)) return rc;
   if (!cache.ring_k || !cache.ring_v || !cache.ring_gate || !cache.total_len || !cache.state_len)
     return fail(KVM_ERR_BAD_ARGUMENT, "decode cache arrays must not be NULL");
-  if (any_update && !n_append_dev) return fail(KVM_ERR_BAD_ARGUMENT, "any_update set but n_append_dev is NULL");
+  UpdateSet upd;
+  upd.arr = n_append_dev;
+  upd.n = 0;
+  if (any_update && n_append_host) {  // the schedule is known here: it travels with the launches as a list, if it fits one
+    int n = 0;
+    for (int b = 0; b < batch; ++b) {
+      if (n_append_host[b] < 0) continue;
+      if (n_append_host[b] > layer->chunk_len) return fail(KVM_ERR_BAD_ARGUMENT, "sequence %d appends %d rows, a block has %d tokens", b, n_append_host[b], layer->chunk_len);
+      if (n < UpdateSet::kMax) {
+        upd.seq[n] = b;
+        upd.rows[n] = (short)n_append_host[b];
+      }
+      ++n;
+    }
+    any_update = n;
+    if (n <= UpdateSet::kMax) {
+      upd.arr = nullptr;
+      upd.n = n;
+    }
+  }
+  LengthSet lens;
+  lens.n = 0;
+  if (total_host && rows_host && batch <= LengthSet::kMax) {
+    // (a captured launch is replayed with whatever the device's lengths are then: no lengths are baked into it)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+      lens.n = batch;
+      for (int b = 0; b < batch; ++b) {
+        lens.total[b] = (int)total_host[b];
+        lens.rows[b] = (int)rows_host[b];
+        if (lens.total[b] <= 0 || lens.rows[b] < 0 || lens.rows[b] > cache.memory.capacity)
+          return fail(KVM_ERR_BAD_ARGUMENT, "sequence %d: %d tokens and %d memory rows do not fit the cache", b, lens.total[b], lens.rows[b]);
+      }
+    }
+  }
+  if (any_update && !upd.arr && upd.n == 0) return fail(KVM_ERR_BAD_ARGUMENT, "any_update set but n_append_dev is NULL");
   if (!out) return fail(KVM_ERR_BAD_ARGUMENT, "out is NULL");
   const int row_bound = cache.memory.capacity + layer->n_bswa_chunks * layer->chunk_len;
   if (max_rows <= 0 || max_rows > row_bound) return fail(KVM_ERR_BAD_ARGUMENT, "max_rows %d outside (0, capacity + window = %d]", max_rows, row_bound);
@@ -421,10 +465,7 @@ static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_dec
   if (!workspace || workspace_bytes < ws.total) return fail(KVM_ERR_CAPACITY, "%s: scratch of %zu bytes available, %zu needed", who, workspace_bytes, ws.total);
   if (((uintptr_t)workspace) % 256) return fail(KVM_ERR_BAD_ARGUMENT, "workspace must be 256-byte aligned");
 
-  DecodeCacheDev c;
-  c.mem = to_dev(cache.memory);
-  c.ring_k = static_cast<bf16*>(cache.ring_k); c.ring_v = static_cast<bf16*>(cache.ring_v);
-  c.ring_g = static_cast<bf16*>(cache.ring_gate); c.total_len = cache.total_len; c.state_len = cache.state_len;
+  const DecodeCacheDev c = to_dev(cache);
   unsigned char* wsb = static_cast<unsigned char*>(workspace);
   if (any_update < 0 || any_update > batch) any_update = batch;  // count unknown: no overlap
   cudaError_t e;
@@ -433,7 +474,7 @@ static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_dec
                         static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, who);
   }
-  e = decode_dispatch(D, to_dev(layer), batch, c, to_dev(q), to_dev(k), to_dev(v), to_dev(gate), n_append_dev,
+  e = decode_dispatch(D, to_dev(layer), batch, c, to_dev(q), to_dev(k), to_dev(v), to_dev(gate), upd, lens,
                                   any_update, max_rows, static_cast<bf16*>(out), route_dev,
                                   reinterpret_cast<bf16*>(wsb + ws.pk), reinterpret_cast<float*>(wsb + ws.partial),
                                   reinterpret_cast<int*>(wsb + ws.counters), ws.nsplit_max, overlap,
@@ -448,6 +489,14 @@ int kvm_decode_step(const kvm_layer* layer, int32_t batch, kvm_decode_cache cach
   g_err[0] = 0;
   return decode_step_impl(layer, batch, cache, q, k, v, gate, n_append_dev, any_update, max_rows, out, route_dev, workspace,
                           workspace_bytes, stream, 1, "kvm_decode_step");
+}
+
+int kvm_decode_step_call(const kvm_decode_call* c, void* stream) {
+  g_err[0] = 0;
+  if (!c) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_decode_step_call: call is NULL");
+  return decode_step_impl(c->layer, c->batch, c->cache, c->q, c->k, c->v, c->gate, c->n_append_dev, c->any_update, c->max_rows,
+                          c->out, c->route_dev, c->workspace, c->workspace_bytes, stream, 1, "kvm_decode_step_call", false,
+                          c->n_append_host, c->total_len_host, c->state_len_host);
 }
 
 int kvm_decode_run(const kvm_layer* layer, int32_t batch, kvm_decode_cache cache, int32_t n_steps, kvm_tensor4 q,

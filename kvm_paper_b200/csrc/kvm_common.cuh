@@ -89,6 +89,38 @@ struct DecodeCacheDev {
   int* state_len;
 };
 
+// Lengths of a decode batch AFTER the token, as the host that plans the schedule knows them: with them a launch derives
+// its work before the previous token's kernel has finished.  n = 0: not given, the kernel reads the device's lengths.
+struct LengthSet {
+  static constexpr int kMax = 256;
+  int n;
+  int total[kMax], rows[kMax];
+};
+
+// The sequences with a memory update at a decode token: either the caller's device array [batch] (-1 = none, else rows to
+// append), or, for up to kMax of them, a list that travels with the launch (no copy to the device per token).
+struct UpdateSet {
+  static constexpr int kMax = 64;
+  const int* arr;  // device array, or null: the list
+  int n;           // entries of the list (0: no sequence updates)
+  int seq[kMax];
+  short rows[kMax];
+  __device__ __forceinline__ int appended(int b) const {
+    if (arr) return arr[b];
+    for (int i = 0; i < n; ++i)
+      if (seq[i] == b) return rows[i];
+    return -1;
+  }
+  // the j-th updating sequence of the batch, -1 if there are fewer
+  __device__ __forceinline__ int nth(int j, int batch) const {
+    if (!arr) return j < n ? seq[j] : -1;
+    int cnt = 0;
+    for (int i = 0; i < batch; ++i)
+      if (arr[i] >= 0 && cnt++ == j) return i;
+    return -1;
+  }
+};
+
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll

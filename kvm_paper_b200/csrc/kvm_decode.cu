@@ -1,64 +1,34 @@
 // Decode kernels: one new token for each of `batch` sequences with ragged lengths.
-//   kvm_decode_pre_kernel   per kv row: memory update for sequences whose window start jumps at this
-//                           token (one full block leaves the window), direct memory append while the
-//                           sequence is shorter than one block, then the ring write of the new token
-//   kvm_decode_attn_kernel  persistent joint attention over [memory ; window]: every CTA streams an equal
-//                           share of all (sequence, kv head, chunk) triples with 16-byte asynchronous
-//                           copies; rows cut by a share boundary are combined by their last CTA, the
-//                           last CTA of the launch advances the sequences' lengths
+//   kvm_decode_update_kernel  per kv row: memory update for sequences whose window start jumps at this
+//                             token (one full block leaves the window)
+//   kvm_decode_attn_kernel    persistent joint attention over [memory ; window]: every CTA streams an equal
+//                             share of all (sequence, kv head, chunk) triples with tiled TMA copies; the CTA
+//                             whose share holds the chunk of a row's new token writes the token into the ring
+//                             (and, while the sequence is shorter than one block, into the memory) right before
+//                             it reads that chunk; rows cut by a share boundary are combined by their last CTA
+// A token without an update is one launch.
 // Follows model/kvm_mixer.py:572-713 (eager single-token step).
-#include <cuda.h>
-
 #include <algorithm>
 #include <mutex>
 
+#include "kvm_decode.cuh"
 #include "kvm_update.cuh"
-#include "kvm_tc.cuh"
-#include "kvm_tma_host.cuh"
 
 namespace kvm {
 
-__device__ __forceinline__ int bswa_begin_dev(int total, int C, int W) {
-  const int end = ((total + C - 1) / C) * C;
-  return max(0, end - W * C);
-}
-
-// Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may start
-// while its predecessor in the stream still runs; pdl_wait() returns once the predecessor has completed
-// and its writes are visible (at once if the launch did not carry the attribute); pdl_trigger() lets the
-// successor start early.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// ------------------------------------------------------------------------------------------- pre
-template <int D, int NT, bool UPDATE, bool SB>
+// ---------------------------------------------------------------------------------------- update
+// The grid covers the kv rows of the updating sequences only (a CTA takes a whole SM): `nc` CTAs (a thread-block
+// cluster) share one kv row, each scans its part of the memory and refreshes its share of the touched rows.
+template <int D, int NT, bool SB>
 __global__ void __launch_bounds__(NT, 1)
-kvm_decode_pre_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 k, Tensor4 v, Tensor4 gate,
-                      const int* __restrict__ n_append_arr, bf16* pk_scr, int* route, int scope, int batch, int nc) {
+kvm_decode_update_kernel(LayerDev L, DecodeCacheDev cache, const __grid_constant__ UpdateSet upd, bf16* pk_scr, int* route,
+                         int batch, int nc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // `nc` CTAs (a thread-block cluster) share one kv row of a memory update: each scans its part of the memory and
-  // refreshes its share of the touched rows; rank 0 alone writes the new token
   const int cta = (int)blockIdx.x / nc, crank = (int)blockIdx.x % nc;
-  int row = cta;
-  if (scope == 2) {
-    // Only the sequences with a memory update at this token, on a grid of just their rows (a CTA of this variant
-    // takes a whole SM: a grid over all rows would queue hundreds of CTAs that return at once behind the few SMs
-    // the attention of the other sequences leaves free): CTA j * Hkv + h belongs to the j-th updating sequence.
-    const int j = cta / L.Hkv;
-    int found = -1, cnt = 0;
-    for (int i = 0; i < batch && found < 0; ++i)
-      if (n_append_arr[i] >= 0 && cnt++ == j) found = i;
-    if (found < 0) return;
-    row = found * L.Hkv + cta % L.Hkv;
-  }
-  const int b = row / L.Hkv, h = row % L.Hkv;
-  pdl_wait();     // the previous token's attention kernel has advanced the lengths
-  pdl_trigger();  // this token's attention kernel may set itself up meanwhile
-  if (scope == 1) {  // only sequences without a memory update at this token
-    const int na = n_append_arr ? n_append_arr[b] : -1;
-    if (na >= 0) return;
-  }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = upd.nth(cta / L.Hkv, batch);  // the cta / Hkv -th updating sequence
+  if (b < 0) return;
+  const int row = b * L.Hkv + cta % L.Hkv;
+  const int n_app = upd.appended(b);
   const int C = L.C, WC = L.W * L.C;
   const int past = cache.total_len[b];
   const int S = cache.state_len[b];
@@ -70,65 +40,25 @@ kvm_decode_pre_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 k, Tensor4 v, Te
   m.vlen = cache.mem.vlen + (size_t)row * cap;
   m.k_attn = cache.mem.k_attn + (size_t)row * cap * D;
   m.v_attn = cache.mem.v_attn + (size_t)row * cap * D;
-  bf16* rk = cache.ring_k + (size_t)row * WC * D;
-  bf16* rv = cache.ring_v + (size_t)row * WC * D;
-  bf16* rg = cache.ring_g + (size_t)row * WC;
-
-  if constexpr (UPDATE) {
-    const int n_app = n_append_arr ? n_append_arr[b] : -1;
-    if (n_app >= 0) {
-      // the block [old_begin, old_begin + C) leaves the window (model/kvm_mixer.py:646-669)
-      UpdateSmem<D> s;
-      s.carve(smem_raw, C, cap, SB);
-      const int old_begin = bswa_begin_dev(past, C, L.W);
-      const int slot0 = old_begin % WC;
-      TokenSrc src;
-      src.k = rk + (size_t)slot0 * D; src.k_st = D;
-      src.v = rv + (size_t)slot0 * D; src.v_st = D;
-      src.g = rg + slot0; src.g_st = 1;
-      src.next_k = nullptr; src.next_v = nullptr;
-      ViewStore view;  // decode keeps one live copy of the attention view: rows are refreshed in place
-      view.k = m.k_attn; view.v = m.v_attn; view.cur = nullptr; view.ver_idx = nullptr; view.pool_next = 0;
-      memory_update<D, NT, SB>(L, src, m, view, cap, S, n_app, pk_scr + (size_t)row * C * D,
-                               route ? route + (size_t)row * C : nullptr, s, nc, crank);
-    }
-  }
-  // the new token (behind the update: its ring slot may be one the leaving block has just been read from; with a
-  // cluster the update ends with a cluster-wide barrier, so every CTA has read the block by now)
-  if (warp == 0 && crank == 0) {
-    const bf16* kp = k.row(b, h, 0);
-    const bf16* vp = v.row(b, h, 0);
-    const bf16 gt = *gate.row(b, h, 0);
-    RowVec<D> kr, vr;
-    load_row<D>(kr, kp, lane);
-    load_row<D>(vr, vp, lane);
-    const int slot = past % WC;
-    store_row<D>(kr, rk + (size_t)slot * D, lane);
-    store_row<D>(vr, rv + (size_t)slot * D, lane);
-    if (lane == 0) rg[slot] = gt;
-    if (past < C && S == past && past < cap) {
-      // still inside the first block: the token becomes memory row `past` directly
-      // (model/kvm_mixer.py:623-638; no gating on this path)
-      RowVec<D> pk;
-      prepare_key_row<D>(L, pk, kp, lane);
-      const float vl = row_norm<D>(vr);
-      store_row<D>(pk, m.k_sum + (size_t)past * D, lane);
-      store_row<D>(vr, m.v_sum + (size_t)past * D, lane);
-      if (lane == 0) m.vlen[past] = vl;
-      refresh_memory_row<D>(L, pk, vr, vl, m.k_attn + (size_t)past * D, m.v_attn + (size_t)past * D, lane);
-    }
-  }
+  // the block [old_begin, old_begin + C) leaves the window (model/kvm_mixer.py:646-669); its ring slots still hold it:
+  // the new token, which takes one of them, is written by the attention kernel behind this one
+  UpdateSmem<D> s;
+  s.carve(smem_raw, C, cap, SB);
+  const int slot0 = bswa_begin_dev(past, C, L.W) % WC;
+  TokenSrc src;
+  src.k = cache.ring_k + ((size_t)row * WC + slot0) * D; src.k_st = D;
+  src.v = cache.ring_v + ((size_t)row * WC + slot0) * D; src.v_st = D;
+  src.g = cache.ring_g + (size_t)row * WC + slot0; src.g_st = 1;
+  src.next_k = nullptr; src.next_v = nullptr;
+  ViewStore view;  // decode keeps one live copy of the attention view: rows are refreshed in place
+  view.k = m.k_attn; view.v = m.v_attn; view.cur = nullptr; view.ver_idx = nullptr; view.pool_next = 0;
+  memory_update<D, NT, SB>(L, src, m, view, cap, S, n_app, pk_scr + (size_t)row * C * D, route ? route + (size_t)row * C : nullptr, s,
+                           nc, crank);
 }
 
 // ------------------------------------------------------------------------------------- attention
+constexpr int kDecPrefetch = 4;                            // chunks of a CTA's range brought into L2 ahead of the previous kernel's end
 constexpr int kDecUpdateCluster = 2;                       // CTAs per kv row of a boundary update on the side stream
-constexpr int kDecConsumers = 8;                           // math warps (16 keys of every chunk each)
-constexpr int kDecThreads = (kDecConsumers + 1) * 32;      // + one producer warp
-constexpr int kDecChunk = kDecConsumers * 16;              // rows per pipeline stage
-constexpr int kDecBoxRows = 16;                            // rows per TMA box: the fetch granularity of a run's tail
-constexpr int kDecMaxBatch = 1024;                         // sequences per launch (their chunk table lives in shared memory)
-constexpr int kDecMaxSmem = 227 * 1024;   // dynamic shared memory one CTA may use (one CTA per SM)
-
 // Shared-memory layout of the attention kernel (byte offsets), for G query heads per kv head.
 // A stage holds the K rows and the V rows of one chunk as TMA boxes: for D >= 64, D/64 blocks of
 // [chunk rows][64 elements] in the 128-byte swizzle (16-byte piece c of row r at position c ^ (r % 8));
@@ -150,51 +80,6 @@ struct DecSmem {
   }
 };
 
-// Chunk geometry of one sequence's kv rows: up to three contiguous runs (memory rows, window part up to
-// the end of the ring, wrapped window part), each cut into chunks of kDecChunk rows.
-struct DecGeo {
-  int S_act, slot0, len_a, len_b, c_mem, c_a, c_b;
-  __device__ __forceinline__ int chunks() const { return c_mem + c_a + c_b; }
-};
-__device__ __forceinline__ DecGeo dec_geometry(int S, int total, int C, int W) {
-  DecGeo g;
-  const int WC = W * C;
-  const int new_begin = bswa_begin_dev(total, C, W);
-  g.S_act = new_begin > 0 ? S : 0;
-  const int n_win = total - new_begin;
-  g.slot0 = new_begin % WC;
-  g.len_a = min(n_win, WC - g.slot0);
-  g.len_b = n_win - g.len_a;
-  g.c_mem = (g.S_act + kDecChunk - 1) / kDecChunk;
-  g.c_a = (g.len_a + kDecChunk - 1) / kDecChunk;
-  g.c_b = (g.len_b + kDecChunk - 1) / kDecChunk;
-  return g;
-}
-
-// The four row arrays of the decode cache as 2-D tensors [all rows][D] with boxes of kDecBoxRows rows.
-struct DecMaps {
-  CUtensorMap mem_k, mem_v, ring_k, ring_v;
-};
-
-// byte offset of the 16-byte piece j of row r inside the K (or V) part of a stage
-template <int D>
-__device__ __forceinline__ uint32_t dec_piece(int r, int j) {
-  if constexpr (D >= 64) return (uint32_t)((j >> 3) * (kDecChunk * 128) + r * 128 + (((j & 7) ^ (r & 7)) << 4));
-  else return (uint32_t)(r * (D * 2) + j * 16);
-}
-
-// Bounded wait that also gives up when another warp of the CTA has given up.
-__device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < tc::kSpinLimit; ++i) {
-    if (tc::mbar_try_wait(bar, parity)) return true;
-    if (i >= 8) {
-      if (*abort_flag) return false;
-      __nanosleep(i < 64 ? 32 : 200);
-    }
-  }
-  return false;
-}
-
 // Joint attention of one new token per sequence over [memory ; window], persistent and bandwidth-bound.
 // All (sequence, kv head, chunk) triples of the launch form one flat list (sequence-major); every CTA
 // (one per SM) takes an equal contiguous range of it.  A producer warp streams the range through a ring
@@ -205,15 +90,18 @@ __device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, volatil
 // query heads of the kv head (G <= 16) on the N dimension, so that a kv head with few query heads costs
 // one 8-wide tile; each warp keeps a running (max, sum, output) that is merged across the warps when the
 // CTA leaves the kv row.  A row that lies inside one CTA's range is finished there; a row cut by a range
-// boundary leaves partial results [m, l, acc[D]] (fp32) and the last of its CTAs combines them.  The last
-// CTA of the launch advances the lengths of the sequences it covered (nobody reads them any more by then).
+// boundary leaves partial results [m, l, acc[D]] (fp32) and the last of its CTAs combines them.
+// The new token of a row belongs to the row's last chunk, which exactly one CTA reads: that CTA's producer writes it
+// into the ring first (a proxy fence orders the write before the TMA read behind it).  Every CTA counts itself once it
+// has read the lengths; the last to do so advances them, while the others already stream.
 // Every wait is bounded; a wait that runs out sets the status word and the CTA drains.
 // `mode`: 0 = all sequences, 1 = only sequences without a memory update at this token, 2 = only those with.
 template <int D, int ST, int NH>
 __global__ void __launch_bounds__(kDecThreads, 1)
-kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* __restrict__ n_append_arr,
-                       float* __restrict__ partial, int* __restrict__ row_counters, int* __restrict__ done_counter,
-                       int* __restrict__ status, bf16* __restrict__ out, float sm_scale, int b0, int nb, int nslots,
+kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, Tensor4 k, Tensor4 v, Tensor4 gate,
+                       const __grid_constant__ UpdateSet upd, const __grid_constant__ LengthSet lens,
+                       float* __restrict__ partial, int* __restrict__ row_counters,
+                       int* __restrict__ done_counter, int* __restrict__ status, bf16* __restrict__ out, float sm_scale, int b0, int nb, int nslots,
                        int per_min, int mode, const __grid_constant__ DecMaps maps) {
   constexpr int STRQ = D + 8;  // padded query rows: conflict-free fragment loads
   constexpr int KS = D / 16;   // k-steps of K Q^T
@@ -259,25 +147,37 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
     s_abort = 0;
     cpre[0] = 0;
   }
+  for (int h = tid; h < L.Hq; h += kDecThreads) {
+    temp_mem[h] = sm_scale * L.state_temp[h] * kLog2e;
+    temp_win[h] = sm_scale * L.front_temp[h] * kLog2e;
+  }
+  // With the lengths from the host everything up to the first copy runs while the previous token's kernel finishes;
+  // otherwise the lengths are that kernel's results and have to be waited for.
+  const bool known = lens.n > 0;
+  if (!known) {
+    pdl_wait();
+    pdl_trigger();  // the next token's kernel may be staged (it waits for this grid to complete)
+  }
   for (int b = tid; b < nb; b += kDecThreads) {
     const int B = b0 + b;
-    const int n_app = n_append_arr ? n_append_arr[B] : -1;
+    const int n_app = upd.appended(B);
     const bool in_scope = mode == 0 || (mode == 1 && n_app < 0) || (mode == 2 && n_app >= 0);
     int cnt = 0, S = 0, total = 0;
     if (in_scope) {
-      const int past = cache.total_len[B];
-      S = cache.state_len[B] + (n_app > 0 ? n_app : 0);
-      if (past < C && S == past) S += 1;  // direct append done by the pre kernel
-      total = past + 1;
+      if (known) {
+        S = lens.rows[B];
+        total = lens.total[B];
+      } else {
+        const int past = cache.total_len[B];
+        S = cache.state_len[B] + (n_app > 0 ? n_app : 0);
+        if (past < C && S == past) S += 1;  // the token becomes a memory row directly
+        total = past + 1;
+      }
       cnt = dec_geometry(S, total, C, W).chunks();
     }
     sq_S[b] = S;
     sq_tot[b] = total;
     cpre[b + 1] = cnt;
-  }
-  for (int h = tid; h < L.Hq; h += kDecThreads) {
-    temp_mem[h] = sm_scale * L.state_temp[h] * kLog2e;
-    temp_win[h] = sm_scale * L.front_temp[h] * kLog2e;
   }
   __syncthreads();
   if (warp == 0) {  // inclusive scan of cpre[1..nb], 32 entries at a time
@@ -305,10 +205,35 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
   const int f_begin = has_work ? cta * per : 0, f_end = has_work ? min(total_f, f_begin + per) : 0;
   const int nloc = f_end - f_begin;
   volatile int* abort_flag = &s_abort;
-  pdl_trigger();  // the next token's ring-write kernel may be staged (it waits for this grid to complete)
+
+  // The device's lengths.  Read from there: they may move once every CTA of the grid (also those without work) has read
+  // them; each counts itself here, behind the barrier that ended its own reads, and the last one advances them.  Known
+  // from the host: nobody reads them, the first CTA writes them.  Done by the last math warp: the producer goes straight
+  // on to its first copies.
+  if (warp == NW - 1) {
+    int writes = known && cta == 0;
+    if (known) {
+      pdl_wait();
+    } else if (lane == 0) {
+      __threadfence();
+      writes = atomicAdd(done_counter, 1) == (int)gridDim.x - 1;
+    }
+    if (__shfl_sync(0xffffffffu, writes, 0)) {
+      for (int b = lane; b < nb; b += 32) {
+        if (cpre[b + 1] != cpre[b]) {
+          cache.total_len[b0 + b] = sq_tot[b];
+          cache.state_len[b0 + b] = sq_S[b];
+        }
+      }
+      if (lane == 0 && !known) *done_counter = 0;
+    }
+  }
 
   if (!has_work) {
-    // nothing to stream
+    if (known && warp == NW) {
+      pdl_wait();
+      pdl_trigger();
+    }
   } else if (warp == NW) {
     // =============================================================== producer warp (lanes in lockstep)
     int pb, ph, pc, pcb;
@@ -326,7 +251,60 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
       pc = rem - ph * pcb;
       pg = dec_geometry(sq_S[pb], sq_tot[pb], C, W);
     }
-    pdl_wait();  // the ring rows of this token are written (everything above only needs the lengths)
+    // rows of the chunk the cursor stands on: their number, the first of them in its array, which array
+    auto chunk_rows = [&](int& n, int& y0) -> bool {
+      const int row = (b0 + pb) * Hkv + ph;
+      if (pc < pg.c_mem) {
+        n = min(CH, pg.S_act - pc * CH);
+        y0 = row * cap + pc * CH;
+        return true;
+      }
+      if (pc < pg.c_mem + pg.c_a) {
+        const int c = pc - pg.c_mem;
+        n = min(CH, pg.len_a - c * CH);
+        y0 = row * WC + pg.slot0 + c * CH;
+      } else {
+        const int c = pc - pg.c_mem - pg.c_a;
+        n = min(CH, pg.len_b - c * CH);
+        y0 = row * WC + c * CH;
+      }
+      return false;
+    };
+    auto advance = [&]() {
+      if (++pc == pcb) {
+        pc = 0;
+        if (++ph == Hkv) {
+          ph = 0;
+          ++pb;
+          while (pb < nb && cpre[pb + 1] == cpre[pb]) ++pb;
+          if (pb < nb) {
+            pcb = cpre[pb + 1] - cpre[pb];
+            pg = dec_geometry(sq_S[pb], sq_tot[pb], C, W);
+          }
+        }
+      }
+    };
+    if (known) {
+      // The previous token's kernel may still be running: nothing of its results may be read, but the rows of the first
+      // chunks can be brought into L2 (a hint: whatever that kernel still writes to them goes through L2 as well).
+      const int pb0 = pb, ph0 = ph, pc0 = pc, pcb0 = pcb;
+      const DecGeo pg0 = pg;
+      for (int i = 0; i < min(nloc, kDecPrefetch); ++i) {
+        int n, y0;
+        const bool is_mem = chunk_rows(n, y0);
+        if (lane * kDecBoxRows < n) {
+#pragma unroll
+          for (int blk = 0; blk < NBLK; ++blk) {
+            prefetch_2d(is_mem ? &maps.mem_k : &maps.ring_k, blk * 64, y0 + lane * kDecBoxRows);
+            prefetch_2d(is_mem ? &maps.mem_v : &maps.ring_v, blk * 64, y0 + lane * kDecBoxRows);
+          }
+        }
+        advance();
+      }
+      pb = pb0; ph = ph0; pc = pc0; pcb = pcb0; pg = pg0;
+      pdl_wait();
+      pdl_trigger();
+    }
     for (int i = 0; i < nloc; ++i) {
       const int s = i % ST;
       if (i >= ST) {  // the math warps are done with the chunk that used this stage
@@ -341,21 +319,15 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
       }
       const int row = (b0 + pb) * Hkv + ph;
       int n, y0;
-      const bool is_mem = pc < pg.c_mem;
-      if (is_mem) {
-        n = min(CH, pg.S_act - pc * CH);
-        y0 = row * cap + pc * CH;
-      } else if (pc < pg.c_mem + pg.c_a) {
-        const int c = pc - pg.c_mem;
-        n = min(CH, pg.len_a - c * CH);
-        y0 = row * WC + pg.slot0 + c * CH;
-      } else {
-        const int c = pc - pg.c_mem - pg.c_a;
-        n = min(CH, pg.len_b - c * CH);
-        y0 = row * WC + c * CH;
-      }
+      const bool is_mem = chunk_rows(n, y0);
       const bool first = i == 0 || pc == 0;
       const bool last = i == nloc - 1 || pc == pcb - 1;
+      if (pc == pcb - 1) {  // the chunk that ends with the row's new token
+        const int past = sq_tot[pb] - 1;
+        write_new_token<D>(L, cache, k, v, gate, b0 + pb, ph, past, past < C && sq_S[pb] == past + 1, lane);
+        fence_proxy_async_all();  // ... and is read back by a TMA copy right below
+        __syncwarp();
+      }
       const int groups = (n + kDecBoxRows - 1) / kDecBoxRows;
       if (lane == 0) {
         int seg = 0, nsegs = 1;
@@ -387,19 +359,7 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
       }
       if (first && lane < G)  // the query rows of this kv head travel with the first chunk of the row segment
         tc::bulk_g2s(qst + ((size_t)s * G + lane) * STRQ, q.row(b0 + pb, ph * G + lane, 0), D * 2, &full[s]);
-      // advance the cursor
-      if (++pc == pcb) {
-        pc = 0;
-        if (++ph == Hkv) {
-          ph = 0;
-          ++pb;
-          while (pb < nb && cpre[pb + 1] == cpre[pb]) ++pb;
-          if (pb < nb) {
-            pcb = cpre[pb + 1] - cpre[pb];
-            pg = dec_geometry(sq_S[pb], sq_tot[pb], C, W);
-          }
-        }
-      }
+      advance();
     }
   } else {
     // ==================================================================================== math warps
@@ -414,6 +374,7 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
     const int krow = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;  // ldmatrix row of the K tile
     const int vrow = warp * 16 + (lane & 7) + (lane >> 4) * 8;         // ldmatrix row of the V tile
     uint32_t fphase = 0;               // phase of the rendezvous barrier
+    // (the math warps touch global memory only behind data that the producer fetched after its own wait)
     bool alive = true;
     // all math warps meet (bounded): false if somebody gave up
     auto rendezvous = [&]() -> bool {
@@ -644,24 +605,6 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, const int* _
     for (int k2 = 0; k2 < 1000; ++k2) __nanosleep(1000);
   }
 
-  // ---- the last CTA of the launch advances the lengths of the sequences in scope: by then every CTA of the
-  //      grid (also those without work) has derived its geometry from the old lengths
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    const int prev = atomicAdd(done_counter, 1);
-    s_flag = (prev == (int)gridDim.x - 1);
-  }
-  __syncthreads();
-  if (s_flag) {
-    for (int b = tid; b < nb; b += kDecThreads) {
-      if (cpre[b + 1] != cpre[b]) {
-        cache.total_len[b0 + b] = sq_tot[b];
-        cache.state_len[b0 + b] = sq_S[b];
-      }
-    }
-    if (tid == 0) *done_counter = 0;
-  }
 }
 
 // Rebuild the attention view of rows [0, state_len[b]) from the carried sums.
@@ -680,9 +623,7 @@ __global__ void kvm_memory_refresh_kernel(LayerDev L, MemoryDev mem, const int* 
 }
 
 // ------------------------------------------------------------------------------------- host side
-constexpr int kMaxDevices = 64;  // device ordinals the per-device caches below cover
-
-static int device_sm_count() {
+int device_sm_count() {
   int dev = 0, n_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       n_sm <= 0)
@@ -700,7 +641,7 @@ static bool encode_rows_map(CUtensorMap* m, const void* base, uint64_t rows, int
 
 // The tensor maps of a decode cache (small cache keyed by the array addresses and sizes: a serving loop
 // calls with the same cache every token).
-static bool decode_maps(const DecodeCacheDev& c, uint64_t kv_rows, int cap, int WC, int D, DecMaps* out) {
+bool decode_maps(const DecodeCacheDev& c, uint64_t kv_rows, int cap, int WC, int D, DecMaps* out) {
   struct Entry {
     const void *mk, *mv, *rk, *rv;
     uint64_t kv_rows;
@@ -757,26 +698,9 @@ static DecodeSide* decode_side() {
   return &d;
 }
 
-// Launch with the programmatic-serialization attribute when `pdl` is set (see pdl_wait above).
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
-                              Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-}
-
 template <int D, int ST, int NH>
-static cudaError_t launch_decode_attn(const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q,
-                                      const int* n_append, int max_rows, bf16* out, float* partial, int* counters,
+static cudaError_t launch_decode_attn(const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q, Tensor4 k,
+                                      Tensor4 v, Tensor4 gate, const UpdateSet& upd, const LengthSet& lens, int max_rows, bf16* out, float* partial, int* counters,
                                       int nslots, int mode, int grid, const DecMaps& maps, bool pdl, int done_slot,
                                       cudaStream_t stream) {
   // The workspace holds `nslots` partial results per query head; a kv row of at most max_chunks chunks cut
@@ -800,12 +724,36 @@ static cudaError_t launch_decode_attn(const LayerDev& L, int batch, const Decode
         smem_set[dev_now] = lay.total;
       }
     }
-    cudaError_t e = launch_pdl(kern, dim3(grid), dim3(kDecThreads), lay.total, stream, pdl && batch <= kDecMaxBatch, L, cache, q,
-                               n_append, partial, counters, counters + rows + done_slot, counters + rows + batch, out,
+    cudaError_t e = launch_pdl(kern, dim3(grid), dim3(kDecThreads), lay.total, stream, pdl && batch <= kDecMaxBatch, L, cache, q, k,
+                               v, gate, upd, lens, partial, counters, counters + rows + done_slot, counters + rows + batch, out,
                                1.0f / sqrtf((float)D), b0, nb, nslots, per_min, mode, maps);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// `ctas` CTAs = clusters of `nc` per kv row of the updating sequences.
+template <int D>
+static cudaError_t launch_update(const LayerDev& L, int batch, const DecodeCacheDev& cache, const UpdateSet& upd, int ctas, int nc,
+                                 bf16* pk_scr, int* route, cudaStream_t stream) {
+  constexpr int NT = 512;
+  const bool sb = update_block_fits_smem<D>(L.C, cache.mem.capacity);
+  auto kern = sb ? kvm_decode_update_kernel<D, NT, true> : kvm_decode_update_kernel<D, NT, false>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = UpdateSmem<D>::bytes(L.C, cache.mem.capacity, sb);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = nc;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchKernelEx(&cfg, kern, L, cache, upd, pk_scr, route, batch, nc);
 }
 
 // `any_update`: number of sequences with a memory update at this token (0: none; any positive value is
@@ -813,10 +761,9 @@ static cudaError_t launch_decode_attn(const LayerDev& L, int batch, const Decode
 // side stream next to the attention of the sequences without one.
 template <int D>
 static cudaError_t launch_decode(const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q, Tensor4 k,
-                                 Tensor4 v, Tensor4 gate, const int* n_append, int any_update, int max_rows, bf16* out,
+                                 Tensor4 v, Tensor4 gate, const UpdateSet& upd, const LengthSet& lens, int any_update, int max_rows, bf16* out,
                                  int* route, bf16* pk_scr, float* partial, int* counters, int nslots,
                                  int overlap, cudaStream_t stream) {
-  constexpr int NT = 512;
   const int rows = batch * L.Hkv, G = L.Hq / L.Hkv;
   if (G > 16) return cudaErrorInvalidValue;  // the query heads of a kv head form one M=16 MMA tile
   const int n_sm = device_sm_count();
@@ -826,94 +773,54 @@ static cudaError_t launch_decode(const LayerDev& L, int batch, const DecodeCache
   if (!decode_maps(cache, (uint64_t)rows, cache.mem.capacity, L.W * L.C, D, &maps)) return cudaErrorInvalidValue;
   // `done_slot`: which launch counter of the workspace the launch uses (two launches that may run at the same
   // time need one each); `st`: the stream it goes to
-  auto attn = [&](int mode, int grid, const int* na, bool pdl = false, int done_slot = 0, cudaStream_t st = nullptr) {
+  auto attn = [&](int mode, int grid, bool pdl = false, int done_slot = 0, cudaStream_t st = nullptr) {
     if (st == nullptr) st = stream;
     if (G <= 8)
-      return st3 ? launch_decode_attn<D, 3, 1>(L, batch, cache, q, na, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st)
-                 : launch_decode_attn<D, 2, 1>(L, batch, cache, q, na, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st);
-    return st3 ? launch_decode_attn<D, 3, 2>(L, batch, cache, q, na, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st)
-               : launch_decode_attn<D, 2, 2>(L, batch, cache, q, na, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st);
+      return st3 ? launch_decode_attn<D, 3, 1>(L, batch, cache, q, k, v, gate, upd, lens, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st)
+                 : launch_decode_attn<D, 2, 1>(L, batch, cache, q, k, v, gate, upd, lens, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st);
+    return st3 ? launch_decode_attn<D, 3, 2>(L, batch, cache, q, k, v, gate, upd, lens, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st)
+               : launch_decode_attn<D, 2, 2>(L, batch, cache, q, k, v, gate, upd, lens, max_rows, out, partial, counters, nslots, mode, grid, maps, pdl, done_slot, st);
   };
   cudaError_t e;
-  {
-    // The ring-write kernel runs between attention kernels that use nearly all shared memory of an SM:
-    // give it the same shared-memory carve-out so that the SMs are not reconfigured twice per token.
-    static bool carve_set[kMaxDevices] = {false};
-    static std::mutex mu;
-    int dev_now = 0;
-    if (cudaGetDevice(&dev_now) == cudaSuccess && dev_now >= 0 && dev_now < kMaxDevices) {
-      std::lock_guard<std::mutex> lock(mu);
-      if (!carve_set[dev_now]) {
-        cudaFuncSetAttribute(kvm_decode_pre_kernel<D, 32, false, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        carve_set[dev_now] = true;
-      }
-    }
-  }
-  if (!any_update) {
-    // plain token: the two kernels are chained with programmatic dependent launches (`overlap` callers only)
-    const bool pdl = overlap != 0;
-    e = launch_pdl(kvm_decode_pre_kernel<D, 32, false, false>, dim3(rows), dim3(32), 0, stream, pdl, L, cache, k, v, gate,
-                   (const int*)nullptr, pk_scr, route, 0, batch, 1);
-    if (e != cudaSuccess) return e;
-    return attn(0, n_sm, nullptr, pdl);
-  }
-  const bool sb = update_block_fits_smem<D>(L.C, cache.mem.capacity);
-  const size_t smem_u = UpdateSmem<D>::bytes(L.C, cache.mem.capacity, sb);
-  auto upd = sb ? kvm_decode_pre_kernel<D, NT, true, true> : kvm_decode_pre_kernel<D, NT, true, false>;
-  e = cudaFuncSetAttribute(upd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_u);
-  if (e != cudaSuccess) return e;
+  // plain token: consecutive tokens are chained with programmatic dependent launches (`overlap` callers only)
+  if (!any_update) return attn(0, n_sm, overlap != 0);
   // A cluster of CTAs per updating kv row while the updating rows are few (the update is a chain of short phases:
   // more CTAs per row shorten it, and the updated sequences' attention behind it gets their SMs)
   int nc = 1;
   for (int c = kDecUpdateCluster; c > 1; c >>= 1)
     if (any_update * L.Hkv * c * 4 <= n_sm) { nc = c; break; }
-  const int upd_sms = any_update * L.Hkv * nc;  // SMs the updating rows occupy (one CTA each)
-  DecodeSide* side = (overlap && any_update < batch && upd_sms * 2 <= n_sm) ? decode_side() : nullptr;
-  if (!side) {  // one stream: update + ring write for every row, then attention over everything
-    upd<<<rows, NT, smem_u, stream>>>(L, cache, k, v, gate, n_append, pk_scr, route, 0, batch, 1);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return attn(0, n_sm, n_append);
+  const int upd_ctas = any_update * L.Hkv * nc;  // SMs the updating rows occupy (one CTA each)
+  DecodeSide* side = (overlap && any_update < batch && upd_ctas * 2 <= n_sm) ? decode_side() : nullptr;
+  // (on one stream a caller's device array decides which sequences update, whatever count came with it)
+  if (!side && upd.arr) nc = 1;
+  const int upd_grid = !side && upd.arr ? rows : upd_ctas;
+  auto update = [&](cudaStream_t st) { return launch_update<D>(L, batch, cache, upd, upd_grid, nc, pk_scr, route, st); };
+  if (!side) {  // one stream: the updates, then attention over everything
+    if ((e = update(stream)) != cudaSuccess) return e;
+    return attn(0, n_sm);
   }
   // fork: the updating sequences' rows on the side stream ...
   if ((e = cudaEventRecord(side->fork, stream)) != cudaSuccess) return e;
   if ((e = cudaStreamWaitEvent(side->stream, side->fork, 0)) != cudaSuccess) return e;
-  {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(upd_sms);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem_u;
-    cfg.stream = side->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = nc;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if ((e = cudaLaunchKernelEx(&cfg, upd, L, cache, k, v, gate, n_append, pk_scr, route, 2, batch, nc)) != cudaSuccess) return e;
-  }
+  if ((e = update(side->stream)) != cudaSuccess) return e;
   // ... followed there by their attention, on the SMs the update leaves (second launch counter of the workspace;
   // the two attention launches touch disjoint sequences, rows, partial slots and outputs)
-  if ((e = attn(2, upd_sms, n_append, false, 1, side->stream)) != cudaSuccess) return e;
+  if ((e = attn(2, upd_ctas, false, 1, side->stream)) != cudaSuccess) return e;
   if ((e = cudaEventRecord(side->join, side->stream)) != cudaSuccess) return e;
-  // ... next to the ring write and the attention of all others, which leave those SMs free
-  kvm_decode_pre_kernel<D, 32, false, false><<<rows, 32, 0, stream>>>(L, cache, k, v, gate, n_append, pk_scr, route, 1, batch, 1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = attn(1, n_sm - upd_sms, n_append)) != cudaSuccess) return e;
+  // ... next to the attention of all others, which leaves those SMs free
+  if ((e = attn(1, n_sm - upd_ctas)) != cudaSuccess) return e;
   // join
   return cudaStreamWaitEvent(stream, side->join, 0);
 }
 
 cudaError_t decode_dispatch(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q, Tensor4 k,
-                            Tensor4 v, Tensor4 gate, const int* n_append, int any_update, int max_rows, bf16* out,
+                            Tensor4 v, Tensor4 gate, const UpdateSet& upd, const LengthSet& lens, int any_update, int max_rows, bf16* out,
                             int* route, bf16* pk_scr, float* partial, int* counters, int nslots, int overlap,
                             cudaStream_t stream) {
   switch (D) {
-    case 32: return launch_decode<32>(L, batch, cache, q, k, v, gate, n_append, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
-    case 64: return launch_decode<64>(L, batch, cache, q, k, v, gate, n_append, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
-    case 128: return launch_decode<128>(L, batch, cache, q, k, v, gate, n_append, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
+    case 32: return launch_decode<32>(L, batch, cache, q, k, v, gate, upd, lens, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
+    case 64: return launch_decode<64>(L, batch, cache, q, k, v, gate, upd, lens, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
+    case 128: return launch_decode<128>(L, batch, cache, q, k, v, gate, upd, lens, any_update, max_rows, out, route, pk_scr, partial, counters, nslots, overlap, stream);
   }
   return cudaErrorInvalidValue;
 }

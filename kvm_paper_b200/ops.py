@@ -25,8 +25,13 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+# address of a device's current stream: the raw query of the torch build, or the stream object where a build lacks it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+
+
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    i = device.index
+    return _raw_stream(torch.cuda.current_device() if i is None else i)
 
 
 def _tensor4(t: torch.Tensor, name: str) -> KvmTensor4:
@@ -48,6 +53,18 @@ def _as_bf16_view(t: torch.Tensor) -> torch.Tensor:
         t = t.to(torch.bfloat16)
     if t.size(-1) > 1 and t.stride(-1) != 1:
         t = t.contiguous()
+    return t
+
+
+def _fill_tensor4(dst: KvmTensor4, t: torch.Tensor, name: str) -> torch.Tensor:
+    """``_tensor4`` into a kept C descriptor; returns the tensor the descriptor points into."""
+    st = t.stride()
+    if t.dtype is not torch.bfloat16 or (st[3] != 1 and t.size(3) > 1):
+        t = _as_bf16_view(t)
+        st = t.stride()
+    if not t.is_cuda:
+        raise RuntimeError(f"{name} must live on a CUDA device")
+    dst.ptr, dst.stride_b, dst.stride_h, dst.stride_t = t.data_ptr(), st[0], st[1], st[2]
     return t
 
 
@@ -469,6 +486,7 @@ class KvmDecodeCache:
     lengths on the device; ``logical_state_dict`` returns the reference's eager cache layout."""
 
     cache_representation = "preallocated memory rows + W*C-token ring, per-sequence lengths on device"
+    _quiet = 0
 
     def __init__(self, params: LayerParams, batch: int, state_capacity: int,
                  desired_state_len: Callable[[int, int, int], int], owner: Any = None):
@@ -492,6 +510,10 @@ class KvmDecodeCache:
         self.out = torch.empty(batch, 1, cfg.n_q_heads * cfg.head_dim, **kw)
         self.route = None
         self._last_any_update, self._last_n_append = False, None
+        self._quiet = 0  # tokens until the next one that may update a memory or grow one directly (see _plan_step)
+        self._max_rows = 0
+        self._q_shape = (self.batch, cfg.n_q_heads, 1, cfg.head_dim)
+        self._kv_shape = (self.batch, cfg.n_kv_heads, 1, cfg.head_dim)
         self._n_append = torch.full((batch,), -1, device=dev, dtype=torch.int32)
         # host staging of the per-step append counts: a small ring of pinned buffers, each guarded by an event
         # recorded behind its copy, so that a later step never overwrites a buffer the copy engine still reads
@@ -506,6 +528,15 @@ class KvmDecodeCache:
         self._ws_bytes = lib.kvm_decode_workspace_bytes(C.byref(self.params.c), self.batch, self._max_rows_bound)
         # the counter region at the head of the workspace must start at zero; the kernels leave it zero
         self._ws = torch.zeros(self._ws_bytes, device=self.device, dtype=torch.uint8)
+        # the kept argument block of kvm_decode_step_call; between tokens only input addresses and launch flags change
+        call = self._call = _lib.KvmDecodeCall()
+        call.layer, call.batch = C.addressof(self.params.c), self.batch
+        call.cache = _CCache(self.memory.c(), self.ring_k.data_ptr(), self.ring_v.data_ptr(), self.ring_gate.data_ptr(),
+                             self.total_len.data_ptr(), self.state_len.data_ptr())
+        call.n_append_dev = self._n_append.data_ptr()
+        call.total_len_host, call.state_len_host = self.total_len_h.ctypes.data, self.state_len_h.ctypes.data
+        call.out, call.workspace, call.workspace_bytes = self.out.data_ptr(), self._ws.data_ptr(), self._ws_bytes
+        self._call_args = (C.addressof(call), call.q, call.k, call.v, call.gate)
 
     # -- construction ---------------------------------------------------------------------------
     def load_sequence(self, b: int, *, k_sum, v_sum, vlen, window_k, window_v, window_gate, total_len: int,
@@ -533,10 +564,12 @@ class KvmDecodeCache:
         self.ring_gate[rows].index_copy_(1, slots, window_gate.reshape(Hkv, R).to(self.device, torch.bfloat16))
         self.total_len_h[b] = total_len
         self.state_len_h[b] = S
+        self._quiet = 0
 
     def commit_lengths(self, refresh_attention_view: bool = False):
         """Upload the host-side lengths after ``load_sequence`` calls; optionally rebuild
         ``k_attn`` / ``v_attn`` from the carried sums (when those were not supplied)."""
+        self._quiet = 0
         self.total_len.copy_(torch.from_numpy(self.total_len_h.astype(np.int32)))
         self.state_len.copy_(torch.from_numpy(self.state_len_h.astype(np.int32)))
         if refresh_attention_view:
@@ -554,71 +587,92 @@ class KvmDecodeCache:
     # -- schedule -------------------------------------------------------------------------------
     def _plan_step(self):
         """Host bookkeeping of one token: which sequences run a memory update and how many rows it
-        appends (reference: model/kvm_mixer.py:617-669).  Returns (n_append array or None, max_rows)."""
+        appends (reference: model/kvm_mixer.py:617-669).  Returns (n_append array or None, max_rows).
+        Between block boundaries of any sequence nothing but the lengths moves: every sequence has one more token in its
+        window.  The walk over the batch is skipped for those tokens (``_quiet`` of them are left)."""
+        if self._quiet > 0:
+            self._quiet -= 1
+            self.total_len_h += 1
+            self._max_rows += 1
+            return None, self._max_rows
         cfg = self.cfg
         Cn, W = cfg.chunk_len, cfg.n_bswa_chunks
         tl, sl = self.total_len_h, self.state_len_h
         cross = (tl % Cn == 0) & (tl // Cn > W)
         n_app = None
         if cross.any():
-            n_app = np.full(self.batch, -1, dtype=np.int32)
-            for b in np.nonzero(cross)[0]:
-                cov = int(tl[b]) - W * Cn          # coverage before this step
-                cur = int(sl[b])
-                desired = int(self.desired_state_len(W * Cn + cov, cov + Cn, cur))
-                na = min(max(desired - cur, 0), Cn)
-                if cur + na <= min(cfg.sink_len, cur + na) and na < Cn:
-                    raise AssertionError("KVM state update requires at least one non-sink slot before merging.")
-                n_app[b] = na
-                sl[b] = cur + na
-            self.update_count += int(cross.sum())
+            n_app = self._plan_updates(np.nonzero(cross)[0])
         direct = (tl < Cn) & (sl == tl)
         sl[direct] += 1
         tl += 1
         begin = np.maximum(0, ((tl + Cn - 1) // Cn) * Cn - W * Cn)
         rows = np.where(begin > 0, sl, 0) + (tl - begin)
-        return n_app, int(rows.max())
+        self._max_rows = int(rows.max())
+        self._quiet = 0 if tl.min() < Cn else int((-tl % Cn).min())
+        return n_app, self._max_rows
+
+    def _plan_updates(self, seqs):
+        """The memory updates of the given sequences, which stand at a block boundary: the rows each appends, [batch]
+        int32 with -1 for all others; their host lengths grow."""
+        cfg = self.cfg
+        Cn, W = cfg.chunk_len, cfg.n_bswa_chunks
+        n_app = np.full(self.batch, -1, dtype=np.int32)
+        for b in seqs:
+            cov = int(self.total_len_h[b]) - W * Cn   # coverage before this step
+            cur = int(self.state_len_h[b])
+            desired = int(self.desired_state_len(W * Cn + cov, cov + Cn, cur))
+            na = min(max(desired - cur, 0), Cn)
+            if cur + na <= min(cfg.sink_len, cur + na) and na < Cn:
+                raise AssertionError("KVM state update requires at least one non-sink slot before merging.")
+            n_app[b] = na
+            self.state_len_h[b] = cur + na
+        self.update_count += len(seqs)
+        return n_app
 
     # -- one token ------------------------------------------------------------------------------
     def step(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, *,
              want_route: bool = False) -> torch.Tensor:
         """One decode token for every sequence: q [B,Hq,1,D], k/v [B,Hkv,1,D], gate [B,Hkv,1,1].
         Returns [B,1,Hq*D] (a buffer owned by the cache, overwritten by the next step)."""
-        lib = _lib.load()
-        cfg = self.cfg
-        B = self.batch
-        if q.shape != (B, cfg.n_q_heads, 1, cfg.head_dim) or k.shape != (B, cfg.n_kv_heads, 1, cfg.head_dim):
+        if q.shape != self._q_shape or k.shape != self._kv_shape:
             raise ValueError(f"decode expects one token per sequence, got q {tuple(q.shape)} k {tuple(k.shape)}")
-        q, k, v, gate = (_as_bf16_view(t) for t in (q, k, v, gate))
         n_app, max_rows = self._plan_step()
-        if int(self.state_len_h.max()) > self.memory.capacity:
-            need = int(self.state_len_h.max())
-            self._reserve(need)
         any_update = n_app is not None
         self._last_any_update, self._last_n_append = any_update, n_app
+        if any_update or self._quiet == 0:
+            need = int(self.state_len_h.max())
+            if need > self.memory.capacity:
+                self._reserve(need)
+        call = self._call
+        addr, cq, ck, cv, cg = self._call_args
+        q, k = _fill_tensor4(cq, q, "q"), _fill_tensor4(ck, k, "k")
+        v, gate = _fill_tensor4(cv, v, "v"), _fill_tensor4(cg, gate, "gate")
+        call.max_rows = max_rows if max_rows < self._max_rows_bound else self._max_rows_bound
         if any_update:
-            slot = self._n_append_slot
-            self._n_append_slot = (slot + 1) % len(self._n_append_pinned)
-            if self._n_append_events[slot] is not None:
-                self._n_append_events[slot].synchronize()
-            self._n_append_pinned[slot].copy_(torch.from_numpy(n_app))
-            self._n_append.copy_(self._n_append_pinned[slot], non_blocking=True)
-            ev = self._n_append_events[slot] or torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(self.device))
-            self._n_append_events[slot] = ev
+            if int((n_app >= 0).sum()) > _lib.UPDATE_LIST_MAX:
+                self._upload_n_append(n_app)
+            call.any_update, call.n_append_host = 1, n_app.ctypes.data
             if want_route:
-                self.route = torch.zeros(self.kv_rows, cfg.chunk_len, device=self.device, dtype=torch.int32)
-        ccache = _CCache(self.memory.c(), self.ring_k.data_ptr(), self.ring_v.data_ptr(), self.ring_gate.data_ptr(),
-                         self.total_len.data_ptr(), self.state_len.data_ptr())
-        rc = lib.kvm_decode_step(
-            C.byref(self.params.c), B, ccache, _tensor4(q, "q"), _tensor4(k, "k"), _tensor4(v, "v"),
-            _tensor4(gate, "gate"), self._n_append.data_ptr() if any_update else None,
-            int((n_app >= 0).sum()) if any_update else 0,
-            min(max_rows, self._max_rows_bound), self.out.data_ptr(),
-            _ptr(self.route) if (any_update and want_route) else None,
-            self._ws.data_ptr(), self._ws_bytes, _stream_ptr(self.device))
-        _lib.check(rc)
+                self.route = torch.zeros(self.kv_rows, self.cfg.chunk_len, device=self.device, dtype=torch.int32)
+                call.route_dev = self.route.data_ptr()
+        rc = _lib.load().kvm_decode_step_call(addr, _stream_ptr(self.device))
+        if any_update:
+            call.any_update, call.n_append_host, call.route_dev = 0, None, None
+        if rc:
+            _lib.check(rc)
         return self.out
+
+    def _upload_n_append(self, n_app):
+        """The step's append counts to the device (for steps at which more sequences update than a launch can list)."""
+        slot = self._n_append_slot
+        self._n_append_slot = (slot + 1) % len(self._n_append_pinned)
+        if self._n_append_events[slot] is not None:
+            self._n_append_events[slot].synchronize()
+        self._n_append_pinned[slot].copy_(torch.from_numpy(n_app))
+        self._n_append.copy_(self._n_append_pinned[slot], non_blocking=True)
+        ev = self._n_append_events[slot] or torch.cuda.Event()
+        ev.record(torch.cuda.current_stream(self.device))
+        self._n_append_events[slot] = ev
 
     def run(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
         """``n`` consecutive decode tokens with inputs already on the device (teacher-forced / synthetic
