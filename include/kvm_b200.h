@@ -281,6 +281,17 @@ typedef struct kvm_decode_call {
 } kvm_decode_call;
 int kvm_decode_step_call(const kvm_decode_call* call, void* stream);
 
+/* Several decode tokens per sequence in one pass over its keys and values, for tokens whose inputs are on the device
+ * (teacher-forced decoding): sequence b decodes `count[b]` tokens (0: none), input `first[b]` onwards, all of them inside
+ * one block; a sequence that stands at a block boundary runs its memory update first.  Arrays [batch], host memory, read
+ * before the call returns.  `call` as for kvm_decode_step_call with the addresses of input and output 0; its host lengths
+ * are those after the span and are required, n_append_host says who updates (>= 0 exactly for the sequences that stand
+ * at a boundary past their window), at most 64 of them.  Token i of the inputs lies i * *_step_stride elements behind
+ * input 0, its output i * out_step_stride elements behind output 0.  count[b] * (query heads per kv head) <= 32, batch
+ * <= 1024.  Same result as the tokens one by one. */
+int kvm_decode_span(const kvm_decode_call* call, const uint8_t* first, const uint8_t* count, int64_t q_step_stride,
+                    int64_t kv_step_stride, int64_t gate_step_stride, int64_t out_step_stride, void* stream);
+
 /* Waits for `stream` and returns what the decode kernels that used `workspace` have reported since the last
  * call: KVM_OK or KVM_ERR_DEVICE_TIMEOUT (a bounded wait of the attention kernel's copy pipeline expired; the
  * kernel drained and returned, that token's output is undefined).  `layer` and `batch` as given to

@@ -73,9 +73,10 @@ EXPORTS = [
     "kvm_prefill_workspace_bytes", "kvm_prefill_forward", "kvm_decode_workspace_bytes", "kvm_decode_step",
     "kvm_memory_refresh", "kvm_last_error_string", "kvm_abi_version", "kvm_decode_step_static", "kvm_prefill_status", "kvm_decode_run",
     "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward",
-    "kvm_prefill_forward_gathered", "kvm_decode_step_call",
+    "kvm_prefill_forward_gathered", "kvm_decode_step_call", "kvm_decode_span",
 ]
 STATIC_SCRATCH_BYTES = 32 << 20
+SPAN_COLUMNS, SPAN_BATCH_MAX = 32, 1024  # tokens x query heads per kv head, and sequences, of one kvm_decode_span
 UPDATE_LIST_MAX = 64  # updating sequences that a decode launch can list by itself
 
 _lib = None
@@ -118,6 +119,8 @@ def load():
         C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
     lib.kvm_decode_step_call.restype = C.c_int
     lib.kvm_decode_step_call.argtypes = [C.c_void_p, C.c_void_p]  # (a kept kvm_decode_call, by its address)
+    lib.kvm_decode_span.restype = C.c_int
+    lib.kvm_decode_span.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]
     lib.kvm_decode_run.restype = C.c_int
     lib.kvm_decode_run.argtypes = [
         LP(KvmLayer), C.c_int32, KvmDecodeCache, C.c_int32, KvmTensor4, KvmTensor4, KvmTensor4, KvmTensor4,

@@ -18,6 +18,11 @@ cudaError_t decode_dispatch(int D, const LayerDev& L, int batch, const DecodeCac
                             Tensor4 v, Tensor4 gate, const UpdateSet& upd, const LengthSet& lens, int any_update, int max_rows, bf16* out,
                             int* route, bf16* pk_scr, float* partial, int* counters, int nslots, int overlap,
                             cudaStream_t stream);
+cudaError_t span_dispatch(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, Tensor4 q, Tensor4 k, Tensor4 v, Tensor4 gate,
+                          long long q_step, long long kv_step, long long gate_step, const SpanSet& spans, int max_count,
+                          const UpdateSet& upd, bf16* pk_scr, float* partial, int* counters, bf16* out, long long out_step,
+                          cudaStream_t stream);
+size_t span_partial_bytes(int D);
 cudaError_t refresh_dispatch(int D, const LayerDev& L, int batch, MemoryDev mem, const int* state_len,
                              cudaStream_t stream);
 }  // namespace kvm
@@ -402,7 +407,7 @@ int kvm_prefill_status(void* workspace, void* stream) {
 
 size_t kvm_decode_workspace_bytes(const kvm_layer* layer, int32_t batch, int32_t max_rows_per_seq) {
   if (!layer || batch <= 0 || max_rows_per_seq <= 0) return 0;
-  return decode_ws(layer, batch, max_rows_per_seq).total;
+  return decode_ws(layer, batch, max_rows_per_seq).total + span_partial_bytes(layer->head_dim);  // (the spans' partial results lie last)
 }
 
 static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_decode_cache& cache, kvm_tensor4 q, kvm_tensor4 k,
@@ -497,6 +502,66 @@ int kvm_decode_step_call(const kvm_decode_call* c, void* stream) {
   return decode_step_impl(c->layer, c->batch, c->cache, c->q, c->k, c->v, c->gate, c->n_append_dev, c->any_update, c->max_rows,
                           c->out, c->route_dev, c->workspace, c->workspace_bytes, stream, 1, "kvm_decode_step_call", false,
                           c->n_append_host, c->total_len_host, c->state_len_host);
+}
+
+int kvm_decode_span(const kvm_decode_call* c, const uint8_t* first, const uint8_t* count, int64_t q_step_stride, int64_t kv_step_stride,
+                    int64_t gate_step_stride, int64_t out_step_stride, void* stream) {
+  g_err[0] = 0;
+  if (!c || !first || !count) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_decode_span: call, first and count must not be NULL");
+  const kvm_layer* layer = c->layer;
+  if (int rc = check_layer(layer)) return rc;
+  const int batch = c->batch, D = layer->head_dim, C = layer->chunk_len, W = layer->n_bswa_chunks;
+  if (batch <= 0 || batch > SpanSet::kMax) return fail(KVM_ERR_UNSUPPORTED, "kvm_decode_span: batch %d must be in [1, %d]", batch, SpanSet::kMax);
+  if (int rc = check_tensor(c->q, "q", D)) return rc;
+  if (int rc = check_tensor(c->k, "k", D)) return rc;
+  if (int rc = check_tensor(c->v, "v", D)) return rc;
+  if (int rc = check_tensor(c->gate, "gate", 1)) return rc;
+  if (q_step_stride % 8 || kv_step_stride % 8) return fail(KVM_ERR_BAD_ARGUMENT, "step strides must be multiples of 16 bytes");
+  if (int rc = check_memory(c->cache.memory, layer)) return rc;
+  if (!c->cache.ring_k || !c->cache.ring_v || !c->cache.ring_gate || !c->cache.total_len || !c->cache.state_len || !c->out ||
+      !c->total_len_host || !c->state_len_host)
+    return fail(KVM_ERR_BAD_ARGUMENT, "kvm_decode_span: cache arrays, host lengths and out must not be NULL");
+  const int G = layer->n_q_heads / layer->n_kv_heads;
+  if (G > 16) return fail(KVM_ERR_UNSUPPORTED, "decode supports at most 16 query heads per kv head, got %d", G);
+  SpanSet spans;
+  UpdateSet upd;
+  upd.arr = nullptr;
+  upd.n = 0;
+  int max_count = 0;
+  for (int b = 0; b < batch; ++b) {
+    const int n = count[b];
+    spans.count[b] = count[b];
+    spans.first[b] = first[b];
+    if (n == 0) continue;
+    // the span lies inside one block of the sequence and its memory holds what it will need
+    const int64_t end = c->total_len_host[b], past = end - n;
+    if (n * G > kSpanColumns || past < 0 || past / C != (end - 1) / C || c->state_len_host[b] < 0 || c->state_len_host[b] > c->cache.memory.capacity)
+      return fail(KVM_ERR_BAD_ARGUMENT, "kvm_decode_span: sequence %d: %d tokens up to %lld, %lld memory rows", b, n, (long long)end,
+                  (long long)c->state_len_host[b]);
+    const int na = c->any_update && c->n_append_host ? c->n_append_host[b] : -1;
+    if ((na >= 0) != (past % C == 0 && past / C > W) || na > C)
+      return fail(KVM_ERR_BAD_ARGUMENT, "kvm_decode_span: sequence %d at token %lld: %d appended rows", b, (long long)past, na);
+    if (na >= 0) {
+      if (upd.n == UpdateSet::kMax) return fail(KVM_ERR_UNSUPPORTED, "kvm_decode_span: more than %d sequences update", UpdateSet::kMax);
+      upd.seq[upd.n] = b;
+      upd.rows[upd.n++] = (short)na;
+    }
+    if (n > max_count) max_count = n;
+  }
+  for (int b = batch; b < SpanSet::kMax; ++b) spans.count[b] = spans.first[b] = 0;
+  if (max_count == 0) return KVM_OK;
+  const DecodeWs ws = decode_ws(layer, batch, c->cache.memory.capacity + W * C);
+  const size_t need = ws.total + span_partial_bytes(D);
+  if (!c->workspace || c->workspace_bytes < need) return fail(KVM_ERR_CAPACITY, "kvm_decode_span: scratch of %zu bytes available, %zu needed", c->workspace_bytes, need);
+  if (((uintptr_t)c->workspace) % 256) return fail(KVM_ERR_BAD_ARGUMENT, "workspace must be 256-byte aligned");
+  unsigned char* wsb = static_cast<unsigned char*>(c->workspace);
+  const cudaError_t e = span_dispatch(D, to_dev(layer), batch, to_dev(c->cache), to_dev(c->q), to_dev(c->k), to_dev(c->v), to_dev(c->gate),
+                                      q_step_stride, kv_step_stride, gate_step_stride, spans, max_count, upd,
+                                      reinterpret_cast<bf16*>(wsb + ws.pk), reinterpret_cast<float*>(wsb + ws.total),
+                                      reinterpret_cast<int*>(wsb + ws.counters), static_cast<bf16*>(c->out), out_step_stride,
+                                      static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "kvm_decode_span");
+  return KVM_OK;
 }
 
 int kvm_decode_run(const kvm_layer* layer, int32_t batch, kvm_decode_cache cache, int32_t n_steps, kvm_tensor4 q,

@@ -121,6 +121,13 @@ struct UpdateSet {
   }
 };
 
+// How many tokens every sequence decodes in one launch over a span of tokens, and which of the inputs its first one is.
+constexpr int kSpanColumns = 32;  // tokens x query heads per kv head of a span, at most
+struct SpanSet {
+  static constexpr int kMax = 1024;
+  unsigned char count[kMax], first[kMax];
+};
+
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll

@@ -756,6 +756,19 @@ static cudaError_t launch_update(const LayerDev& L, int batch, const DecodeCache
   return cudaLaunchKernelEx(&cfg, kern, L, cache, upd, pk_scr, route, batch, nc);
 }
 
+cudaError_t decode_update(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, const UpdateSet& upd, bf16* pk_scr,
+                          cudaStream_t stream) {
+  const int rows = upd.n * L.Hkv, n_sm = device_sm_count();
+  int nc = kMaxCluster;  // as many CTAs per row as the GPU has SMs for
+  while (nc > 1 && rows * nc > n_sm) nc >>= 1;
+  switch (D) {
+    case 32: return launch_update<32>(L, batch, cache, upd, rows * nc, nc, pk_scr, nullptr, stream);
+    case 64: return launch_update<64>(L, batch, cache, upd, rows * nc, nc, pk_scr, nullptr, stream);
+    case 128: return launch_update<128>(L, batch, cache, upd, rows * nc, nc, pk_scr, nullptr, stream);
+  }
+  return cudaErrorInvalidValue;
+}
+
 // `any_update`: number of sequences with a memory update at this token (0: none; any positive value is
 // treated as "some" when the count is not known).  `overlap`: a boundary update may run on the library's
 // side stream next to the attention of the sequences without one.

@@ -117,6 +117,10 @@ int device_sm_count();
 // The tensor maps of a decode cache (kept between calls, keyed by the arrays' addresses and sizes).
 bool decode_maps(const DecodeCacheDev& c, uint64_t kv_rows, int cap, int WC, int D, DecMaps* out);
 
+// The boundary updates of the listed sequences (nothing else runs on the GPU meanwhile).
+cudaError_t decode_update(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, const UpdateSet& upd, bf16* pk_scr,
+                          cudaStream_t stream);
+
 // Launch with the programmatic-serialization attribute when `pdl` is set (see pdl_wait above).
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,

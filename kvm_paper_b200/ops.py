@@ -677,46 +677,56 @@ class KvmDecodeCache:
     def run(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
         """``n`` consecutive decode tokens with inputs already on the device (teacher-forced / synthetic
         decoding): q [n,B,Hq,1,D], k/v [n,B,Hkv,1,D], gate [n,B,Hkv,1,1], contiguous.  Returns [n,B,Hq*D].
-        The host walks the per-sequence schedule a piece of 32 tokens at a time and issues one C call per piece, so
-        that the device works on one piece while the next is planned."""
-        lib = _lib.load()
+        Tokens of one block see the same memory, so a sequence's keys and values are read once for a span of tokens
+        (up to its next block boundary, and as many as a launch has columns for); the sequences advance independently."""
         cfg, B = self.cfg, self.batch
         n = q.size(0)
-        if q.shape != (n, B, cfg.n_q_heads, 1, cfg.head_dim) or k.shape != (n, B, cfg.n_kv_heads, 1, cfg.head_dim):
+        if q.shape != (n, *self._q_shape) or k.shape != (n, *self._kv_shape):
             raise ValueError(f"run expects [n,B,H,1,D] inputs, got q {tuple(q.shape)} k {tuple(k.shape)}")
         q, k, v, gate = (t.to(torch.bfloat16).contiguous() for t in (q, k, v, gate))
         out = torch.empty(n, B, cfg.n_q_heads * cfg.head_dim, device=self.device, dtype=torch.bfloat16)
-        keep = [q, k, v, gate]
-        # The schedule is walked and issued in pieces: while the device works on one piece the host plans the next
-        # (a walk of all n tokens up front would leave the device idle for its whole duration).
-        piece = 32
+        if B > _lib.SPAN_BATCH_MAX:
+            for i in range(n):
+                out[i] = self.step(q[i], k[i], v[i], gate[i]).view(B, -1)
+            return out
+        lib, stream = _lib.load(), _stream_ptr(self.device)
+        Cn, WC = cfg.chunk_len, self.ring_capacity
+        span = _lib.SPAN_COLUMNS // (cfg.n_q_heads // cfg.n_kv_heads)
+        tl, sl = self.total_len_h, self.state_len_h
+        self._quiet = 0
+        piece = 128  # (a token's place inside a piece fits a byte)
         for lo in range(0, n, piece):
             m = min(piece, n - lo)
-            n_app = np.full((m, B), -1, dtype=np.int32)
-            any_upd = (C.c_int32 * m)()
-            max_rows = (C.c_int32 * m)()
-            for i in range(m):
-                na, mr = self._plan_step()
-                if na is not None:
-                    n_app[i] = na
-                    any_upd[i] = int((na >= 0).sum())
-                max_rows[i] = min(mr, self.memory.capacity + self.ring_capacity)
-            if int(self.state_len_h.max()) > self.memory.capacity:
-                self._reserve(int(self.state_len_h.max()))
-                bound = self.memory.capacity + self.ring_capacity
-                for i in range(m):
-                    max_rows[i] = min(max_rows[i], bound)
-            n_app_dev = torch.from_numpy(n_app).to(self.device, non_blocking=True) if any(any_upd) else None
-            ccache = _CCache(self.memory.c(), self.ring_k.data_ptr(), self.ring_v.data_ptr(), self.ring_gate.data_ptr(),
-                             self.total_len.data_ptr(), self.state_len.data_ptr())
-            rc = lib.kvm_decode_run(
-                C.byref(self.params.c), B, ccache, m, _tensor4(q[lo], "q"), _tensor4(k[lo], "k"), _tensor4(v[lo], "v"),
-                _tensor4(gate[lo], "gate"), q.stride(0), k.stride(0), gate.stride(0),
-                n_app_dev.data_ptr() if n_app_dev is not None else None, any_upd, max_rows,
-                out[lo].data_ptr(), self._ws.data_ptr(), self._ws_bytes, _stream_ptr(self.device))
-            _lib.check(rc)
-            keep.append(n_app_dev)
-        self._keepalive = tuple(keep)
+            done = np.zeros(B, dtype=np.int64)
+            while True:
+                at = tl % Cn
+                count = np.minimum(np.minimum(m - done, Cn - at), span)
+                if not count.any():
+                    break
+                cross = np.nonzero((count > 0) & (at == 0) & (tl > WC))[0]
+                if cross.size > _lib.UPDATE_LIST_MAX:  # the others wait for the next launch
+                    count[cross[_lib.UPDATE_LIST_MAX:]] = 0
+                    cross = cross[:_lib.UPDATE_LIST_MAX]
+                n_app = self._plan_updates(cross) if cross.size else None
+                direct = (tl < Cn) & (sl == tl)
+                sl[direct] += count[direct]
+                tl += count
+                need = int(sl.max())
+                if need > self.memory.capacity:
+                    self._reserve(need)
+                call = self._call
+                addr, cq, ck, cv, cg = self._call_args
+                for dst, t, name in ((cq, q, "q"), (ck, k, "k"), (cv, v, "v"), (cg, gate, "gate")):
+                    _fill_tensor4(dst, t[lo], name)
+                call.out = out[lo].data_ptr()
+                if n_app is not None:
+                    call.any_update, call.n_append_host = 1, n_app.ctypes.data
+                first8, count8 = done.astype(np.uint8), count.astype(np.uint8)
+                rc = lib.kvm_decode_span(addr, first8.ctypes.data, count8.ctypes.data, q.stride(0), k.stride(0), gate.stride(0),
+                                         out.stride(0), stream)
+                call.out, call.any_update, call.n_append_host = self.out.data_ptr(), 0, None
+                _lib.check(rc)
+                done += count
         return out
 
     def check_status(self) -> None:
