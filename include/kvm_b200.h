@@ -203,6 +203,14 @@ typedef struct kvm_prologue {
   const void* cos;
   const void* sin;
   int64_t rope_stride_b;
+  int64_t q_stride_t, k_stride_t, v_stride_t, gate_stride_t; /* elements from token to token (the outputs of one GEMM over all
+                                                  projections: rows wider than one of them); 0: contiguous.  A batch row
+                                                  is T such strides */
+  int64_t prev_q_stride_b, prev_k_stride_b, prev_v_stride_b; /* elements from batch row to batch row; 0: contiguous */
+  const void* v_first;     /* value residual before the token shift: v + (v_first - v) * sigmoid(v_gate0 + v_gate), */
+  const void* v_gate;      /* v_first [B,T,Hkv*D] contiguous, v_gate [B,T,Hkv*D] contiguous, v_gate0 [Hkv*D]; all */
+  const void* v_gate0;     /* three NULL: none (model/value_residual_mixin.py:173-218) */
+  void* v_last;            /* [B,Hkv*D] out, may be NULL: the last token's value behind the residual, before the shift */
 } kvm_prologue;
 /*   q_out [B,T,Hq,D], k_out, v_out [B,T,Hkv,D]   the operator's inputs (pass them on as [B,H,T,D] views)
  *   gate_out [B,Hkv,T]                           merge gate
@@ -215,6 +223,14 @@ typedef struct kvm_prologue {
 int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in,
                          void* q_out, void* k_out, void* v_out, void* gate_out, int64_t total_version_rows,
                          void* workspace, size_t workspace_bytes, void* stream);
+
+/* Linear layers (no bias) over few rows, for the projections of decode tokens: out[m, :] = (x[m, :] W_0^T, x[m, :] W_1^T, ..)
+ * for 1 <= n_rows <= 64 rows of `width` (a multiple of 32) bf16 values, x_stride elements apart, and up to eight weights
+ * [weight_rows[i], width] bf16 contiguous; out rows are out_stride elements apart.  fp32 sums, one rounding to bf16.
+ * Replaces the module calls c_q / c_k / c_v / v_gate1 / v_gate2 / key_weighting / c_proj of a cached single-token step
+ * (model/value_residual_mixin.py:173-218, model/kvm_mixer.py:381-395, 701-713). */
+int kvm_project(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights,
+                const int32_t* weight_rows, int32_t n_weights, void* out, int64_t out_stride, void* stream);
 
 /* The decode-time cache of one layer for `batch` sequences with ragged lengths (all device memory,
  * caller-owned).  Replaces TritonKVMDecodeCache (model/kvm_triton_decode.py:34-400); unlike the
@@ -334,6 +350,13 @@ int kvm_decode_step_static(const kvm_layer* layer, int32_t batch, kvm_decode_cac
                            kvm_tensor4 q, kvm_tensor4 k, kvm_tensor4 v, kvm_tensor4 gate,
                            const int32_t* n_append_dev, int32_t any_update, int32_t max_rows,
                            void* out, int32_t* route_dev, void* stream);
+
+/* Decode cache of a batch right after a prefill of `seq_len` tokens per sequence: the window's keys, values and gates into
+ * the rings, the lengths, the zeroed counters at the head of a decode workspace (NULL: none) and, unless `from` names
+ * the cache's own arrays, the first `rows` memory rows of every kv row.
+ * Replaces TritonKVMDecodeCache.reset_ (model/kvm_triton_decode.py:264-317). */
+int kvm_decode_cache_fill(const kvm_layer* layer, int32_t batch, int64_t seq_len, kvm_tensor4 k, kvm_tensor4 v, kvm_tensor4 gate,
+                          kvm_memory from, int32_t rows, kvm_decode_cache cache, void* workspace, void* stream);
 
 /* Build k_attn / v_attn from k_sum / v_sum / vlen for rows [0, state_len[b]) of every sequence
  * (used when a cache is initialised from the reference's eager cache layout).

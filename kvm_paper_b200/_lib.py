@@ -53,7 +53,10 @@ class KvmPrefillLayout(C.Structure):
 class KvmPrologue(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("q_lin", "k_lin", "v_lin", "gate_lin", "shift_q", "shift_k", "shift_v",
                                           "prev_q", "prev_k", "prev_v", "ln_q_w", "ln_q_b", "ln_k_w", "ln_k_b")] + [
-        ("ln_qk_eps", C.c_float), ("cos", C.c_void_p), ("sin", C.c_void_p), ("rope_stride_b", C.c_int64)]
+        ("ln_qk_eps", C.c_float), ("cos", C.c_void_p), ("sin", C.c_void_p), ("rope_stride_b", C.c_int64),
+        ("q_stride_t", C.c_int64), ("k_stride_t", C.c_int64), ("v_stride_t", C.c_int64), ("gate_stride_t", C.c_int64),
+        ("prev_q_stride_b", C.c_int64), ("prev_k_stride_b", C.c_int64), ("prev_v_stride_b", C.c_int64),
+        ("v_first", C.c_void_p), ("v_gate", C.c_void_p), ("v_gate0", C.c_void_p), ("v_last", C.c_void_p)]
 
 
 class KvmDecodeCache(C.Structure):
@@ -74,8 +77,10 @@ EXPORTS = [
     "kvm_memory_refresh", "kvm_last_error_string", "kvm_abi_version", "kvm_decode_step_static", "kvm_prefill_status", "kvm_decode_run",
     "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward",
     "kvm_prefill_forward_gathered", "kvm_decode_step_call", "kvm_decode_span",
+    "kvm_decode_cache_fill", "kvm_project",
 ]
 STATIC_SCRATCH_BYTES = 32 << 20
+PROJECT_ROWS_MAX = 64  # rows of one kvm_project
 SPAN_COLUMNS, SPAN_BATCH_MAX = 32, 1024  # tokens x query heads per kv head, and sequences, of one kvm_decode_span
 UPDATE_LIST_MAX = 64  # updating sequences that a decode launch can list by itself
 
@@ -121,6 +126,9 @@ def load():
     lib.kvm_decode_step_call.argtypes = [C.c_void_p, C.c_void_p]  # (a kept kvm_decode_call, by its address)
     lib.kvm_decode_span.restype = C.c_int
     lib.kvm_decode_span.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]
+    lib.kvm_decode_cache_fill.restype = C.c_int
+    lib.kvm_decode_cache_fill.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, KvmTensor4, KvmTensor4, KvmTensor4, KvmMemory, C.c_int32,
+                                          KvmDecodeCache, C.c_void_p, C.c_void_p]
     lib.kvm_decode_run.restype = C.c_int
     lib.kvm_decode_run.argtypes = [
         LP(KvmLayer), C.c_int32, KvmDecodeCache, C.c_int32, KvmTensor4, KvmTensor4, KvmTensor4, KvmTensor4,
@@ -136,6 +144,9 @@ def load():
     lib.kvm_prologue_forward.restype = C.c_int
     lib.kvm_prologue_forward.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, LP(KvmPrologue), C.c_void_p, C.c_void_p, C.c_void_p,
                                          C.c_void_p, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.kvm_project.restype = C.c_int
+    lib.kvm_project.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_int32, LP(C.c_void_p), LP(C.c_int32), C.c_int32, C.c_void_p,
+                                C.c_int64, C.c_void_p]
     lib.kvm_interleave_shards.restype = C.c_int
     lib.kvm_interleave_shards.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_void_p]
     lib.kvm_last_error_string.restype = C.c_char_p

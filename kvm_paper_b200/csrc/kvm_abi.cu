@@ -23,6 +23,8 @@ cudaError_t span_dispatch(int D, const LayerDev& L, int batch, const DecodeCache
                           const UpdateSet& upd, bf16* pk_scr, float* partial, int* counters, bf16* out, long long out_step,
                           cudaStream_t stream);
 size_t span_partial_bytes(int D);
+cudaError_t cache_fill_dispatch(int D, const LayerDev& L, int batch, long long T, Tensor4 k, Tensor4 v, Tensor4 gate, MemoryDev from,
+                                int rows, const DecodeCacheDev& cache, int* counters, int n_counters, cudaStream_t stream);
 cudaError_t refresh_dispatch(int D, const LayerDev& L, int batch, MemoryDev mem, const int* state_len,
                              cudaStream_t stream);
 }  // namespace kvm
@@ -202,6 +204,7 @@ int static_scratch_for_current_device(void** out) {
 namespace kvm {
 cudaError_t launch_prologue(int D, const LayerDev& L, const PrologueDev& p, int batch, long long T, cudaStream_t stream);
 cudaError_t launch_interleave_shards(void* dst, const void* src, int n_shards, long long n_tokens, long long shard_bytes, cudaStream_t stream);
+cudaError_t launch_project(const ProjectArgs& a, cudaStream_t stream);
 }
 using kvm::launch_interleave_shards;
 
@@ -209,7 +212,7 @@ extern "C" {
 
 const char* kvm_last_error_string(void) { return g_err; }
 
-int kvm_abi_version(void) { return 100; }
+int kvm_abi_version(void) { return 101; }
 
 size_t kvm_prefill_workspace_bytes(const kvm_layer* layer, int32_t batch, int64_t seq_len, int64_t total_version_rows) {
   if (!layer || batch <= 0 || total_version_rows < 0) return 0;
@@ -329,11 +332,25 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   if (in->cos && in->rope_stride_b != 0 && in->rope_stride_b != seq_len * D)
     return fail(KVM_ERR_BAD_ARGUMENT, "rope_stride_b %lld must be 0 or seq_len*head_dim", (long long)in->rope_stride_b);
   const void* aligned[] = {in->q_lin, in->k_lin, in->v_lin, in->shift_q, in->shift_k, in->shift_v, in->prev_q, in->prev_k, in->prev_v,
-                           in->cos, in->sin, q_out, k_out, v_out, in->ln_q_w, in->ln_q_b, in->ln_k_w, in->ln_k_b,
+                           in->cos, in->sin, in->v_first, in->v_gate, in->v_gate0, in->v_last, q_out, k_out, v_out, in->ln_q_w, in->ln_q_b, in->ln_k_w, in->ln_k_b,
                            layer->ln_weight_dev, layer->ln_bias_dev};
   for (const void* a : aligned)
     if (((uintptr_t)a) % 16) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: tensors must be 16-byte aligned");
+  const int n_mix = (in->v_first != nullptr) + (in->v_gate != nullptr) + (in->v_gate0 != nullptr);
+  if (n_mix != 0 && n_mix != 3) return fail(KVM_ERR_BAD_ARGUMENT, "the value residual needs v_first, v_gate and v_gate0");
+  const long long width_q = (long long)layer->n_q_heads * D, width_kv = (long long)layer->n_kv_heads * D;
   kvm::PrologueDev p = {};
+  const int64_t given[6] = {in->q_stride_t, in->k_stride_t, in->v_stride_t, in->prev_q_stride_b, in->prev_k_stride_b, in->prev_v_stride_b};
+  for (int i = 0; i < 6; ++i) {
+    const long long width = i % 3 == 0 ? width_q : width_kv, st = given[i] ? given[i] : width;
+    if (st < width || st % 8) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: stride %lld must be a multiple of 8 and at least %lld", st, width);
+    (i < 3 ? p.st[i] : p.prev_sb[i - 3]) = st;
+  }
+  p.gate_st = in->gate_stride_t ? in->gate_stride_t : layer->n_kv_heads;
+  p.v_first = static_cast<const bf16*>(in->v_first);
+  p.v_gate = static_cast<const bf16*>(in->v_gate);
+  p.v_gate0 = static_cast<const bf16*>(in->v_gate0);
+  p.v_last = static_cast<bf16*>(in->v_last);
   p.q_lin = static_cast<const bf16*>(in->q_lin);
   p.k_lin = static_cast<const bf16*>(in->k_lin);
   p.v_lin = static_cast<const bf16*>(in->v_lin);
@@ -370,6 +387,36 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   }
   const cudaError_t e = kvm::launch_prologue(D, to_dev(layer), p, batch, seq_len, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "kvm_prologue_forward");
+  return KVM_OK;
+}
+
+int kvm_project(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights, const int32_t* weight_rows,
+                int32_t n_weights, void* out, int64_t out_stride, void* stream) {
+  g_err[0] = 0;
+  if (!x || !weights || !weight_rows || !out) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: arguments must not be NULL");
+  if (n_rows <= 0 || n_rows > kProjectRows || n_weights <= 0 || n_weights > kProjectParts || width <= 0 || width % 32)
+    return fail(KVM_ERR_UNSUPPORTED, "kvm_project: %d rows (1..%d), %d layers (1..%d), width %d (a multiple of 32)", n_rows, kProjectRows,
+                n_weights, kProjectParts, width);
+  if (((uintptr_t)x) % 16 || x_stride % 8 || x_stride < width) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: input rows must be 16-byte aligned");
+  ProjectArgs a = {};
+  a.x = static_cast<const bf16*>(x);
+  a.x_stride = x_stride;
+  a.M = n_rows;
+  a.K = width;
+  a.n_parts = n_weights;
+  int64_t cols = 0;
+  for (int i = 0; i < n_weights; ++i) {
+    if (!weights[i] || ((uintptr_t)weights[i]) % 16 || weight_rows[i] <= 0)
+      return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: weights of layer %d must be 16-byte aligned and not empty", i);
+    a.weight[i] = static_cast<const bf16*>(weights[i]);
+    a.rows[i] = weight_rows[i];
+    cols += weight_rows[i];
+  }
+  if (out_stride < cols) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: output stride %lld below %lld columns", (long long)out_stride, (long long)cols);
+  a.out = static_cast<bf16*>(out);
+  a.out_stride = out_stride;
+  const cudaError_t e = kvm::launch_project(a, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "kvm_project");
   return KVM_OK;
 }
 
@@ -636,6 +683,28 @@ int kvm_memory_refresh(const kvm_layer* layer, int32_t batch, kvm_memory memory,
     return fail(KVM_ERR_BAD_ARGUMENT, "memory arrays must not be NULL");
   cudaError_t e = refresh_dispatch(layer->head_dim, to_dev(layer), batch, to_dev(memory), state_len_dev, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "kvm_memory_refresh");
+  return KVM_OK;
+}
+
+int kvm_decode_cache_fill(const kvm_layer* layer, int32_t batch, int64_t seq_len, kvm_tensor4 k, kvm_tensor4 v, kvm_tensor4 gate,
+                          kvm_memory from, int32_t rows, kvm_decode_cache cache, void* workspace, void* stream) {
+  g_err[0] = 0;
+  if (int rc = check_layer(layer)) return rc;
+  if (batch <= 0 || seq_len <= 0 || rows <= 0) return fail(KVM_ERR_BAD_ARGUMENT, "batch %d, seq_len %lld and rows %d must be positive", batch, (long long)seq_len, rows);
+  const int D = layer->head_dim;
+  if (int rc = check_tensor(k, "k", D)) return rc;
+  if (int rc = check_tensor(v, "v", D)) return rc;
+  if (int rc = check_tensor(gate, "gate", 1)) return rc;
+  if (int rc = check_memory(from, layer)) return rc;
+  if (int rc = check_memory(cache.memory, layer)) return rc;
+  if (!cache.ring_k || !cache.ring_v || !cache.ring_gate || !cache.total_len || !cache.state_len)
+    return fail(KVM_ERR_BAD_ARGUMENT, "decode cache arrays must not be NULL");
+  if (rows > from.capacity || rows > cache.memory.capacity)
+    return fail(KVM_ERR_CAPACITY, "%d memory rows do not fit capacities %d and %d", rows, from.capacity, cache.memory.capacity);
+  const cudaError_t e = cache_fill_dispatch(D, to_dev(layer), batch, seq_len, to_dev(k), to_dev(v), to_dev(gate), to_dev(from), rows,
+                                            to_dev(cache), static_cast<int*>(workspace),
+                                            batch * layer->n_kv_heads + batch + 1, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "kvm_decode_cache_fill");
   return KVM_OK;
 }
 

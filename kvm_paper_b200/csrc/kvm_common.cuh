@@ -62,6 +62,12 @@ struct PrologueDev {
   const bf16* cos;
   const bf16* sin;
   long long rope_stride_b;
+  long long st[3], gate_st;   // q, k, v, gate: elements from token to token
+  long long prev_sb[3];       // cached tokens: elements from batch row to batch row
+  const bf16* v_first;
+  const bf16* v_gate;
+  const bf16* v_gate0;
+  bf16* v_last;
   bf16* q_out;
   bf16* k_out;
   bf16* v_out;
@@ -69,6 +75,18 @@ struct PrologueDev {
   bf16* pk_all;
   bf16* gk_all;
   long long n_tok;  // tokens per kv row in pk_all / gk_all
+};
+
+// Linear layers over the same few rows (kvm_project): part i's outputs are the columns behind those of part i - 1.
+constexpr int kProjectParts = 8, kProjectRows = 64;
+struct ProjectArgs {
+  const bf16* x;
+  long long x_stride;
+  int M, K, n_parts;
+  const bf16* weight[kProjectParts];
+  int rows[kProjectParts];
+  bf16* out;
+  long long out_stride;
 };
 
 struct MemoryDev {

@@ -1,10 +1,10 @@
 // Fused prologue of the mixer: everything between the q/k/v/gate projections and the operator's inputs in one pass.
 //
-// Per token and head: token shift against the previous token, per-head LayerNorm of q and k, rotary embedding,
+// Per token and head: value residual (values only), token shift against the previous token, per-head LayerNorm of q and k, rotary embedding,
 // the merge gate 1 + elu(.), and (for the keys that a memory update will consume) the prepared key
 // bf16(LayerNorm(key with its rotary dims zeroed)) and the gated key bf16(prepared * gate) in the layout the chain
 // kernels read, so that the prefill can skip its own pass over the keys.
-// Follows model/tokenshift.py:11-37, model/value_residual_mixin.py:219-235 (token shift, ln_q / ln_k),
+// Follows model/tokenshift.py:11-37, model/value_residual_mixin.py:173-235 (value residual, token shift, ln_q / ln_k),
 // model/rwkv7_backbone.py:76-88 (rotary on interleaved pairs), model/kvm_mixer.py:381-399 (merge gate, head-major
 // views), model/kvm_mixer.py:120-129 (prepared key).  Every operation of the reference's bf16 module rounds its result
 // to bf16; the kernel rounds at the same points.
@@ -93,6 +93,23 @@ __device__ __forceinline__ void store_raw(const uint32_t (&w)[EPL / 2], bf16* p)
 __device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t u) { return *reinterpret_cast<__nv_bfloat162*>(&u); }
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
+// Value residual of a lane's share of a value row, in bf16 arithmetic as below: v + (v_first - v) * sigmoid(v_gate0 + v_gate),
+// the sigmoid in fp32, rounded once.
+template <int EPL>
+__device__ __forceinline__ void mix_values(uint32_t (&x)[EPL / 2], const PrologueDev& p, size_t row, int col) {
+  uint32_t f[EPL / 2], g[EPL / 2], g0[EPL / 2];
+  load_raw<EPL>(f, p.v_first + row + col);
+  load_raw<EPL>(g, p.v_gate + row + col);
+  load_raw<EPL>(g0, p.v_gate0 + col);
+#pragma unroll
+  for (int i = 0; i < EPL / 2; ++i) {
+    const float2 a = __bfloat1622float2(__hadd2_rn(as_bf162(g0[i]), as_bf162(g[i])));
+    const __nv_bfloat162 s = as_bf162(pack_bf16(1.0f / (1.0f + expf(-a.x)), 1.0f / (1.0f + expf(-a.y))));
+    const __nv_bfloat162 v = as_bf162(x[i]);
+    x[i] = as_u32(__hadd2_rn(v, __hmul2_rn(__hsub2_rn(as_bf162(f[i]), v), s)));
+  }
+}
+
 // Token shift and rotary embedding are bf16 arithmetic in the reference (every product, difference and sum rounded
 // to bf16): they run on packed pairs with the hardware's bf16 instructions (exact result rounded once, which is what
 // "compute in fp32, round to bf16" gives for one operation on bf16 operands; the _rn forms are never contracted into
@@ -120,14 +137,29 @@ kvm_prologue_kernel(LayerDev L, PrologueDev p, long long T) {
   bf16* out = kind == 0 ? p.q_out : (kind == 1 ? p.k_out : p.v_out);
   const size_t row_off = ((size_t)b * T + t) * H * D + (size_t)h * D + gl * EPL;  // this lane's share of the row
 
+  // ... of the projections, whose rows may be parts of wider ones
+  const int col = h * D + gl * EPL;
+  const bf16* src = lin + ((size_t)b * T + t) * p.st[kind] + col;
+  const size_t v_row = ((size_t)b * T + t) * H * D;
+  const bool mixed = kind == 2 && p.v_first != nullptr;
+
   uint32_t x[EPL / 2];
-  load_raw<EPL>(x, lin + row_off);
+  load_raw<EPL>(x, src);
+  if (mixed) {
+    mix_values<EPL>(x, p, v_row, col);
+    if (p.v_last && valid && t == T - 1) store_raw<EPL>(x, p.v_last + (size_t)b * H * D + col);
+  }
   if (shift) {
     // x + scale * (previous token - x); the first token of a call uses the cached token, or itself
     uint32_t xp[EPL / 2], sc[EPL / 2];
-    const bf16* pr = t > 0 ? lin + row_off - (size_t)H * D : (prev ? prev + (size_t)b * H * D + (size_t)h * D + gl * EPL : lin + row_off);
-    load_raw<EPL>(xp, pr);
-    load_raw<EPL>(sc, shift + (size_t)h * D + gl * EPL);
+    if (t > 0 || prev) {
+      load_raw<EPL>(xp, t > 0 ? src - p.st[kind] : prev + (size_t)b * p.prev_sb[kind] + col);
+      if (mixed && t > 0) mix_values<EPL>(xp, p, v_row - (size_t)H * D, col);
+    } else {
+#pragma unroll
+      for (int i = 0; i < EPL / 2; ++i) xp[i] = x[i];
+    }
+    load_raw<EPL>(sc, shift + col);
 #pragma unroll
     for (int i = 0; i < EPL / 2; ++i) {
       const __nv_bfloat162 xi = as_bf162(x[i]);
@@ -167,7 +199,7 @@ kvm_prologue_kernel(LayerDev L, PrologueDev p, long long T) {
   // merge gate 1 + elu(g) of this (token, kv head), in the head-major layout [B, Hkv, T]
   float g = 1.0f;
   if (p.gate_lin && is_key) {
-    const float gl_in = __bfloat162float(p.gate_lin[((size_t)b * T + t) * L.Hkv + h]);
+    const float gl_in = __bfloat162float(p.gate_lin[((size_t)b * T + t) * p.gate_st + h]);
     const float e = bf16_round(gl_in > 0.f ? gl_in : expf(gl_in) - 1.0f);
     g = bf16_round(1.0f + e);
   }

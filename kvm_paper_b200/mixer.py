@@ -22,7 +22,7 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
-from . import ops
+from . import _lib, ops
 
 
 def set_label(label: str, module, mup_d_in_ratio=None):
@@ -203,7 +203,8 @@ class SequenceMixer(nn.Module):
             self.state_head_temp = set_label("scalars", nn.Parameter(torch.ones(H)))
         if self.chunk_len % 16 or not (16 <= self.chunk_len <= 512):
             raise ValueError(f"kvm_b200 mixer needs chunk_len to be a multiple of 16 in [16, 512], got {self.chunk_len}")
-        self._params_cache: tuple | None = None
+        self._params_cache: tuple | None = None      # what is laid out once from the parameters (see layer_params,
+        self._prologue_cache: tuple | None = None    # _prologue_params_kept)
 
     # ------------------------------------------------------------------ schedule (host integers)
     def _desired_state_len(self, ctx_len: int, available_context: int, current_state_len: int) -> int:
@@ -236,7 +237,7 @@ class SequenceMixer(nn.Module):
     def layer_params(self, device) -> ops.LayerParams:
         """fp32 device copies of ln_s_k and the head temperatures, rebuilt when a parameter changes."""
         temps = (self.front_head_temp, self.state_head_temp) if self.config.kvm_use_head_temps else (None, None)
-        key = (str(device), self.ln_s_k.weight._version, self.ln_s_k.bias._version,
+        key = (device, self.ln_s_k.weight._version, self.ln_s_k.bias._version,
                self.ln_s_k.weight.data_ptr(), *(0 if t is None else t._version for t in temps))
         if self._params_cache is None or self._params_cache[0] != key:
             cfg = ops.LayerConfig(
@@ -313,46 +314,104 @@ class SequenceMixer(nn.Module):
                                   shift_v=self.x_v if shift else None, ln_q=self.ln_q if ln else None,
                                   ln_k=self.ln_k if ln else None, ln_eps=self.ln_q.eps if ln else 1e-5)
 
+    def _prologue_params_kept(self, device) -> ops.PrologueParams:
+        """``prologue_params``, rebuilt when a parameter changes."""
+        src = [t for m in (self.ln_q, self.ln_k) if isinstance(m, nn.LayerNorm) for t in (m.weight, m.bias)]
+        if self.tokenshift_mode == "rwkv":
+            src += [self.x_q, self.x_k, self.x_v]
+        key = (device, *((t.data_ptr(), t._version) for t in src))
+        if self._prologue_cache is None or self._prologue_cache[0] != key:
+            self._prologue_cache = (key, self.prologue_params(device))
+        return self._prologue_cache[1]
+
     def fused_prologue_applies(self, x: torch.Tensor) -> bool:
         """The one-kernel prologue covers bf16 modules on CUDA with head dims the kernel is built for and a value
         path without the post-shift residual (that variant mixes values after the token shift)."""
         return (x.is_cuda and x.dtype == torch.bfloat16 and self.c_q.weight.dtype == torch.bfloat16
                 and self.d_qk_head in (32, 64, 128) and self.value_projection_size == self.num_key_value_heads * self.d_qk_head
-                and self.value_residual_mode != "rwkv_post_tokenshift")
+                and self.value_residual_mode != "rwkv_post_tokenshift"
+                and (self.value_residual_mode != "rwkv" or self.v_gate0.dtype == torch.bfloat16))
+
+    @staticmethod
+    def _plain_linear(m, x) -> bool:
+        """A linear layer that ``ops.project`` may stand in for: bf16, no bias, nothing hooked onto it."""
+        return (type(m) is nn.Linear and m.bias is None and m.weight.dtype is torch.bfloat16 and m.weight.is_contiguous()
+                and m.weight.data_ptr() % 16 == 0 and m.in_features % 32 == 0 and m.weight.device == x.device and not m._forward_hooks and not m._forward_pre_hooks)
+
+    def _few_rows(self, x) -> bool:
+        """Up to 64 rows (tokens x sequences) the linear layers are bound by reading the weights and by launches: the
+        library's kernel takes all layers of one input at once.  More rows are left to the library GEMMs."""
+        return (x.size(0) * x.size(1) <= _lib.PROJECT_ROWS_MAX and x.is_cuda and x.dtype is torch.bfloat16
+                and not torch.is_grad_enabled())
+
+    def _project(self, x):
+        """q, k, v projections, output of ``v_gate2`` and merge-gate logits (the last two None where the layer has none)."""
+        B, T, _ = x.shape
+        gated = self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values
+        mixed = self.value_residual_mode == "rwkv"
+        lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
+        if not (self._few_rows(x) and all(self._plain_linear(m, x) for m in lins) and (not mixed or self._plain_linear(self.v_gate2, x))):
+            return (self.c_q(x).contiguous(), self.c_k(x).contiguous(), self.c_v(x).contiguous(),
+                    self.v_gate2(self.v_gate1(x)) if mixed else None, self.key_weighting(x) if gated else None)
+        y = ops.project(x.reshape(B * T, -1), [m.weight for m in lins])
+        parts, at = [], 0
+        for m in lins:  # (every range but the merge gate's starts on a 16-byte boundary)
+            parts.append(y[:, at:at + m.out_features])
+            at += m.out_features
+        v_gate = ops.project(parts[3], [self.v_gate2.weight]).view(B, T, -1) if mixed else None
+        q, k, v = (t.view(B, T, -1) for t in parts[:3])
+        return q, k, v, v_gate, parts[-1].view(B, T, -1) if gated else None
+
+    def _output(self, y):
+        """``c_proj``."""
+        B, T, _ = y.shape
+        if self._few_rows(y) and self._plain_linear(self.c_proj, y) and self.c_proj.out_features % 8 == 0:
+            return ops.project(y.view(B * T, -1), [self.c_proj.weight]).view(B, T, -1)
+        return self.c_proj(y)
 
     def forward_prefix_fused(self, x, v_first, position_embeddings, past_key_values=None, runner=None):
-        """``forward_prefix`` with everything behind the projections in one kernel (``kvm_prologue_forward``): the
-        projections and the value residual are torch GEMMs / elementwise ops as in ``calc_qkv``; token shift, q/k
-        LayerNorm, rotary embedding and merge gate run fused, and with ``runner`` the prepared keys of the prompt are
-        written into its workspace (reference: model/value_residual_mixin.py:173-237, model/kvm_mixer.py:367-401)."""
+        """``forward_prefix`` with everything behind the projections in one kernel (``kvm_prologue_forward``): value
+        residual, token shift, q/k LayerNorm, rotary embedding and merge gate run fused, and with ``runner`` (a prefill
+        runner, or a function that makes one while the projections run) the prepared keys of the prompt are written into
+        its workspace (reference: model/value_residual_mixin.py:173-237, model/kvm_mixer.py:367-401)."""
         B, T, _ = x.size()
         states = past_key_values.get_states(self.layer_idx) if past_key_values is not None else {}
         past_len = past_key_values.get_seq_length(self.layer_idx) if past_key_values is not None else 0
         if past_len > 0 and T != 1:
             raise AssertionError("cached decode expects single-token inputs.")
-        q, k, v = self.c_q(x), self.c_k(x), self.c_v(x)
+        q, k, v, v_gate, gate_lin = self._project(x)
+        residual = v_last = None
         if self.value_residual_mode == "linear":
-            v = (1 - self.lamb) * v + self.lamb * v_first.view_as(v)
+            v = ((1 - self.lamb) * v + self.lamb * v_first.view_as(v)).contiguous()
         elif self.value_residual_mode == "rwkv":
-            v = v + (v_first.to(v.dtype) - v) * self._value_gate(x).to(v.dtype)
+            residual = (v_first, v_gate, self.v_gate0)
+            v_last = torch.empty(B, 1, self.value_projection_size, device=x.device, dtype=x.dtype)
+        dev = x.device
         prev = None
         if past_key_values is not None:
             prev = (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL))
+            v_final = v[:, -1:].detach() if residual is None else v_last
             past_key_values.update(self.layer_idx, offset=0, states_dict={
                 self._CACHE_Q_FINAL: q[:, -1:].detach(), self._CACHE_K_FINAL: k[:, -1:].detach(),
-                self._CACHE_V_FINAL: v[:, -1:].detach(), self._CACHE_X_FINAL: x[:, -1:].detach()})
-        gated = self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values
-        gate_lin = self.key_weighting(x) if gated else None
-        dev = x.device
-        return ops.prologue_forward(self.layer_params(dev), self.prologue_params(dev), q.contiguous(), k.contiguous(),
-                                    v.contiguous(), gate_lin, position_embeddings, prev=prev, runner=runner)
+                self._CACHE_V_FINAL: v_final, self._CACHE_X_FINAL: x[:, -1:].detach()})
+        if callable(runner):
+            runner = runner()
+        return ops.prologue_forward(self.layer_params(dev), self._prologue_params_kept(dev), q, k, v, gate_lin, position_embeddings,
+                                    prev=prev, runner=runner, value_residual=residual, v_last=v_last)
 
     # ------------------------------------------------------------------ module entry points
     def _prompt_fused(self, x, v_first, position_embeddings, attention_mask, past_key_values, **kwargs):
         """A prompt through the one-kernel prologue, which also leaves the prepared keys in the prefill's workspace."""
-        params = self.layer_params(x.device)
-        runner = ops.PrefillRunner(params, x.size(0), self.make_prefill_plan(int(x.size(1))), want_route=self.capture_routes)
-        q, k, v, gate = self.forward_prefix_fused(x, v_first, position_embeddings, past_key_values, runner=runner)
+        runner = None
+
+        def make_runner():  # called while the projections run; its memory has room for a decode cache to go on in it
+            nonlocal runner
+            plan = self.make_prefill_plan(int(x.size(1)))
+            runner = ops.PrefillRunner(self.layer_params(x.device), x.size(0), plan, want_route=self.capture_routes,
+                                       memory_capacity=plan.final_state_len + self.chunk_len, zero_memory=False)
+            return runner
+
+        q, k, v, gate = self.forward_prefix_fused(x, v_first, position_embeddings, past_key_values, runner=make_runner)
         return self.forward_prefill(q, k, v, gate, v_first, position_embeddings, attention_mask, past_key_values,
                                     _prefill_runner=runner, **kwargs)
 
@@ -397,17 +456,18 @@ class SequenceMixer(nn.Module):
         if attention_mask is not None:
             raise ValueError("kvm_b200 mixer does not support attention_mask")
         T = int(q.size(2))
-        res = self.prefill_raw(q, k, v, merge_gate, want_route=self.capture_routes, runner=kwargs.pop("_prefill_runner", None))
+        runner = kwargs.pop("_prefill_runner", None)
+        res = self.prefill_raw(q, k, v, merge_gate, want_route=self.capture_routes, runner=runner)
         if self.capture_routes:
             self.last_route = res.route
-        y = self.c_proj(res.out.to(q.dtype))
+        y = self._output(res.out.to(q.dtype))
         if past_key_values is not None:
             plan = res.plan
             init_len = min(T, self.chunk_len)
             if plan.final_coverage != max(init_len, self._bswa_begin_for_total_len(T)):
                 raise AssertionError("KVM prefill state progression drifted from the decode-state bookkeeping.")
             cache = ops.decode_cache_from_prefill(self.layer_params(q.device), res, k, v, merge_gate,
-                                                  self._desired_state_len, owner=self)
+                                                  self._desired_state_len, owner=self, adopt_memory=runner is not None)
             past_key_values.update(self.layer_idx, offset=T, states_dict={self._CACHE_DECODE: cache})
         return y
 
@@ -445,7 +505,7 @@ class SequenceMixer(nn.Module):
             raise RuntimeError("KVM cache is missing its decode state; run a prefill with this cache before decoding")
         if cache.owner is not self:
             raise RuntimeError("KVM decode cache belongs to another mixer")
-        if int(cache.total_len_h[0]) != past_len or len(set(cache.total_len_h.tolist())) != 1:
+        if not (cache.total_len_h == past_len).all():
             raise AssertionError(f"KVM decode cache length disagrees with the layer cache: {cache.total_len_h.tolist()} != {past_len}")
         out = cache.step(q, k, v, merge_gate, want_route=self.capture_routes)
         if self.capture_routes:
@@ -453,7 +513,7 @@ class SequenceMixer(nn.Module):
         if self.check_device_status:
             cache.check_status()
         past_key_values.update(self.layer_idx, offset=1, states_dict={self._CACHE_DECODE: cache})
-        return self.c_proj(out.to(q.dtype))
+        return self._output(out.to(q.dtype))
 
 
 def _ramp(n: int) -> torch.Tensor:

@@ -138,9 +138,9 @@ class PrefillPlan:
         return arr
 
     def to_tensor(self, device) -> torch.Tensor:
-        t = torch.tensor([[sb, na, vr, 0] for sb, na, vr in zip(self.state_before, self.n_append, self.version_row)],
-                         dtype=torch.int32)
-        return t.to(device, non_blocking=True)
+        t = np.zeros((len(self.n_append), 4), dtype=np.int32)
+        t[:, 0], t[:, 1], t[:, 2] = self.state_before, self.n_append, self.version_row
+        return torch.from_numpy(t).to(device, non_blocking=True)
 
 
 def build_prefill_plan(seq_len: int, chunk_len: int, n_bswa_chunks: int,
@@ -184,16 +184,18 @@ def _round8(x: int) -> int:
 # ----------------------------------------------------------------------------------------- memory
 
 class MemoryBuffers:
-    """The compressed memory of ``n_rows`` kv rows with ``capacity`` rows each."""
+    """The compressed memory of ``n_rows`` kv rows with ``capacity`` rows each (``zero``: rows past the live ones read as
+    zeros; the kernels never look at them)."""
 
-    def __init__(self, n_rows: int, capacity: int, head_dim: int, device):
+    def __init__(self, n_rows: int, capacity: int, head_dim: int, device, zero: bool = True):
         self.n_rows, self.capacity, self.head_dim = n_rows, int(capacity), head_dim
+        make = torch.zeros if zero else torch.empty
         kw = dict(device=device, dtype=torch.bfloat16)
-        self.k_sum = torch.zeros(n_rows, capacity, head_dim, **kw)
-        self.v_sum = torch.zeros(n_rows, capacity, head_dim, **kw)
-        self.vlen = torch.zeros(n_rows, capacity, device=device, dtype=torch.float32)
-        self.k_attn = torch.zeros(n_rows, capacity, head_dim, **kw)
-        self.v_attn = torch.zeros(n_rows, capacity, head_dim, **kw)
+        self.k_sum = make(n_rows, capacity, head_dim, **kw)
+        self.v_sum = make(n_rows, capacity, head_dim, **kw)
+        self.vlen = make(n_rows, capacity, device=device, dtype=torch.float32)
+        self.k_attn = make(n_rows, capacity, head_dim, **kw)
+        self.v_attn = make(n_rows, capacity, head_dim, **kw)
 
     def c(self) -> KvmMemory:
         return KvmMemory(self.k_sum.data_ptr(), self.v_sum.data_ptr(), self.vlen.data_ptr(),
@@ -233,48 +235,76 @@ class PrologueParams:
         if ln_q is not None:
             self.ln = tuple(t.detach().to(dev, torch.float32).contiguous() for t in (ln_q.weight, ln_q.bias, ln_k.weight, ln_k.bias))
         self.ln_eps = float(ln_eps)
+        self.shift_ptrs = tuple(_ptr(t) for t in (self.shift_q, self.shift_k, self.shift_v))
+        self.ln_ptrs = None if self.ln is None else tuple(t.data_ptr() for t in self.ln)
+
+
+def _token_stride(t: torch.Tensor, B: int, T: int, width: int, name: str) -> int:
+    """Elements from token to token of a [B,T,width] bf16 projection output: contiguous, or a column range of wider rows."""
+    if t.dtype is not torch.bfloat16 or not t.is_cuda or t.shape != (B, T, width):
+        raise ValueError(f"{name} projection must be a bf16 CUDA tensor [B,T,{width}], got {tuple(t.shape)} {t.dtype}")
+    st = t.stride()
+    step = st[1] if T > 1 else (st[0] if B > 1 else (width + 7) // 8 * 8)
+    if (st[2] != 1 and width > 1) or (B > 1 and st[0] != T * step):
+        raise ValueError(f"{name} projection must be contiguous or a column range of contiguous rows, got strides {st}")
+    return step
 
 
 def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tensor, k_lin: torch.Tensor, v_lin: torch.Tensor,
                      gate_lin: torch.Tensor | None, position_embeddings, *, prev=None, runner: "PrefillRunner | None" = None,
-                     out: tuple | None = None):
-    """Token shift, q/k LayerNorm, rotary embedding and merge gate in one kernel over the projection outputs
-    ([B,T,H*D] bf16).  Returns q [B,Hq,T,D], k, v [B,Hkv,T,D], gate [B,Hkv,T,1] as views of [B,T,H,D] / [B,Hkv,T]
+                     out: tuple | None = None, value_residual: tuple | None = None, v_last: torch.Tensor | None = None):
+    """Value residual, token shift, q/k LayerNorm, rotary embedding and merge gate in one kernel over the projection
+    outputs ([B,T,H*D] bf16, contiguous or column ranges of one wider GEMM output).  Returns q [B,Hq,T,D], k, v
+    [B,Hkv,T,D], gate [B,Hkv,T,1] as views of [B,T,H,D] / [B,Hkv,T]
     buffers, the layouts the reference hands its mixer (model/kvm_mixer.py:397-399).  With ``runner`` the prepared
     keys of the tokens that memory updates consume are written into that runner's workspace, and its ``run`` may
     be called with ``keys_prepared=True``.  ``prev`` = (q, k, v) rows [B,1,H*D] of the previous call's last token.
-    ``out`` = preallocated (q [B,T,Hq,D], k, v [B,T,Hkv,D], gate [B,Hkv,T]) bf16 buffers to write into."""
+    ``out`` = preallocated (q [B,T,Hq,D], k, v [B,T,Hkv,D], gate [B,Hkv,T]) bf16 buffers to write into.
+    ``value_residual`` = (v_first, output of v_gate2, v_gate0) of the "rwkv" value residual; ``v_last`` [B,1,Hkv*D]
+    receives the last token's value behind it (what the next call's ``prev`` needs)."""
     cfg = params.cfg
     B, T, _ = q_lin.shape
     D, Hq, Hkv = cfg.head_dim, cfg.n_q_heads, cfg.n_kv_heads
-    for name, t, h in (("q", q_lin, Hq), ("k", k_lin, Hkv), ("v", v_lin, Hkv)):
-        if t.dtype != torch.bfloat16 or not t.is_cuda or not t.is_contiguous() or t.shape != (B, T, h * D):
-            raise ValueError(f"{name} projection must be a contiguous bf16 CUDA tensor [B,T,{h * D}], got {tuple(t.shape)} {t.dtype}")
+    dev = q_lin.device
     keep = []
     arg = _lib.KvmPrologue()
     arg.q_lin, arg.k_lin, arg.v_lin = q_lin.data_ptr(), k_lin.data_ptr(), v_lin.data_ptr()
+    arg.q_stride_t, arg.k_stride_t, arg.v_stride_t = (
+        _token_stride(t, B, T, h * D, n) for n, t, h in (("q", q_lin, Hq), ("k", k_lin, Hkv), ("v", v_lin, Hkv)))
     if gate_lin is not None:
-        gate_lin = gate_lin.to(torch.bfloat16).reshape(B, T, Hkv).contiguous()
-        keep.append(gate_lin)
-        arg.gate_lin = gate_lin.data_ptr()
+        if gate_lin.dtype is not torch.bfloat16 or gate_lin.shape != (B, T, Hkv):
+            gate_lin = gate_lin.to(torch.bfloat16).reshape(B, T, Hkv).contiguous()
+            keep.append(gate_lin)
+        arg.gate_lin, arg.gate_stride_t = gate_lin.data_ptr(), _token_stride(gate_lin, B, T, Hkv, "gate")
+    if value_residual is not None:
+        v_first, v_gate, v_gate0 = (t.to(torch.bfloat16).contiguous() for t in value_residual)
+        if v_first.numel() != B * T * Hkv * D or v_gate.numel() != B * T * Hkv * D or v_gate0.numel() != Hkv * D:
+            raise ValueError(f"value residual: v_first and v_gate must have {Hkv * D} values per token, v_gate0 {Hkv * D}")
+        keep += [v_first, v_gate, v_gate0]
+        arg.v_first, arg.v_gate, arg.v_gate0 = v_first.data_ptr(), v_gate.data_ptr(), v_gate0.data_ptr()
+        if v_last is not None:
+            arg.v_last = v_last.data_ptr()
     if pro.shift_q is not None:
-        arg.shift_q, arg.shift_k, arg.shift_v = pro.shift_q.data_ptr(), pro.shift_k.data_ptr(), pro.shift_v.data_ptr()
+        arg.shift_q, arg.shift_k, arg.shift_v = pro.shift_ptrs
         if prev is not None and all(t is not None for t in prev):
-            pv = [t.to(q_lin.device, torch.bfloat16).reshape(B, -1).contiguous() for t in prev]
+            pv = [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.stride(2) == 1 and t.stride(0) % 8 == 0
+                  and t.data_ptr() % 16 == 0 else t.to(dev, torch.bfloat16).reshape(B, 1, -1).contiguous() for t in prev]
             keep += pv
             arg.prev_q, arg.prev_k, arg.prev_v = (t.data_ptr() for t in pv)
+            if B > 1:
+                arg.prev_q_stride_b, arg.prev_k_stride_b, arg.prev_v_stride_b = (t.stride(0) for t in pv)
     if pro.ln is not None:
-        arg.ln_q_w, arg.ln_q_b, arg.ln_k_w, arg.ln_k_b = (t.data_ptr() for t in pro.ln)
+        arg.ln_q_w, arg.ln_q_b, arg.ln_k_w, arg.ln_k_b = pro.ln_ptrs
         arg.ln_qk_eps = pro.ln_eps
     if position_embeddings is not None:
-        cos, sin = position_embeddings
-        cs = [t.to(q_lin.device, torch.bfloat16).reshape(-1, T, D).contiguous() for t in (cos, sin)]
-        if cs[0].size(0) not in (1, B):
-            raise ValueError(f"rotary tables must have batch 1 or {B}, got {cs[0].size(0)}")
+        cs = [t if t.dtype is torch.bfloat16 and t.device == dev and t.is_contiguous() else t.to(dev, torch.bfloat16).contiguous()
+              for t in position_embeddings]
+        n_rope = cs[0].numel() // (T * D)
+        if n_rope not in (1, B) or cs[0].numel() != n_rope * T * D or cs[1].numel() != cs[0].numel():
+            raise ValueError(f"rotary tables must be [1 or {B}, {T}, .., {D}], got {tuple(cs[0].shape)} and {tuple(cs[1].shape)}")
         keep += cs
         arg.cos, arg.sin = cs[0].data_ptr(), cs[1].data_ptr()
-        arg.rope_stride_b = 0 if cs[0].size(0) == 1 else T * D
-    dev = q_lin.device
+        arg.rope_stride_b = 0 if n_rope == 1 else T * D
     if out is not None:
         q, k, v, gate = out
         for t, shape in ((q, (B, T, Hq, D)), (k, (B, T, Hkv, D)), (v, (B, T, Hkv, D)), (gate, (B, Hkv, T))):
@@ -292,9 +322,25 @@ def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tens
         ws_ptr, ws_bytes, ver_rows = runner.ws.data_ptr(), runner.ws_bytes, runner.plan.total_version_rows
     rc = _lib.load().kvm_prologue_forward(C.byref(params.c), B, T, C.byref(arg), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                           gate.data_ptr(), ver_rows, ws_ptr, ws_bytes, _stream_ptr(dev))
-    _lib.check(rc)
+    if rc:
+        _lib.check(rc)
     del keep  # (the kernel is enqueued on the current stream: torch's allocator keeps the blocks until it has run)
     return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), gate.unsqueeze(-1)
+
+
+def project(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
+    """[rows, width] bf16 (at most 64 rows, inner stride 1) times the transposed weights, side by side:
+    [rows, sum of the weights' rows], in one launch."""
+    rows, width = x.shape
+    n = len(weights)
+    sizes = [w.size(0) for w in weights]
+    cols = (sum(sizes) + 7) // 8 * 8  # (16-byte aligned rows)
+    out = torch.empty(rows, cols, device=x.device, dtype=torch.bfloat16)
+    rc = _lib.load().kvm_project(x.data_ptr(), x.stride(0), rows, width, (C.c_void_p * n)(*[w.data_ptr() for w in weights]),
+                                 (C.c_int32 * n)(*sizes), n, out.data_ptr(), cols, _stream_ptr(x.device))
+    if rc:
+        _lib.check(rc)
+    return out
 
 
 class PrefillRunner:
@@ -303,13 +349,13 @@ class PrefillRunner:
     ``run`` only enqueues kernels on the current stream; nothing is allocated per call."""
 
     def __init__(self, params: LayerParams, batch: int, plan: PrefillPlan, *, memory_capacity: int | None = None,
-                 want_route: bool = False):
+                 want_route: bool = False, zero_memory: bool = True):
         lib = _lib.load()
         cfg = params.cfg
         self.params, self.plan, self.batch = params, plan, int(batch)
         dev = params.device
         cap = max(plan.final_state_len, 1) if memory_capacity is None else int(memory_capacity)
-        self.memory = MemoryBuffers(batch * cfg.n_kv_heads, cap, cfg.head_dim, dev)
+        self.memory = MemoryBuffers(batch * cfg.n_kv_heads, cap, cfg.head_dim, dev, zero_memory)
         self.ws_bytes = lib.kvm_prefill_workspace_bytes(C.byref(params.c), batch, plan.seq_len, plan.total_version_rows)
         self.ws = torch.empty(self.ws_bytes, device=dev, dtype=torch.uint8)
         self.out = torch.empty(batch, plan.seq_len, cfg.n_q_heads * cfg.head_dim, device=dev, dtype=torch.bfloat16)
@@ -489,7 +535,8 @@ class KvmDecodeCache:
     _quiet = 0
 
     def __init__(self, params: LayerParams, batch: int, state_capacity: int,
-                 desired_state_len: Callable[[int, int, int], int], owner: Any = None):
+                 desired_state_len: Callable[[int, int, int], int], owner: Any = None, *, _memory: MemoryBuffers | None = None):
+        """``_memory``: buffers to live in instead of new ones; the caller fills the cache before it is used (``_fill``)."""
         cfg = params.cfg
         self.params, self.cfg, self.batch, self.owner = params, cfg, int(batch), owner
         self.desired_state_len = desired_state_len
@@ -497,13 +544,14 @@ class KvmDecodeCache:
         self.device = dev
         self.kv_rows = batch * cfg.n_kv_heads
         self.ring_capacity = cfg.n_bswa_chunks * cfg.chunk_len
-        self.memory = MemoryBuffers(self.kv_rows, max(int(state_capacity), 1), cfg.head_dim, dev)
+        self.memory = MemoryBuffers(self.kv_rows, max(int(state_capacity), 1), cfg.head_dim, dev) if _memory is None else _memory
+        make = torch.zeros if _memory is None else torch.empty
         kw = dict(device=dev, dtype=torch.bfloat16)
-        self.ring_k = torch.zeros(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
-        self.ring_v = torch.zeros(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
-        self.ring_gate = torch.zeros(self.kv_rows, self.ring_capacity, **kw)
-        self.total_len = torch.zeros(batch, device=dev, dtype=torch.int32)
-        self.state_len = torch.zeros(batch, device=dev, dtype=torch.int32)
+        self.ring_k = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
+        self.ring_v = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
+        self.ring_gate = make(self.kv_rows, self.ring_capacity, **kw)
+        self._lens = make(2, batch, device=dev, dtype=torch.int32)
+        self.total_len, self.state_len = self._lens[0], self._lens[1]
         self.total_len_h = np.zeros(batch, dtype=np.int64)
         self.state_len_h = np.zeros(batch, dtype=np.int64)
         self.update_count = 0
@@ -514,26 +562,27 @@ class KvmDecodeCache:
         self._max_rows = 0
         self._q_shape = (self.batch, cfg.n_q_heads, 1, cfg.head_dim)
         self._kv_shape = (self.batch, cfg.n_kv_heads, 1, cfg.head_dim)
-        self._n_append = torch.full((batch,), -1, device=dev, dtype=torch.int32)
-        # host staging of the per-step append counts: a small ring of pinned buffers, each guarded by an event
-        # recorded behind its copy, so that a later step never overwrites a buffer the copy engine still reads
-        self._n_append_pinned = [torch.full((batch,), -1, dtype=torch.int32).pin_memory() for _ in range(4)]
-        self._n_append_events = [None] * 4
+        # Append counts on the device and their host staging, for batches in which more sequences may update at a token
+        # than a launch can list: a small ring of pinned buffers, each guarded by an event recorded behind its copy, so
+        # that a later step never overwrites a buffer the copy engine still reads
+        self._n_append = torch.full((batch,), -1, device=dev, dtype=torch.int32) if _memory is None or batch > _lib.UPDATE_LIST_MAX else None
+        self._n_append_pinned = None
         self._n_append_slot = 0
-        self._alloc_workspace()
+        self._alloc_workspace(clear=_memory is None)
 
-    def _alloc_workspace(self):
+    def _alloc_workspace(self, clear: bool = True):
         lib = _lib.load()
         self._max_rows_bound = self.memory.capacity + self.ring_capacity
         self._ws_bytes = lib.kvm_decode_workspace_bytes(C.byref(self.params.c), self.batch, self._max_rows_bound)
-        # the counter region at the head of the workspace must start at zero; the kernels leave it zero
-        self._ws = torch.zeros(self._ws_bytes, device=self.device, dtype=torch.uint8)
+        self._ws = torch.empty(self._ws_bytes, device=self.device, dtype=torch.uint8)
+        if clear:  # the counter region at the head of the workspace must start at zero; the kernels leave it zero
+            self._ws[:4 * (self.kv_rows + self.batch + 1)].zero_()
         # the kept argument block of kvm_decode_step_call; between tokens only input addresses and launch flags change
         call = self._call = _lib.KvmDecodeCall()
         call.layer, call.batch = C.addressof(self.params.c), self.batch
         call.cache = _CCache(self.memory.c(), self.ring_k.data_ptr(), self.ring_v.data_ptr(), self.ring_gate.data_ptr(),
                              self.total_len.data_ptr(), self.state_len.data_ptr())
-        call.n_append_dev = self._n_append.data_ptr()
+        call.n_append_dev = _ptr(self._n_append)
         call.total_len_host, call.state_len_host = self.total_len_h.ctypes.data, self.state_len_h.ctypes.data
         call.out, call.workspace, call.workspace_bytes = self.out.data_ptr(), self._ws.data_ptr(), self._ws_bytes
         self._call_args = (C.addressof(call), call.q, call.k, call.v, call.gate)
@@ -664,6 +713,9 @@ class KvmDecodeCache:
 
     def _upload_n_append(self, n_app):
         """The step's append counts to the device (for steps at which more sequences update than a launch can list)."""
+        if self._n_append_pinned is None:
+            self._n_append_pinned = [torch.full((self.batch,), -1, dtype=torch.int32).pin_memory() for _ in range(4)]
+            self._n_append_events = [None] * 4
         slot = self._n_append_slot
         self._n_append_slot = (slot + 1) % len(self._n_append_pinned)
         if self._n_append_events[slot] is not None:
@@ -779,24 +831,19 @@ class KvmDecodeCache:
 
 
 def decode_cache_from_prefill(params: LayerParams, res: PrefillResult, k: torch.Tensor, v: torch.Tensor,
-                              gate: torch.Tensor, desired_state_len, owner=None, extra_capacity: int | None = None) -> KvmDecodeCache:
-    """Build the decode cache of a batch right after its prefill (uniform lengths)."""
+                              gate: torch.Tensor, desired_state_len, owner=None, extra_capacity: int | None = None, *,
+                              adopt_memory: bool = False) -> KvmDecodeCache:
+    """Build the decode cache of a batch right after its prefill (uniform lengths), with one launch.  ``adopt_memory``: the
+    cache goes on in the prefill's own memory buffers instead of a copy (the result's memory then changes with it)."""
     cfg = params.cfg
     B, Hkv, T, D = k.shape
-    plan = res.plan
-    S = plan.final_state_len
+    S = res.plan.final_state_len
     extra = cfg.chunk_len if extra_capacity is None else extra_capacity
-    cache = KvmDecodeCache(params, B, S + extra, desired_state_len, owner)
-    mem = res.memory
-    n = min(mem.capacity, cache.memory.capacity)
-    for name in ("k_sum", "v_sum", "vlen", "k_attn", "v_attn"):
-        getattr(cache.memory, name)[:, :n].copy_(getattr(mem, name)[:, :n])
-    bb = plan.bswa_begin
-    slots = torch.arange(bb, T, device=k.device) % cache.ring_capacity
-    cache.ring_k.index_copy_(1, slots, k[:, :, bb:].reshape(B * Hkv, T - bb, D).to(torch.bfloat16))
-    cache.ring_v.index_copy_(1, slots, v[:, :, bb:].reshape(B * Hkv, T - bb, D).to(torch.bfloat16))
-    cache.ring_gate.index_copy_(1, slots, gate[:, :, bb:].reshape(B * Hkv, T - bb).to(torch.bfloat16))
+    cache = KvmDecodeCache(params, B, S + extra, desired_state_len, owner, _memory=res.memory if adopt_memory else None)
+    k, v, gate = (_as_bf16_view(t) for t in (k, v, gate))
+    rc = _lib.load().kvm_decode_cache_fill(C.byref(params.c), B, T, _tensor4(k, "k"), _tensor4(v, "v"), _tensor4(gate, "gate"),
+                                           res.memory.c(), S, cache._call.cache, cache._ws.data_ptr(), _stream_ptr(cache.device))
+    _lib.check(rc)
     cache.total_len_h[:] = T
     cache.state_len_h[:] = S
-    cache.commit_lengths()
     return cache
