@@ -225,7 +225,7 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
                          void* workspace, size_t workspace_bytes, void* stream);
 
 /* Linear layers (no bias) over few rows, for the projections of decode tokens: out[m, :] = (x[m, :] W_0^T, x[m, :] W_1^T, ..)
- * for 1 <= n_rows <= 64 rows of `width` (a multiple of 32) bf16 values, x_stride elements apart, and up to eight weights
+ * for 1 <= n_rows <= 128 rows of `width` (a multiple of 32) bf16 values, x_stride elements apart, and up to eight weights
  * [weight_rows[i], width] bf16 contiguous; out rows are out_stride elements apart.  fp32 sums, one rounding to bf16.
  * Replaces the module calls c_q / c_k / c_v / v_gate1 / v_gate2 / key_weighting / c_proj of a cached single-token step
  * (model/value_residual_mixin.py:173-218, model/kvm_mixer.py:381-395, 701-713). */
@@ -357,6 +357,52 @@ int kvm_decode_step_static(const kvm_layer* layer, int32_t batch, kvm_decode_cac
  * Replaces TritonKVMDecodeCache.reset_ (model/kvm_triton_decode.py:264-317). */
 int kvm_decode_cache_fill(const kvm_layer* layer, int32_t batch, int64_t seq_len, kvm_tensor4 k, kvm_tensor4 v, kvm_tensor4 gate,
                           kvm_memory from, int32_t rows, kvm_decode_cache cache, void* workspace, void* stream);
+
+/* One cached token of the whole mixer from the hidden states: projections, value residual, token shift, q/k LayerNorm,
+ * rotary embedding, merge gate, decode step and output projection, one call.  Same results as kvm_project,
+ * kvm_prologue_forward, kvm_decode_step_call and kvm_project one after the other; batch <= 128.
+ * Replaces SequenceMixer.forward_inference of a cached single-token step (model/kvm_mixer.py:527-570, 572-713). */
+typedef struct kvm_token_call {
+  kvm_decode_call decode;      /* q, k, v, gate and out are not read */
+  kvm_prologue prologue;       /* parameters, rotary tables, cached tokens, v_first, v_gate0, v_last; projection outputs and v_gate not read */
+  const void* x;               /* [batch, hidden] bf16, rows x_stride elements apart */
+  int64_t x_stride;
+  int32_t hidden;
+  int32_t n_weights;
+  const void* weights[5];      /* c_q, c_k, c_v, then v_gate1 (with v_gate2), then key_weighting (if gated) */
+  int32_t weight_rows[5];
+  int32_t gated;
+  int32_t out_features;
+  const void* v_gate2;         /* [Hkv*D, rows of v_gate1] or NULL: no value residual */
+  const void* c_proj;          /* [out_features, Hq*D] */
+  void* lin;                   /* [batch, lin_stride] out: the projections (the next token's cached rows) */
+  int64_t lin_stride;
+  void* scratch;               /* kvm_token_scratch_bytes */
+  size_t scratch_bytes;
+  void* y;                     /* [batch, out_features] bf16 */
+} kvm_token_call;
+size_t kvm_token_scratch_bytes(const kvm_layer* layer, int32_t batch);
+int kvm_mixer_token(const kvm_token_call* call, void* stream);
+
+/* A prompt of the whole mixer between the projections and c_proj: kvm_prologue_forward, kvm_prefill_forward and (unless
+ * cache.ring_k is NULL) kvm_decode_cache_fill in one call; the schedule is taken from plan_host and need not stay.
+ * `memory` receives the memory (the cache may live in the same arrays), `out` [B,T,Hq*D] the attention's output. */
+typedef struct kvm_prompt_call {
+  const kvm_layer* layer;
+  int32_t batch, n_updates;
+  int64_t seq_len, total_version_rows;
+  const kvm_update_plan* plan_host;
+  kvm_prologue prologue;
+  kvm_memory memory;
+  kvm_decode_cache cache;
+  void* decode_workspace;
+  void* out;
+  void* workspace;             /* kvm_prompt_workspace_bytes; a prefill workspace lies at its start */
+  size_t workspace_bytes;
+} kvm_prompt_call;
+size_t kvm_prompt_workspace_bytes(const kvm_layer* layer, int32_t batch, int64_t seq_len, int32_t n_updates,
+                                  int64_t total_version_rows);
+int kvm_mixer_prompt(const kvm_prompt_call* call, void* stream);
 
 /* Build k_attn / v_attn from k_sum / v_sum / vlen for rows [0, state_len[b]) of every sequence
  * (used when a cache is initialised from the reference's eager cache layout).

@@ -72,15 +72,30 @@ class KvmDecodeCall(C.Structure):
                 ("out", C.c_void_p), ("route_dev", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)]
 
 
+class KvmTokenCall(C.Structure):
+    _fields_ = [("decode", KvmDecodeCall), ("prologue", KvmPrologue), ("x", C.c_void_p), ("x_stride", C.c_int64), ("hidden", C.c_int32),
+                ("n_weights", C.c_int32), ("weights", C.c_void_p * 5), ("weight_rows", C.c_int32 * 5), ("gated", C.c_int32),
+                ("out_features", C.c_int32), ("v_gate2", C.c_void_p), ("c_proj", C.c_void_p), ("lin", C.c_void_p),
+                ("lin_stride", C.c_int64), ("scratch", C.c_void_p), ("scratch_bytes", C.c_size_t), ("y", C.c_void_p)]
+
+
+class KvmPromptCall(C.Structure):
+    _fields_ = [("layer", C.c_void_p), ("batch", C.c_int32), ("n_updates", C.c_int32), ("seq_len", C.c_int64),
+                ("total_version_rows", C.c_int64), ("plan_host", C.c_void_p), ("prologue", KvmPrologue), ("memory", KvmMemory),
+                ("cache", KvmDecodeCache), ("decode_workspace", C.c_void_p), ("out", C.c_void_p), ("workspace", C.c_void_p),
+                ("workspace_bytes", C.c_size_t)]
+
+
 EXPORTS = [
     "kvm_prefill_workspace_bytes", "kvm_prefill_forward", "kvm_decode_workspace_bytes", "kvm_decode_step",
     "kvm_memory_refresh", "kvm_last_error_string", "kvm_abi_version", "kvm_decode_step_static", "kvm_prefill_status", "kvm_decode_run",
     "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward",
     "kvm_prefill_forward_gathered", "kvm_decode_step_call", "kvm_decode_span",
-    "kvm_decode_cache_fill", "kvm_project",
+    "kvm_decode_cache_fill", "kvm_project", "kvm_token_scratch_bytes", "kvm_mixer_token",
+    "kvm_prompt_workspace_bytes", "kvm_mixer_prompt",
 ]
 STATIC_SCRATCH_BYTES = 32 << 20
-PROJECT_ROWS_MAX = 64  # rows of one kvm_project
+PROJECT_ROWS_MAX = 128  # rows of one kvm_project
 SPAN_COLUMNS, SPAN_BATCH_MAX = 32, 1024  # tokens x query heads per kv head, and sequences, of one kvm_decode_span
 UPDATE_LIST_MAX = 64  # updating sequences that a decode launch can list by itself
 
@@ -144,6 +159,14 @@ def load():
     lib.kvm_prologue_forward.restype = C.c_int
     lib.kvm_prologue_forward.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, LP(KvmPrologue), C.c_void_p, C.c_void_p, C.c_void_p,
                                          C.c_void_p, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.kvm_token_scratch_bytes.restype = C.c_size_t
+    lib.kvm_token_scratch_bytes.argtypes = [LP(KvmLayer), C.c_int32]
+    lib.kvm_mixer_token.restype = C.c_int
+    lib.kvm_mixer_token.argtypes = [C.c_void_p, C.c_void_p]  # (kept calls, by their addresses)
+    lib.kvm_prompt_workspace_bytes.restype = C.c_size_t
+    lib.kvm_prompt_workspace_bytes.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, C.c_int32, C.c_int64]
+    lib.kvm_mixer_prompt.restype = C.c_int
+    lib.kvm_mixer_prompt.argtypes = [C.c_void_p, C.c_void_p]
     lib.kvm_project.restype = C.c_int
     lib.kvm_project.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_int32, LP(C.c_void_p), LP(C.c_int32), C.c_int32, C.c_void_p,
                                 C.c_int64, C.c_void_p]

@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libkvm_b200.so")
 SOURCES = ["kvm_abi.cu", "kvm_prefill.cu", "kvm_chain_tc.cu", "kvm_vpass.cu", "kvm_attn_tc.cu", "kvm_decode.cu", "kvm_decode_span.cu", "kvm_prologue.cu", "kvm_project.cu"]
-HEADERS = ["kvm_common.cuh", "kvm_decode.cuh", "kvm_update.cuh", "kvm_tc.cuh", "kvm_tma_host.cuh", "kvm_vdelta.cuh", os.path.join("..", "..", "include", "kvm_b200.h")]
+HEADERS = ["kvm_common.cuh", "kvm_pdl.cuh", "kvm_decode.cuh", "kvm_update.cuh", "kvm_tc.cuh", "kvm_tma_host.cuh", "kvm_vdelta.cuh", os.path.join("..", "..", "include", "kvm_b200.h")]
 
 
 def _nvcc() -> str:

@@ -202,9 +202,9 @@ int static_scratch_for_current_device(void** out) {
 }  // namespace
 
 namespace kvm {
-cudaError_t launch_prologue(int D, const LayerDev& L, const PrologueDev& p, int batch, long long T, cudaStream_t stream);
+cudaError_t launch_prologue(int D, const LayerDev& L, const PrologueDev& p, int batch, long long T, cudaStream_t stream, bool pdl);
 cudaError_t launch_interleave_shards(void* dst, const void* src, int n_shards, long long n_tokens, long long shard_bytes, cudaStream_t stream);
-cudaError_t launch_project(const ProjectArgs& a, cudaStream_t stream);
+cudaError_t launch_project(const ProjectArgs& a, cudaStream_t stream, bool pdl);
 }
 using kvm::launch_interleave_shards;
 
@@ -314,10 +314,10 @@ int kvm_prefill_forward_gathered(const kvm_layer* layer, int32_t batch, int64_t 
                               out_bases[rank], route_dev, workspace, workspace_bytes, phases, stream, &gd);
 }
 
-int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out,
-                         void* k_out, void* v_out, void* gate_out, int64_t total_version_rows, void* workspace,
-                         size_t workspace_bytes, void* stream) {
-  g_err[0] = 0;
+// Checked arguments of the prologue; workspace == nullptr: no prepared keys.
+static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out, void* k_out,
+                         void* v_out, void* gate_out, int64_t total_version_rows, void* workspace, size_t workspace_bytes,
+                         kvm::PrologueDev* dev) {
   if (int rc = check_layer(layer)) return rc;
   if (batch <= 0 || seq_len <= 0) return fail(KVM_ERR_BAD_ARGUMENT, "batch %d and seq_len %lld must be positive", batch, (long long)seq_len);
   if (!in || !in->q_lin || !in->k_lin || !in->v_lin || !q_out || !k_out || !v_out || !gate_out)
@@ -339,7 +339,8 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   const int n_mix = (in->v_first != nullptr) + (in->v_gate != nullptr) + (in->v_gate0 != nullptr);
   if (n_mix != 0 && n_mix != 3) return fail(KVM_ERR_BAD_ARGUMENT, "the value residual needs v_first, v_gate and v_gate0");
   const long long width_q = (long long)layer->n_q_heads * D, width_kv = (long long)layer->n_kv_heads * D;
-  kvm::PrologueDev p = {};
+  kvm::PrologueDev& p = *dev;
+  p = {};
   const int64_t given[6] = {in->q_stride_t, in->k_stride_t, in->v_stride_t, in->prev_q_stride_b, in->prev_k_stride_b, in->prev_v_stride_b};
   for (int i = 0; i < 6; ++i) {
     const long long width = i % 3 == 0 ? width_q : width_kv, st = given[i] ? given[i] : width;
@@ -385,14 +386,23 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
     p.gk_all = ws.route > ws.gk_all ? reinterpret_cast<bf16*>(wsb + ws.gk_all) : nullptr;  // present for the tensor-core chain's shapes
     p.n_tok = n_plan * C;
   }
-  const cudaError_t e = kvm::launch_prologue(D, to_dev(layer), p, batch, seq_len, static_cast<cudaStream_t>(stream));
+  return KVM_OK;
+}
+
+int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out,
+                         void* k_out, void* v_out, void* gate_out, int64_t total_version_rows, void* workspace,
+                         size_t workspace_bytes, void* stream) {
+  g_err[0] = 0;
+  kvm::PrologueDev p;
+  if (int rc = prologue_args(layer, batch, seq_len, in, q_out, k_out, v_out, gate_out, total_version_rows, workspace, workspace_bytes, &p))
+    return rc;
+  const cudaError_t e = kvm::launch_prologue(layer->head_dim, to_dev(layer), p, batch, seq_len, static_cast<cudaStream_t>(stream), false);
   if (e != cudaSuccess) return cuda_fail(e, "kvm_prologue_forward");
   return KVM_OK;
 }
 
-int kvm_project(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights, const int32_t* weight_rows,
-                int32_t n_weights, void* out, int64_t out_stride, void* stream) {
-  g_err[0] = 0;
+static int project_impl(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights,
+                        const int32_t* weight_rows, int32_t n_weights, void* out, int64_t out_stride, void* stream, bool pdl) {
   if (!x || !weights || !weight_rows || !out) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: arguments must not be NULL");
   if (n_rows <= 0 || n_rows > kProjectRows || n_weights <= 0 || n_weights > kProjectParts || width <= 0 || width % 32)
     return fail(KVM_ERR_UNSUPPORTED, "kvm_project: %d rows (1..%d), %d layers (1..%d), width %d (a multiple of 32)", n_rows, kProjectRows,
@@ -415,9 +425,15 @@ int kvm_project(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, 
   if (out_stride < cols) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_project: output stride %lld below %lld columns", (long long)out_stride, (long long)cols);
   a.out = static_cast<bf16*>(out);
   a.out_stride = out_stride;
-  const cudaError_t e = kvm::launch_project(a, static_cast<cudaStream_t>(stream));
+  const cudaError_t e = kvm::launch_project(a, static_cast<cudaStream_t>(stream), pdl);
   if (e != cudaSuccess) return cuda_fail(e, "kvm_project");
   return KVM_OK;
+}
+
+int kvm_project(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights, const int32_t* weight_rows,
+                int32_t n_weights, void* out, int64_t out_stride, void* stream) {
+  g_err[0] = 0;
+  return project_impl(x, x_stride, n_rows, width, weights, weight_rows, n_weights, out, out_stride, stream, false);
 }
 
 int kvm_prefill_workspace_layout(const kvm_layer* layer, int32_t batch, int64_t seq_len, int64_t total_version_rows,
@@ -706,6 +722,113 @@ int kvm_decode_cache_fill(const kvm_layer* layer, int32_t batch, int64_t seq_len
                                             batch * layer->n_kv_heads + batch + 1, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "kvm_decode_cache_fill");
   return KVM_OK;
+}
+
+// q, k, v, gate of `tokens` tokens per sequence behind `base`; v_gate and the attention output of a decode token behind them
+struct MixerScratch {
+  size_t q, k, v, gate, v_gate, att, total;
+};
+static MixerScratch mixer_scratch(const kvm_layer* l, int batch, int64_t tokens) {
+  const size_t n = (size_t)batch * tokens * 2, dq = (size_t)l->n_q_heads * l->head_dim, dk = (size_t)l->n_kv_heads * l->head_dim;
+  MixerScratch m;
+  size_t off = 0;
+  m.q = off; off = align_up(off + n * dq, 256);
+  m.k = off; off = align_up(off + n * dk, 256);
+  m.v = off; off = align_up(off + n * dk, 256);
+  m.gate = off; off = align_up(off + n * l->n_kv_heads, 256);
+  m.v_gate = off; off = align_up(off + n * dk, 256);
+  m.att = off; off = align_up(off + n * dq, 256);
+  m.total = off;
+  return m;
+}
+
+size_t kvm_token_scratch_bytes(const kvm_layer* layer, int32_t batch) {
+  return layer && batch > 0 ? mixer_scratch(layer, batch, 1).total : 0;
+}
+
+int kvm_mixer_token(const kvm_token_call* c, void* stream) {
+  g_err[0] = 0;
+  if (!c) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_mixer_token: call is NULL");
+  const kvm_layer* layer = c->decode.layer;
+  if (int rc = check_layer(layer)) return rc;
+  const int batch = c->decode.batch, D = layer->head_dim, Hq = layer->n_q_heads, Hkv = layer->n_kv_heads;
+  if (batch <= 0 || batch > kProjectRows) return fail(KVM_ERR_UNSUPPORTED, "kvm_mixer_token: batch %d must be in [1, %d]", batch, kProjectRows);
+  const bool mixed = c->v_gate2 != nullptr;
+  if (c->n_weights != 3 + (mixed ? 1 : 0) + (c->gated ? 1 : 0) || c->weight_rows[0] != Hq * D || c->weight_rows[1] != Hkv * D ||
+      c->weight_rows[2] != Hkv * D || (c->gated && c->weight_rows[c->n_weights - 1] != Hkv))
+    return fail(KVM_ERR_BAD_ARGUMENT, "kvm_mixer_token: the layers must be q, k, v, v_gate1 (with v_gate2) and the merge gate (if gated)");
+  const MixerScratch m = mixer_scratch(layer, batch, 1);
+  if (!c->scratch || c->scratch_bytes < m.total || ((uintptr_t)c->scratch) % 256) return fail(KVM_ERR_CAPACITY, "kvm_mixer_token: scratch of %zu bytes available, %zu needed", c->scratch_bytes, m.total);
+  if (!c->lin || ((uintptr_t)c->lin) % 16 || c->lin_stride % 8 || !c->y) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_mixer_token: lin must be 16-byte aligned, y not NULL");
+  unsigned char* w = static_cast<unsigned char*>(c->scratch);
+  if (int rc = project_impl(c->x, c->x_stride, batch, c->hidden, c->weights, c->weight_rows, c->n_weights, c->lin, c->lin_stride, stream, false))
+    return rc;
+  const bf16* lin = static_cast<const bf16*>(c->lin);
+  kvm_prologue pro = c->prologue;
+  pro.q_lin = lin;
+  pro.k_lin = lin + Hq * D;
+  pro.v_lin = lin + (Hq + Hkv) * D;
+  pro.q_stride_t = pro.k_stride_t = pro.v_stride_t = pro.gate_stride_t = c->lin_stride;
+  const bf16* behind = lin + (Hq + 2 * Hkv) * D;
+  pro.v_gate = nullptr;
+  if (mixed) {
+    const int32_t rows = Hkv * D;
+    if (int rc = project_impl(behind, c->lin_stride, batch, c->weight_rows[3], &c->v_gate2, &rows, 1, w + m.v_gate, rows, stream, true)) return rc;
+    pro.v_gate = w + m.v_gate;
+    behind += c->weight_rows[3];
+  }
+  pro.gate_lin = c->gated ? behind : nullptr;
+  kvm::PrologueDev p;
+  if (int rc = prologue_args(layer, batch, 1, &pro, w + m.q, w + m.k, w + m.v, w + m.gate, 0, nullptr, 0, &p)) return rc;
+  const cudaError_t e = kvm::launch_prologue(D, to_dev(layer), p, batch, 1, static_cast<cudaStream_t>(stream), true);
+  if (e != cudaSuccess) return cuda_fail(e, "kvm_mixer_token");
+  const kvm_decode_call& d = c->decode;
+  const int64_t dq = (int64_t)Hq * D, dk = (int64_t)Hkv * D;
+  if (int rc = decode_step_impl(layer, batch, d.cache, {w + m.q, dq, D, dq}, {w + m.k, dk, D, dk}, {w + m.v, dk, D, dk},
+                                {w + m.gate, Hkv, 1, 1}, d.n_append_dev, d.any_update, d.max_rows, w + m.att, d.route_dev, d.workspace,
+                                d.workspace_bytes, stream, 1, "kvm_mixer_token", false, d.n_append_host, d.total_len_host, d.state_len_host))
+    return rc;
+  return project_impl(w + m.att, dq, batch, Hq * D, &c->c_proj, &c->out_features, 1, c->y, c->out_features, stream, true);
+}
+
+size_t kvm_prompt_workspace_bytes(const kvm_layer* layer, int32_t batch, int64_t seq_len, int32_t n_updates, int64_t total_version_rows) {
+  if (!layer || batch <= 0 || seq_len <= 0 || n_updates < 0 || total_version_rows < 0) return 0;
+  return align_up(prefill_ws(layer, batch, seq_len, total_version_rows).total, 256) + align_up((size_t)(n_updates + 1) * sizeof(kvm_update_plan), 256) +
+         mixer_scratch(layer, batch, seq_len).v_gate;
+}
+
+int kvm_mixer_prompt(const kvm_prompt_call* c, void* stream) {
+  g_err[0] = 0;
+  if (!c) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_mixer_prompt: call is NULL");
+  const kvm_layer* layer = c->layer;
+  if (int rc = check_layer(layer)) return rc;
+  const int batch = c->batch, D = layer->head_dim, Hq = layer->n_q_heads, Hkv = layer->n_kv_heads;
+  const int64_t T = c->seq_len;
+  const size_t need = kvm_prompt_workspace_bytes(layer, batch, T, c->n_updates, c->total_version_rows);
+  if (!need || !c->plan_host) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_mixer_prompt: batch, seq_len and plan must be given");
+  if (!c->workspace || c->workspace_bytes < need || ((uintptr_t)c->workspace) % 256)
+    return fail(KVM_ERR_CAPACITY, "kvm_mixer_prompt: workspace of %zu bytes given, %zu needed (256-byte aligned)", c->workspace_bytes, need);
+  unsigned char* ws = static_cast<unsigned char*>(c->workspace);
+  const size_t ws_bytes = align_up(prefill_ws(layer, batch, T, c->total_version_rows).total, 256);
+  kvm_update_plan* plan_dev = reinterpret_cast<kvm_update_plan*>(ws + ws_bytes);
+  unsigned char* w = ws + ws_bytes + align_up((size_t)(c->n_updates + 1) * sizeof(kvm_update_plan), 256);
+  const MixerScratch m = mixer_scratch(layer, batch, T);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  kvm::PrologueDev p;
+  if (int rc = prologue_args(layer, batch, T, &c->prologue, w + m.q, w + m.k, w + m.v, w + m.gate, c->total_version_rows, ws, ws_bytes, &p)) return rc;
+  // (the table is in pageable host memory: the copy has taken it over when the call returns)
+  cudaError_t e = cudaMemcpyAsync(plan_dev, c->plan_host, (size_t)(c->n_updates + 1) * sizeof(kvm_update_plan), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = kvm::launch_prologue(D, to_dev(layer), p, batch, T, st, false);
+  if (e != cudaSuccess) return cuda_fail(e, "kvm_mixer_prompt");
+  const int64_t dq = (int64_t)Hq * D, dk = (int64_t)Hkv * D;
+  const kvm_tensor4 q4 = {w + m.q, T * dq, D, dq}, k4 = {w + m.k, T * dk, D, dk}, v4 = {w + m.v, T * dk, D, dk}, g4 = {w + m.gate, Hkv * T, T, 1};
+  if (int rc = prefill_forward_impl(layer, batch, T, q4, k4, v4, g4, plan_dev, c->plan_host, c->n_updates, c->total_version_rows, c->memory,
+                                    c->out, nullptr, ws, ws_bytes, KVM_PREFILL_CHAIN | KVM_PREFILL_ATTENTION | KVM_PREFILL_KEYS_PREPARED,
+                                    stream, nullptr))
+    return rc;
+  if (!c->cache.ring_k) return KVM_OK;
+  const kvm_update_plan& last = c->plan_host[c->n_updates];
+  return kvm_decode_cache_fill(layer, batch, T, k4, v4, g4, c->memory, last.state_before + last.n_append, c->cache, c->decode_workspace, stream);
 }
 
 int kvm_interleave_shards(void* dst, const void* src, int32_t n_shards, int64_t n_tokens, int64_t shard_bytes, void* stream) {

@@ -78,7 +78,7 @@ struct PrologueDev {
 };
 
 // Linear layers over the same few rows (kvm_project): part i's outputs are the columns behind those of part i - 1.
-constexpr int kProjectParts = 8, kProjectRows = 64;
+constexpr int kProjectParts = 8, kProjectRows = 128;
 struct ProjectArgs {
   const bf16* x;
   long long x_stride;

@@ -73,7 +73,7 @@ struct DecSmem {
     ored = off;   off += (size_t)kDecConsumers * G * D * 4;          // [warp][query head][D] fp32
     wred = off;   off += (size_t)2 * kDecConsumers * 16 * 4;         // per-warp running max / sum
     meta = off;   off += (size_t)ST * 32;                            // per-stage chunk description (8 ints)
-    bars = off;   off += (size_t)(2 * ST + 1) * 8;                   // full[ST], empty[ST], rendezvous
+    bars = off;   off += (size_t)(2 * ST + 2) * 8;                   // full[ST], empty[ST], rendezvous, scales
     temps = off;  off += (size_t)2 * Hq * 4;                         // folded softmax scales per query head
     seq = off;    off += (size_t)(3 * nb + 4) * 4;                   // per sequence: S, total, chunk prefix
     total = (off + 15) & ~(size_t)15;
@@ -123,6 +123,7 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, Tensor4 k, T
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + lay.bars);  // [ST] chunk landed (transaction bytes)
   uint64_t* empty = full + ST;                                        // [ST] chunk consumed (one arrival per math warp)
   uint64_t* fbar = empty + ST;                                        // rendezvous of the math warps
+  uint64_t* tbar = fbar + 1;                                          // the softmax scales are in shared memory
   float* temp_mem = reinterpret_cast<float*>(smem_raw + lay.temps);   // [Hq]
   float* temp_win = temp_mem + L.Hq;                                  // [Hq]
   int* sq_S = reinterpret_cast<int*>(smem_raw + lay.seq);             // [nb]
@@ -143,13 +144,10 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, Tensor4 k, T
       tc::mbar_init(&empty[s], NW);
     }
     tc::mbar_init(fbar, NW);
+    tc::mbar_init(tbar, 1);
     tc::fence_barrier_init();
     s_abort = 0;
     cpre[0] = 0;
-  }
-  for (int h = tid; h < L.Hq; h += kDecThreads) {
-    temp_mem[h] = sm_scale * L.state_temp[h] * kLog2e;
-    temp_win[h] = sm_scale * L.front_temp[h] * kLog2e;
   }
   // With the lengths from the host everything up to the first copy runs while the previous token's kernel finishes;
   // otherwise the lengths are that kernel's results and have to be waited for.
@@ -226,6 +224,14 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, Tensor4 k, T
         }
       }
       if (lane == 0 && !known) *done_counter = 0;
+    }
+    if (has_work) {  // the layer's parameters, like everything an earlier kernel may have written: behind the wait
+      for (int h = lane; h < L.Hq; h += 32) {
+        temp_mem[h] = sm_scale * L.state_temp[h] * kLog2e;
+        temp_win[h] = sm_scale * L.front_temp[h] * kLog2e;
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tbar);
     }
   }
 
@@ -375,7 +381,7 @@ kvm_decode_attn_kernel(LayerDev L, DecodeCacheDev cache, Tensor4 q, Tensor4 k, T
     const int vrow = warp * 16 + (lane & 7) + (lane >> 4) * 8;         // ldmatrix row of the V tile
     uint32_t fphase = 0;               // phase of the rendezvous barrier
     // (the math warps touch global memory only behind data that the producer fetched after its own wait)
-    bool alive = true;
+    bool alive = __all_sync(0xffffffffu, dec_wait(tbar, 0, abort_flag));
     // all math warps meet (bounded): false if somebody gave up
     auto rendezvous = [&]() -> bool {
       __syncwarp();

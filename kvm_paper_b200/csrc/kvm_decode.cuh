@@ -4,7 +4,7 @@
 
 #include <cuda.h>
 
-#include "kvm_common.cuh"
+#include "kvm_pdl.cuh"
 #include "kvm_tc.cuh"
 #include "kvm_tma_host.cuh"
 
@@ -15,14 +15,8 @@ __device__ __forceinline__ int bswa_begin_dev(int total, int C, int W) {
   return max(0, end - W * C);
 }
 
-// Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may start
-// while its predecessor in the stream still runs; pdl_wait() returns once the predecessor has completed
-// and its writes are visible (at once if the launch did not carry the attribute); pdl_trigger() lets the
-// successor start early.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Writes of this thread (also to global memory) -> visible to its later asynchronous copies.
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One box of a 2-D tensor into L2 (a hint: nothing is waited for).
 __device__ __forceinline__ void prefetch_2d(const CUtensorMap* m, int x, int y) {
@@ -120,22 +114,5 @@ bool decode_maps(const DecodeCacheDev& c, uint64_t kv_rows, int cap, int WC, int
 // The boundary updates of the listed sequences (nothing else runs on the GPU meanwhile).
 cudaError_t decode_update(int D, const LayerDev& L, int batch, const DecodeCacheDev& cache, const UpdateSet& upd, bf16* pk_scr,
                           cudaStream_t stream);
-
-// Launch with the programmatic-serialization attribute when `pdl` is set (see pdl_wait above).
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
-                              Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-}
 
 }  // namespace kvm

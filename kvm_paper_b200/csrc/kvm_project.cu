@@ -1,4 +1,4 @@
-// Linear layers over a handful of rows (decode tokens): y[m, n] = sum_k x[m, k] * w[n, k] for up to 64 rows of x and
+// Linear layers over few rows (decode tokens, short prompts): y[m, n] = sum_k x[m, k] * w[n, k] for up to 128 rows of x and
 // several weight matrices at once.
 //
 // Bound by reading the weights once (33 MB around a 2048-wide mixer: 5 us at the copy bandwidth) and by launches, so all
@@ -7,8 +7,9 @@
 // the first is used.  Warp-level MMAs with the weight rows on M and the input rows on N.  The order of k inside a 32-wide
 // slice is permuted alike in both operands (thread t of a quad holds k = 8t .. 8t+7), so that fragments are loaded
 // straight from global memory with 16-byte accesses.  Sums: fp32, warps in order, rounded once to bf16.
-// Measured, B200, 8 rows x 2048 -> 6256 + 2048 columns: see the table of the design notes.
-#include "kvm_common.cuh"
+// More than 64 rows take a second layer of CTAs (the weights then come from L2).  The first loads of the weights are issued
+// before the wait for the previous kernel, whose results are only the input rows.
+#include "kvm_pdl.cuh"
 
 namespace kvm {
 
@@ -32,23 +33,30 @@ kvm_project_kernel(const __grid_constant__ ProjectArgs a) {
   const int n_rows = a.rows[part], r0 = tile * 16;
   const bf16* w_lo = a.weight[part] + (size_t)min(r0 + g, n_rows - 1) * a.K + t * 8;  // rows past the end repeat the last one
   const bf16* w_hi = a.weight[part] + (size_t)min(r0 + g + 8, n_rows - 1) * a.K + t * 8;
+  const int m0 = blockIdx.y * NT * 8;
   const bf16* xp[NT];
 #pragma unroll
-  for (int n = 0; n < NT; ++n) xp[n] = a.x + (size_t)min(n * 8 + g, a.M - 1) * a.x_stride + t * 8;
+  for (int n = 0; n < NT; ++n) xp[n] = a.x + (size_t)min(m0 + n * 8 + g, a.M - 1) * a.x_stride + t * 8;
   float acc[NT][4];
 #pragma unroll
   for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
   const int slices = a.K / 32, per = (slices + kProjWarps - 1) / kProjWarps;
   const int s_end = min(slices, (warp + 1) * per);
   constexpr int kAhead = NT <= 2 ? 8 : 4;  // slices whose loads are issued together
+  pdl_trigger();
+  bool waited = false;
   for (int s0 = warp * per; s0 < s_end; s0 += kAhead) {
     uint4 wl[kAhead], wh[kAhead];
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       if (s0 + i < s_end) {
-        wl[i] = __ldcs(reinterpret_cast<const uint4*>(w_lo + (s0 + i) * 32));
-        wh[i] = __ldcs(reinterpret_cast<const uint4*>(w_hi + (s0 + i) * 32));
+        wl[i] = __ldg(reinterpret_cast<const uint4*>(w_lo + (s0 + i) * 32));
+        wh[i] = __ldg(reinterpret_cast<const uint4*>(w_hi + (s0 + i) * 32));
       }
+    }
+    if (!waited) {
+      pdl_wait();
+      waited = true;
     }
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
@@ -71,25 +79,24 @@ kvm_project_kernel(const __grid_constant__ ProjectArgs a) {
     red[warp][g + 8][n * 8 + t * 2 + 1] = acc[n][3];
   }
   __syncthreads();
-  for (int e = tid; e < 16 * a.M; e += kProjWarps * 32) {  // consecutive threads: consecutive columns of one output row
+  if (!waited) pdl_wait();  // (a warp without a share of k: nothing is written ahead of the previous kernel's end)
+  for (int e = tid; e < 16 * min(NT * 8, a.M - m0); e += kProjWarps * 32) {  // consecutive threads: consecutive columns of an output row
     const int r = e & 15, m = e >> 4;
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < kProjWarps; ++w) s += red[w][r][m];
-    if (r0 + r < n_rows) a.out[(size_t)m * a.out_stride + col0 + r0 + r] = __float2bfloat16_rn(s);
+    if (r0 + r < n_rows) a.out[(size_t)(m0 + m) * a.out_stride + col0 + r0 + r] = __float2bfloat16_rn(s);
   }
 }
 
 }  // namespace
 
-cudaError_t launch_project(const ProjectArgs& a, cudaStream_t stream) {
+cudaError_t launch_project(const ProjectArgs& a, cudaStream_t stream, bool pdl) {
   int ctas = 0;
   for (int i = 0; i < a.n_parts; ++i) ctas += (a.rows[i] + 15) / 16;
-  if (a.M <= 8) kvm_project_kernel<1><<<ctas, kProjWarps * 32, 0, stream>>>(a);
-  else if (a.M <= 16) kvm_project_kernel<2><<<ctas, kProjWarps * 32, 0, stream>>>(a);
-  else if (a.M <= 32) kvm_project_kernel<4><<<ctas, kProjWarps * 32, 0, stream>>>(a);
-  else kvm_project_kernel<8><<<ctas, kProjWarps * 32, 0, stream>>>(a);
-  return cudaGetLastError();
+  const int nt = a.M <= 8 ? 1 : a.M <= 16 ? 2 : a.M <= 32 ? 4 : 8;
+  auto kern = nt == 1 ? kvm_project_kernel<1> : nt == 2 ? kvm_project_kernel<2> : nt == 4 ? kvm_project_kernel<4> : kvm_project_kernel<8>;
+  return launch_pdl(kern, dim3(ctas, (a.M + nt * 8 - 1) / (nt * 8)), dim3(kProjWarps * 32), 0, stream, pdl, a);
 }
 
 }  // namespace kvm

@@ -12,7 +12,7 @@
 // One group of 8 lanes per (token, head) row, D/8 contiguous elements per lane (16-byte accesses; a rotary pair never
 // straddles lanes).  The kernel is a single streaming pass: q, k, v are read once (plus the previous token's
 // row, which the neighbouring group has just read: an L1/L2 hit) and written once.
-#include "kvm_common.cuh"
+#include "kvm_pdl.cuh"
 
 namespace kvm {
 
@@ -118,6 +118,8 @@ template <int D>
 __global__ void __launch_bounds__(256)
 kvm_prologue_kernel(LayerDev L, PrologueDev p, long long T) {
   constexpr int EPL = D / GL;
+  pdl_trigger();
+  pdl_wait();
   const int gl = threadIdx.x % GL;
   const int HS = L.Hq + 2 * L.Hkv;  // rows per token: query heads, key heads, value heads
   // (the lane groups of a warp reduce with full-warp shuffles: every group runs the same sequence of reductions, on
@@ -232,16 +234,15 @@ kvm_prologue_kernel(LayerDev L, PrologueDev p, long long T) {
 
 }  // namespace
 
-cudaError_t launch_prologue(int D, const LayerDev& L, const PrologueDev& p, int batch, long long T, cudaStream_t stream) {
+cudaError_t launch_prologue(int D, const LayerDev& L, const PrologueDev& p, int batch, long long T, cudaStream_t stream, bool pdl) {
   const long long units = T * (L.Hq + 2 * L.Hkv);
   const dim3 grid((unsigned)((units + 256 / GL - 1) / (256 / GL)), (unsigned)batch);
   switch (D) {
-    case 32: kvm_prologue_kernel<32><<<grid, 256, 0, stream>>>(L, p, T); break;
-    case 64: kvm_prologue_kernel<64><<<grid, 256, 0, stream>>>(L, p, T); break;
-    case 128: kvm_prologue_kernel<128><<<grid, 256, 0, stream>>>(L, p, T); break;
-    default: return cudaErrorInvalidValue;
+    case 32: return launch_pdl(kvm_prologue_kernel<32>, grid, dim3(256), 0, stream, pdl, L, p, T);
+    case 64: return launch_pdl(kvm_prologue_kernel<64>, grid, dim3(256), 0, stream, pdl, L, p, T);
+    case 128: return launch_pdl(kvm_prologue_kernel<128>, grid, dim3(256), 0, stream, pdl, L, p, T);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace kvm

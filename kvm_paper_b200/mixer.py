@@ -402,6 +402,8 @@ class SequenceMixer(nn.Module):
     # ------------------------------------------------------------------ module entry points
     def _prompt_fused(self, x, v_first, position_embeddings, attention_mask, past_key_values, **kwargs):
         """A prompt through the one-kernel prologue, which also leaves the prepared keys in the prefill's workspace."""
+        if not kwargs and self._unwatched("forward_prefill"):
+            return self._prompt(x, v_first, position_embeddings, past_key_values)
         runner = None
 
         def make_runner():  # called while the projections run; its memory has room for a decode cache to go on in it
@@ -415,6 +417,72 @@ class SequenceMixer(nn.Module):
         return self.forward_prefill(q, k, v, gate, v_first, position_embeddings, attention_mask, past_key_values,
                                     _prefill_runner=runner, **kwargs)
 
+    def _unwatched(self, stage: str) -> bool:
+        """Nobody looks at the tensors between the stages of a call (no hook, no override of the stage behind the prefix):
+        the stages may run as one library call."""
+        return not (self.capture_routes or self.check_device_status or torch.is_grad_enabled() or stage in self.__dict__
+                    or "forward_prefix_fused" in self.__dict__ or getattr(type(self), stage) is not getattr(SequenceMixer, stage)
+                    or type(self).forward_prefix_fused is not SequenceMixer.forward_prefix_fused)
+
+    def _prompt(self, x, v_first, position_embeddings, past_key_values):
+        """``forward_prefix_fused`` and ``forward_prefill`` of a prompt in one library call between the linear layers; the
+        schedule is planned while the projections run."""
+        B, T, _ = x.size()
+        if past_key_values is not None and past_key_values.get_seq_length(self.layer_idx) > 0 and T != 1:
+            raise AssertionError("cached decode expects single-token inputs.")
+        dev = x.device
+        q, k, v, v_gate, gate_lin = self._project(x)
+        residual = v_last = None
+        if self.value_residual_mode == "linear":
+            v = ((1 - self.lamb) * v + self.lamb * v_first.view_as(v)).contiguous()
+        elif self.value_residual_mode == "rwkv":
+            residual = (v_first, v_gate, self.v_gate0)
+            v_last = torch.empty(B, 1, self.value_projection_size, device=dev, dtype=x.dtype)
+        params, pro = self.layer_params(dev), self._prologue_params_kept(dev)
+        prev = None
+        if past_key_values is not None:
+            states = past_key_values.get_states(self.layer_idx)
+            prev = (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL))
+        cache, y = ops.prompt_forward(params, pro, q, k, v, gate_lin, position_embeddings, self.make_prefill_plan(T), prev=prev,
+                                      value_residual=residual, v_last=v_last, desired_state_len=self._desired_state_len, owner=self,
+                                      want_cache=past_key_values is not None)
+        if past_key_values is not None:
+            past_key_values.update(self.layer_idx, offset=T, states_dict={
+                self._CACHE_Q_FINAL: q[:, -1:].detach(), self._CACHE_K_FINAL: k[:, -1:].detach(),
+                self._CACHE_V_FINAL: v[:, -1:].detach() if v_last is None else v_last, self._CACHE_X_FINAL: x[:, -1:].detach(),
+                self._CACHE_DECODE: cache})
+        return self._output(y)
+
+    def _token(self, x, v_first, position_embeddings, past_key_values):
+        """One cached token as one library call (``kvm_mixer_token``), or None where a stage has to run by itself."""
+        if not self._unwatched("forward_single") or x.dim() != 3 or x.size(1) != 1 or not self._few_rows(x):
+            return None
+        states = past_key_values.get_states(self.layer_idx)
+        cache = states.get(self._CACHE_DECODE)
+        B = x.size(0)
+        mixed = self.value_residual_mode == "rwkv"
+        gated = bool(self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values)
+        lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
+        c_proj = self.c_proj
+        if (not isinstance(cache, ops.KvmDecodeCache) or cache.owner is not self or cache.batch != B or self.value_residual_mode == "linear"
+                or not (cache.total_len_h == past_key_values.get_seq_length(self.layer_idx)).all()
+                or not all(self._plain_linear(m, x) for m in lins) or not self._plain_linear(c_proj, x) or c_proj.out_features % 8
+                or (mixed and not self._plain_linear(self.v_gate2, x))):
+            return None
+        dev = x.device
+        call = ops.TokenCall.of(cache, self.layer_params(dev), self._prologue_params_kept(dev))
+        y, lin, v_last = call.run(x, [m.weight for m in lins], self.v_gate2.weight if mixed else None, c_proj.weight, gated,
+                                  (v_first, self.v_gate0) if mixed else None, position_embeddings,
+                                  (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL)))
+        dq, dk = self.q_projection_size, self.k_projection_size
+        v_final = v_last if mixed else lin[..., dq + dk:dq + 2 * dk]
+        finals = (lin[..., :dq], lin[..., dq:dq + dk], v_final)
+        call.produced(finals)
+        past_key_values.update(self.layer_idx, offset=1, states_dict={
+            self._CACHE_Q_FINAL: finals[0], self._CACHE_K_FINAL: finals[1], self._CACHE_V_FINAL: v_final, self._CACHE_X_FINAL: x,
+            self._CACHE_DECODE: cache})
+        return y
+
     def forward(self, x, v_first, position_embeddings, attention_mask, past_key_values=None, **kwargs):
         if self.use_fused_prologue and attention_mask is None and self.fused_prologue_applies(x):
             return self._prompt_fused(x, v_first, position_embeddings, attention_mask, past_key_values, **kwargs)
@@ -427,6 +495,9 @@ class SequenceMixer(nn.Module):
             return self._prompt_fused(x, v_first, position_embeddings, attention_mask, past_key_values, **kwargs)
         if past_len > 0 and self.use_fused_prologue and attention_mask is None and self.fused_prologue_applies(x):
             # cached single-token step: the same kernel, shifting against the previous call's last token
+            y = self._token(x, v_first, position_embeddings, past_key_values) if not kwargs else None
+            if y is not None:
+                return y
             q, k, v, gate = self.forward_prefix_fused(x, v_first, position_embeddings, past_key_values)
         else:
             q, k, v, gate = self.forward_prefix(x, v_first, position_embeddings, attention_mask, past_key_values, **kwargs)

@@ -137,10 +137,14 @@ class PrefillPlan:
             arr[i] = KvmUpdatePlan(sb, na, vr, 0)
         return arr
 
-    def to_tensor(self, device) -> torch.Tensor:
+    def to_array(self) -> np.ndarray:
+        """The table as the C side reads it (kvm_update_plan)."""
         t = np.zeros((len(self.n_append), 4), dtype=np.int32)
         t[:, 0], t[:, 1], t[:, 2] = self.state_before, self.n_append, self.version_row
-        return torch.from_numpy(t).to(device, non_blocking=True)
+        return t
+
+    def to_tensor(self, device) -> torch.Tensor:
+        return torch.from_numpy(self.to_array()).to(device, non_blocking=True)
 
 
 def build_prefill_plan(seq_len: int, chunk_len: int, n_bswa_chunks: int,
@@ -250,18 +254,19 @@ def _token_stride(t: torch.Tensor, B: int, T: int, width: int, name: str) -> int
     return step
 
 
-def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tensor, k_lin: torch.Tensor, v_lin: torch.Tensor,
-                     gate_lin: torch.Tensor | None, position_embeddings, *, prev=None, runner: "PrefillRunner | None" = None,
-                     out: tuple | None = None, value_residual: tuple | None = None, v_last: torch.Tensor | None = None):
-    """Value residual, token shift, q/k LayerNorm, rotary embedding and merge gate in one kernel over the projection
-    outputs ([B,T,H*D] bf16, contiguous or column ranges of one wider GEMM output).  Returns q [B,Hq,T,D], k, v
-    [B,Hkv,T,D], gate [B,Hkv,T,1] as views of [B,T,H,D] / [B,Hkv,T]
-    buffers, the layouts the reference hands its mixer (model/kvm_mixer.py:397-399).  With ``runner`` the prepared
-    keys of the tokens that memory updates consume are written into that runner's workspace, and its ``run`` may
-    be called with ``keys_prepared=True``.  ``prev`` = (q, k, v) rows [B,1,H*D] of the previous call's last token.
-    ``out`` = preallocated (q [B,T,Hq,D], k, v [B,T,Hkv,D], gate [B,Hkv,T]) bf16 buffers to write into.
-    ``value_residual`` = (v_first, output of v_gate2, v_gate0) of the "rwkv" value residual; ``v_last`` [B,1,Hkv*D]
-    receives the last token's value behind it (what the next call's ``prev`` needs)."""
+def rotary_tables_arg(position_embeddings, B: int, T: int, D: int, dev):
+    """(cos, sin) as contiguous bf16 tables on the device, and whether every sequence has its own."""
+    cs = [t if t.dtype is torch.bfloat16 and t.device == dev and t.is_contiguous() else t.to(dev, torch.bfloat16).contiguous()
+          for t in position_embeddings]
+    n = cs[0].numel() // (T * D)
+    if n not in (1, B) or cs[0].numel() != n * T * D or cs[1].numel() != cs[0].numel():
+        raise ValueError(f"rotary tables must be [1 or {B}, {T}, .., {D}], got {tuple(cs[0].shape)} and {tuple(cs[1].shape)}")
+    return cs[0], cs[1], n > 1
+
+
+def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin, gate_lin, position_embeddings, prev, value_residual,
+                  v_last):
+    """The C argument block of the prologue and the tensors it points into (see ``prologue_forward``)."""
     cfg = params.cfg
     B, T, _ = q_lin.shape
     D, Hq, Hkv = cfg.head_dim, cfg.n_q_heads, cfg.n_kv_heads
@@ -297,14 +302,29 @@ def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tens
         arg.ln_q_w, arg.ln_q_b, arg.ln_k_w, arg.ln_k_b = pro.ln_ptrs
         arg.ln_qk_eps = pro.ln_eps
     if position_embeddings is not None:
-        cs = [t if t.dtype is torch.bfloat16 and t.device == dev and t.is_contiguous() else t.to(dev, torch.bfloat16).contiguous()
-              for t in position_embeddings]
-        n_rope = cs[0].numel() // (T * D)
-        if n_rope not in (1, B) or cs[0].numel() != n_rope * T * D or cs[1].numel() != cs[0].numel():
-            raise ValueError(f"rotary tables must be [1 or {B}, {T}, .., {D}], got {tuple(cs[0].shape)} and {tuple(cs[1].shape)}")
-        keep += cs
-        arg.cos, arg.sin = cs[0].data_ptr(), cs[1].data_ptr()
-        arg.rope_stride_b = 0 if n_rope == 1 else T * D
+        cos, sin, own = rotary_tables_arg(position_embeddings, B, T, D, dev)
+        keep += [cos, sin]
+        arg.cos, arg.sin, arg.rope_stride_b = cos.data_ptr(), sin.data_ptr(), T * D if own else 0
+    return arg, keep
+
+
+def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tensor, k_lin: torch.Tensor, v_lin: torch.Tensor,
+                     gate_lin: torch.Tensor | None, position_embeddings, *, prev=None, runner: "PrefillRunner | None" = None,
+                     out: tuple | None = None, value_residual: tuple | None = None, v_last: torch.Tensor | None = None):
+    """Value residual, token shift, q/k LayerNorm, rotary embedding and merge gate in one kernel over the projection
+    outputs ([B,T,H*D] bf16, contiguous or column ranges of one wider GEMM output).  Returns q [B,Hq,T,D], k, v
+    [B,Hkv,T,D], gate [B,Hkv,T,1] as views of [B,T,H,D] / [B,Hkv,T]
+    buffers, the layouts the reference hands its mixer (model/kvm_mixer.py:397-399).  With ``runner`` the prepared
+    keys of the tokens that memory updates consume are written into that runner's workspace, and its ``run`` may
+    be called with ``keys_prepared=True``.  ``prev`` = (q, k, v) rows [B,1,H*D] of the previous call's last token.
+    ``out`` = preallocated (q [B,T,Hq,D], k, v [B,T,Hkv,D], gate [B,Hkv,T]) bf16 buffers to write into.
+    ``value_residual`` = (v_first, output of v_gate2, v_gate0) of the "rwkv" value residual; ``v_last`` [B,1,Hkv*D]
+    receives the last token's value behind it (what the next call's ``prev`` needs)."""
+    cfg = params.cfg
+    B, T, _ = q_lin.shape
+    D, Hq, Hkv = cfg.head_dim, cfg.n_q_heads, cfg.n_kv_heads
+    dev = q_lin.device
+    arg, keep = _prologue_arg(params, pro, q_lin, k_lin, v_lin, gate_lin, position_embeddings, prev, value_residual, v_last)
     if out is not None:
         q, k, v, gate = out
         for t, shape in ((q, (B, T, Hq, D)), (k, (B, T, Hkv, D)), (v, (B, T, Hkv, D)), (gate, (B, Hkv, T))):
@@ -533,6 +553,7 @@ class KvmDecodeCache:
 
     cache_representation = "preallocated memory rows + W*C-token ring, per-sequence lengths on device"
     _quiet = 0
+    _token = None  # the mixer's kept arguments of kvm_mixer_token for this cache
 
     def __init__(self, params: LayerParams, batch: int, state_capacity: int,
                  desired_state_len: Callable[[int, int, int], int], owner: Any = None, *, _memory: MemoryBuffers | None = None):
@@ -685,21 +706,14 @@ class KvmDecodeCache:
         Returns [B,1,Hq*D] (a buffer owned by the cache, overwritten by the next step)."""
         if q.shape != self._q_shape or k.shape != self._kv_shape:
             raise ValueError(f"decode expects one token per sequence, got q {tuple(q.shape)} k {tuple(k.shape)}")
-        n_app, max_rows = self._plan_step()
+        n_app = self._begin_step()
         any_update = n_app is not None
-        self._last_any_update, self._last_n_append = any_update, n_app
-        if any_update or self._quiet == 0:
-            need = int(self.state_len_h.max())
-            if need > self.memory.capacity:
-                self._reserve(need)
         call = self._call
         addr, cq, ck, cv, cg = self._call_args
         q, k = _fill_tensor4(cq, q, "q"), _fill_tensor4(ck, k, "k")
         v, gate = _fill_tensor4(cv, v, "v"), _fill_tensor4(cg, gate, "gate")
-        call.max_rows = max_rows if max_rows < self._max_rows_bound else self._max_rows_bound
+        call.max_rows = min(self._max_rows, self._max_rows_bound)
         if any_update:
-            if int((n_app >= 0).sum()) > _lib.UPDATE_LIST_MAX:
-                self._upload_n_append(n_app)
             call.any_update, call.n_append_host = 1, n_app.ctypes.data
             if want_route:
                 self.route = torch.zeros(self.kv_rows, self.cfg.chunk_len, device=self.device, dtype=torch.int32)
@@ -710,6 +724,19 @@ class KvmDecodeCache:
         if rc:
             _lib.check(rc)
         return self.out
+
+    def _begin_step(self):
+        """The host side of a token ahead of its launch: schedule, room for the rows it appends.  Returns the append counts
+        (None: no sequence updates its memory)."""
+        n_app, _ = self._plan_step()
+        self._last_any_update, self._last_n_append = n_app is not None, n_app
+        if n_app is not None or self._quiet == 0:
+            need = int(self.state_len_h.max())
+            if need > self.memory.capacity:
+                self._reserve(need)
+            if n_app is not None and int((n_app >= 0).sum()) > _lib.UPDATE_LIST_MAX:
+                self._upload_n_append(n_app)
+        return n_app
 
     def _upload_n_append(self, n_app):
         """The step's append counts to the device (for steps at which more sequences update than a launch can list)."""
@@ -847,3 +874,133 @@ def decode_cache_from_prefill(params: LayerParams, res: PrefillResult, k: torch.
     cache.total_len_h[:] = T
     cache.state_len_h[:] = S
     return cache
+
+
+def prompt_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tensor, k_lin: torch.Tensor, v_lin: torch.Tensor,
+                   gate_lin: torch.Tensor | None, position_embeddings, plan: PrefillPlan, *, prev=None, value_residual=None, v_last=None,
+                   desired_state_len=None, owner=None, want_cache: bool = True) -> tuple[KvmDecodeCache | None, torch.Tensor]:
+    """A prompt from the projection outputs to the input of ``c_proj`` in one library call: ``prologue_forward``, prefill and
+    the decode cache behind it (which lives in the prefill's memory).  Returns (cache or None, [B,T,Hq*D])."""
+    lib = _lib.load()
+    cfg = params.cfg
+    B, T, _ = q_lin.shape
+    dev = q_lin.device
+    if plan.seq_len != T:
+        raise ValueError("plan was built for another sequence length")
+    S = plan.final_state_len
+    memory = MemoryBuffers(B * cfg.n_kv_heads, S + cfg.chunk_len, cfg.head_dim, dev, zero=False)
+    out = torch.empty(B, T, cfg.n_q_heads * cfg.head_dim, device=dev, dtype=torch.bfloat16)
+    call = _lib.KvmPromptCall()
+    call.layer, call.batch, call.n_updates, call.seq_len = C.addressof(params.c), B, plan.n_updates, T
+    call.total_version_rows = plan.total_version_rows
+    call.workspace_bytes = lib.kvm_prompt_workspace_bytes(C.byref(params.c), B, T, plan.n_updates, plan.total_version_rows)
+    ws = torch.empty(call.workspace_bytes, device=dev, dtype=torch.uint8)
+    table = plan.to_array()
+    call.plan_host, call.workspace, call.out, call.memory = table.ctypes.data, ws.data_ptr(), out.data_ptr(), memory.c()
+    arg, keep = _prologue_arg(params, pro, q_lin, k_lin, v_lin, gate_lin, position_embeddings, prev, value_residual, v_last)
+    call.prologue = arg
+    cache = None
+    if want_cache:
+        cache = KvmDecodeCache(params, B, S + cfg.chunk_len, desired_state_len, owner, _memory=memory)
+        call.cache, call.decode_workspace = cache._call.cache, cache._ws.data_ptr()
+        cache.total_len_h[:] = T
+        cache.state_len_h[:] = S
+    rc = lib.kvm_mixer_prompt(C.addressof(call), _stream_ptr(dev))
+    if rc:
+        _lib.check(rc)
+    del keep  # (enqueued on the current stream: torch's allocator keeps the blocks until the kernels have run)
+    return cache, out
+
+
+class TokenCall:
+    """The kept argument block of ``kvm_mixer_token`` for one decode cache: between tokens only a few addresses change."""
+
+    def __init__(self, cache: KvmDecodeCache, params: LayerParams, pro: PrologueParams):
+        self.cache, self.params, self.pro, self.decode_src = cache, params, pro, cache._call
+        c = self.c = _lib.KvmTokenCall()
+        c.decode = cache._call
+        c.scratch_bytes = _lib.load().kvm_token_scratch_bytes(C.byref(params.c), cache.batch)
+        self._scratch = torch.empty(c.scratch_bytes, device=cache.device, dtype=torch.uint8)
+        c.scratch = self._scratch.data_ptr()
+        p = c.prologue
+        if pro.shift_q is not None:
+            p.shift_q, p.shift_k, p.shift_v = pro.shift_ptrs
+        if pro.ln is not None:
+            p.ln_q_w, p.ln_q_b, p.ln_k_w, p.ln_k_b = pro.ln_ptrs
+            p.ln_qk_eps = pro.ln_eps
+        self._views = (C.addressof(c), c.decode, p, c.weights, c.weight_rows)
+        self._finals = (None, None, None)
+
+    @staticmethod
+    def of(cache: KvmDecodeCache, params: LayerParams, pro: PrologueParams) -> "TokenCall":
+        t = cache._token
+        if t is None or t.params is not params or t.pro is not pro:
+            t = cache._token = TokenCall(cache, params, pro)
+        return t
+
+    def produced(self, finals):
+        """The tensors handed out as the token's cached rows: the next call recognises them."""
+        self._finals = finals
+
+    def run(self, x, weights, v_gate2, c_proj, gated, residual, position_embeddings, prev):
+        """x [B,1,hidden]; returns (y [B,1,out], projections [B,1,..], last values behind the residual or None)."""
+        cache, cfg = self.cache, self.cache.cfg
+        addr, decode, p, w, rows = self._views
+        c, B, dev = self.c, cache.batch, cache.device
+        keep = []
+        if not x.is_contiguous():
+            x = x.contiguous()
+        cos = sin = None
+        if position_embeddings is not None:
+            cos, sin, own = rotary_tables_arg(position_embeddings, B, 1, cfg.head_dim, x.device)
+            p.cos, p.sin, p.rope_stride_b = cos.data_ptr(), sin.data_ptr(), cfg.head_dim if own else 0
+        else:
+            p.cos, p.sin = None, None
+        v_last = None
+        if residual is not None:
+            v_first, v_gate0 = residual
+            if v_first.dtype is not torch.bfloat16 or not v_first.is_contiguous():
+                v_first = v_first.to(torch.bfloat16).contiguous()
+            if v_first.numel() != B * cfg.n_kv_heads * cfg.head_dim:
+                raise ValueError(f"value residual: v_first must have {cfg.n_kv_heads * cfg.head_dim} values per token")
+            keep.append(v_first)
+            v_last = torch.empty(B, 1, cfg.n_kv_heads * cfg.head_dim, device=x.device, dtype=torch.bfloat16)
+            p.v_first, p.v_gate0, p.v_last = v_first.data_ptr(), v_gate0.data_ptr(), v_last.data_ptr()
+        if self.pro.shift_q is not None:
+            mine = self._finals
+            if prev[0] is not None and prev[0] is mine[0] and prev[1] is mine[1] and prev[2] is mine[2]:
+                pv = prev
+            elif all(t is not None for t in prev):
+                pv = [t.to(x.device, torch.bfloat16).reshape(B, 1, -1).contiguous() for t in prev]
+            else:
+                pv = None
+            if pv is None:
+                p.prev_q, p.prev_k, p.prev_v = None, None, None
+            else:
+                keep.append(pv)
+                p.prev_q, p.prev_k, p.prev_v = pv[0].data_ptr(), pv[1].data_ptr(), pv[2].data_ptr()
+                if B > 1:
+                    p.prev_q_stride_b, p.prev_k_stride_b, p.prev_v_stride_b = pv[0].stride(0), pv[1].stride(0), pv[2].stride(0)
+        cols = 0
+        for i, t in enumerate(weights):
+            w[i], rows[i] = t.data_ptr(), t.size(0)
+            cols += t.size(0)
+        cols = (cols + 7) // 8 * 8
+        lin = torch.empty(B, 1, cols, device=x.device, dtype=torch.bfloat16)
+        y = torch.empty(B, 1, c_proj.size(0), device=x.device, dtype=torch.bfloat16)
+        c.x, c.x_stride, c.hidden, c.n_weights, c.gated = x.data_ptr(), x.size(2), x.size(2), len(weights), gated
+        c.v_gate2 = None if v_gate2 is None else v_gate2.data_ptr()
+        c.c_proj, c.out_features = c_proj.data_ptr(), c_proj.size(0)
+        c.lin, c.lin_stride, c.y = lin.data_ptr(), cols, y.data_ptr()
+        n_app = cache._begin_step()
+        if self.decode_src is not cache._call:  # (the memory has been moved to larger arrays)
+            c.decode = self.decode_src = cache._call
+        decode.max_rows = min(cache._max_rows, cache._max_rows_bound)
+        if n_app is not None:
+            decode.any_update, decode.n_append_host = 1, n_app.ctypes.data
+        rc = _lib.load().kvm_mixer_token(addr, _stream_ptr(dev))
+        if n_app is not None:
+            decode.any_update, decode.n_append_host = 0, None
+        if rc:
+            _lib.check(rc)
+        return y, lin, v_last
