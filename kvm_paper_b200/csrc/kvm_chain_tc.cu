@@ -16,19 +16,23 @@
 //                                             per token; both partial results exchanged between the CTAs in one
 //                                             go (st.async into the peers' shared memory); the n_append tokens of
 //                                             lowest bf16-rounded novelty are appended (LayerNorm by one warp per
-//                                             row) and scored against every token (dot products, or a small third
-//                                             MMA pass); a new row wins a token only with a strictly larger logit
+//                                             row) and scored against every token (warp-level MMAs, a token warp its
+//                                             own 32 tokens); a new row wins a token only with a strictly larger logit
 //                                             (with many appended rows: novelty pass, appends, then one logits pass
 //                                             against the memory after the appends)
 //                           2. scatter        delta[rows x D] = onehot[rows x tokens] x gk[tokens x D] on the
 //                                             tensor cores (touched rows compacted onto the 128 accumulator
-//                                             lanes; the one-hot operand lives in the buffer of the prepared keys,
-//                                             cleared by the copy engine; products are exact, the accumulation order
-//                                             is the hardware's and fixed), then row = bf16(row + bf16(delta)),
+//                                             lanes; a row's first token stands for it: it names its accumulator lane and
+//                                             its pool row; the one-hot operand lives in the buffer of the prepared
+//                                             keys, cleared by the copy engine; products are exact, the accumulation
+//                                             order is the hardware's and fixed), then row = bf16(row + bf16(delta)),
 //                                             LayerNorm refresh of the touched rows into shared memory and into the
-//                                             row pool
+//                                             row pool, staged so that global memory sees whole rows
+//                         What only a token needs (exchange, selection, new rows, routing table, one-hot) runs on the
+//                         C / 32 warps whose threads stand for the tokens, with barriers of just those.
 //                         Prepared keys pk and gated keys gk = bf16(pk * gate) of every token come from a parallel
-//                         pre-pass and arrive by tiled TMA, issued as soon as the scatter has read the buffers.
+//                         pre-pass and arrive by tiled TMA, issued as soon as the buffers are free (prepared keys only
+//                         for blocks that append rows).
 //                         CTAs of the launch beyond the routing's (whole clusters on the SMs it leaves free) work on
 //                         the value side meanwhile: see kvm_vdelta.cuh.
 //   value side            which no later update reads: value deltas per (kv row, update) on the tensor cores
@@ -36,6 +40,9 @@
 //                         the variant for a chain of which only the final memory is wanted (no versions): one warp
 //                         per memory row walks the routing decisions of all updates and accumulates the gated
 //                         values routed to its row in token order.
+// The code of an update is walked through once per update by warps that wait for one another, so instruction fetch is part of
+// its latency: what an update touches is kept small enough to stay in the SM's instruction cache (rolled loops, the loops of
+// waits and the read-back of accumulators not inlined, shifts instead of divisions by the cluster size).
 // Every wait is bounded; a wait that runs out sets the status word, all roles and all CTAs of the cluster leave
 // through the common exit, tensor memory is freed.
 #include <algorithm>
@@ -57,9 +64,8 @@ constexpr int kIssuers = 2;                   // issuing threads (one warp each)
 constexpr int kThreads = kWorkers + kIssuers * 32;
 constexpr int kChunk = 256;                   // memory rows per MMA instruction and per tensor-memory chunk (the N limit)
 constexpr int kRowPad = 64;                   // granularity of the resident rows per CTA
-constexpr int kLoaderThread = 15 * 32;        // the worker thread that issues the next block's copies
 constexpr int kNewRows = 16;                  // up to this many appended rows per update take the logits-first order
-constexpr int kDirectNew = 2;                 // ... and up to this many are scored with plain dot products instead of an MMA pass
+constexpr int kTokenBits = 9;                 // bits of a token's place inside its block
 constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxSmem = 226 * 1024;          // dynamic part; the kernel also holds 1 KB of static shared memory
 
@@ -73,14 +79,14 @@ struct Layout {
     Rcap = ceil_div(ceil_div(s_max, nc), kRowPad) * kRowPad;
     uint32_t off = 0;
     R = off;    off += 2u * Rcap * 128u;                 // [2 halves of D][Rcap][64] bf16, 128-byte swizzle
-    P = off;    off += (uint32_t)C * 256u;               // prepared keys of the block; later the one-hot operand
+    P = off;    off += (uint32_t)C * 256u;               // prepared keys of the block; then the one-hot operand; then the staged sums
     G = off;    off += (uint32_t)C * 256u;               // gated keys of the block
-    xbuf = off; off += 2u * nc * C * 8u;                 // [parity][source CTA][token] {value, row}
-    part = off; off += (2u * C * 8u > 4096u ? 2u * C * 8u : 4096u);                      // [column half][token] {value, row}: the two halves of a chunk (4 KB at least: see stat)
-    tok = off;  off += 4u * C * 4u;                      // nov[C] f32, idx[C], pos[C], list[C]
+    xbuf = off; off += 2u * nc * C * 8u;                 // [parity][source CTA][token] {value, row | novelty}
+    part = off; off += (2u * C * 8u > 4096u ? 2u * C * 8u : 4096u);  // [column half][token]: the two halves of a chunk; small operand of the appended rows
+    tok = off;  off += 2u * C * 4u;                      // nov[C] f32, list[C]
     const uint32_t sp = (uint32_t)((s_max + 63) & ~31);  // padded row count: every region below stays 16-byte aligned
-    rowi = off; off += sp * 4u + sp * 2u + ((2u * Rcap + 15u) & ~15u);  // cur[sp] i32, gci[sp] i16, lci[Rcap] i16 (by local row)
-    tloc = off; off += ((2u * C + 15u) & ~15u) + 2u * sp;  // touched_local[C] u16, stamps[sp] u16 (update that last touched the row)
+    rowi = off; off += sp * 4u + (uint32_t)Rcap * 8u;    // lead[sp] i32; cur[Rcap], lci[Rcap] i32 (by local row)
+    tloc = off; off += (4u * C + 15u) & ~15u;            // touched rows of this CTA by accumulator lane
     stat = part;                                         // LayerNorm partial sums of the scatter epilogue (the routing partials are dead by then)
     bars = off; off += 448u;
     total = (off + 15u) & ~15u;
@@ -94,25 +100,27 @@ struct Bars {
   // index), so that a pass is issued while the workers still read the one before it
   uint64_t tm_full[2][2];
   uint64_t tm_empty[2][2];
-  uint64_t w2i;                         // workers -> issuer: shared-memory operands are ready
+  uint64_t w2i;                         // all worker warps -> issuer: the resident rows are final for the next pass
+  uint64_t t2i;                         // token warps -> issuer: prepared keys dead / one-hot operand ready
+  uint64_t idle;                        // all worker warps (and the second issuer) -> issuer: the update is in global memory,
+                                        // its staging buffer free
   uint64_t sc_done;                     // scatter MMAs complete
   uint64_t xbar[2];                     // arrivals of the peers' partial results (two in flight)
   uint64_t zero_done;                   // the copy engine has cleared the one-hot operand
   uint32_t tmem_base;
   int abort;                            // somebody in the cluster gave up
-  int n_pass;                           // scatter passes of the current update (workers -> issuer)
-  float red_v[32];
+  int n_loc;                            // touched rows of this CTA in the current update
+  float red_v[16];
   int red_t[32];
 };
 
-static_assert(kNewRows <= kWorkerWarps, "one warp per appended row in the short path");
 static_assert(sizeof(Bars) <= 448, "the barrier block outgrew its shared-memory region");
 
 struct Args {
   LayerDev L;
   const kvm_update_plan* plan;
   int n_plan;
-  int nc;
+  int nc, lg;            // CTAs per kv row (a power of two) and its logarithm
   int s_max;             // final number of memory rows
   long long n_tok;       // tokens per kv row in pk_all / gk_all
   bf16* k_sum;           // [rows][capacity][D]
@@ -138,6 +146,10 @@ __device__ __align__(128) unsigned char g_zeros[256 * 256];
 
 // ------------------------------------------------------------------------------------------------ primitives
 __device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
+// barrier of the first `n` worker threads (one per token of the block)
+__device__ __forceinline__ void tsync(int n) { asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory"); }
+// barrier of the four warps that share an accumulator lane quarter
+__device__ __forceinline__ void qsync(int quarter) { asm volatile("bar.sync %0, 128;" ::"r"(3 + quarter) : "memory"); }
 // uniform AND over the worker threads
 __device__ __forceinline__ bool wvote(bool ok) {
   uint32_t r;
@@ -162,9 +174,10 @@ __device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity)
       : "memory");
   return ok != 0;
 }
-// Bounded wait; also gives up when somebody else has.
-template <bool CLUSTER = false>
-__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* abort) {
+// Bounded wait; also gives up when somebody else has.  The first attempt is inlined, the loop is not: the code an update
+// walks through has to stay small (see above).
+template <bool CLUSTER>
+__device__ __noinline__ bool wait_loop(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* abort) {
   for (uint32_t i = 0; i < limit; ++i) {
     if (CLUSTER ? try_wait_cluster(bar, parity) : tc::mbar_try_wait(bar, parity)) return true;
     if ((i & 63) == 63) {  // try_wait suspends the thread for a while by itself; look at the abort flag now and then
@@ -173,6 +186,11 @@ __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, uint32_t li
     }
   }
   return false;
+}
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* abort) {
+  if (CLUSTER ? try_wait_cluster(bar, parity) : tc::mbar_try_wait(bar, parity)) return true;
+  return wait_loop<CLUSTER>(bar, parity, limit, abort);
 }
 __device__ __forceinline__ uint32_t peer_addr(const void* local, int peer) {
   uint32_t a = tc::smem_u32(local), r;
@@ -198,24 +216,48 @@ __device__ __forceinline__ uint32_t piece(int rows, int r, int c) {
   return (uint32_t)((c >> 3) * rows * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
 }
 
-// rows r < S owned by CTA `rank` (r % nc == rank)
-__device__ __forceinline__ int n_local(int S, int nc, int rank) { return S > rank ? (S - rank + nc - 1) / nc : 0; }
+// rows r < S owned by CTA `rank` of 2^lg (r % 2^lg == rank)
+__device__ __forceinline__ int n_local(int S, int lg, int rank) { return S > rank ? (S - rank + (1 << lg) - 1) >> lg : 0; }
 
-// One thread: tiled TMA copies of block u of a kv row (prepared and gated keys, two 64-element halves each) into the
-// block buffers.  The gated keys first: the logits pass, which opens an update, reads them.
-__device__ __forceinline__ void issue_block_loads(unsigned char* smem, const Layout& lay, Bars* bars, const CUtensorMap* map_pk,
-                                                  const CUtensorMap* map_gk, int row, long long n_tok, int C, int u) {
-  const int y = (int)((long long)row * n_tok + (long long)u * C);
-  tc::mbar_arrive_expect_tx(&bars->full_g, (uint32_t)C * 256u);
-  tc::tma_load_2d(smem + lay.G, map_gk, 0, y, &bars->full_g);
-  tc::tma_load_2d(smem + lay.G + C * 128, map_gk, 64, y, &bars->full_g);
-  tc::mbar_arrive_expect_tx(&bars->full_p, (uint32_t)C * 256u);
-  tc::tma_load_2d(smem + lay.P, map_pk, 0, y, &bars->full_p);
-  tc::tma_load_2d(smem + lay.P + C * 128, map_pk, 64, y, &bars->full_p);
+// One thread's share of a routing pass: `groups` groups of 16 accumulator columns from tensor-memory address `at`, column 0
+// = local row l0; rows outside [l_min, n_rows) do not count.  ARG: first maximum {value, local row or -1}; otherwise the
+// maximum.  (Not inlined: three call sites.)
+template <bool ARG>
+__device__ __noinline__ float2 read_columns(uint32_t at, int groups, int l0, int l_min, int n_rows) {
+  float best = -INFINITY;
+  int where = -1;
+#pragma unroll 1
+  for (; groups > 0; --groups, at += 16, l0 += 16) {
+    uint32_t r[16];
+    tc::tmem_ld16(at, r);
+    tc::tmem_ld_wait();
+    if (l0 < l_min || l0 + 16 > n_rows) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (l0 + j < l_min || l0 + j >= n_rows) r[j] = 0xff800000u;  // -inf
+    }
+    if (ARG) {
+      // two runs of eight, each with its first maximum; strictly greater replaces, so the first of equal values stays
+      float v0 = -INFINITY, v1 = -INFINITY;
+      int j0 = -1, j1 = -1;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float x0 = __uint_as_float(r[j]), x1 = __uint_as_float(r[8 + j]);
+        if (x0 > v0) { v0 = x0; j0 = j; }
+        if (x1 > v1) { v1 = x1; j1 = 8 + j; }
+      }
+      if (v1 > v0) { v0 = v1; j0 = j1; }
+      if (v0 > best) { best = v0; where = l0 + j0; }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) best = fmaxf(best, fmaxf(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
+    }
+  }
+  return make_float2(best, __int_as_float(where));
 }
 
 // ------------------------------------------------------------------------------------------------ the issuer
-// One thread: TMA copies of the next block, the MMAs of the routing passes and of the scatter.
+// One thread per token tile: the MMAs of that tile's routing passes.  The first also issues all copies and the scatter.
 struct Issuer {
   const Args& a;
   unsigned char* smem;
@@ -227,13 +269,19 @@ struct Issuer {
   const CUtensorMap* map_gk;
   int which;             // 0: token tile 0, all copies, the scatter; 1: token tile 1 of the routing passes only
   uint32_t g = 0;        // chunks issued so far
-  uint32_t n_w2i = 0, n_sc = 0, n_load = 0, n_zero = 0;
+  uint32_t n_w2i = 0, n_t2i = 0, n_idle = 0, n_sc = 0, n_g = 0, n_p = 0, n_zero = 0;
   volatile int* abort;
   // accumulator half and per-barrier phase of chunk number gg (see Bars::tm_full): with at most 128 resident rows per
   // CTA consecutive chunks alternate between the halves of a token tile's 256 columns
   __device__ __forceinline__ int acc_half(uint32_t gg) const { return lay.Rcap <= 128 ? (int)(gg & 1u) : 0; }
   __device__ __forceinline__ int acc_phase(uint32_t gg) const { return lay.Rcap <= 128 ? (int)(gg >> 1) : (int)gg; }
 
+  __device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t& n) {
+    const bool ok = wait(bar, n & 1, a.wait_limit, abort);
+    ++n;
+    tc::tc_fence_after_sync();
+    return ok;
+  }
   // Update u of this CTA's rows is complete in global memory (routes, version table): tell the CTAs that work on the
   // value side.  Called behind a wait for all worker warps, whose writes this thread's fence makes visible with the flag.
   __device__ __forceinline__ void publish(int u) {
@@ -241,33 +289,29 @@ struct Issuer {
     __threadfence();
     *reinterpret_cast<volatile int*>(a.progress + (size_t)row * a.nc + crank) = u;
   }
-  __device__ __forceinline__ bool wait_workers() {
-    const bool ok = wait(&bars->w2i, n_w2i & 1, a.wait_limit, abort);
-    ++n_w2i;
-    tc::tc_fence_after_sync();
-    return ok;
-  }
+  __device__ __forceinline__ int block_row(int u) const { return (int)((long long)row * a.n_tok + (long long)u * a.L.C); }
   // warm L2 with a later block (the copy into shared memory then does not wait for DRAM)
-  __device__ __forceinline__ void prefetch_block(int u) {
-    const int C = a.L.C;
-    const int y = (int)((long long)row * a.n_tok + (long long)u * C);
+  __device__ __forceinline__ void prefetch(const CUtensorMap* map, int u) {
+    const int y = block_row(u);
 #pragma unroll
-    for (int x = 0; x < 128; x += 64) {
-      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map_pk), "r"(x), "r"(y) : "memory");
-      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map_gk), "r"(x), "r"(y) : "memory");
-    }
+    for (int x = 0; x < 128; x += 64)
+      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
   }
-  __device__ __forceinline__ void load_block(int u) { issue_block_loads(smem, lay, bars, map_pk, map_gk, row, a.n_tok, a.L.C, u); }
+  __device__ __forceinline__ void load(const CUtensorMap* map, uint32_t off, uint64_t* bar, int u) {
+    const int C = a.L.C, y = block_row(u);
+    tc::mbar_arrive_expect_tx(bar, (uint32_t)C * 256u);
+    tc::tma_load_2d(smem + off, map, 0, y, bar);
+    tc::tma_load_2d(smem + off + C * 128, map, 64, y, bar);
+  }
   // Operand descriptors and strides that never change, built once (the per-update code of this thread stays short: it
   // runs alone, so every instruction-cache line it touches for the first time in an update is a wait of its own).
-  uint64_t d_p, d_g, d_r, d_new, d_gmn;  // prepared keys / one-hot (K-major), gated keys (K-major), resident rows, new rows, gated keys (MN-major)
+  uint64_t d_p, d_g, d_r, d_gmn;         // prepared keys / one-hot (K-major), gated keys (K-major), resident rows, gated keys (MN-major)
   uint32_t a_half, r_half;               // second 64-element half of an operand, in descriptor units (16 bytes)
   __device__ __forceinline__ void setup() {
     const int C = a.L.C;
     d_p = tc::make_desc(tc::smem_u32(smem + lay.P), 16, 1024);
     d_g = tc::make_desc(tc::smem_u32(smem + lay.G), 16, 1024);
     d_r = tc::make_desc(tc::smem_u32(smem + lay.R), 16, 1024);
-    d_new = tc::make_desc(tc::smem_u32(smem + lay.part), 16, 1024);
     d_gmn = tc::make_desc(tc::smem_u32(smem + lay.G), (uint32_t)C * 128u, 1024);
     a_half = (uint32_t)(C * 128) >> 4;
     r_half = (uint32_t)(lay.Rcap * 128) >> 4;
@@ -299,28 +343,6 @@ struct Issuer {
     }
     return true;
   }
-  // Logits of every token against the rows that were just appended (at most kNewRows of them), which every CTA keeps
-  // as a small operand of its own: S[tokens x 16] = gk[tokens x D] * newk[16 x D]^T
-  __device__ __forceinline__ bool pass_new_rows() {
-    const int n_mt = a.L.C / 128;
-    constexpr uint32_t idesc = tc::make_idesc(128, kNewRows, 0, 0);
-    constexpr uint32_t n_half = (uint32_t)(kNewRows * 128) >> 4;
-    for (int m = which; m < n_mt; m += kIssuers) {
-      const int hb = acc_half(g), ph = acc_phase(g);
-      if (ph >= 1 && !wait(&bars->tm_empty[hb][m], (ph - 1) & 1, a.wait_limit, abort)) return false;
-      tc::tc_fence_after_sync();
-      const uint64_t da0 = d_g + (uint64_t)((uint32_t)(m * 128 * 128) >> 4);
-      const uint32_t d = tmem + (uint32_t)(m * kChunk + hb * 128);
-#pragma unroll 1
-      for (int ks = 0; ks < HD / 16; ++ks) {
-        const uint32_t lo = (uint32_t)(ks & 3) * 2u;
-        tc::mma_ss(d, da0 + (uint64_t)(((ks >> 2) ? a_half : 0u) + lo), d_new + (uint64_t)(((ks >> 2) ? n_half : 0u) + lo), idesc, ks > 0);
-      }
-      tc::mma_commit_own_cta(&bars->tm_full[hb][m]);
-    }
-    ++g;
-    return true;
-  }
   // delta[128 compacted rows x D] = onehot[rows x C tokens] * gk[C tokens x D]
   // (one-hot: K-major [C/64][128][64] in the buffer of the prepared keys; gated keys: MN-major)
   __device__ __forceinline__ void scatter() {
@@ -331,87 +353,84 @@ struct Issuer {
       tc::mma_ss(tmem, d_p + (uint64_t)((uint32_t)(ks >> 2) * (128u * 128u >> 4) + (uint32_t)(ks & 3) * 2u), d_gmn + (uint64_t)((uint32_t)ks * (2048u >> 4)), idesc, ks > 0);
     tc::mma_commit_own_cta(&bars->sc_done);
   }
+  __device__ __forceinline__ void clear_onehot() {
+    tc::mbar_arrive_expect_tx(&bars->zero_done, (uint32_t)a.L.C * 256u);
+    tc::bulk_g2s(smem + lay.P, g_zeros, (uint32_t)a.L.C * 256u, &bars->zero_done);
+  }
 
   __device__ bool run() {
     const int C = a.L.C, nc = a.nc;
-    // The second issuer follows the same schedule and takes part in the same handshakes, but only issues the routing
-    // MMAs of its token tile.
     const bool primary = which == 0;
+    if (which >= C / 128) return true;
     setup();
-    // block 0 (the initial memory) needs the prepared keys only; the gated keys travel with it to keep the barriers in step
-    if (primary) load_block(0);
+    if (primary) {  // block 0 (the initial memory): prepared keys, or the gated ones where the layer gates the initial memory
+      load(map_pk, lay.P, &bars->full_p, 0);
+      load(map_gk, lay.G, &bars->full_g, 0);
+    }
+    ++n_p; ++n_g;
     kvm_update_plan pl_next = a.plan[0];  // fetched one update ahead: the table lives in global memory
     for (int u = 0; u < a.n_plan; ++u) {
       const kvm_update_plan pl = pl_next;
       if (u + 1 < a.n_plan) pl_next = a.plan[u + 1];
       const int S0 = pl.state_before, na = pl.n_append, S1 = S0 + na, nm = C - na;
-      if (u == 0) {
-        // the workers build the initial memory from the prepared keys and report when the block buffers are free
-        if (!wait_workers()) return false;
-        if (primary) publish(0);
-        n_load = 1;
-        if (primary && a.n_plan > 1) load_block(1);
-        if (primary && a.n_plan > 2 && crank == 0) prefetch_block(2);
-        continue;
-      }
-      const bool has_nov = na > 0 && nm > 0;
-      if (primary && u + 2 < a.n_plan && crank == (u & (nc - 1))) prefetch_block(u + 2);  // one CTA of the cluster asks, all profit
-      const bool withhold = (a.test_flags & 1u) && u == 1;
-      if (nm > 0 && na <= kNewRows) {
-        // few appended rows: the logits against the OLD memory do not depend on them, so they go first and the
-        // novelty MMAs follow behind (the workers read one result while the tensor core produces the next); the
-        // logits against the new rows are a small third pass once the workers have chosen and stored them
-        if (!wait(&bars->full_g, n_load & 1, a.wait_limit, abort)) return false;
-        if (!pass(d_g, n_local(S0, nc, crank), withhold)) return false;
-        if (has_nov) {
-          if (!wait(&bars->full_p, n_load & 1, a.wait_limit, abort)) return false;
-          if (!pass(d_p, n_local(S0, nc, crank), false)) return false;
+      const bool fast = na <= kNewRows, has_nov = na > 0 && nm > 0;
+      if (u > 0) {
+        if (!wait_on(&bars->w2i, n_w2i)) return false;  // the resident rows of the previous update are final
+        if (!primary) tc::mbar_arrive(&bars->idle);     // (no worker runs two updates ahead of this thread)
+        if (primary && u == 1) load(map_gk, lay.G, &bars->full_g, 1);
+        const bool withhold = (a.test_flags & 1u) && u == 1;
+        if (!wait(&bars->full_g, n_g & 1, a.wait_limit, abort)) return false;
+        ++n_g;
+        // Few appended rows: the logits against the OLD memory do not depend on them, so they go first and the novelty
+        // follows behind; many: the novelty first, then the logits against the memory after the appends.
+        for (int k = 0; k < 2; ++k) {
+          const bool logits = (k == 0) == fast;
+          if (!logits) {
+            if (primary) {
+              if (!wait_on(&bars->idle, n_idle)) return false;  // the previous update is in global memory, its staging buffer free
+              publish(u - 1);
+              if (na > 0) load(map_pk, lay.P, &bars->full_p, u);
+              else clear_onehot();
+            }
+            if (na > 0) {
+              if (has_nov && !wait(&bars->full_p, n_p & 1, a.wait_limit, abort)) return false;
+              ++n_p;
+            }
+          } else if (!fast && nm > 0 && !wait_on(&bars->w2i, n_w2i)) {  // the appended rows are in the resident memory
+            return false;
+          }
+          if ((logits ? nm > 0 : has_nov) &&
+              !pass(logits ? d_g : d_p, n_local(logits && !fast ? S1 : S0, a.lg, crank), withhold && logits)) return false;
         }
-        // The workers report when nobody reads the prepared keys any more (novelty read back, appended rows stored, the
-        // new rows in every CTA's small operand): the copy engine clears their buffer, which becomes the one-hot operand
-        // of the scatter, while the workers score the new rows and build the routing table.
-        if (!wait_workers()) return false;
-        if (primary) {
-          // (an update without appends never looked at the prepared keys: their copy must have landed before the buffer is reused)
-          if (!has_nov && !wait(&bars->full_p, n_load & 1, a.wait_limit, abort)) return false;
-          tc::mbar_arrive_expect_tx(&bars->zero_done, (uint32_t)C * 256u);
-          tc::bulk_g2s(smem + lay.P, g_zeros, (uint32_t)C * 256u, &bars->zero_done);
+        if (primary && fast && na > 0) {
+          // nobody reads the prepared keys any more (novelty read back, appended rows stored): their buffer is cleared by
+          // the copy engine and becomes the one-hot operand of the scatter while the workers score the new rows
+          if (!wait_on(&bars->t2i, n_t2i)) return false;
+          clear_onehot();
         }
-        if (has_nov && na > kDirectNew && !pass_new_rows()) return false;  // (one or two new rows are scored by the workers with plain dot products)
-      } else {
-        if (has_nov) {
-          if (!wait(&bars->full_p, n_load & 1, a.wait_limit, abort)) return false;
-          if (!pass(d_p, n_local(S0, nc, crank), false)) return false;
-          if (!wait_workers()) return false;  // the appended rows are in the resident memory
-        }
-        if (nm > 0) {
-          if (!wait(&bars->full_g, n_load & 1, a.wait_limit, abort)) return false;
-          if (!pass(d_g, n_local(S1, nc, crank), withhold)) return false;
+        if (primary && nm > 0) {
+          // scatter passes (their number is known once the routing is final)
+          if (!wait_on(&bars->t2i, n_t2i)) return false;
+          const int n_pass = ceil_div(*reinterpret_cast<volatile int*>(&bars->n_loc), 128);
+          for (int p = 0; p < n_pass; ++p) {
+            if (p > 0 && !wait_on(&bars->t2i, n_t2i)) return false;
+            scatter();
+            if (!wait(&bars->sc_done, n_sc & 1, a.wait_limit, abort)) return false;
+            ++n_sc;
+          }
         }
       }
-      // scatter passes (their number is decided by the workers once the routing is final)
-      if (!wait_workers()) return false;
-      const int n_pass = *reinterpret_cast<volatile int*>(&bars->n_pass);
-      for (int p = 0; p < n_pass; ++p) {
-        if (p > 0 && !wait_workers()) return false;
-        if (primary) scatter();
-        ++n_sc;
+      // every routing pass was read back before the scatter was asked for: the gated keys of this block are dead
+      if (primary && u > 0 && u + 1 < a.n_plan) load(map_gk, lay.G, &bars->full_g, u + 1);
+      if (primary && u + 2 < a.n_plan && crank == (u & (nc - 1))) {  // one CTA of the cluster asks, all profit
+        prefetch(map_gk, u + 2);
+        if (a.plan[u + 2].n_append > 0) prefetch(map_pk, u + 2);
       }
-      if (n_pass == 0) {  // nothing routed to this CTA's rows: the logits MMAs must still be complete before G is overwritten
-        if (primary) tc::mma_commit_own_cta(&bars->sc_done);
-        ++n_sc;
-      }
-      // (all routing MMAs were read back by the workers before they asked for the scatter, so the commit of the
-      // primary issuer covers what the block buffers are needed for)
-      if (primary && !wait(&bars->sc_done, (n_sc - 1) & 1, a.wait_limit, abort)) return false;
-      if (nm > 0 && na <= kNewRows) {  // the clearing copy has landed, too (nobody may have waited for it: no row of this CTA touched)
-        if (primary && !wait(&bars->zero_done, n_zero & 1, a.wait_limit, abort)) return false;
-        ++n_zero;
-      }
-      ++n_load;  // the loads of this update have been consumed; a worker thread has issued the next block's (see there)
-      // the next routing pass reads the resident memory the workers are refreshing now
-      if (!wait_workers()) return false;
-      if (primary) publish(u);
+    }
+    if (!primary) tc::mbar_arrive(&bars->idle);
+    if (primary && a.n_plan > 1) {
+      if (!wait_on(&bars->idle, n_idle)) return false;
+      publish(a.n_plan - 1);
     }
     return true;
   }
@@ -429,175 +448,76 @@ struct Workers {
   const float* ln_b;
   volatile int* abort;
   int tid, warp, lane;
-  const CUtensorMap* map_pk;
-  const CUtensorMap* map_gk;
-  uint32_t g = 0, n_sc = 0, n_x = 0, n_load = 0, n_zero = 0;
-  int pool_next = 0;
-  unsigned mine_mask = 0;  // lanes whose row (a multiple of 32 + lane) belongs to this CTA
-  // accumulator half and per-barrier phase of chunk number gg (see Bars::tm_full): with at most 128 resident rows per
-  // CTA consecutive chunks alternate between the halves of a token tile's 256 columns
+  uint32_t g = 0, n_sc = 0, n_x = 0, n_p = 0, n_zero = 0;
+  // accumulator half and per-barrier phase of chunk number gg (see Issuer)
   __device__ __forceinline__ int acc_half(uint32_t gg) const { return lay.Rcap <= 128 ? (int)(gg & 1u) : 0; }
   __device__ __forceinline__ int acc_phase(uint32_t gg) const { return lay.Rcap <= 128 ? (int)(gg >> 1) : (int)gg; }
 
   __device__ __forceinline__ float* nov() const { return reinterpret_cast<float*>(smem + lay.tok); }
-  __device__ __forceinline__ int* idx() const { return reinterpret_cast<int*>(smem + lay.tok) + a.L.C; }
-  __device__ __forceinline__ int* pos() const { return reinterpret_cast<int*>(smem + lay.tok) + 2 * a.L.C; }
-  __device__ __forceinline__ int* list() const { return reinterpret_cast<int*>(smem + lay.tok) + 3 * a.L.C; }
-  __device__ __forceinline__ int* cur() const { return reinterpret_cast<int*>(smem + lay.rowi); }
-  __device__ __forceinline__ int padded_rows() const { return (a.s_max + 63) & ~31; }
-  __device__ __forceinline__ short* gci() const { return reinterpret_cast<short*>(smem + lay.rowi + (uint32_t)padded_rows() * 4u); }
-  __device__ __forceinline__ short* lci() const { return gci() + padded_rows(); }  // indexed by the local row r / nc
-  __device__ __forceinline__ unsigned short* tloc() const { return reinterpret_cast<unsigned short*>(smem + lay.tloc); }
-  __device__ __forceinline__ unsigned short* tf() const { return reinterpret_cast<unsigned short*>(smem + lay.tloc + ((2u * a.L.C + 15u) & ~15u)); }
+  __device__ __forceinline__ int* list() const { return reinterpret_cast<int*>(smem + lay.tok) + a.L.C; }
+  // per memory row: (update that last touched it) << kTokenBits | (its first token in that update, counted from the end);
+  // the maximum over an update's tokens wins, later updates win over earlier ones, nothing is ever cleared
+  __device__ __forceinline__ int* lead() const { return reinterpret_cast<int*>(smem + lay.rowi); }
+  __device__ __forceinline__ int* cur() const { return lead() + ((a.s_max + 63) & ~31); }  // [local row] pool row of the current view
+  __device__ __forceinline__ int* lci() const { return cur() + lay.Rcap; }                 // [local row] accumulator lane in this update
+  __device__ __forceinline__ int* tloc() const { return reinterpret_cast<int*>(smem + lay.tloc); }
   __device__ __forceinline__ float2* part(int half) const { return reinterpret_cast<float2*>(smem + lay.part) + half * a.L.C; }
   __device__ __forceinline__ float2* xb(int parity, int src) const { return reinterpret_cast<float2*>(smem + lay.xbuf) + (size_t)(parity * a.nc + src) * a.L.C; }
   __device__ __forceinline__ float* stat(int which) const { return reinterpret_cast<float*>(smem + lay.stat) + which * 4 * 128; }
 
-  __device__ __forceinline__ void signal_issuer() {
-    tc::fence_proxy_async();   // shared-memory writes of this thread -> visible to the tensor core / TMA
+  // this warp's shared-memory writes are visible to the tensor core and the copy engine; it arrives on `bar`
+  __device__ __forceinline__ void signal(uint64_t* bar) {
+    tc::fence_proxy_async();
     tc::tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) tc::mbar_arrive(&bars->w2i);
+    if (lane == 0) tc::mbar_arrive(bar);
   }
 
-  // Read back the chunks of a routing pass.  ARG = false: running maximum (novelty); true: running first-argmax of
-  // rows >= `protected_rows`.  Warp w reads token tile (w / 4) % 2, lanes 32 (w % 4).., and one half of the chunk's
-  // 32-column groups; leaves per token the CTA's partial result in part(half)[token].
-  template <bool ARG>
-  __device__ __forceinline__ bool read_pass(int n_rows, int protected_rows) {
-    float v;
-    int i;
-    const bool ok = read_regs<ARG>(n_rows, protected_rows, v, i);
-    const int half = warp >> 3, mt = (warp >> 2) & 1, quarter = warp & 3;
-    if (mt * 128 < a.L.C) part(half)[mt * 128 + quarter * 32 + lane] = make_float2(v, __int_as_float(i));
-    return wvote(ok);
-  }
-  // The same, the thread's result (value; global row or -1) left in registers, no vote.
+  // Read back the chunks of a routing pass: maximum (ARG = false: novelty) or first maximum over rows >= `protected_rows`
+  // (true), the thread's result (value; global row or -1) left in registers.  Warp w reads token tile (w / 4) % 2, lanes
+  // 32 (w % 4).., and one half of the chunk's 16-column groups.
   template <bool ARG>
   __device__ __forceinline__ bool read_regs(int n_rows, int protected_rows, float& v_out, int& i_out) {
-    const int C = a.L.C, nc = a.nc;
-    const int half = warp >> 3, mt = (warp >> 2) & 1, quarter = warp & 3;
-    const bool active = mt * 128 < C;
+    const int half = warp >> 3, mt = (warp >> 2) & 1;
     const int n_chunks = ceil_div(n_rows, kChunk);
     // first local row that counts: global row l * nc + crank >= protected_rows
-    const int l_min = ARG ? (protected_rows > crank ? (protected_rows - crank + nc - 1) / nc : 0) : 0;
-    float bv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    int bi[4] = {-1, -1, -1, -1};
+    const int l_min = ARG ? n_local(protected_rows, a.lg, crank) : 0;
+    float best = -INFINITY;
+    int where = -1;
     bool ok = true;
+#pragma unroll 1
     for (int c = 0; c < n_chunks; ++c, ++g) {
-      if (!active) continue;
+      if (mt * 128 >= a.L.C) continue;
       const int hb = acc_half(g), ph = acc_phase(g);
       ok = ok && wait(&bars->tm_full[hb][mt], ph & 1, a.wait_limit, abort);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;  // the caller aborts
       tc::tc_fence_after_sync();
-      const int n = min(kChunk, n_rows - c * kChunk);
-      const int n_groups = ceil_div(n, 32), g_half = (n_groups + 1) / 2;
-      const int g_begin = half ? g_half : 0, g_end = half ? n_groups : g_half;
-      for (int gi = g_begin; gi < g_end; ++gi) {
-        uint32_t r[32];
-        tc::tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mt * kChunk + hb * 128 + gi * 32), r);
-        tc::tmem_ld_wait();
-        const int l0 = c * kChunk + gi * 32;  // local row of column 0
-        const bool full = l0 + 32 <= n_rows && l0 >= l_min;
-        if (!ARG) {
-          if (full) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) bv[j & 3] = fmaxf(bv[j & 3], __uint_as_float(r[j]));
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (l0 + j < n_rows) bv[j & 3] = fmaxf(bv[j & 3], __uint_as_float(r[j]));
-          }
-        } else {
-          if (full) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float x = __uint_as_float(r[j]);  // strictly greater replaces: the first of equal values stays
-              if (x > bv[j & 3]) { bv[j & 3] = x; bi[j & 3] = l0 + j; }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float x = __uint_as_float(r[j]);
-              const int l = l0 + j;
-              if (l < n_rows && l >= l_min && x > bv[j & 3]) { bv[j & 3] = x; bi[j & 3] = l; }
-            }
-          }
-        }
-      }
+      const int n_groups = ceil_div(min(kChunk, n_rows - c * kChunk), 16), g_half = (n_groups + 1) / 2;
+      const int g_begin = half ? g_half : 0, n_mine = half ? n_groups - g_half : g_half;
+      const float2 f = read_columns<ARG>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * kChunk + hb * 128 + g_begin * 16), n_mine,
+                                         c * kChunk + g_begin * 16, l_min, n_rows);
+      if (f.x > best) { best = f.x; where = __float_as_int(f.y); }
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars->tm_empty[hb][mt]);
     }
-    float v = bv[0];
-    int i = bi[0];
-    if (!ARG) {
-      v = fmaxf(fmaxf(bv[0], bv[1]), fmaxf(bv[2], bv[3]));
-    } else {
-#pragma unroll
-      for (int j = 1; j < 4; ++j)  // first maximum in row order: larger value, or equal value at a lower row
-        if (bi[j] >= 0 && (i < 0 || bv[j] > v || (bv[j] == v && bi[j] < i))) { v = bv[j]; i = bi[j]; }
-      if (i >= 0) i = i * nc + crank;  // local -> global row
-    }
-    v_out = v;
-    i_out = i;
+    v_out = best;
+    i_out = where >= 0 ? (where << a.lg) + crank : -1;
     return ok;
   }
-
-  // Merge the two column halves, exchange the CTA's partial results with the peers, combine.
-  // ARG = false: nov()[t] = bf16(max); true: idx()[t] = first row with the largest logit.
-  template <bool ARG>
-  __device__ __forceinline__ bool exchange() {
-    const int C = a.L.C, nc = a.nc;
-    const int parity = n_x & 1;
-    float v = -INFINITY;
-    int i = -1;
-    if (tid < C) {
-      const float2 p0 = part(0)[tid], p1 = part(1)[tid];
-      v = p0.x;
-      i = __float_as_int(p0.y);
-      const int i1 = __float_as_int(p1.y);
-      if (!ARG) {
-        v = fmaxf(p0.x, p1.x);
-      } else if (i1 >= 0 && (i < 0 || p1.x > v || (p1.x == v && i1 < i))) {
-        v = p1.x;
-        i = i1;
-      }
+  // This thread's share of the routing results of its token -> shared memory.  {best logit over the old rows, row (16
+  // bits, 0xffff = none) | novelty maximum as bf16 << 16}; the bf16 rounding of the novelty commutes with the maximum.
+  __device__ __forceinline__ void store_part(float v, int i, float nv) {
+    const int mt = (warp >> 2) & 1;
+    if (mt * 128 < a.L.C) {
+      const unsigned packed = ((unsigned)i & 0xffffu) | ((unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(nv)) << 16);
+      part(warp >> 3)[mt * 128 + (warp & 3) * 32 + lane] = make_float2(v, __uint_as_float(packed));
     }
-    bool ok = true;
-    if (nc > 1) {
-      // every token's partial result goes to the same token's slot in every peer; this CTA expects the peers' bytes
-      if (tid == 0) tc::mbar_arrive_expect_tx(&bars->xbar[parity], (uint32_t)((nc - 1) * C * 8));
-      if (tid < C) {
-        const float2* slot = &xb(parity, crank)[tid];
-        for (int p = 0; p < nc; ++p)
-          if (p != crank) st_async_v2(peer_addr(slot, p), v, i, peer_addr(&bars->xbar[parity], p));
-      }
-      ok = tid < C ? wait<true>(&bars->xbar[parity], (n_x >> 1) & 1, a.wait_limit, abort) : true;
-      if (ok && tid < C) {
-        for (int p = 0; p < nc; ++p) {
-          if (p == crank) continue;
-          const float2 q = xb(parity, p)[tid];
-          const int qi = __float_as_int(q.y);
-          if (!ARG) v = fmaxf(v, q.x);
-          else if (qi >= 0 && (i < 0 || q.x > v || (q.x == v && qi < i))) { v = q.x; i = qi; }
-        }
-      }
-    }
-    ++n_x;
-    if (tid < C) {
-      if (!ARG) nov()[tid] = bf16_round(v);
-      else idx()[tid] = i;
-    }
-    return wvote(ok);
   }
-
-  // Both routing results of the logits-first order in one exchange.  part(half)[token] holds {best logit over the
-  // old rows, row (16 bits, 0xffff = none) | novelty maximum as bf16 << 16}; the bf16 rounding of the novelty commutes
-  // with the maximum.  Leaves the novelty in nov()[token] and the best old row in the token thread's registers.
-  __device__ __forceinline__ bool exchange_both(float& best_v, int& best_i) {
-    const int C = a.L.C, nc = a.nc;
+  // Token threads: merge the two column halves, exchange the CTA's partial result with the peers, combine.
+  __device__ __forceinline__ bool exchange(float& best_v, int& best_i, float& novelty) {
+    const int C = a.L.C, nc = 1 << a.lg;
     const int parity = n_x & 1;
     float v = -INFINITY, nv = -INFINITY;
     int i = -1;
@@ -607,102 +527,85 @@ struct Workers {
       nv = fmaxf(nv, __uint_as_float(w & 0xffff0000u));
       if (pi >= 0 && (i < 0 || p.x > v || (p.x == v && pi < i))) { v = p.x; i = pi; }
     };
-    if (tid < C) {
-      take(part(0)[tid]);
-      take(part(1)[tid]);
-    }
+    take(part(0)[tid]);
+    take(part(1)[tid]);
     bool ok = true;
     if (nc > 1) {
+      // every token's partial result goes to the same token's slot in every peer; this CTA expects the peers' bytes
       if (tid == 0) tc::mbar_arrive_expect_tx(&bars->xbar[parity], (uint32_t)((nc - 1) * C * 8));
-      if (tid < C) {
-        const float2* slot = &xb(parity, crank)[tid];
-        const int packed = (int)(((unsigned)i & 0xffffu) | (__float_as_uint(nv) & 0xffff0000u));
-        for (int p = 0; p < nc; ++p)
-          if (p != crank) st_async_v2(peer_addr(slot, p), v, packed, peer_addr(&bars->xbar[parity], p));
-      }
-      ok = tid < C ? wait<true>(&bars->xbar[parity], (n_x >> 1) & 1, a.wait_limit, abort) : true;
-      if (ok && tid < C)
+      const float2* slot = &xb(parity, crank)[tid];
+      const int packed = (int)(((unsigned)i & 0xffffu) | (__float_as_uint(nv) & 0xffff0000u));
+#pragma unroll 1
+      for (int p = 0; p < nc; ++p)
+        if (p != crank) st_async_v2(peer_addr(slot, p), v, packed, peer_addr(&bars->xbar[parity], p));
+      ok = wait<true>(&bars->xbar[parity], (n_x >> 1) & 1, a.wait_limit, abort);
+      if (ok)
+#pragma unroll 1
         for (int p = 0; p < nc; ++p)
           if (p != crank) take(xb(parity, p)[tid]);
     }
-    ++n_x;
-    if (tid < C) nov()[tid] = nv;
     best_v = v;
     best_i = i;
-    return wvote(ok);
+    novelty = nv;
+    return ok;
   }
 
-  // LayerNorm view of one memory row (8 lanes per row): source `x`, written to the resident memory (if local) and
-  // to a pool row / the carried sums.
-  // `new_row` >= 0: also row `new_row` of the small operand every CTA keeps of the rows appended in this update.
-  __device__ __forceinline__ void store_key_row(RowVec<HD, 8>& x, int r, int slot, int gl, bool mine, int new_row = -1) {
-    const size_t grow = (size_t)row * a.capacity + r;
-    if (mine) store_row<HD, 8>(x, a.k_sum + grow * HD, gl);
-    layer_norm_row<HD, 8>(x, ln_w, ln_b, a.L.ln_eps, gl);
-    uint4 u0, u1;
-    u0.x = pack_bf16(x.x[0], x.x[1]); u0.y = pack_bf16(x.x[2], x.x[3]); u0.z = pack_bf16(x.x[4], x.x[5]); u0.w = pack_bf16(x.x[6], x.x[7]);
-    u1.x = pack_bf16(x.x[8], x.x[9]); u1.y = pack_bf16(x.x[10], x.x[11]); u1.z = pack_bf16(x.x[12], x.x[13]); u1.w = pack_bf16(x.x[14], x.x[15]);
-    if (new_row >= 0) {
-      *reinterpret_cast<uint4*>(smem + lay.part + piece(kNewRows, new_row, 2 * gl)) = u0;
-      *reinterpret_cast<uint4*>(smem + lay.part + piece(kNewRows, new_row, 2 * gl + 1)) = u1;
-    }
-    if (mine) {
-      const int l = r / a.nc;
-      *reinterpret_cast<uint4*>(smem + lay.R + piece(lay.Rcap, l, 2 * gl)) = u0;
-      *reinterpret_cast<uint4*>(smem + lay.R + piece(lay.Rcap, l, 2 * gl + 1)) = u1;
-      if (a.pool_k) {
-        bf16* dst = a.pool_k + ((size_t)row * a.pool_rows + slot) * HD + gl * 16;
-        *reinterpret_cast<uint4*>(dst) = u0;
-        *reinterpret_cast<uint4*>(dst + 8) = u1;
-      }
-    }
-  }
   // the 16 elements of lane gl of row t of a block operand (prepared or gated keys)
-  __device__ __forceinline__ void load_block_row(RowVec<HD, 8>& x, uint32_t off, int t, int gl) { load_block_row_n(x, off, a.L.C, t, gl); }
-  // ... of an operand of `rows` rows
-  __device__ __forceinline__ void load_block_row_n(RowVec<HD, 8>& x, uint32_t off, int rows, int t, int gl) {
-    const int C = rows;
+  __device__ __forceinline__ void load_block_row(RowVec<HD, 8>& x, uint32_t off, int t, int gl) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const uint4 u = *reinterpret_cast<const uint4*>(smem + off + piece(C, t, 2 * gl + h));
+      const uint4 u = *reinterpret_cast<const uint4*>(smem + off + piece(a.L.C, t, 2 * gl + h));
       const float2 p0 = unpack_bf16(u.x), p1 = unpack_bf16(u.y), p2 = unpack_bf16(u.z), p3 = unpack_bf16(u.w);
       x.x[h * 8 + 0] = p0.x; x.x[h * 8 + 1] = p0.y; x.x[h * 8 + 2] = p1.x; x.x[h * 8 + 3] = p1.y;
       x.x[h * 8 + 4] = p2.x; x.x[h * 8 + 5] = p2.y; x.x[h * 8 + 6] = p3.x; x.x[h * 8 + 7] = p3.y;
     }
   }
-
-  // rows [S0, S0 + na) from the tokens list()[0..na): `src_off` = operand holding what is stored (prepared or gated keys)
-  // `all_ctas`: every CTA also keeps the rows' view in its small operand of new rows (na <= kNewRows)
-  __device__ __forceinline__ void append_rows(int S0, int na, uint32_t src_off, int u, bool all_ctas = false) {
+  // Rows [S0, S0 + na) from the tokens list()[0..na), all warps, eight lanes per row: carried sums, resident view, pool
+  // row (a row lives in the pool row of its token).  `src_off`: operand holding what is stored (prepared or gated keys).
+  __device__ __forceinline__ void append_rows(int S0, int na, uint32_t src_off, int u) {
     const int gl = tid & 7, grp = tid >> 3;
+#pragma unroll 1
     for (int base = 0; base < na; base += kWorkers / 8) {  // whole warps stay together: the LayerNorm uses group shuffles
       const int p = base + grp;
-      const bool act = p < na;
-      if (!__any_sync(0xffffffffu, act && (all_ctas || (S0 + p) % a.nc == crank))) continue;  // nothing for this warp to store
-      const int r = S0 + (act ? p : 0);
-      const int t = list()[act ? p : 0];
+      const bool mine = p < na && ((S0 + p) & (a.nc - 1)) == crank;
+      if (!__any_sync(0xffffffffu, mine)) continue;  // nothing for this warp to store
+      const int r = S0 + (p < na ? p : 0), t = list()[p < na ? p : 0];
       RowVec<HD, 8> x;
       load_block_row(x, src_off, t, gl);
-      const bool mine = act && (r % a.nc == crank);
-      store_key_row(x, r, pool_next + p, gl, mine, (all_ctas && act) ? p : -1);
-      if (mine && gl == 0 && a.born) a.born[(size_t)row * a.s_max + r] = u * a.L.C + t;
+      if (mine) store_row<HD, 8>(x, a.k_sum + ((size_t)row * a.capacity + r) * HD, gl);
+      layer_norm_row<HD, 8>(x, ln_w, ln_b, a.L.ln_eps, gl);
+      if (mine) {
+        uint4 u0, u1;
+        u0.x = pack_bf16(x.x[0], x.x[1]); u0.y = pack_bf16(x.x[2], x.x[3]); u0.z = pack_bf16(x.x[4], x.x[5]); u0.w = pack_bf16(x.x[6], x.x[7]);
+        u1.x = pack_bf16(x.x[8], x.x[9]); u1.y = pack_bf16(x.x[10], x.x[11]); u1.z = pack_bf16(x.x[12], x.x[13]); u1.w = pack_bf16(x.x[14], x.x[15]);
+        const int l = r >> a.lg;
+        *reinterpret_cast<uint4*>(smem + lay.R + piece(lay.Rcap, l, 2 * gl)) = u0;
+        *reinterpret_cast<uint4*>(smem + lay.R + piece(lay.Rcap, l, 2 * gl + 1)) = u1;
+        if (a.pool_k) {
+          bf16* dst = a.pool_k + ((size_t)row * a.pool_rows + (size_t)u * a.L.C + t) * HD + gl * 16;
+          *reinterpret_cast<uint4*>(dst) = u0;
+          *reinterpret_cast<uint4*>(dst + 8) = u1;
+        }
+        if (gl == 0) {
+          cur()[l] = u * a.L.C + t;
+          if (a.born) a.born[(size_t)row * a.s_max + r] = u * a.L.C + t;
+        }
+      }
     }
-    for (int i = tid; i < na; i += kWorkers) cur()[S0 + i] = pool_next + i;
-    pool_next += na;
   }
-
-  // The same for at most kWorkerWarps rows, one warp per row and four elements per lane, every CTA keeping the rows' view
-  // in its small operand of new rows: the few warps that store rows run alone, and what they wait for is mostly their
-  // own instructions, so the code is kept short.
+  // The same for at most kNewRows rows by the token warps, one warp per row and four elements per lane, every CTA keeping
+  // the rows' view in its small operand of new rows: the few warps that store rows run alone, and what they wait for is
+  // mostly their own instructions, so the code is kept short.
   __device__ __forceinline__ void append_rows_warp(int S0, int na, uint32_t src_off, int u) {
-    if (warp < na) {
-      const int p = warp, r = S0 + p, t = list()[p], pc = lane >> 1;
+#pragma unroll 1
+    for (int p = warp; p < na; p += a.L.C / 32) {
+      const int r = S0 + p, t = list()[p], pc = lane >> 1;
       const uint32_t sub = (uint32_t)(lane & 1) * 8u;  // which half of a 16-byte piece
       const uint2 raw = *reinterpret_cast<const uint2*>(smem + src_off + piece(a.L.C, t, pc) + sub);
       RowVec<HD, 32> x;
       const float2 e0 = unpack_bf16(raw.x), e1 = unpack_bf16(raw.y);
       x.x[0] = e0.x; x.x[1] = e0.y; x.x[2] = e1.x; x.x[3] = e1.y;
-      const bool mine = r % a.nc == crank;
+      const bool mine = (r & (a.nc - 1)) == crank;
       if (mine) *reinterpret_cast<uint2*>(a.k_sum + ((size_t)row * a.capacity + r) * HD + lane * 4) = raw;  // the carried sum is the token's row
       layer_norm_row<HD, 32>(x, ln_w, ln_b, a.L.ln_eps, lane);
       uint2 o;
@@ -710,380 +613,388 @@ struct Workers {
       o.y = pack_bf16(x.x[2], x.x[3]);
       *reinterpret_cast<uint2*>(smem + lay.part + piece(kNewRows, p, pc) + sub) = o;
       if (mine) {
-        *reinterpret_cast<uint2*>(smem + lay.R + piece(lay.Rcap, r / a.nc, pc) + sub) = o;
-        if (a.pool_k) *reinterpret_cast<uint2*>(a.pool_k + ((size_t)row * a.pool_rows + pool_next + p) * HD + lane * 4) = o;
-        if (lane == 0 && a.born) a.born[(size_t)row * a.s_max + r] = u * a.L.C + t;
+        *reinterpret_cast<uint2*>(smem + lay.R + piece(lay.Rcap, r >> a.lg, pc) + sub) = o;
+        if (a.pool_k) *reinterpret_cast<uint2*>(a.pool_k + ((size_t)row * a.pool_rows + (size_t)u * a.L.C + t) * HD + lane * 4) = o;
+        if (lane == 0) {
+          cur()[r >> a.lg] = u * a.L.C + t;
+          if (a.born) a.born[(size_t)row * a.s_max + r] = u * a.L.C + t;
+        }
       }
     }
-    if (tid < na) cur()[S0 + tid] = pool_next + tid;
-    pool_next += na;
+  }
+  // A token warp: logits of its 32 tokens against the rows that were just appended (the small operand), warp-level MMAs;
+  // a new row has a higher index than every old one, it wins only with a strictly larger logit.
+  __device__ __forceinline__ void score_new_rows(int S0, int na, int protected_rows, float& best_v, int& best_i) {
+    const int gq = lane >> 2, tq = lane & 3;
+    for (int n0 = 0; n0 < na; n0 += 8) {
+      float acc[2][4];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+#pragma unroll 2
+      for (int ks = 0; ks < HD / 16; ++ks) {
+        const unsigned char* nb = smem + lay.part;
+        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(nb + piece(kNewRows, n0 + gq, ks * 2) + tq * 4);
+        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(nb + piece(kNewRows, n0 + gq, ks * 2 + 1) + tq * 4);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          uint32_t ka[4];
+          ldmatrix_x4(ka, smem + lay.G + piece(a.L.C, warp * 32 + m * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, ks * 2 + (lane >> 4)));
+          mma_bf16_16816(acc[m], ka, b0, b1);
+        }
+      }
+      const int src = (lane & 7) * 4, e_mine = lane >> 3;  // a token's own lane = tile * 16 + upper half * 8 + quad
+      if (na == 1) {  // column 0 only
+        float x = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float sv = __shfl_sync(0xffffffffu, acc[k >> 1][(k & 1) * 2], src);
+          if (k == e_mine) x = sv;
+        }
+        if (S0 >= protected_rows && (x > best_v || best_i < 0)) { best_v = x; best_i = S0; }
+        return;
+      }
+      // first maximum over the new rows: this thread's columns 2 tq, 2 tq + 1, then the quad; tokens gq and gq + 8 of a tile
+      float v[4];
+      int j[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {  // e = tile * 2 + upper half
+        const int c = n0 + tq * 2;
+        const float x0 = acc[e >> 1][(e & 1) * 2], x1 = acc[e >> 1][(e & 1) * 2 + 1];
+        const bool ok0 = c < na && S0 + c >= protected_rows, ok1 = c + 1 < na && S0 + c + 1 >= protected_rows;
+        v[e] = ok0 ? x0 : -INFINITY;
+        j[e] = ok0 ? c : -1;
+        if (ok1 && (j[e] < 0 || x1 > v[e])) { v[e] = x1; j[e] = c + 1; }
+#pragma unroll
+        for (int off = 1; off <= 2; off <<= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, v[e], off);
+          const int oj = __shfl_xor_sync(0xffffffffu, j[e], off);
+          if (oj >= 0 && (j[e] < 0 || ov > v[e] || (ov == v[e] && oj < j[e]))) { v[e] = ov; j[e] = oj; }
+        }
+      }
+      float tv = -INFINITY;
+      int tj = -1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float sv = __shfl_sync(0xffffffffu, v[k], src);
+        const int sj = __shfl_sync(0xffffffffu, j[k], src);
+        if (k == e_mine) { tv = sv; tj = sj; }
+      }
+      if (tj >= 0 && (tv > best_v || best_i < 0)) { best_v = tv; best_i = S0 + tj; }
+    }
+  }
+  // Token threads: the na tokens of lowest novelty, lowest index among equals; returns this token's place in the append
+  // list (token order) or -1, fills list().
+  __device__ __forceinline__ int select(float novelty, int na) {
+    const int C = a.L.C, n_warps = C / 32;
+    if (na == 1) {
+      float bv = novelty;
+      int bt = tid;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+        const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
+        if (ov < bv || (ov == bv && ot < bt)) { bv = ov; bt = ot; }
+      }
+      if (lane == 0) { bars->red_v[warp] = bv; bars->red_t[warp] = bt; }
+      tsync(C);
+      bv = bars->red_v[lane & (n_warps - 1)];
+      bt = bars->red_t[lane & (n_warps - 1)];
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+        const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
+        if (ov < bv || (ov == bv && ot < bt)) { bv = ov; bt = ot; }
+      }
+      if (tid == 0) list()[0] = bt;
+      return tid == bt ? 0 : -1;
+    }
+    nov()[tid] = novelty;
+    tsync(C);
+    int rank = 0;
+#pragma unroll 4
+    for (int u0 = 0; u0 < C; u0 += 4) {  // stable rank of the novelty scores
+      const float4 q = *reinterpret_cast<const float4*>(nov() + u0);
+      rank += (q.x < novelty || (q.x == novelty && u0 + 0 < tid)) ? 1 : 0;
+      rank += (q.y < novelty || (q.y == novelty && u0 + 1 < tid)) ? 1 : 0;
+      rank += (q.z < novelty || (q.z == novelty && u0 + 2 < tid)) ? 1 : 0;
+      rank += (q.w < novelty || (q.w == novelty && u0 + 3 < tid)) ? 1 : 0;
+    }
+    const bool f = rank < na;
+    const unsigned bal = __ballot_sync(0xffffffffu, f);
+    if (lane == 0) bars->red_t[warp] = __popc(bal);
+    tsync(C);
+    int p = __popc(bal & ((1u << lane) - 1u));
+#pragma unroll 1
+    for (int w = 0; w < warp; ++w) p += bars->red_t[w];
+    if (f) list()[p] = tid;
+    return f ? p : -1;
+  }
+
+  // The 128 touched rows of scatter pass p: carried sums, LayerNorm refresh into the resident memory and the row pool.
+  // The four warps of an accumulator lane quarter work on its 32 rows by themselves (qsync).  Rows are scattered over the
+  // carried sums and the pool, so they travel between global memory and a staging buffer (the one-hot operand's, dead
+  // by now) as whole rows, while the arithmetic runs one row per thread and 32 columns per warp, as tensor memory has
+  // them: row per lane straight to global memory touches 32 lines per instruction, which alone took 6 000 cycles.
+  // `last`: the resident rows are final behind this pass, the next update's routing may start.
+  __device__ __forceinline__ bool epilogue(int p, int n_loc, bool last) {
+    const int quarter = warp & 3, colq = warp >> 2;
+    // whole rows: sixteen threads per row, this one the piece pc of the quarter's rows r8, r8 + 8, ..
+    constexpr int kPieces = HD / 8, kShare = 32 * kPieces / 128;
+    const int qt = colq * 32 + lane, pc = qt % kPieces, r8 = quarter * 32 + qt / kPieces;
+    unsigned char* stage = smem + lay.P;
+    unsigned char* const mine = stage + piece(128, r8, pc);   // (+ 1024 bytes per further row: the swizzle repeats every 8 rows)
+    const int* const rows = tloc() + p * 128 + r8;
+    const int n_share = ceil_div(n_loc - p * 128 - r8, 8);    // how many of them are live
+    bf16* const sums = a.k_sum + (size_t)row * a.capacity * HD + pc * 8;
+    uint4 old[kShare];
+#pragma unroll
+    for (int k = 0; k < kShare; ++k)
+      if (k < n_share) old[k] = *reinterpret_cast<const uint4*>(sums + (size_t)rows[k * 8] * HD);
+    const bool ok = wait(&bars->sc_done, n_sc & 1, a.wait_limit, abort);
+    ++n_sc;
+    tc::tc_fence_after_sync();
+#pragma unroll
+    for (int k = 0; k < kShare; ++k)
+      if (k < n_share) *reinterpret_cast<uint4*>(mine + k * 1024) = old[k];
+    const int ci = quarter * 32 + lane;
+    const bool act = p * 128 + ci < n_loc;
+    const int l = act ? tloc()[p * 128 + ci] >> a.lg : 0;
+    // Three short sweeps over this thread's 32 columns, the row's new sum (bf16, exact) kept in the staging buffer between
+    // them: row = bf16(row + bf16(delta)) on packed pairs (the sum of two bf16 numbers rounded once), variance, output
+    unsigned char* const at0 = stage + (colq >> 1) * (128 * 128) + ci * 128;
+    auto at = [&](int j) { return reinterpret_cast<uint4*>(at0 + ((((colq & 1) * 4 + j) ^ (ci & 7)) << 4)); };
+    qsync(quarter);
+    float s1 = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < 4; j += 2) {
+      uint32_t d[16];
+      tc::tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(colq * 32 + j * 8), d);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint4 o4 = *at(j + h);
+        uint32_t* w = reinterpret_cast<uint32_t*>(&o4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = h * 8 + e * 2;
+          const __nv_bfloat162 dl = __floats2bfloat162_rn(__uint_as_float(d[c]), __uint_as_float(d[c + 1]));
+          const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]), dl);
+          w[e] = *reinterpret_cast<const uint32_t*>(&sum);
+          const float2 f2 = __bfloat1622float2(sum);
+          s1 += f2.x + f2.y;
+        }
+        *at(j + h) = o4;
+      }
+    }
+    tc::tc_fence_before_sync();
+    stat(0)[colq * 128 + ci] = s1;
+    qsync(quarter);
+    const float mean = (stat(0)[ci] + stat(0)[128 + ci] + stat(0)[256 + ci] + stat(0)[384 + ci]) * (1.0f / HD);
+    float s2 = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      const uint4 o4 = *at(j);
+      const uint32_t w[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f2 = unpack_bf16(w[e]);
+        const float x0 = f2.x - mean, x1 = f2.y - mean;
+        s2 += x0 * x0;
+        s2 += x1 * x1;
+      }
+    }
+    stat(1)[colq * 128 + ci] = s2;
+    qsync(quarter);
+    const float var = (stat(1)[ci] + stat(1)[128 + ci] + stat(1)[256 + ci] + stat(1)[384 + ci]) * (1.0f / HD);
+    const float rstd = 1.0f / sqrtf(var + a.L.ln_eps);
+    if (act) {
+      unsigned char* const dst = smem + lay.R + (colq >> 1) * lay.Rcap * 128 + l * 128;
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const uint4 o4 = *at(j);
+        const uint32_t w[4] = {o4.x, o4.y, o4.z, o4.w};
+        uint32_t y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f2 = unpack_bf16(w[e]);
+          const float2 lw = *reinterpret_cast<const float2*>(ln_w + colq * 32 + j * 8 + e * 2), lb = *reinterpret_cast<const float2*>(ln_b + colq * 32 + j * 8 + e * 2);
+          y[e] = pack_bf16((f2.x - mean) * rstd * lw.x + lb.x, (f2.y - mean) * rstd * lw.y + lb.y);
+        }
+        *reinterpret_cast<uint4*>(dst + ((((colq & 1) * 4 + j) ^ (l & 7)) << 4)) = make_uint4(y[0], y[1], y[2], y[3]);
+      }
+    }
+    if (last) signal(&bars->w2i);  // behind this the next update's routing reads the resident memory
+    qsync(quarter);
+    // out to global memory, whole rows again
+#pragma unroll 1
+    for (int k = 0; k < kShare && k < n_share; ++k) {
+      const int r = rows[k * 8], lr = r >> a.lg;
+      *reinterpret_cast<uint4*>(sums + (size_t)r * HD) = *reinterpret_cast<const uint4*>(mine + k * 1024);
+      if (a.pool_k)
+        *reinterpret_cast<uint4*>(a.pool_k + ((size_t)row * a.pool_rows + cur()[lr]) * HD + pc * 8) =
+            *reinterpret_cast<const uint4*>(smem + lay.R + piece(lay.Rcap, lr, pc));
+    }
+    return ok;
   }
 
   __device__ bool run() {
     const int C = a.L.C, nc = a.nc;
-    for (int l = crank; l < 32; l += nc) mine_mask |= 1u << l;
+    const bool token = tid < C;  // (whole warps)
     int* route_row = a.route + (size_t)row * a.n_plan * C;
     kvm_update_plan pl_next = a.plan[0];  // fetched one update ahead
+    // (a wait that ran out shows in `ok` and ends the walk at the next vote: nobody leaves a barrier of the others alone)
+    bool ok = true;
     for (int u = 0; u < a.n_plan; ++u) {
       const kvm_update_plan pl = pl_next;
       if (u + 1 < a.n_plan) pl_next = a.plan[u + 1];
       const int S0 = pl.state_before, na = pl.n_append, S1 = S0 + na, nm = C - na;
       int* ver = (a.ver_idx && pl.version_row >= 0) ? a.ver_idx + (size_t)row * a.ver_rows + pl.version_row : nullptr;
-      bool ok = true;
-      if (u == 0) {
-        // ---- initial memory: the first C tokens row for row (model/kvm_mixer.py:434-447)
-        ok = wait(&bars->full_p, 0, a.wait_limit, abort) && wait(&bars->full_g, 0, a.wait_limit, abort);
+      if (u == 0 || nm == 0) {
+        // ---- the block becomes memory rows token by token: the initial memory (model/kvm_mixer.py:434-447), or a block
+        // that is appended as a whole
+        ok = ok && wait(&bars->full_p, n_p & 1, a.wait_limit, abort) && (u > 0 || wait(&bars->full_g, 0, a.wait_limit, abort));
+        ++n_p;
+        if (token) list()[tid] = tid;
         if (!wvote(ok)) return false;
-        if (tid < C) list()[tid] = tid;
-        wsync();
-        append_rows(0, na, (a.L.gate_initial && a.L.gate_keys) ? lay.G : lay.P, 0);
+        append_rows(S0, na, ((u == 0 ? a.L.gate_initial : a.L.gate_appends) && a.L.gate_keys) ? lay.G : lay.P, u);
         if (crank == 0)
-          for (int i = tid; i < C; i += kWorkers) route_row[i] = i < na ? -(1 + i) : 0;
+#pragma unroll 1
+          for (int i = tid; i < C; i += kWorkers) route_row[(size_t)u * C + i] = i < na ? -(1 + S0 + i) : 0;
+        signal(&bars->w2i);
         wsync();
-        if (ver)
-          for (int i = tid + crank * kWorkers; i < S1; i += kWorkers * nc) ver[i] = cur()[i];
-        n_load = 1;
-        signal_issuer();
-        continue;
-      }
-      const bool has_nov = na > 0 && nm > 0;
-      const int protected_rows = min(a.L.sink_len, S1);
-      // few appended rows: logits against the old memory first, the novelty behind them, both exchanged together,
-      // the logits against the new rows last (see the issuer)
-      const bool fast = nm > 0 && na <= kNewRows;
-      float best_v = -INFINITY;  // (fast) this token's best logit and row so far
-      int best_i = -1;
-      // ---- 1. novelty of every token against the old memory; the n_append least similar tokens are appended
-      if (fast) {
-        float vl_, vn_ = -INFINITY;
-        int il_, unused;
-        bool okr = read_regs<true>(n_local(S0, nc, crank), protected_rows, vl_, il_);
-        if (has_nov) okr = read_regs<false>(n_local(S0, nc, crank), 0, vn_, unused) && okr;
-        const int mt = (warp >> 2) & 1;
-        if (mt * 128 < C) {
-          const unsigned packed = ((unsigned)il_ & 0xffffu) | ((unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(vn_)) << 16);
-          part(warp >> 3)[mt * 128 + (warp & 3) * 32 + lane] = make_float2(vl_, __uint_as_float(packed));
-        }
-        if (!wvote(okr)) return false;
-        if (!exchange_both(best_v, best_i)) return false;
-      } else if (has_nov) {
-        if (!read_pass<false>(n_local(S0, nc, crank), 0)) return false;
-        if (!exchange<false>()) return false;
-      }
-      if (na > 0) {
-        if (!has_nov) {  // the whole block is appended
-          ok = wait(&bars->full_p, n_load & 1, a.wait_limit, abort);
-          if (!wvote(ok)) return false;
-          if (tid < C) { pos()[tid] = tid; list()[tid] = tid; idx()[tid] = -1; }
-        } else if (na == 1) {
-          // the token with the lowest novelty, lowest index among equals
-          float bv = tid < C ? nov()[tid] : INFINITY;
-          int bt = tid < C ? tid : 0x7fffffff;
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
-            if (ov < bv || (ov == bv && ot < bt)) { bv = ov; bt = ot; }
-          }
-          if (lane == 0) { bars->red_v[warp] = bv; bars->red_t[warp] = bt; }
-          wsync();
-          bv = bars->red_v[lane & 15];
-          bt = bars->red_t[lane & 15];
-#pragma unroll
-          for (int off = 8; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
-            if (ov < bv || (ov == bv && ot < bt)) { bv = ov; bt = ot; }
-          }
-          if (tid < C) pos()[tid] = tid == bt ? 0 : -1;
-          if (tid == 0) list()[0] = bt;
-        } else {
-          // stable rank of the novelty scores: the na lowest are appended, in token order
-          int f = 0;
-          if (tid < C) {
-            const float si = nov()[tid];
-            int rank = 0;
-#pragma unroll 4
-            for (int u0 = 0; u0 < C; u0 += 4) {
-              const float4 q = *reinterpret_cast<const float4*>(nov() + u0);
-              rank += (q.x < si || (q.x == si && u0 + 0 < tid)) ? 1 : 0;
-              rank += (q.y < si || (q.y == si && u0 + 1 < tid)) ? 1 : 0;
-              rank += (q.z < si || (q.z == si && u0 + 2 < tid)) ? 1 : 0;
-              rank += (q.w < si || (q.w == si && u0 + 3 < tid)) ? 1 : 0;
-            }
-            f = rank < na ? 1 : 0;
-          }
-          const unsigned bal = __ballot_sync(0xffffffffu, f != 0);
-          if (lane == 0) bars->red_t[warp] = __popc(bal);
-          wsync();
-          if (tid < C) {
-            int p = __popc(bal & ((1u << lane) - 1u));
-            for (int w = 0; w < warp; ++w) p += bars->red_t[w];
-            pos()[tid] = f ? p : -1;
-            if (f) list()[p] = tid;
-          }
-        }
-        wsync();
-        if (fast) append_rows_warp(S0, na, (a.L.gate_appends && a.L.gate_keys) ? lay.G : lay.P, u);
-        else append_rows(S0, na, (a.L.gate_appends && a.L.gate_keys) ? lay.G : lay.P, u);
-        if (!fast && has_nov) signal_issuer();  // the appended rows are in place: the pass against them may start
-      } else if (tid < C) {
-        pos()[tid] = -1;
-      }
-      // The prepared keys are dead from here on: their buffer becomes the one-hot operand of the scatter.
-      if (fast) {
-        signal_issuer();  // the issuer has the copy engine clear it (and may start the pass against the new rows)
-      } else if (nm > 0) {
-        wsync();  // the warps that store appended rows have read their prepared keys
-        uint4* o = reinterpret_cast<uint4*>(smem + lay.P);
-        for (int i = tid; i < C * 16; i += kWorkers) o[i] = make_uint4(0, 0, 0, 0);  // while the tensor core works on the logits
-      }
-      // ---- 2. merge target of every token: first argmax of the fp32 logits over the memory after the appends
-      if (fast) {
-        bool okm = true;
-        if (na > 0 && na <= kDirectNew) {
-          // one or two new rows: fp32 dot products of every token's gated key with them, eight lanes per token (fixed
-          // summation order); the rows are read from the small operand every CTA keeps of them
-          // (results in the novelty and append-list arrays, which nobody reads any more in this update)
-          wsync();  // the new rows are in the small operand (stored by the warps that appended them)
-          float* dots_row[2] = {nov(), reinterpret_cast<float*>(list())};
-          static_assert(kDirectNew <= 2, "two scratch rows");
-          const int gl = tid & 7, grp = tid >> 3;
-          for (int j = 0; j < na; ++j) {
-            RowVec<HD, 8> nr;
-            load_block_row_n(nr, lay.part, kNewRows, j, gl);
-            for (int base = 0; base < C; base += kWorkers / 8) {
-              const int t = base + grp;
-              RowVec<HD, 8> kr;
-              load_block_row(kr, lay.G, t, gl);
-              float acc = 0.f;
-#pragma unroll
-              for (int e = 0; e < HD / 8; ++e) acc = fmaf(kr.x[e], nr.x[e], acc);
-              acc = group_sum<8>(acc);
-              if (gl == 0) dots_row[j][t] = acc;
-            }
-          }
-          wsync();
-          if (tid < C)
-            for (int j = 0; j < na; ++j) {
-              const float x = dots_row[j][tid];
-              if (S0 + j >= protected_rows && (x > best_v || best_i < 0)) { best_v = x; best_i = S0 + j; }
-            }
-        } else if (na > 0) {
-          // the new rows (columns 0 .. na-1 of the small pass) against this token's best old row: a new row has the
-          // higher index, it wins only with a strictly larger logit
-          const int mt = (warp >> 2) & 1;
-          if (mt * 128 < C) {
-            const int hb = acc_half(g), ph = acc_phase(g);
-            okm = wait(&bars->tm_full[hb][mt], ph & 1, a.wait_limit, abort);
-            okm = __all_sync(0xffffffffu, okm);
-            if (okm && warp * 32 < C) {
-              tc::tc_fence_after_sync();
-              uint32_t r16[16];
-              tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * kChunk + hb * 128), r16);
-              tc::tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < kNewRows; ++j) {
-                const float x = __uint_as_float(r16[j]);
-                if (j < na && S0 + j >= protected_rows && (x > best_v || best_i < 0)) { best_v = x; best_i = S0 + j; }
-              }
-              tc::tc_fence_before_sync();
-            }
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&bars->tm_empty[hb][mt]);
-          }
-          ++g;
-        }
-        if (tid < C) idx()[tid] = best_i;
-        if (!wvote(okm)) return false;
-      } else if (nm > 0) {
-        if (!read_pass<true>(n_local(S1, nc, crank), protected_rows)) return false;
-        if (!exchange<true>()) return false;
-      }
-      // ---- 3. routing table, touched rows and their pool slots
-      int my = -1;
-      if (tid < C) {
-        const int p = pos()[tid];
-        my = p >= 0 ? -1 : idx()[tid];
-        if (crank == 0) route_row[(size_t)u * C + tid] = p >= 0 ? -(1 + S0 + p) : my;
-      }
-      // a row is touched in this update iff its stamp equals the update's number (no clearing between updates)
-      if (my >= 0) tf()[my] = (unsigned short)u;
-      wsync();
-      int n_touched = 0, n_touched_local = 0;
-      {
-        // compact index of every touched row among all touched rows (pool slot) and among this CTA's (accumulator lane)
-        int base_all = 0, base_loc = 0;
-        for (int r0 = 0; r0 < S1; r0 += kWorkers) {
-          const int r = r0 + tid;
-          const bool t = r < S1 && tf()[r] == (unsigned short)u;
-          const unsigned bal = __ballot_sync(0xffffffffu, t);
-          if (lane == 0) {
-            bars->red_t[warp] = __popc(bal);
-            bars->red_t[16 + warp] = __popc(bal & mine_mask);
-          }
-          wsync();
-          // lanes 0..15 hold the counts of all rows, lanes 16..31 of this CTA's rows: inclusive scan over each half
-          int cnt = bars->red_t[lane];
-#pragma unroll
-          for (int d = 1; d < 16; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, cnt, d, 16);
-            if ((lane & 15) >= d) cnt += y;
-          }
-          const int ta = __shfl_sync(0xffffffffu, cnt, 15), tl = __shfl_sync(0xffffffffu, cnt, 31);
-          const int ea = __shfl_sync(0xffffffffu, cnt, max(warp - 1, 0)), el = __shfl_sync(0xffffffffu, cnt, 16 + max(warp - 1, 0));
-          const int pa = base_all + (warp > 0 ? ea : 0), pl_ = base_loc + (warp > 0 ? el : 0);
-          if (t) {
-            const unsigned lt = (1u << lane) - 1u;
-            const int ga = pa + __popc(bal & lt);
-            gci()[r] = (short)ga;
-            if (r % nc == crank) {
-              const int ll = pl_ + __popc(bal & mine_mask & lt);
-              lci()[r / nc] = (short)ll;
-              tloc()[ll] = (unsigned short)r;
-            }
-          }
-          base_all += ta;
-          base_loc += tl;
-          wsync();
-        }
-        n_touched = base_all;
-        n_touched_local = base_loc;
-      }
-      // ---- 4. scatter: delta of the touched rows on the tensor cores, 128 compacted rows per pass
-      const int n_pass = ceil_div(n_touched_local, 128);
-      if (tid == 0) bars->n_pass = n_pass;
-      if (n_pass == 0) {
-        signal_issuer();
-        ++n_sc;  // the issuer still commits once
-        // No row of this CTA was touched: every MMA that read the block buffers has been read back, only the clearing
-        // copy may still be on its way.
-        if (tid == kLoaderThread && u + 1 < a.n_plan) {
-          const bool okl = fast ? wait(&bars->zero_done, n_zero & 1, a.wait_limit, abort) : true;
-          if (okl) issue_block_loads(smem, lay, bars, map_pk, map_gk, row, a.n_tok, C, u + 1);  // (a wait that ran out shows up at the next one)
-        }
-      }
-      bool okz = true;
-      for (int p = 0; p < n_pass; ++p) {
-        {  // one-hot operand [C/64][128 rows][64 tokens] (in the buffer of the prepared keys, which are dead by now)
-          if (p > 0) {  // a further pass: clear what the previous one set
-            uint4* o = reinterpret_cast<uint4*>(smem + lay.P);
-            for (int i = tid; i < C * 16; i += kWorkers) o[i] = make_uint4(0, 0, 0, 0);
-            wsync();
-          }
-          if (p == 0 && fast) okz = wait(&bars->zero_done, n_zero & 1, a.wait_limit, abort);  // the cleared buffer has landed
-          if (okz && my >= 0 && my % nc == crank) {
-            const int ll = lci()[my / nc] - p * 128;
-            if (ll >= 0 && ll < 128) {
-              const uint32_t off = (uint32_t)(tid >> 6) * (128u * 128u) + tc::sw128_offset(ll, tid & 63);
-              *reinterpret_cast<unsigned short*>(smem + lay.P + off) = 0x3F80;  // bf16 1.0
-            }
-          }
-        }
-        signal_issuer();
-        // this thread's share of the epilogue: row = accumulator lane quarter*32 + lane, 32 of its 128 elements
-        const int quarter = warp & 3, colq = warp >> 2;
-        const int ci = quarter * 32 + lane;
-        const bool act = p * 128 + ci < n_touched_local;
-        const int r = act ? tloc()[p * 128 + ci] : 0;
-        const size_t grow = (size_t)row * a.capacity + r;
-        uint4 old[4];
-        if (act) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) old[j] = *reinterpret_cast<const uint4*>(a.k_sum + grow * HD + colq * 32 + j * 8);
-        }
-        ok = wait(&bars->sc_done, n_sc & 1, a.wait_limit, abort) && okz;
-        ++n_sc;
-        // The scatter was the last reader of the block buffers: one thread has the next block copied in right away (both
-        // operands of every block, also where an update needs only one: the two barriers stay in step).
-        if (ok && p == n_pass - 1 && tid == kLoaderThread && u + 1 < a.n_plan)
-          issue_block_loads(smem, lay, bars, map_pk, map_gk, row, a.n_tok, C, u + 1);
-        if (!wvote(ok)) return false;
-        tc::tc_fence_after_sync();
-        float x[32];
+      } else {
+        const int protected_rows = min(a.L.sink_len, S1);
+        // few appended rows: logits against the old memory first, the novelty behind them, both exchanged together, the
+        // logits against the new rows last (see the issuer); many: novelty, appends, then all logits
+        const bool fast = na <= kNewRows;
+        // ---- 1. routing passes, partial results of the CTAs, appended rows
+        float best_v = -INFINITY, novelty = -INFINITY;  // this token's best logit and row so far
+        int best_i = -1, app = -1;                      // ... and its place among the appended ones
         {
-          uint32_t d[32];
-          tc::tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(colq * 32), d);
-          tc::tmem_ld_wait();
-          tc::tc_fence_before_sync();
-          // row = bf16(row + bf16(delta)) on packed pairs: one conversion per two elements (conversions are the
-          // slowest instructions of this loop), the sum of two bf16 numbers rounded once
-          float s1 = 0.f;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t w4[4] = {old[j].x, old[j].y, old[j].z, old[j].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int c = j * 8 + e * 2;
-              const __nv_bfloat162 dl = __floats2bfloat162_rn(__uint_as_float(d[c]), __uint_as_float(d[c + 1]));
-              uint32_t ow = act ? w4[e] : 0u;
-              const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&ow), dl);
-              const float2 f2 = __bfloat1622float2(sum);
-              x[c] = f2.x;
-              x[c + 1] = f2.y;
-              s1 += f2.x + f2.y;
+          float vl = -INFINITY, vn = -INFINITY;
+          int il = -1, unused;
+          if (fast) ok = read_regs<true>(n_local(S0, a.lg, crank), protected_rows, vl, il) && ok;
+          if (na > 0) ok = read_regs<false>(n_local(S0, a.lg, crank), 0, vn, unused) && ok;
+          store_part(vl, il, vn);
+        }
+        wsync();
+        if (token) {
+          ok = exchange(best_v, best_i, novelty) && ok;
+          if (na > 0) {
+            app = select(novelty, na);
+            tsync(C);
+          }
+        }
+        ++n_x;
+        if (na > 0) {
+          ++n_p;
+          const uint32_t src = (a.L.gate_appends && a.L.gate_keys) ? lay.G : lay.P;
+          if (fast) {
+            if (token) {
+              append_rows_warp(S0, na, src, u);
+              signal(&bars->t2i);  // the prepared keys are dead: the copy engine may clear their buffer
+              tsync(C);
+              score_new_rows(S0, na, protected_rows, best_v, best_i);
+            }
+          } else {
+            wsync();
+            append_rows(S0, na, src, u);
+            signal(&bars->w2i);  // the appended rows are in place: the pass against them may start
+            wsync();             // ... and the prepared keys dead: cleared while the tensor core works on the logits
+            uint4* o = reinterpret_cast<uint4*>(smem + lay.P);
+#pragma unroll 1
+            for (int i = tid; i < C * 16; i += kWorkers) o[i] = make_uint4(0, 0, 0, 0);
+            tc::fence_proxy_async();
+            float vl;
+            int il;
+            ok = read_regs<true>(n_local(S1, a.lg, crank), protected_rows, vl, il) && ok;
+            store_part(vl, il, -INFINITY);
+            wsync();
+            if (token) {
+              float unused;
+              ok = exchange(best_v, best_i, unused) && ok;
+            }
+            ++n_x;
+          }
+        }
+        // ---- 2. routing table; touched rows of this CTA, an accumulator lane and a pool row for each
+        const int my = app >= 0 ? -1 : best_i;
+        if (token) {
+          if (crank == 0) route_row[(size_t)u * C + tid] = app >= 0 ? -(1 + S0 + app) : my;
+          const int key = (u << kTokenBits) | ((1 << kTokenBits) - 1 - tid);
+          if (my >= 0) atomicMax(lead() + my, key);
+          tsync(C);
+          const bool mine = my >= 0 && (my & (a.nc - 1)) == crank;
+          const bool leads = mine && lead()[my] == key;
+          const unsigned bal = __ballot_sync(0xffffffffu, leads);
+          if (lane == 0) bars->red_t[16 + warp] = __popc(bal);
+          tsync(C);
+          int before = 0, total = 0;
+#pragma unroll 1
+          for (int w = 0; w < C / 32; ++w) {
+            const int c = bars->red_t[16 + w];
+            if (w < warp) before += c;
+            total += c;
+          }
+          if (leads) {
+            const int ll = before + __popc(bal & ((1u << lane) - 1u)), l = my >> a.lg;
+            lci()[l] = ll;
+            tloc()[ll] = my;
+            cur()[l] = u * C + tid;  // the row moves to the pool row of its first token
+          }
+          if (tid == 0) bars->n_loc = total;
+          tsync(C);
+          // one-hot operand [C/64][128 rows][64 tokens] of the first 128 touched rows, in the cleared buffer
+          if (fast) ok = wait(&bars->zero_done, n_zero & 1, a.wait_limit, abort) && ok;
+          if (ok && mine) {
+            const int ll = lci()[my >> a.lg];
+            if (ll < 128)
+              *reinterpret_cast<unsigned short*>(smem + lay.P + (uint32_t)(tid >> 6) * (128u * 128u) + tc::sw128_offset(ll, tid & 63)) = 0x3F80;  // bf16 1.0
+          }
+          signal(&bars->t2i);
+        }
+        if (fast) ++n_zero;
+        if (!wvote(ok)) return false;
+        // ---- 3. scatter: delta of the touched rows on the tensor cores, 128 rows per pass
+        const int n_loc = bars->n_loc, n_pass = ceil_div(n_loc, 128);
+        if (n_pass == 0) signal(&bars->w2i);
+#pragma unroll 1
+        for (int p = 0; p < n_pass; ++p) {
+          if (p > 0) {  // a further pass: the buffer holds staged sums, clear it and set the next rows
+            wsync();
+            uint4* o = reinterpret_cast<uint4*>(smem + lay.P);
+#pragma unroll 1
+            for (int i = tid; i < C * 16; i += kWorkers) o[i] = make_uint4(0, 0, 0, 0);
+            tc::fence_proxy_async();
+            wsync();
+            if (token) {
+              if (my >= 0 && (my & (a.nc - 1)) == crank) {
+                const int ll = lci()[my >> a.lg] - p * 128;
+                if (ll >= 0 && ll < 128)
+                  *reinterpret_cast<unsigned short*>(smem + lay.P + (uint32_t)(tid >> 6) * (128u * 128u) + tc::sw128_offset(ll, tid & 63)) = 0x3F80;
+              }
+              signal(&bars->t2i);
             }
           }
-          stat(0)[colq * 128 + ci] = s1;
+          ok = epilogue(p, n_loc, p == n_pass - 1) && ok;
         }
-        if (act) {  // the carried sums
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 o;
-            o.x = pack_bf16(x[j * 8 + 0], x[j * 8 + 1]); o.y = pack_bf16(x[j * 8 + 2], x[j * 8 + 3]);
-            o.z = pack_bf16(x[j * 8 + 4], x[j * 8 + 5]); o.w = pack_bf16(x[j * 8 + 6], x[j * 8 + 7]);
-            *reinterpret_cast<uint4*>(a.k_sum + grow * HD + colq * 32 + j * 8) = o;
-          }
-        }
-        wsync();
-        const float mean = (stat(0)[ci] + stat(0)[128 + ci] + stat(0)[256 + ci] + stat(0)[384 + ci]) * (1.0f / HD);
-        float s2 = 0.f;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          x[c] -= mean;
-          s2 += x[c] * x[c];
-        }
-        stat(1)[colq * 128 + ci] = s2;
-        wsync();
-        const float var = (stat(1)[ci] + stat(1)[128 + ci] + stat(1)[256 + ci] + stat(1)[384 + ci]) * (1.0f / HD);
-        const float rstd = 1.0f / sqrtf(var + a.L.ln_eps);
-        if (act) {
-          const int l = r / nc;
-          const int slot = pool_next + gci()[r];
-          bf16* pdst = a.pool_k ? a.pool_k + ((size_t)row * a.pool_rows + slot) * HD + colq * 32 : nullptr;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float y[8];
-            const float4 w0 = *reinterpret_cast<const float4*>(ln_w + colq * 32 + j * 8), w1 = *reinterpret_cast<const float4*>(ln_w + colq * 32 + j * 8 + 4);
-            const float4 b0 = *reinterpret_cast<const float4*>(ln_b + colq * 32 + j * 8), b1 = *reinterpret_cast<const float4*>(ln_b + colq * 32 + j * 8 + 4);
-            const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, bv8[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = x[j * 8 + e] * rstd * wv[e] + bv8[e];
-            uint4 o;
-            o.x = pack_bf16(y[0], y[1]); o.y = pack_bf16(y[2], y[3]); o.z = pack_bf16(y[4], y[5]); o.w = pack_bf16(y[6], y[7]);
-            *reinterpret_cast<uint4*>(smem + lay.R + piece(lay.Rcap, l, colq * 4 + j)) = o;
-            if (pdst) *reinterpret_cast<uint4*>(pdst + j * 8) = o;
-          }
-        }
+        if (!ok) *abort = 1;
       }
-      if (fast) ++n_zero;
-      // ---- 5. the version: every touched row moved to a fresh pool row
-      for (int i = tid; i < S1; i += kWorkers)
-        if (tf()[i] == (unsigned short)u) cur()[i] = pool_next + gci()[i];
-      pool_next += n_touched;
-      wsync();
+      // ---- 4. the version: pool rows of this CTA's memory rows
       if (ver)
-        for (int i = tid + crank * kWorkers; i < S1; i += kWorkers * nc) ver[i] = cur()[i];
-      ++n_load;
-      signal_issuer();  // the resident memory is final for the next update
+#pragma unroll 1
+        for (int l = tid; l < n_local(S1, a.lg, crank); l += kWorkers) ver[(l << a.lg) + crank] = cur()[l];
+      signal(&bars->idle);
     }
     // final attention view of the keys, row order, for whoever continues from this memory (the decode cache)
     {
       const kvm_update_plan pl = a.plan[a.n_plan - 1];
       const int S = pl.state_before + pl.n_append;
-      for (int i = tid; i < n_local(S, nc, crank) * 16; i += kWorkers) {
+      if (!wvote(ok)) return false;
+#pragma unroll 1
+      for (int i = tid; i < n_local(S, a.lg, crank) * 16; i += kWorkers) {
         const int l = i >> 4, c = i & 15;
-        const int r = l * nc + crank;
+        const int r = (l << a.lg) + crank;
         *reinterpret_cast<uint4*>(a.k_attn + ((size_t)row * a.capacity + r) * HD + c * 8) =
             *reinterpret_cast<const uint4*>(smem + lay.R + piece(lay.Rcap, l, c));
       }
@@ -1127,9 +1038,7 @@ kvm_chain_tc_kernel(const __grid_constant__ Args a, const __grid_constant__ Maps
   {  // resident memory starts as zeros: rows past the live ones feed the MMAs, too (their scores are masked)
     uint4* r4 = reinterpret_cast<uint4*>(smem + lay.R);
     for (int i = tid; i < lay.Rcap * 16; i += kThreads) r4[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < a.s_max; i += kThreads) reinterpret_cast<int*>(smem + lay.rowi)[i] = 0;
-    unsigned short* stamps = reinterpret_cast<unsigned short*>(smem + lay.tloc + ((2u * a.L.C + 15u) & ~15u));
-    for (int i = tid; i < a.s_max; i += kThreads) stamps[i] = 0;  // update numbers start at 1
+    for (int i = tid; i < a.s_max; i += kThreads) reinterpret_cast<int*>(smem + lay.rowi)[i] = 0;  // update numbers start at 1
   }
   if (tid == 0) {
     tc::mbar_init(&bars->full_p, 1);
@@ -1141,12 +1050,14 @@ kvm_chain_tc_kernel(const __grid_constant__ Args a, const __grid_constant__ Maps
       }
     }
     tc::mbar_init(&bars->w2i, kWorkerWarps);
+    tc::mbar_init(&bars->t2i, a.L.C / 32);
+    tc::mbar_init(&bars->idle, kWorkerWarps + (a.L.C > 128 ? 1 : 0));  // ... and the second issuer
     tc::mbar_init(&bars->sc_done, 1);
     tc::mbar_init(&bars->xbar[0], 1);  // one local arrival that states the bytes the peers will store
     tc::mbar_init(&bars->xbar[1], 1);
     tc::mbar_init(&bars->zero_done, 1);
     bars->abort = 0;
-    bars->n_pass = 0;
+    bars->n_loc = 0;
     tc::fence_barrier_init();
   }
   if (warp == kWorkerWarps) tc::tmem_alloc(&bars->tmem_base, kTmemCols);
@@ -1166,7 +1077,7 @@ kvm_chain_tc_kernel(const __grid_constant__ Args a, const __grid_constant__ Maps
       ok = is.run();
     }
   } else {
-    Workers w{a, smem, lay, bars, tmem, crank, row, ln_s, ln_s + HD, abort, tid, warp, lane, &maps.pk, &maps.gk};
+    Workers w{a, smem, lay, bars, tmem, crank, row, ln_s, ln_s + HD, abort, tid, warp, lane};
     ok = w.run();
   }
   if (!ok) {
@@ -1454,7 +1365,7 @@ cudaError_t launch_chain_tc(const LayerDev& L, int batch, long long T, Tensor4 v
       return cudaErrorInvalidValue;
   }
   Args a;
-  a.L = L; a.plan = plan_dev; a.n_plan = n_plan; a.nc = nc; a.s_max = s_max; a.n_tok = n_tok;
+  a.L = L; a.plan = plan_dev; a.n_plan = n_plan; a.nc = nc; a.lg = nc == 8 ? 3 : nc == 4 ? 2 : nc == 2 ? 1 : 0; a.s_max = s_max; a.n_tok = n_tok;
   a.k_sum = mem.k_sum; a.k_attn = mem.k_attn; a.capacity = mem.capacity;
   a.pool_k = ver_idx ? pool_k : nullptr; a.pool_rows = pool_rows; a.ver_idx = ver_idx; a.ver_rows = ver_rows;
   a.route = route; a.born = born; a.status = status; a.wait_limit = wait_limit; a.test_flags = test_flags;
