@@ -181,7 +181,7 @@ int kvm_prefill_workspace_layout(const kvm_layer* layer, int32_t batch, int64_t 
  *   shift_q [Hq*D], shift_k, shift_v [Hkv*D]      token-shift scales, all three NULL: no token shift
  *   prev_q [B,Hq*D], prev_k, prev_v [B,Hkv*D]     last token of the previous call (cached decode), NULL: the first
  *                                                 token is shifted against itself
- *   ln_q_w, ln_q_b, ln_k_w, ln_k_b [D] fp32       per-head LayerNorm of q and k, all four NULL: none
+ *   ln_q_w, ln_q_b, ln_k_w, ln_k_b [D] fp32       per-head LayerNorm of q and k (bf16 with ln_bf16), all four NULL: none
  *   cos, sin [B or 1, T, D]                       rotary tables as RotaryEmbedding returns them (the sign of the
  *                                                 odd sin entries folded in); rope_stride_b = T*D or 0; NULL: none */
 typedef struct kvm_prologue {
@@ -195,14 +195,18 @@ typedef struct kvm_prologue {
   const void* prev_q;
   const void* prev_k;
   const void* prev_v;
-  const float* ln_q_w;
-  const float* ln_q_b;
-  const float* ln_k_w;
-  const float* ln_k_b;
+  const void* ln_q_w;
+  const void* ln_q_b;
+  const void* ln_k_w;
+  const void* ln_k_b;
   float ln_qk_eps;
   const void* cos;
   const void* sin;
   int64_t rope_stride_b;
+} kvm_prologue;
+/* The same with more that the kernel can take over; all zero: exactly kvm_prologue. */
+typedef struct kvm_prologue_ext {
+  kvm_prologue base;
   int64_t q_stride_t, k_stride_t, v_stride_t, gate_stride_t; /* elements from token to token (the outputs of one GEMM over all
                                                   projections: rows wider than one of them); 0: contiguous.  A batch row
                                                   is T such strides */
@@ -211,7 +215,8 @@ typedef struct kvm_prologue {
   const void* v_gate;      /* v_first [B,T,Hkv*D] contiguous, v_gate [B,T,Hkv*D] contiguous, v_gate0 [Hkv*D]; all */
   const void* v_gate0;     /* three NULL: none (model/value_residual_mixin.py:173-218) */
   void* v_last;            /* [B,Hkv*D] out, may be NULL: the last token's value behind the residual, before the shift */
-} kvm_prologue;
+  int32_t ln_bf16;         /* ln_q_w .. ln_k_b are bf16 (else fp32) */
+} kvm_prologue_ext;
 /*   q_out [B,T,Hq,D], k_out, v_out [B,T,Hkv,D]   the operator's inputs (pass them on as [B,H,T,D] views)
  *   gate_out [B,Hkv,T]                           merge gate
  *   workspace  a prefill workspace for this shape (kvm_prefill_workspace_bytes) or NULL.  When given and the
@@ -223,6 +228,9 @@ typedef struct kvm_prologue {
 int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in,
                          void* q_out, void* k_out, void* v_out, void* gate_out, int64_t total_version_rows,
                          void* workspace, size_t workspace_bytes, void* stream);
+int kvm_prologue_forward_ext(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue_ext* in,
+                             void* q_out, void* k_out, void* v_out, void* gate_out, int64_t total_version_rows,
+                             void* workspace, size_t workspace_bytes, void* stream);
 
 /* Linear layers (no bias) over few rows, for the projections of decode tokens: out[m, :] = (x[m, :] W_0^T, x[m, :] W_1^T, ..)
  * for 1 <= n_rows <= 128 rows of `width` (a multiple of 32) bf16 values, x_stride elements apart, and up to eight weights
@@ -364,7 +372,7 @@ int kvm_decode_cache_fill(const kvm_layer* layer, int32_t batch, int64_t seq_len
  * Replaces SequenceMixer.forward_inference of a cached single-token step (model/kvm_mixer.py:527-570, 572-713). */
 typedef struct kvm_token_call {
   kvm_decode_call decode;      /* q, k, v, gate and out are not read */
-  kvm_prologue prologue;       /* parameters, rotary tables, cached tokens, v_first, v_gate0, v_last; projection outputs and v_gate not read */
+  kvm_prologue_ext prologue;       /* parameters, rotary tables, cached tokens, v_first, v_gate0, v_last; projection outputs and v_gate not read */
   const void* x;               /* [batch, hidden] bf16, rows x_stride elements apart */
   int64_t x_stride;
   int32_t hidden;
@@ -392,7 +400,7 @@ typedef struct kvm_prompt_call {
   int32_t batch, n_updates;
   int64_t seq_len, total_version_rows;
   const kvm_update_plan* plan_host;
-  kvm_prologue prologue;
+  kvm_prologue_ext prologue;
   kvm_memory memory;
   kvm_decode_cache cache;
   void* decode_workspace;

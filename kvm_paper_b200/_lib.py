@@ -53,10 +53,16 @@ class KvmPrefillLayout(C.Structure):
 class KvmPrologue(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("q_lin", "k_lin", "v_lin", "gate_lin", "shift_q", "shift_k", "shift_v",
                                           "prev_q", "prev_k", "prev_v", "ln_q_w", "ln_q_b", "ln_k_w", "ln_k_b")] + [
-        ("ln_qk_eps", C.c_float), ("cos", C.c_void_p), ("sin", C.c_void_p), ("rope_stride_b", C.c_int64),
+        ("ln_qk_eps", C.c_float), ("cos", C.c_void_p), ("sin", C.c_void_p), ("rope_stride_b", C.c_int64)]
+
+
+class KvmPrologueExt(C.Structure):
+    _anonymous_ = ("base",)
+    _fields_ = [
+        ("base", KvmPrologue),
         ("q_stride_t", C.c_int64), ("k_stride_t", C.c_int64), ("v_stride_t", C.c_int64), ("gate_stride_t", C.c_int64),
         ("prev_q_stride_b", C.c_int64), ("prev_k_stride_b", C.c_int64), ("prev_v_stride_b", C.c_int64),
-        ("v_first", C.c_void_p), ("v_gate", C.c_void_p), ("v_gate0", C.c_void_p), ("v_last", C.c_void_p)]
+        ("v_first", C.c_void_p), ("v_gate", C.c_void_p), ("v_gate0", C.c_void_p), ("v_last", C.c_void_p), ("ln_bf16", C.c_int32)]
 
 
 class KvmDecodeCache(C.Structure):
@@ -73,7 +79,7 @@ class KvmDecodeCall(C.Structure):
 
 
 class KvmTokenCall(C.Structure):
-    _fields_ = [("decode", KvmDecodeCall), ("prologue", KvmPrologue), ("x", C.c_void_p), ("x_stride", C.c_int64), ("hidden", C.c_int32),
+    _fields_ = [("decode", KvmDecodeCall), ("prologue", KvmPrologueExt), ("x", C.c_void_p), ("x_stride", C.c_int64), ("hidden", C.c_int32),
                 ("n_weights", C.c_int32), ("weights", C.c_void_p * 5), ("weight_rows", C.c_int32 * 5), ("gated", C.c_int32),
                 ("out_features", C.c_int32), ("v_gate2", C.c_void_p), ("c_proj", C.c_void_p), ("lin", C.c_void_p),
                 ("lin_stride", C.c_int64), ("scratch", C.c_void_p), ("scratch_bytes", C.c_size_t), ("y", C.c_void_p)]
@@ -81,7 +87,7 @@ class KvmTokenCall(C.Structure):
 
 class KvmPromptCall(C.Structure):
     _fields_ = [("layer", C.c_void_p), ("batch", C.c_int32), ("n_updates", C.c_int32), ("seq_len", C.c_int64),
-                ("total_version_rows", C.c_int64), ("plan_host", C.c_void_p), ("prologue", KvmPrologue), ("memory", KvmMemory),
+                ("total_version_rows", C.c_int64), ("plan_host", C.c_void_p), ("prologue", KvmPrologueExt), ("memory", KvmMemory),
                 ("cache", KvmDecodeCache), ("decode_workspace", C.c_void_p), ("out", C.c_void_p), ("workspace", C.c_void_p),
                 ("workspace_bytes", C.c_size_t)]
 
@@ -89,7 +95,7 @@ class KvmPromptCall(C.Structure):
 EXPORTS = [
     "kvm_prefill_workspace_bytes", "kvm_prefill_forward", "kvm_decode_workspace_bytes", "kvm_decode_step",
     "kvm_memory_refresh", "kvm_last_error_string", "kvm_abi_version", "kvm_decode_step_static", "kvm_prefill_status", "kvm_decode_run",
-    "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward",
+    "kvm_decode_status", "kvm_prefill_workspace_layout", "kvm_interleave_shards", "kvm_prologue_forward", "kvm_prologue_forward_ext",
     "kvm_prefill_forward_gathered", "kvm_decode_step_call", "kvm_decode_span",
     "kvm_decode_cache_fill", "kvm_project", "kvm_token_scratch_bytes", "kvm_mixer_token",
     "kvm_prompt_workspace_bytes", "kvm_mixer_prompt",
@@ -156,9 +162,10 @@ def load():
         C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.kvm_memory_refresh.restype = C.c_int
     lib.kvm_memory_refresh.argtypes = [LP(KvmLayer), C.c_int32, KvmMemory, C.c_void_p, C.c_void_p]
-    lib.kvm_prologue_forward.restype = C.c_int
-    lib.kvm_prologue_forward.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, LP(KvmPrologue), C.c_void_p, C.c_void_p, C.c_void_p,
-                                         C.c_void_p, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]
+    for fn, arg in ((lib.kvm_prologue_forward, KvmPrologue), (lib.kvm_prologue_forward_ext, KvmPrologueExt)):
+        fn.restype = C.c_int
+        fn.argtypes = [LP(KvmLayer), C.c_int32, C.c_int64, LP(arg), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
+                       C.c_void_p, C.c_size_t, C.c_void_p]
     lib.kvm_token_scratch_bytes.restype = C.c_size_t
     lib.kvm_token_scratch_bytes.argtypes = [LP(KvmLayer), C.c_int32]
     lib.kvm_mixer_token.restype = C.c_int

@@ -315,12 +315,14 @@ int kvm_prefill_forward_gathered(const kvm_layer* layer, int32_t batch, int64_t 
 }
 
 // Checked arguments of the prologue; workspace == nullptr: no prepared keys.
-static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out, void* k_out,
+static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue_ext* ext, void* q_out, void* k_out,
                          void* v_out, void* gate_out, int64_t total_version_rows, void* workspace, size_t workspace_bytes,
                          kvm::PrologueDev* dev) {
+  if (!ext) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: in is NULL");
+  const kvm_prologue* in = &ext->base;
   if (int rc = check_layer(layer)) return rc;
   if (batch <= 0 || seq_len <= 0) return fail(KVM_ERR_BAD_ARGUMENT, "batch %d and seq_len %lld must be positive", batch, (long long)seq_len);
-  if (!in || !in->q_lin || !in->k_lin || !in->v_lin || !q_out || !k_out || !v_out || !gate_out)
+  if (!in->q_lin || !in->k_lin || !in->v_lin || !q_out || !k_out || !v_out || !gate_out)
     return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: projections and outputs must not be NULL");
   const int D = layer->head_dim;
   if (D != 32 && D != 64 && D != 128) return fail(KVM_ERR_UNSUPPORTED, "kvm_prologue_forward: head_dim %d (supported: 32, 64, 128)", D);
@@ -332,26 +334,26 @@ static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   if (in->cos && in->rope_stride_b != 0 && in->rope_stride_b != seq_len * D)
     return fail(KVM_ERR_BAD_ARGUMENT, "rope_stride_b %lld must be 0 or seq_len*head_dim", (long long)in->rope_stride_b);
   const void* aligned[] = {in->q_lin, in->k_lin, in->v_lin, in->shift_q, in->shift_k, in->shift_v, in->prev_q, in->prev_k, in->prev_v,
-                           in->cos, in->sin, in->v_first, in->v_gate, in->v_gate0, in->v_last, q_out, k_out, v_out, in->ln_q_w, in->ln_q_b, in->ln_k_w, in->ln_k_b,
+                           in->cos, in->sin, ext->v_first, ext->v_gate, ext->v_gate0, ext->v_last, q_out, k_out, v_out, in->ln_q_w, in->ln_q_b, in->ln_k_w, in->ln_k_b,
                            layer->ln_weight_dev, layer->ln_bias_dev};
   for (const void* a : aligned)
     if (((uintptr_t)a) % 16) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: tensors must be 16-byte aligned");
-  const int n_mix = (in->v_first != nullptr) + (in->v_gate != nullptr) + (in->v_gate0 != nullptr);
+  const int n_mix = (ext->v_first != nullptr) + (ext->v_gate != nullptr) + (ext->v_gate0 != nullptr);
   if (n_mix != 0 && n_mix != 3) return fail(KVM_ERR_BAD_ARGUMENT, "the value residual needs v_first, v_gate and v_gate0");
   const long long width_q = (long long)layer->n_q_heads * D, width_kv = (long long)layer->n_kv_heads * D;
   kvm::PrologueDev& p = *dev;
   p = {};
-  const int64_t given[6] = {in->q_stride_t, in->k_stride_t, in->v_stride_t, in->prev_q_stride_b, in->prev_k_stride_b, in->prev_v_stride_b};
+  const int64_t given[6] = {ext->q_stride_t, ext->k_stride_t, ext->v_stride_t, ext->prev_q_stride_b, ext->prev_k_stride_b, ext->prev_v_stride_b};
   for (int i = 0; i < 6; ++i) {
     const long long width = i % 3 == 0 ? width_q : width_kv, st = given[i] ? given[i] : width;
     if (st < width || st % 8) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: stride %lld must be a multiple of 8 and at least %lld", st, width);
     (i < 3 ? p.st[i] : p.prev_sb[i - 3]) = st;
   }
-  p.gate_st = in->gate_stride_t ? in->gate_stride_t : layer->n_kv_heads;
-  p.v_first = static_cast<const bf16*>(in->v_first);
-  p.v_gate = static_cast<const bf16*>(in->v_gate);
-  p.v_gate0 = static_cast<const bf16*>(in->v_gate0);
-  p.v_last = static_cast<bf16*>(in->v_last);
+  p.gate_st = ext->gate_stride_t ? ext->gate_stride_t : layer->n_kv_heads;
+  p.v_first = static_cast<const bf16*>(ext->v_first);
+  p.v_gate = static_cast<const bf16*>(ext->v_gate);
+  p.v_gate0 = static_cast<const bf16*>(ext->v_gate0);
+  p.v_last = static_cast<bf16*>(ext->v_last);
   p.q_lin = static_cast<const bf16*>(in->q_lin);
   p.k_lin = static_cast<const bf16*>(in->k_lin);
   p.v_lin = static_cast<const bf16*>(in->v_lin);
@@ -367,6 +369,7 @@ static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   p.ln_k_w = in->ln_k_w;
   p.ln_k_b = in->ln_k_b;
   p.ln_qk_eps = in->ln_qk_eps;
+  p.ln_bf16 = ext->ln_bf16;
   p.cos = static_cast<const bf16*>(in->cos);
   p.sin = static_cast<const bf16*>(in->sin);
   p.rope_stride_b = in->rope_stride_b;
@@ -389,9 +392,9 @@ static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   return KVM_OK;
 }
 
-int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out,
-                         void* k_out, void* v_out, void* gate_out, int64_t total_version_rows, void* workspace,
-                         size_t workspace_bytes, void* stream) {
+int kvm_prologue_forward_ext(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue_ext* in, void* q_out,
+                             void* k_out, void* v_out, void* gate_out, int64_t total_version_rows, void* workspace,
+                             size_t workspace_bytes, void* stream) {
   g_err[0] = 0;
   kvm::PrologueDev p;
   if (int rc = prologue_args(layer, batch, seq_len, in, q_out, k_out, v_out, gate_out, total_version_rows, workspace, workspace_bytes, &p))
@@ -399,6 +402,15 @@ int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len,
   const cudaError_t e = kvm::launch_prologue(layer->head_dim, to_dev(layer), p, batch, seq_len, static_cast<cudaStream_t>(stream), false);
   if (e != cudaSuccess) return cuda_fail(e, "kvm_prologue_forward");
   return KVM_OK;
+}
+
+int kvm_prologue_forward(const kvm_layer* layer, int32_t batch, int64_t seq_len, const kvm_prologue* in, void* q_out,
+                         void* k_out, void* v_out, void* gate_out, int64_t total_version_rows, void* workspace,
+                         size_t workspace_bytes, void* stream) {
+  kvm_prologue_ext ext = {};
+  if (in) ext.base = *in;
+  return kvm_prologue_forward_ext(layer, batch, seq_len, in ? &ext : nullptr, q_out, k_out, v_out, gate_out, total_version_rows, workspace,
+                                  workspace_bytes, stream);
 }
 
 static int project_impl(const void* x, int64_t x_stride, int32_t n_rows, int32_t width, const void* const* weights,
@@ -764,10 +776,10 @@ int kvm_mixer_token(const kvm_token_call* c, void* stream) {
   if (int rc = project_impl(c->x, c->x_stride, batch, c->hidden, c->weights, c->weight_rows, c->n_weights, c->lin, c->lin_stride, stream, false))
     return rc;
   const bf16* lin = static_cast<const bf16*>(c->lin);
-  kvm_prologue pro = c->prologue;
-  pro.q_lin = lin;
-  pro.k_lin = lin + Hq * D;
-  pro.v_lin = lin + (Hq + Hkv) * D;
+  kvm_prologue_ext pro = c->prologue;
+  pro.base.q_lin = lin;
+  pro.base.k_lin = lin + Hq * D;
+  pro.base.v_lin = lin + (Hq + Hkv) * D;
   pro.q_stride_t = pro.k_stride_t = pro.v_stride_t = pro.gate_stride_t = c->lin_stride;
   const bf16* behind = lin + (Hq + 2 * Hkv) * D;
   pro.v_gate = nullptr;
@@ -777,7 +789,7 @@ int kvm_mixer_token(const kvm_token_call* c, void* stream) {
     pro.v_gate = w + m.v_gate;
     behind += c->weight_rows[3];
   }
-  pro.gate_lin = c->gated ? behind : nullptr;
+  pro.base.gate_lin = c->gated ? behind : nullptr;
   kvm::PrologueDev p;
   if (int rc = prologue_args(layer, batch, 1, &pro, w + m.q, w + m.k, w + m.v, w + m.gate, 0, nullptr, 0, &p)) return rc;
   const cudaError_t e = kvm::launch_prologue(D, to_dev(layer), p, batch, 1, static_cast<cudaStream_t>(stream), true);

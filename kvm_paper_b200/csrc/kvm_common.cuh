@@ -54,11 +54,12 @@ struct PrologueDev {
   const bf16* prev_q;
   const bf16* prev_k;
   const bf16* prev_v;
-  const float* ln_q_w;
-  const float* ln_q_b;
-  const float* ln_k_w;
-  const float* ln_k_b;
+  const void* ln_q_w;
+  const void* ln_q_b;
+  const void* ln_k_w;
+  const void* ln_k_b;
   float ln_qk_eps;
+  int ln_bf16;
   const bf16* cos;
   const bf16* sin;
   long long rope_stride_b;

@@ -628,17 +628,17 @@ __global__ void kvm_memory_refresh_kernel(LayerDev L, MemoryDev mem, const int* 
   refresh_memory_row<D>(L, ks, vs, mem.vlen[(size_t)row * mem.capacity + r], mem.k_attn + off, mem.v_attn + off, lane);
 }
 
-// Decode cache after a prefill: CTA (x, kv row) copies its share of the row's window tokens and memory rows, 16 bytes per
+// Decode cache after a prefill: each of `per_row` CTAs of a kv row copies its share of the row's window tokens and memory rows, 16 bytes per
 // thread and step; the first CTA also writes the lengths and clears the counters.
 template <int D>
 __global__ void __launch_bounds__(256)
 kvm_cache_fill_kernel(LayerDev L, long long T, Tensor4 k, Tensor4 v, Tensor4 gate, MemoryDev from, int rows, DecodeCacheDev cache, int batch,
-                      int* __restrict__ counters, int n_counters) {
+                      int* __restrict__ counters, int n_counters, int per_row) {
   constexpr int CPR = D / 8;
-  const int row = blockIdx.y, b = row / L.Hkv, h = row % L.Hkv, WC = L.W * L.C;
+  const int row = blockIdx.x / per_row, x = blockIdx.x % per_row, b = row / L.Hkv, h = row % L.Hkv, WC = L.W * L.C;
   const long long begin = bswa_begin_dev((int)T, L.C, L.W);
   const int n_win = (int)(T - begin);
-  const int at = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+  const int at = x * 256 + threadIdx.x, step = per_row * 256;
   for (int i = at; i < n_win * CPR; i += step) {
     const int w = i / CPR, c = i % CPR;
     const size_t dst = ((size_t)row * WC + (int)((begin + w) % WC)) * D + c * 8;
@@ -656,7 +656,7 @@ kvm_cache_fill_kernel(LayerDev L, long long T, Tensor4 k, Tensor4 v, Tensor4 gat
             *reinterpret_cast<const uint4*>(src[a] + (size_t)row * from.capacity * D + i * 8);
     for (int i = at; i < rows; i += step) cache.mem.vlen[(size_t)row * cache.mem.capacity + i] = from.vlen[(size_t)row * from.capacity + i];
   }
-  if (row == 0 && blockIdx.x == 0) {
+  if (blockIdx.x == 0) {
     for (int i = threadIdx.x; i < batch; i += 256) {
       cache.total_len[i] = (int)T;
       cache.state_len[i] = rows;
@@ -886,11 +886,11 @@ cudaError_t cache_fill_dispatch(int D, const LayerDev& L, int batch, long long T
                                 int rows, const DecodeCacheDev& cache, int* counters, int n_counters, cudaStream_t stream) {
   // enough CTAs per kv row to fill the GPU when the rows are few, at most one per 1024 pieces of 16 bytes
   const int kv_rows = batch * L.Hkv, pieces = std::max(L.W * L.C, rows) * (D / 8);
-  dim3 grid(std::max(1, std::min((pieces + 1023) / 1024, 4 * device_sm_count() / kv_rows)), kv_rows);
+  const int per_row = std::max(1, std::min((pieces + 1023) / 1024, 4 * device_sm_count() / kv_rows)), grid = per_row * kv_rows;
   switch (D) {
-    case 32: kvm_cache_fill_kernel<32><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters); break;
-    case 64: kvm_cache_fill_kernel<64><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters); break;
-    case 128: kvm_cache_fill_kernel<128><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters); break;
+    case 32: kvm_cache_fill_kernel<32><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters, per_row); break;
+    case 64: kvm_cache_fill_kernel<64><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters, per_row); break;
+    case 128: kvm_cache_fill_kernel<128><<<grid, 256, 0, stream>>>(L, T, k, v, gate, from, rows, cache, batch, counters, n_counters, per_row); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

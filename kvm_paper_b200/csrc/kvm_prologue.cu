@@ -46,11 +46,17 @@ __device__ __forceinline__ void load_raw(uint32_t (&w)[EPL / 2], const bf16* p) 
   }
 }
 
+__device__ __forceinline__ float4 load_weights(const void* w, int i, int is_bf16) {  // four of them, from the i-th
+  if (!is_bf16) return __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(w) + i));
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const bf16*>(w) + i));
+  const float2 lo = unpack_bf16(u.x), hi = unpack_bf16(u.y);
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
 // LayerNorm as the reference's module evaluates it on bf16 rows: moments in fp32, y = (x*rstd - mean*rstd)*w + b with
 // every product and sum rounded on its own, one rounding to bf16 at the end.
 template <int D>
-__device__ __forceinline__ void qk_layer_norm(RowVec<D, GL>& r, const float* __restrict__ w, const float* __restrict__ b, float eps,
-                                              int gl) {
+__device__ __forceinline__ void qk_layer_norm(RowVec<D, GL>& r, const void* __restrict__ w, const void* __restrict__ b, int is_bf16,
+                                              float eps, int gl) {
   constexpr int EPL = D / GL;
   float s = 0.f;
 #pragma unroll
@@ -65,12 +71,10 @@ __device__ __forceinline__ void qk_layer_norm(RowVec<D, GL>& r, const float* __r
   const float var = group_sum<GL>(q) * (1.0f / D);
   const float rstd = 1.0f / sqrtf(fmaxf(var, 0.f) + eps);
   const float bias = __fmul_rn(-mean, rstd);
-  // (weights by 16-byte loads: a lane's share starts at a multiple of four elements)
-  const float4* w4 = reinterpret_cast<const float4*>(w + gl * EPL);
-  const float4* b4 = reinterpret_cast<const float4*>(b + gl * EPL);
+  // (weights by 16-byte loads, 8 bytes of bf16: a lane's share starts at a multiple of four elements)
 #pragma unroll
   for (int i = 0; i < EPL; i += 4) {
-    const float4 wv = __ldg(w4 + i / 4), bv = __ldg(b4 + i / 4);
+    const float4 wv = load_weights(w, gl * EPL + i, is_bf16), bv = load_weights(b, gl * EPL + i, is_bf16);
     r.x[i] = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(r.x[i], rstd), bias), wv.x), bv.x);
     r.x[i + 1] = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(r.x[i + 1], rstd), bias), wv.y), bv.y);
     r.x[i + 2] = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(r.x[i + 2], rstd), bias), wv.z), bv.z);
@@ -178,7 +182,7 @@ kvm_prologue_kernel(LayerDev L, PrologueDev p, long long T) {
       y.x[2 * i] = f.x;
       y.x[2 * i + 1] = f.y;
     }
-    qk_layer_norm<D>(y, kind == 0 ? p.ln_q_w : p.ln_k_w, kind == 0 ? p.ln_q_b : p.ln_k_b, p.ln_qk_eps, gl);
+    qk_layer_norm<D>(y, kind == 0 ? p.ln_q_w : p.ln_k_w, kind == 0 ? p.ln_q_b : p.ln_k_b, p.ln_bf16, p.ln_qk_eps, gl);
     if (kind < 2) {
 #pragma unroll
       for (int i = 0; i < EPL / 2; ++i) x[i] = pack_bf16(y.x[2 * i], y.x[2 * i + 1]);

@@ -21,6 +21,7 @@ from typing import Any
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules import module as _module
 
 from . import _lib, ops
 
@@ -307,21 +308,26 @@ class SequenceMixer(nn.Module):
             gate = torch.ones((B, self.num_key_value_heads, T, 1), device=x.device, dtype=torch.float)
         return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), gate
 
-    def prologue_params(self, device) -> ops.PrologueParams:
+    def prologue_params(self, device, share_ln: bool = False) -> ops.PrologueParams:
         ln = isinstance(self.ln_q, nn.LayerNorm)
         shift = self.tokenshift_mode == "rwkv"
         return ops.PrologueParams(device, shift_q=self.x_q if shift else None, shift_k=self.x_k if shift else None,
                                   shift_v=self.x_v if shift else None, ln_q=self.ln_q if ln else None,
-                                  ln_k=self.ln_k if ln else None, ln_eps=self.ln_q.eps if ln else 1e-5)
+                                  ln_k=self.ln_k if ln else None, ln_eps=self.ln_q.eps if ln else 1e-5, share_ln=share_ln)
 
     def _prologue_params_kept(self, device) -> ops.PrologueParams:
-        """``prologue_params``, rebuilt when a parameter changes."""
+        """``prologue_params``, kept as long as it consists of views of the parameters (a copy would miss what is written
+        to a parameter behind autograd's back)."""
+        ln = isinstance(self.ln_q, nn.LayerNorm)
         src = [t for m in (self.ln_q, self.ln_k) if isinstance(m, nn.LayerNorm) for t in (m.weight, m.bias)]
         if self.tokenshift_mode == "rwkv":
             src += [self.x_q, self.x_k, self.x_v]
-        key = (device, *((t.data_ptr(), t._version) for t in src))
+        key = (device, self.ln_q.eps if ln else None, *((t.data_ptr(), t.dtype) for t in src))
         if self._prologue_cache is None or self._prologue_cache[0] != key:
-            self._prologue_cache = (key, self.prologue_params(device))
+            pro = self.prologue_params(device, share_ln=True)
+            if not pro.shared:
+                return pro
+            self._prologue_cache = (key, pro)
         return self._prologue_cache[1]
 
     def fused_prologue_applies(self, x: torch.Tensor) -> bool:
@@ -335,14 +341,20 @@ class SequenceMixer(nn.Module):
     @staticmethod
     def _plain_linear(m, x) -> bool:
         """A linear layer that ``ops.project`` may stand in for: bf16, no bias, nothing hooked onto it."""
-        return (type(m) is nn.Linear and m.bias is None and m.weight.dtype is torch.bfloat16 and m.weight.is_contiguous()
-                and m.weight.data_ptr() % 16 == 0 and m.in_features % 32 == 0 and m.weight.device == x.device and not m._forward_hooks and not m._forward_pre_hooks)
+        if type(m) is not nn.Linear or m.bias is not None:
+            return False
+        w = m.weight
+        return (type(w) in (nn.Parameter, torch.Tensor) and w.dtype is torch.bfloat16
+                and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.size(1) % 32 == 0 and w.device == x.device
+                and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__)
 
     def _few_rows(self, x) -> bool:
-        """Up to 64 rows (tokens x sequences) the linear layers are bound by reading the weights and by launches: the
-        library's kernel takes all layers of one input at once.  More rows are left to the library GEMMs."""
-        return (x.size(0) * x.size(1) <= _lib.PROJECT_ROWS_MAX and x.is_cuda and x.dtype is torch.bfloat16
-                and not torch.is_grad_enabled())
+        """Up to 128 rows (tokens x sequences) the linear layers are bound by reading the weights and by launches: the
+        library's kernel takes all layers of one input at once.  More rows are left to the library GEMMs, and so is
+        whatever else looks at the modules' calls (autocast, hooks on all modules)."""
+        return (0 < x.size(0) * x.size(1) <= _lib.PROJECT_ROWS_MAX and x.is_cuda and x.dtype is torch.bfloat16
+                and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+                and not (_module._global_forward_hooks or _module._global_forward_pre_hooks))
 
     def _project(self, x):
         """q, k, v projections, output of ``v_gate2`` and merge-gate logits (the last two None where the layer has none)."""
@@ -420,9 +432,9 @@ class SequenceMixer(nn.Module):
     def _unwatched(self, stage: str) -> bool:
         """Nobody looks at the tensors between the stages of a call (no hook, no override of the stage behind the prefix):
         the stages may run as one library call."""
-        return not (self.capture_routes or self.check_device_status or torch.is_grad_enabled() or stage in self.__dict__
-                    or "forward_prefix_fused" in self.__dict__ or getattr(type(self), stage) is not getattr(SequenceMixer, stage)
-                    or type(self).forward_prefix_fused is not SequenceMixer.forward_prefix_fused)
+        stages = (stage, "forward_prefix_fused", "prefill_raw", "_value_gate")
+        return not (self.capture_routes or self.check_device_status or torch.is_grad_enabled()
+                    or any(n in self.__dict__ or getattr(type(self), n) is not getattr(SequenceMixer, n) for n in stages))
 
     def _prompt(self, x, v_first, position_embeddings, past_key_values):
         """``forward_prefix_fused`` and ``forward_prefill`` of a prompt in one library call between the linear layers; the
@@ -443,7 +455,10 @@ class SequenceMixer(nn.Module):
         if past_key_values is not None:
             states = past_key_values.get_states(self.layer_idx)
             prev = (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL))
-        cache, y = ops.prompt_forward(params, pro, q, k, v, gate_lin, position_embeddings, self.make_prefill_plan(T), prev=prev,
+        plan = self.make_prefill_plan(T)
+        if past_key_values is not None and plan.final_coverage != max(min(T, self.chunk_len), self._bswa_begin_for_total_len(T)):
+            raise AssertionError("KVM prefill state progression drifted from the decode-state bookkeeping.")
+        cache, y = ops.prompt_forward(params, pro, q, k, v, gate_lin, position_embeddings, plan, prev=prev,
                                       value_residual=residual, v_last=v_last, desired_state_len=self._desired_state_len, owner=self,
                                       want_cache=past_key_values is not None)
         if past_key_values is not None:
@@ -477,7 +492,6 @@ class SequenceMixer(nn.Module):
         dq, dk = self.q_projection_size, self.k_projection_size
         v_final = v_last if mixed else lin[..., dq + dk:dq + 2 * dk]
         finals = (lin[..., :dq], lin[..., dq:dq + dk], v_final)
-        call.produced(finals)
         past_key_values.update(self.layer_idx, offset=1, states_dict={
             self._CACHE_Q_FINAL: finals[0], self._CACHE_K_FINAL: finals[1], self._CACHE_V_FINAL: v_final, self._CACHE_X_FINAL: x,
             self._CACHE_DECODE: cache})

@@ -59,6 +59,8 @@ def _as_bf16_view(t: torch.Tensor) -> torch.Tensor:
 def _fill_tensor4(dst: KvmTensor4, t: torch.Tensor, name: str) -> torch.Tensor:
     """``_tensor4`` into a kept C descriptor; returns the tensor the descriptor points into."""
     st = t.stride()
+    if len(st) != 4:
+        raise ValueError(f"{name} must be 4-dimensional, got {tuple(t.shape)}")
     if t.dtype is not torch.bfloat16 or (st[3] != 1 and t.size(3) > 1):
         t = _as_bf16_view(t)
         st = t.stride()
@@ -223,21 +225,29 @@ class PrefillResult:
 
 
 class PrologueParams:
-    """Device copies of what the fused prologue reads besides the projections: token-shift scales (bf16),
-    per-head LayerNorm of q and k (fp32), all optional as in the reference module
-    (model/value_residual_mixin.py:60-98)."""
+    """What the fused prologue reads besides the projections, on the device: token-shift scales (bf16),
+    per-head LayerNorm of q and k (a fp32 copy), all optional as in the reference module
+    (model/value_residual_mixin.py:60-98).  ``share_ln``: the kernel reads bf16 LayerNorm weights where they are instead
+    of a copy; ``shared`` then says whether all of it lives in the parameters themselves, whatever is written to them."""
 
-    def __init__(self, device, *, shift_q=None, shift_k=None, shift_v=None, ln_q=None, ln_k=None, ln_eps: float = 1e-5):
+    def __init__(self, device, *, shift_q=None, shift_k=None, shift_v=None, ln_q=None, ln_k=None, ln_eps: float = 1e-5,
+                 share_ln: bool = False):
         dev = torch.device(device)
+        given = [shift_q, shift_k, shift_v]
         shifts = [None if t is None else t.detach().to(dev, torch.bfloat16).reshape(-1).contiguous() for t in (shift_q, shift_k, shift_v)]
         if any(t is None for t in shifts) and not all(t is None for t in shifts):
             raise ValueError("token-shift scales must be given for q, k and v or for none")
         self.shift_q, self.shift_k, self.shift_v = shifts
         if (ln_q is None) != (ln_k is None):
             raise ValueError("LayerNorm must be given for q and k or for neither")
-        self.ln = None
+        self.ln, self.ln_bf16 = None, 0
         if ln_q is not None:
-            self.ln = tuple(t.detach().to(dev, torch.float32).contiguous() for t in (ln_q.weight, ln_q.bias, ln_k.weight, ln_k.bias))
+            ln = (ln_q.weight, ln_q.bias, ln_k.weight, ln_k.bias)
+            given += ln
+            self.ln_bf16 = int(share_ln and all(t.dtype is torch.bfloat16 and t.device == dev and t.is_contiguous()
+                                                and t.data_ptr() % 16 == 0 for t in ln))
+            self.ln = tuple(t.detach() if self.ln_bf16 else t.detach().to(dev, torch.float32).contiguous() for t in ln)
+        self.shared = share_ln and all(a is None or a.data_ptr() == b.data_ptr() for a, b in zip(given, [*shifts, *(self.ln or ())]))
         self.ln_eps = float(ln_eps)
         self.shift_ptrs = tuple(_ptr(t) for t in (self.shift_q, self.shift_k, self.shift_v))
         self.ln_ptrs = None if self.ln is None else tuple(t.data_ptr() for t in self.ln)
@@ -264,6 +274,27 @@ def rotary_tables_arg(position_embeddings, B: int, T: int, D: int, dev):
     return cs[0], cs[1], n > 1
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary, by a copy where it is not."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _first_values(v_first: torch.Tensor, B: int, T: int, width: int, dev) -> torch.Tensor:
+    """The first layer's values [B,T,width] as the value residual's kernels read them: broadcast, bf16, contiguous, aligned."""
+    if v_first.device != dev:
+        raise RuntimeError(f"v_first must be on {dev}, got {v_first.device}")
+    if v_first.shape != (B, T, width):
+        v_first = v_first.expand(B, T, width)
+    return _aligned(v_first.to(torch.bfloat16))
+
+
+def _prev_rows(prev, B: int, dev) -> list[torch.Tensor]:
+    """The cached rows [B,1,width] of the previous token as the prologue kernel reads them."""
+    return [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.stride(2) == 1 and t.stride(0) % 8 == 0
+            and t.stride(0) >= t.size(2) and t.data_ptr() % 16 == 0 else _aligned(t.to(dev, torch.bfloat16).reshape(B, 1, -1)) for t in prev]
+
+
 def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin, gate_lin, position_embeddings, prev, value_residual,
                   v_last):
     """The C argument block of the prologue and the tensors it points into (see ``prologue_forward``)."""
@@ -272,7 +303,7 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
     D, Hq, Hkv = cfg.head_dim, cfg.n_q_heads, cfg.n_kv_heads
     dev = q_lin.device
     keep = []
-    arg = _lib.KvmPrologue()
+    arg = _lib.KvmPrologueExt()
     arg.q_lin, arg.k_lin, arg.v_lin = q_lin.data_ptr(), k_lin.data_ptr(), v_lin.data_ptr()
     arg.q_stride_t, arg.k_stride_t, arg.v_stride_t = (
         _token_stride(t, B, T, h * D, n) for n, t, h in (("q", q_lin, Hq), ("k", k_lin, Hkv), ("v", v_lin, Hkv)))
@@ -282,9 +313,10 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
             keep.append(gate_lin)
         arg.gate_lin, arg.gate_stride_t = gate_lin.data_ptr(), _token_stride(gate_lin, B, T, Hkv, "gate")
     if value_residual is not None:
-        v_first, v_gate, v_gate0 = (t.to(torch.bfloat16).contiguous() for t in value_residual)
-        if v_first.numel() != B * T * Hkv * D or v_gate.numel() != B * T * Hkv * D or v_gate0.numel() != Hkv * D:
-            raise ValueError(f"value residual: v_first and v_gate must have {Hkv * D} values per token, v_gate0 {Hkv * D}")
+        v_first = _first_values(value_residual[0], B, T, Hkv * D, dev)
+        v_gate, v_gate0 = (_aligned(t.to(dev, torch.bfloat16)) for t in value_residual[1:])
+        if v_gate.numel() != B * T * Hkv * D or v_gate0.numel() != Hkv * D:
+            raise ValueError(f"value residual: v_gate must have {Hkv * D} values per token, v_gate0 {Hkv * D}")
         keep += [v_first, v_gate, v_gate0]
         arg.v_first, arg.v_gate, arg.v_gate0 = v_first.data_ptr(), v_gate.data_ptr(), v_gate0.data_ptr()
         if v_last is not None:
@@ -292,15 +324,14 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
     if pro.shift_q is not None:
         arg.shift_q, arg.shift_k, arg.shift_v = pro.shift_ptrs
         if prev is not None and all(t is not None for t in prev):
-            pv = [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.stride(2) == 1 and t.stride(0) % 8 == 0
-                  and t.data_ptr() % 16 == 0 else t.to(dev, torch.bfloat16).reshape(B, 1, -1).contiguous() for t in prev]
+            pv = _prev_rows(prev, B, dev)
             keep += pv
             arg.prev_q, arg.prev_k, arg.prev_v = (t.data_ptr() for t in pv)
             if B > 1:
                 arg.prev_q_stride_b, arg.prev_k_stride_b, arg.prev_v_stride_b = (t.stride(0) for t in pv)
     if pro.ln is not None:
         arg.ln_q_w, arg.ln_q_b, arg.ln_k_w, arg.ln_k_b = pro.ln_ptrs
-        arg.ln_qk_eps = pro.ln_eps
+        arg.ln_qk_eps, arg.ln_bf16 = pro.ln_eps, pro.ln_bf16
     if position_embeddings is not None:
         cos, sin, own = rotary_tables_arg(position_embeddings, B, T, D, dev)
         keep += [cos, sin]
@@ -340,7 +371,7 @@ def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tens
         if runner.batch != B or runner.plan.seq_len != T:
             raise ValueError("runner was built for another batch or sequence length")
         ws_ptr, ws_bytes, ver_rows = runner.ws.data_ptr(), runner.ws_bytes, runner.plan.total_version_rows
-    rc = _lib.load().kvm_prologue_forward(C.byref(params.c), B, T, C.byref(arg), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+    rc = _lib.load().kvm_prologue_forward_ext(C.byref(params.c), B, T, C.byref(arg), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                           gate.data_ptr(), ver_rows, ws_ptr, ws_bytes, _stream_ptr(dev))
     if rc:
         _lib.check(rc)
@@ -349,9 +380,11 @@ def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tens
 
 
 def project(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
-    """[rows, width] bf16 (at most 64 rows, inner stride 1) times the transposed weights, side by side:
+    """[rows, width] bf16 (at most ``PROJECT_ROWS_MAX`` rows) times the transposed weights, side by side:
     [rows, sum of the weights' rows], in one launch."""
     rows, width = x.shape
+    if x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < width or x.data_ptr() % 16:
+        x = x.clone(memory_format=torch.contiguous_format)
     n = len(weights)
     sizes = [w.size(0) for w in weights]
     cols = (sum(sizes) + 7) // 8 * 8  # (16-byte aligned rows)
@@ -770,7 +803,7 @@ class KvmDecodeCache:
             return out
         lib, stream = _lib.load(), _stream_ptr(self.device)
         Cn, WC = cfg.chunk_len, self.ring_capacity
-        span = _lib.SPAN_COLUMNS // (cfg.n_q_heads // cfg.n_kv_heads)
+        span = max(1, _lib.SPAN_COLUMNS // (cfg.n_q_heads // cfg.n_kv_heads))  # (more query heads: refused by the library)
         tl, sl = self.total_len_h, self.state_len_h
         self._quiet = 0
         piece = 128  # (a token's place inside a piece fits a byte)
@@ -927,9 +960,8 @@ class TokenCall:
             p.shift_q, p.shift_k, p.shift_v = pro.shift_ptrs
         if pro.ln is not None:
             p.ln_q_w, p.ln_q_b, p.ln_k_w, p.ln_k_b = pro.ln_ptrs
-            p.ln_qk_eps = pro.ln_eps
+            p.ln_qk_eps, p.ln_bf16 = pro.ln_eps, pro.ln_bf16
         self._views = (C.addressof(c), c.decode, p, c.weights, c.weight_rows)
-        self._finals = (None, None, None)
 
     @staticmethod
     def of(cache: KvmDecodeCache, params: LayerParams, pro: PrologueParams) -> "TokenCall":
@@ -938,45 +970,34 @@ class TokenCall:
             t = cache._token = TokenCall(cache, params, pro)
         return t
 
-    def produced(self, finals):
-        """The tensors handed out as the token's cached rows: the next call recognises them."""
-        self._finals = finals
-
     def run(self, x, weights, v_gate2, c_proj, gated, residual, position_embeddings, prev):
         """x [B,1,hidden]; returns (y [B,1,out], projections [B,1,..], last values behind the residual or None)."""
         cache, cfg = self.cache, self.cache.cfg
         addr, decode, p, w, rows = self._views
         c, B, dev = self.c, cache.batch, cache.device
         keep = []
-        if not x.is_contiguous():
-            x = x.contiguous()
+        x = _aligned(x)
         cos = sin = None
         if position_embeddings is not None:
             cos, sin, own = rotary_tables_arg(position_embeddings, B, 1, cfg.head_dim, x.device)
+            if (cos.data_ptr() | sin.data_ptr()) % 16:
+                raise ValueError("rotary tables must be 16-byte aligned")
             p.cos, p.sin, p.rope_stride_b = cos.data_ptr(), sin.data_ptr(), cfg.head_dim if own else 0
         else:
             p.cos, p.sin = None, None
         v_last = None
         if residual is not None:
             v_first, v_gate0 = residual
-            if v_first.dtype is not torch.bfloat16 or not v_first.is_contiguous():
-                v_first = v_first.to(torch.bfloat16).contiguous()
-            if v_first.numel() != B * cfg.n_kv_heads * cfg.head_dim:
-                raise ValueError(f"value residual: v_first must have {cfg.n_kv_heads * cfg.head_dim} values per token")
-            keep.append(v_first)
+            v_first = _first_values(v_first, B, 1, cfg.n_kv_heads * cfg.head_dim, x.device)
+            v_gate0 = _aligned(v_gate0.to(x.device))
+            keep += [v_first, v_gate0]
             v_last = torch.empty(B, 1, cfg.n_kv_heads * cfg.head_dim, device=x.device, dtype=torch.bfloat16)
             p.v_first, p.v_gate0, p.v_last = v_first.data_ptr(), v_gate0.data_ptr(), v_last.data_ptr()
         if self.pro.shift_q is not None:
-            mine = self._finals
-            if prev[0] is not None and prev[0] is mine[0] and prev[1] is mine[1] and prev[2] is mine[2]:
-                pv = prev
-            elif all(t is not None for t in prev):
-                pv = [t.to(x.device, torch.bfloat16).reshape(B, 1, -1).contiguous() for t in prev]
-            else:
-                pv = None
-            if pv is None:
+            if any(t is None for t in prev):
                 p.prev_q, p.prev_k, p.prev_v = None, None, None
             else:
+                pv = _prev_rows(prev, B, x.device)
                 keep.append(pv)
                 p.prev_q, p.prev_k, p.prev_v = pv[0].data_ptr(), pv[1].data_ptr(), pv[2].data_ptr()
                 if B > 1:

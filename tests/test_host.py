@@ -190,3 +190,34 @@ def test_mixer_error_conventions():
         SequenceMixer(bad, 0)._desired_state_len(100, 100, 0)
     # every parameter carries the optimizer label the reference's trainer asserts on
     assert all(getattr(p, "label", None) for p in m.parameters())
+
+
+def test_layouts_that_kernels_cannot_read_are_copied_or_refused():
+    """What reaches the one-call paths: a 16-byte boundary, the device of the call, four dimensions, a broadcast first value."""
+    flat = torch.arange(1 + 2 * 1 * 64).bfloat16()
+    off = flat[1:].view(2, 1, 64)
+    for t in (ops._aligned(off), ops._first_values(off, 2, 1, 64, off.device), *ops._prev_rows((off,), 2, off.device)):
+        assert t.data_ptr() % 16 == 0 and torch.equal(t, off)
+    wide = torch.randn(2, 1, 72).bfloat16()
+    assert ops._prev_rows((wide[..., :64],), 2, wide.device)[0].data_ptr() == wide.data_ptr()  # a range of wider rows stays one
+    one = torch.randn(1, 1, 64)
+    assert torch.equal(ops._first_values(one, 3, 1, 64, one.device), one.bfloat16().expand(3, 1, 64))
+    with pytest.raises(RuntimeError):
+        ops._first_values(torch.randn(2, 1, 32), 2, 1, 64, torch.device("cpu"))
+    with pytest.raises(RuntimeError):
+        ops._first_values(one, 1, 1, 64, torch.device("cuda", 0))
+    with pytest.raises(ValueError):
+        ops._fill_tensor4(_lib.KvmTensor4(), torch.zeros(2, 2, 2), "v")
+
+
+def test_prologue_parameters_are_read_where_they_are():
+    """Kept parameters are views: what is written to a parameter through ``.data`` is seen; fp32 ones are laid out per call."""
+    cfg, m = _mixer_from_fixture(load_fixture("powerlaw_bf16"))
+    pro = m._prologue_params_kept(torch.device("cpu"))
+    assert pro.shared and pro.ln_bf16 and m._prologue_params_kept(torch.device("cpu")) is pro
+    m.ln_q.weight.data.add_(1.0)
+    assert torch.equal(pro.ln[0], m.ln_q.weight) and pro.ln_ptrs[0] == m.ln_q.weight.data_ptr()
+    m.ln_q.float()
+    a = m._prologue_params_kept(torch.device("cpu"))
+    assert not a.shared and not a.ln_bf16 and m._prologue_params_kept(torch.device("cpu")) is not a
+    assert not ops.PrologueParams("cpu", ln_q=m.ln_k, ln_k=m.ln_k).ln_bf16  # a caller's own block keeps its copy
