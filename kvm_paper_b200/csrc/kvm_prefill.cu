@@ -55,7 +55,7 @@ kvm_prepare_keys_kernel(LayerDev L, Tensor4 k, Tensor4 gate, bf16* __restrict__ 
 // One CTA (or a cluster of up to 4 CTAs) per kv row walks the whole prompt: initial memory, then one update per token block.  The
 // attention view of the memory is kept in a row pool with per-version index tables (see ViewStore);
 // after the last update the final view is gathered into `mem.k_attn` / `mem.v_attn`.
-template <int D, int NT, bool SB>
+template <int D, int NT, bool SB, bool WIDE>
 __global__ void __launch_bounds__(NT, 1)
 kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate, const kvm_update_plan* __restrict__ plan,
                  int n_plan, MemoryDev mem, bf16* pool_k, bf16* pool_v, long long pool_rows, int* ver_idx,
@@ -74,11 +74,11 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
   L.ln_b = ln_s + D;
   __syncthreads();
   UpdateSmem<D> s;
-  s.carve(smem_raw, L.C, mem.capacity, SB);
+  s.carve(smem_raw, L.C, mem.capacity, SB, WIDE);
   s.status = status;
   bool has_tmem = false;
-  if constexpr (SB && D == 128 && NT == 512) {
-    if (L.C == 128 || L.C == 256) {  // tcgen05 routing scan: its two barriers and tensor memory, once per kernel
+  if constexpr ((SB || WIDE) && D == 128 && NT == 512) {
+    if (WIDE || L.C == 128 || L.C == 256) {  // tcgen05 routing scan: its two barriers and tensor memory, once per kernel
       if (threadIdx.x == 0) {
         tc::mbar_init(&s.bars[0], 1);
         tc::mbar_init(&s.bars[1], 1);
@@ -165,7 +165,7 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
       const bool has_next = u + 1 < n_plan;
       src.next_k = has_next ? src.k + (size_t)C * D : nullptr;
       src.next_v = has_next ? v.row(b, h, (long long)(u + 1) * C) : nullptr;
-      memory_update<D, NT, SB, true>(L, src, m, view, mem.capacity, pl.state_before, pl.n_append, pk,
+      memory_update<D, NT, SB, true, WIDE>(L, src, m, view, mem.capacity, pl.state_before, pl.n_append, pk,
                                route ? route + ((size_t)row * n_plan + u) * C : nullptr, s, nc, crank);
     }
   }
@@ -471,8 +471,13 @@ static cudaError_t launch_prefill(const LayerDev& L, int batch, long long T, Ten
     if (e != cudaSuccess) return e;
   } else if (phases & KVM_PREFILL_CHAIN) {
     const bool sb = update_block_fits_smem<D>(L.C, mem.capacity);
-    const size_t smem_u = UpdateSmem<D>::bytes(L.C, mem.capacity, sb);
-    auto kern = sb ? kvm_chain_kernel<D, NT, true> : kvm_chain_kernel<D, NT, false>;
+    auto kern = sb ? kvm_chain_kernel<D, NT, true, false> : kvm_chain_kernel<D, NT, false, false>;
+    bool wide = false;
+    if constexpr (D == 128) {
+      wide = update_scan_wide<D>(L.C, mem.capacity);
+      if (wide) kern = kvm_chain_kernel<D, NT, false, true>;
+    }
+    const size_t smem_u = UpdateSmem<D>::bytes(L.C, mem.capacity, sb, wide);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_u);
     if (e != cudaSuccess) return e;
     // A cluster of CTAs per kv row when the GPU has room for it (the chain is latency-bound per row): the largest

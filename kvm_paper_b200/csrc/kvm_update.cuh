@@ -25,6 +25,8 @@ namespace kvm {
 
 constexpr int kScanTile = 64;  // memory rows per shared-memory tile of the routing GEMM
 constexpr int kMaxCluster = 4; // CTAs that may share one kv row
+constexpr int kWideTokens = 256; // wide scan: tokens per pass ...
+constexpr int kWideTile = 128;   // ... and memory rows per tile
 constexpr int kDirectRows = 4; // up to this many appended rows are scored with plain dot products
 
 struct TokenSrc {  // the C tokens consumed by one update; token t at base + t*stride
@@ -69,7 +71,7 @@ __host__ __device__ constexpr int scan_tile_stride() { return D + 8; }
 // Shared-memory carve-up of the update (sizes depend on C, the memory capacity and SB).
 template <int D>
 struct UpdateSmem {
-  bf16* btile;   // [2][kScanTile][D+8]
+  bf16* btile;   // [2][kScanTile][D+8]; wide scan: the token operand [kWideTokens][D] and two tiles [kWideTile][D]
   bf16* pk_s;    // [C][D+8]   (SB only)
   bf16* v_s;     // [C][D]     (SB only)
   float* g_s;    // [C] gates
@@ -95,17 +97,20 @@ struct UpdateSmem {
   uint32_t tc_tiles;  // tiles issued so far by the tcgen05 scan: tile n signals barrier n%2 with phase parity (n/2)%2
   int* status;     // device status word (a bounded wait that ran out is reported here), or null
   static constexpr int kTokenArrays = 13 + 3 * kMaxCluster;
-  __host__ __device__ static size_t bytes(int C, int capacity, bool sb) {
-    size_t b = (size_t)2 * kScanTile * scan_tile_stride<D>() * sizeof(bf16);
+  __host__ __device__ static size_t tile_bytes(bool wide) {
+    return wide ? (size_t)(kWideTokens + 2 * kWideTile) * D * sizeof(bf16) : (size_t)2 * kScanTile * scan_tile_stride<D>() * sizeof(bf16);
+  }
+  __host__ __device__ static size_t bytes(int C, int capacity, bool sb, bool wide = false) {
+    size_t b = tile_bytes(wide);
     if (sb) b += (size_t)C * (D + 8) * sizeof(bf16) + (size_t)C * D * sizeof(bf16);
     b += (size_t)C * 4 * kTokenArrays;
     b += (size_t)((capacity + 3) / 4 * 4) * 4;
     b += 36 * 4 + 32;
     return b;
   }
-  __device__ void carve(unsigned char* base, int C, int capacity, bool sb) {
+  __device__ void carve(unsigned char* base, int C, int capacity, bool sb, bool wide = false) {
     btile = reinterpret_cast<bf16*>(base);
-    base += (size_t)2 * kScanTile * scan_tile_stride<D>() * sizeof(bf16);
+    base += tile_bytes(wide);
     pk_s = v_s = nullptr;
     if (sb) {
       pk_s = reinterpret_cast<bf16*>(base); base += (size_t)C * (D + 8) * sizeof(bf16);
@@ -136,6 +141,12 @@ constexpr size_t kSmemLimit = 225 * 1024;  // dynamic part: the kernels also hol
 template <int D>
 __host__ __device__ inline bool update_block_fits_smem(int C, int capacity) {
   return UpdateSmem<D>::bytes(C, capacity, true) <= kSmemLimit;
+}
+// Blocks that are not staged but are whole accumulators of 128 tokens: the routing scan goes to tcgen05 a part of the
+// block at a time (see scan_memory_wide), as long as its operands fit next to the table of the memory rows.
+template <int D>
+__host__ __device__ inline bool update_scan_wide(int C, int capacity) {
+  return D == 128 && C % 128 == 0 && !update_block_fits_smem<D>(C, capacity) && UpdateSmem<D>::bytes(C, capacity, false, true) <= kSmemLimit;
 }
 
 // A cluster of up to kMaxCluster CTAs may share one kv row: the memory rows of the routing scan and the
@@ -338,7 +349,7 @@ __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, i
               const int r = e >> 1;
               const int n = tile_base + (nt + h) * 8 + t * 2 + (e & 1);
               if (n < n_end) {
-                if (want_app) amax[r] = fmaxf(amax[r], bf16_round(cp[h][e]));
+                if (want_app) amax[r] = fmaxf(amax[r], cp[h][e]);  // (rounded below: rounding keeps the order)
                 if (n >= protected_rows && (cg[h][e] > bbest[r] || bidx[r] < 0)) {
                   bbest[r] = cg[h][e];
                   bidx[r] = n;
@@ -366,7 +377,7 @@ __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, i
         }
         if (t == 0) {
           const int row = mt * 16 + g + r * 8;
-          if (want_app) s.app[row] = amax[r];
+          if (want_app) s.app[row] = bf16_round(amax[r]);
           if (bidx[r] >= 0 && (s.idx[row] < 0 || bbest[r] > s.best[row])) {
             s.best[row] = bbest[r];
             s.idx[row] = bidx[r];
@@ -467,11 +478,11 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
         if (op == 0) {
           if (full) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) am[c & 3] = fmaxf(am[c & 3], bf16_round(__uint_as_float(r[c])));
+            for (int c = 0; c < 32; ++c) am[c & 3] = fmaxf(am[c & 3], __uint_as_float(r[c]));
           } else {
 #pragma unroll
             for (int c = 0; c < 32; ++c)
-              if (n0 + c < n_end) am[c & 3] = fmaxf(am[c & 3], bf16_round(__uint_as_float(r[c])));
+              if (n0 + c < n_end) am[c & 3] = fmaxf(am[c & 3], __uint_as_float(r[c]));
           }
         } else {
           if (full) {
@@ -559,7 +570,7 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
   if (epi) {
     const int row = mt * 128 + (warp & 3) * 32 + lane;
     if (op == 0) {
-      s.app[row] = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
+      s.app[row] = bf16_round(fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3])));  // (rounding keeps the order)
     } else {
       float bbest = bb[0];
       int bidx = bi[0];
@@ -576,6 +587,188 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
     }
   }
   __syncthreads();
+  return true;
+}
+
+// The same routing GEMM for blocks that do not fit shared memory (D = 128, C a multiple of 128; prepared keys in global
+// memory).  Same contract as scan_memory_tc.  A pass takes up to 256 tokens and one operand (prepared keys for the novelty,
+// gated keys for the logits) through all memory rows, in tiles of 128 rows: at N = 128 an MMA reads its two operands from
+// shared memory as fast as it multiplies them (64 cycles, N = 64: 48 for half of the work).  Two tiles and two accumulator
+// buffers of 2 x 128 columns: while the tensor core works on one tile, all 16 warps read the other accumulators back (warp
+// w: lanes 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..) and the tile behind it is fetched.  The memory
+// rows are read from L2 once per pass; a block of 512 tokens that only merges takes two passes.
+// Block 512, up to 4096 rows, four CTAs per kv row: an update's scan takes 95 K cycles; as warp-level MMAs, which read their
+// B fragments from shared memory once per 16 tokens, 227 K (262144 tokens, 32 heads: 106.8 -> 64.2 ms).
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+template <int D, int NT>
+__device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_keys, int C, const bf16* __restrict__ k_attn,
+                                              const int* slots, int n_begin, int n_end, bool want_app, int protected_rows,
+                                              UpdateSmem<D>& s) {
+  static_assert(D == 128 && NT == 512, "wide routing scan: head dimension 128, 16 warps");
+  constexpr int TN = kWideTile;
+  constexpr uint32_t kWaitLimit = 1u << 16;
+  constexpr uint32_t kTileBytes = TN * 256, kHalfA = kWideTokens * 128, kHalfB = TN * 128;
+  constexpr uint32_t idesc = tc::make_idesc(128, TN, 0, 0);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_tiles = (n_end - n_begin + TN - 1) / TN;
+  if (n_tiles <= 0) return true;
+  unsigned char* A = reinterpret_cast<unsigned char*>(s.btile);  // [2 k-halves][kWideTokens][128 B], swizzled
+  unsigned char* B = A + 2 * kHalfA;                              // two tiles, [2 k-halves][TN][128 B] each
+  const bool issuer = tid == NT - 32;
+  const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64;
+  const uint32_t t_lane = s.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * TN + col0);
+  bool ok = true;
+
+  auto load_tile = [&](int it) {
+    unsigned char* dst = B + (size_t)(it & 1) * kTileBytes;
+    const int row0 = n_begin + it * TN;
+#pragma unroll
+    for (int i = 0; i < TN * 16 / NT; ++i) {
+      const int c = tid + i * NT, r = c >> 4, cc = c & 15, row = row0 + r;
+      const bool in = row < n_end;
+      const int slot = in ? (slots ? slots[row] : row) : 0;
+      cp_async16(dst + (cc >> 3) * kHalfB + r * 128 + (((cc & 7) ^ (r & 7)) << 4), k_attn + (size_t)slot * D + cc * 8, in ? 16 : 0);
+    }
+    cp_async_commit();
+  };
+
+  for (int m0 = 0; m0 < C; m0 += kWideTokens) {
+    const int n_mt = min(kWideTokens, C - m0) / 128;
+    for (int op = want_app ? 0 : 1; op < 2; ++op) {  // 0: prepared keys (novelty), 1: gated keys (merge logits)
+      const uint32_t g0 = s.tc_tiles;
+      for (int it = 0; it < 2 && it < n_tiles; ++it) load_tile(it);
+      if (op == 0 || !want_app || gate_keys) {  // (without gates both operands are the same)
+        uint4 u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int c = tid + i * NT;
+          if (i < n_mt * 4) u[i] = *reinterpret_cast<const uint4*>(blk.pk + (size_t)(m0 + (c >> 4)) * blk.pk_st + (c & 15) * 8);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i >= n_mt * 4) break;
+          const int c = tid + i * NT, r = c >> 4, cc = c & 15;
+          if (op == 1 && gate_keys) {
+            const __nv_bfloat162 g2 = __float2bfloat162_rn(blk.g[m0 + r]);
+            u[i].x = mul_bf16x2(u[i].x, g2);
+            u[i].y = mul_bf16x2(u[i].y, g2);
+            u[i].z = mul_bf16x2(u[i].z, g2);
+            u[i].w = mul_bf16x2(u[i].w, g2);
+          }
+          *reinterpret_cast<uint4*>(A + (cc >> 3) * kHalfA + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = u[i];
+        }
+      }
+      auto issue_mmas = [&](int it) {
+        tc::tc_fence_after_sync();
+        const uint64_t da0 = tc::make_desc(tc::smem_u32(A), 16, 1024);
+        const uint64_t db0 = tc::make_desc(tc::smem_u32(B) + (uint32_t)(it & 1) * kTileBytes, 16, 1024);
+        for (int m = 0; m < n_mt; ++m) {
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks)
+            tc::mma_ss(s.tmem + (uint32_t)((it & 1) * 256 + m * TN),
+                       da0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfA + (uint32_t)m * 128 * 128 + (uint32_t)(ks & 3) * 32u) >> 4),
+                       db0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfB + (uint32_t)(ks & 3) * 32u) >> 4), idesc, ks > 0);
+        }
+        tc::mma_commit_own_cta(&s.bars[(g0 + it) & 1]);
+      };
+      cp_async_wait<0>();
+      tc::fence_proxy_async();
+      __syncthreads();
+      if (issuer)
+        for (int it = 0; it < 2 && it < n_tiles; ++it) issue_mmas(it);
+
+      // Running maximum of this thread's columns.  The read-back is bound by the rate of comparisons and selections (half
+      // of an add's): eight columns at a time go through three-input maxima, and only the first column of the group that
+      // holds the maximum is noted, with the group's eight values, among which the column is looked up at the end.
+      float best = -INFINITY, held[8];
+      int at = -1;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) held[j] = -INFINITY;
+      const bool epi = mt < n_mt;
+      for (int it = 0; it < n_tiles; ++it) {
+        ok = ok && tc::mbar_wait_limit(&s.bars[(g0 + it) & 1], ((g0 + it) >> 1) & 1, kWaitLimit);
+        const bool more = it + 2 < n_tiles;
+        if (more) load_tile(it + 2);  // (the MMAs of tile `it` are done with its buffer)
+        if (epi) {
+          tc::tc_fence_after_sync();
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int n0 = n_begin + it * TN + col0 + half * 32;
+            if (n0 >= n_end) continue;
+            uint32_t r[32];
+            tc::tmem_ld32(t_lane + (uint32_t)((it & 1) * 256 + half * 32), r);
+            tc::tmem_ld_wait();
+            const int lo = op == 0 ? 0 : protected_rows;
+            if (n0 + 32 > n_end || n0 < lo) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c)
+                if (n0 + c >= n_end || n0 + c < lo) r[c] = 0xff800000u;  // -inf
+            }
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) {
+              float x[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[c + j]);
+              const float m = fmaxf(max3(max3(x[0], x[1], x[2]), x[6], x[7]), max3(x[3], x[4], x[5]));
+              if (op == 0) {
+                best = fmaxf(best, m);
+              } else if (m > best) {
+                best = m;
+                at = n0 + c;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) held[j] = x[j];
+              }
+            }
+          }
+          tc::tc_fence_before_sync();
+        }
+        if (more) {
+          cp_async_wait<0>();
+          tc::fence_proxy_async();
+          __syncthreads();  // tile it + 2 is complete, the accumulators of tile `it` have been read
+          if (issuer) issue_mmas(it + 2);
+        }
+      }
+      s.tc_tiles = g0 + (uint32_t)n_tiles;
+      if (!__syncthreads_and(ok ? 1 : 0)) return false;
+      // the column inside the group, then the two threads of a token (columns 0..63 and 64..127 of every tile), who
+      // exchange through a tile's buffer
+      float bv = op == 0 ? bf16_round(best) : best;  // (rounding keeps the order)
+      int bi = at;
+      if (op == 1 && at >= 0) {
+#pragma unroll
+        for (int j = 7; j >= 0; --j)
+          if (held[j] == best) bi = at + j;
+      }
+      if (op == 1 && at < 0 && col0 == 0 && max(n_begin, protected_rows) < n_end) bi = max(n_begin, protected_rows);  // (no number above -inf)
+      float* xv = reinterpret_cast<float*>(B);
+      int* xi = reinterpret_cast<int*>(B) + kWideTokens;
+      const int tok = mt * 128 + (warp & 3) * 32 + lane;
+      if (epi && col0 != 0) {
+        xv[tok] = bv;
+        xi[tok] = bi;
+      }
+      __syncthreads();
+      if (epi && col0 == 0) {
+        const float ov = xv[tok];
+        const int oi = xi[tok], row = m0 + tok;
+        if (op == 0) {
+          s.app[row] = fmaxf(bv, ov);
+        } else {
+          if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
+          if (bi >= 0 && (s.idx[row] < 0 || bv > s.best[row])) {
+            s.best[row] = bv;
+            s.idx[row] = bi;
+          }
+        }
+      }
+      __syncthreads();  // (the next pass fetches its first tiles over the exchange buffer)
+    }
+  }
   return true;
 }
 
@@ -598,7 +791,7 @@ struct ViewStore {
 // their source.  `route_out` ([C] int32, may be null) receives the decision for every token.
 // Requires C <= NT.
 // PKR: `src.k` already holds prepared keys (a parallel pre-pass ran the LayerNorm), phase 1 is skipped.
-template <int D, int NT, bool SB, bool PKR = false>
+template <int D, int NT, bool SB, bool PKR = false, bool WIDE = false>
 __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const MemoryRowPtrs& mem, ViewStore& view, int capacity,
                               int S_before, int n_append, bf16* pk_scr, int* route_out, UpdateSmem<D>& s, int nc = 1,
                               int crank = 0) {
@@ -613,9 +806,10 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
   const int n_merge = C - n_append;
   const bool pool = view.cur != nullptr;
   // this CTA scans the tiles [crank, crank+1) * n_tiles / nc of the old memory
-  const int n_tiles_all = (S_before + kScanTile - 1) / kScanTile;
-  const int scan_b = min(S_before, (crank * n_tiles_all / nc) * kScanTile);
-  const int scan_e = min(S_before, ((crank + 1) * n_tiles_all / nc) * kScanTile);
+  constexpr int kTile = WIDE ? kWideTile : kScanTile;
+  const int n_tiles_all = (S_before + kTile - 1) / kTile;
+  const int scan_b = min(S_before, (crank * n_tiles_all / nc) * kTile);
+  const int scan_e = min(S_before, ((crank + 1) * n_tiles_all / nc) * kTile);
   // routing scan of the old memory on tcgen05: the prepared keys are staged in the swizzled operand layout, the
   // gated operand borrows the value staging area (the values are fetched after the scan)
   bool use_tc = false;
@@ -709,6 +903,15 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
         scanned = scan_memory_tc<D, NT>(blk, L.gate_keys != 0, C, view.k, view.cur, scan_b, scan_e, n_append > 0, protected_rows,
                                         s, tiles_in_flight);
         if (!scanned) {  // report, and stay on the warp-level path for the rest of this kernel
+          if (tid == 0 && s.status) atomicExch(s.status, KVM_ERR_DEVICE_TIMEOUT);
+          s.use_tc = false;
+        }
+      }
+    }
+    if constexpr (WIDE) {
+      if (s.use_tc) {
+        scanned = scan_memory_wide<D, NT>(blk, L.gate_keys != 0, C, view.k, view.cur, scan_b, scan_e, n_append > 0, protected_rows, s);
+        if (!scanned) {
           if (tid == 0 && s.status) atomicExch(s.status, KVM_ERR_DEVICE_TIMEOUT);
           s.use_tc = false;
         }
@@ -893,7 +1096,38 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
   __syncthreads();
   bool is_leader = false;
   int ltok = 0;  // the token this thread leads (valid if is_leader)
-  {
+  if constexpr (WIDE) {
+    // A table over the memory rows (where the scan's tiles were): (first token + 1) << 16 | tokens so far.  Tokens of a warp
+    // with the same target are matched, then the warps enter their counts one after the other.  Block 512: 26 K -> 6 K cycles
+    // against every token's comparison with every other, which blocks of 256 and less do as fast with their two threads per
+    // token.  (The memory rows fit: they are fewer than kSmemLimit / 4 - tile bytes, the tiles 32768 ints.)
+    int* tab = reinterpret_cast<int*>(s.btile);
+    for (int i = tid; i < S_after; i += NT) tab[i] = 0;
+    const int mine = tid < C ? s.idx[tid] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, mine >= 0 ? mine : -2 - lane);
+    const int head = __ffs(same) - 1;  // the lane that enters for all of them
+    int base = 0;
+    __syncthreads();
+    for (int w = 0; w < (C + 31) / 32; ++w) {
+      if (warp == w && mine >= 0 && lane == head) {
+        base = tab[mine];
+        tab[mine] = (base == 0 ? (tid + 1) << 16 : base) + __popc(same);
+      }
+      __syncthreads();
+    }
+    base = __shfl_sync(0xffffffffu, base, head) & 0xffff;
+    if (mine >= 0) {
+      const int all = tab[mine], ord = base + __popc(same & ((1u << lane) - 1u));
+      s.ord[tid] = ord;
+      s.lead[tid] = (all >> 16) - 1;
+      if (ord == 0) {
+        s.tcnt[tid] = all & 0xffff;
+        s.tstart[tid] = atomicAdd(&s.counters[0], all & 0xffff);
+        is_leader = true;
+        ltok = tid;
+      }
+    }
+  } else {
     // per merged token: how many tokens with the same target come before it, how many there are, which is
     // the first.  With 2C <= NT two threads share a token, each counting over one half of the block.
     const bool pair = 2 * C <= NT;
