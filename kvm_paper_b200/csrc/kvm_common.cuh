@@ -362,7 +362,8 @@ __device__ __forceinline__ void divide_by(float (&x)[N], float n) {
 // Attention view of one memory row: k_attn = LN(k_sum), v_attn = v_sum / max(|v_sum|, 1e-12) * vlen.
 template <int D, int GL = 32>
 __device__ __forceinline__ void refresh_memory_row(const LayerDev& L, RowVec<D, GL> ks, RowVec<D, GL> vs, float vlen,
-                                                   bf16* k_attn_row, bf16* v_attn_row, int gl, bool do_store = true) {
+                                                   bf16* k_attn_row, bf16* v_attn_row, int gl, bool do_store = true,
+                                                   bf16* k_copy = nullptr) {
   layer_norm_row<D, GL>(ks, L.ln_w, L.ln_b, L.ln_eps, gl);
   float n = fmaxf(row_norm<D, GL>(vs), 1e-12f);
   divide_by(vs.x, n);
@@ -370,6 +371,7 @@ __device__ __forceinline__ void refresh_memory_row(const LayerDev& L, RowVec<D, 
   for (int i = 0; i < D / GL; ++i) vs.x[i] *= vlen;
   if (do_store) {
     store_row<D, GL>(ks, k_attn_row, gl);
+    if (k_copy) store_row<D, GL>(ks, k_copy, gl);
     store_row<D, GL>(vs, v_attn_row, gl);
   }
 }

@@ -6,6 +6,7 @@
 //
 // The memory trajectory depends only on k, v and the merge gate (model/kvm_mixer.py:478-487), never on
 // attention outputs, so the chain runs ahead and attention over all blocks runs in parallel behind it.
+#include "kvm_tma_host.cuh"
 #include "kvm_update.cuh"
 
 namespace kvm {
@@ -55,11 +56,12 @@ kvm_prepare_keys_kernel(LayerDev L, Tensor4 k, Tensor4 gate, bf16* __restrict__ 
 // One CTA (or a cluster of up to 4 CTAs) per kv row walks the whole prompt: initial memory, then one update per token block.  The
 // attention view of the memory is kept in a row pool with per-version index tables (see ViewStore);
 // after the last update the final view is gathered into `mem.k_attn` / `mem.v_attn`.
-template <int D, int NT, bool SB, bool WIDE>
+template <int D, int NT, bool SB, int WIDE>
 __global__ void __launch_bounds__(NT, 1)
 kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate, const kvm_update_plan* __restrict__ plan,
                  int n_plan, MemoryDev mem, bf16* pool_k, bf16* pool_v, long long pool_rows, int* ver_idx,
-                 long long ver_rows, bf16* pk_scr, const bf16* __restrict__ pk_all, int* route, int nc, int* status) {
+                 long long ver_rows, bf16* pk_scr, const bf16* __restrict__ pk_all, int* route, int nc, int* status,
+                 const __grid_constant__ CUtensorMap rows_map) {
   extern __shared__ __align__(1024) unsigned char chain_smem[];
   unsigned char* smem_raw = chain_smem;
   // LayerNorm weights in shared memory: almost all of the SM's L1 is carved out as shared memory, so every
@@ -82,6 +84,10 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
       if (threadIdx.x == 0) {
         tc::mbar_init(&s.bars[0], 1);
         tc::mbar_init(&s.bars[1], 1);
+        if (WIDE) {
+          for (int i = 0; i < 3; ++i) tc::mbar_init(&s.bars[3 + i], 1);
+          for (int i = 0; i < 2; ++i) tc::mbar_init(&s.bars[6 + i], NT / 32 - 1);
+        }
         tc::fence_barrier_init();
       }
       if (threadIdx.x < 32) tc::tmem_alloc(reinterpret_cast<uint32_t*>(s.bars + 2), kTcTmemCols);
@@ -95,6 +101,8 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
   }
   const int row = blockIdx.x / nc;     // the nc CTAs of a cluster share one kv row
   const int crank = blockIdx.x % nc;
+  s.rows_map = &rows_map;
+  s.rows_at = row * mem.capacity;
   const int b = row / L.Hkv, h = row % L.Hkv;
   const int tid = threadIdx.x;
   const int C = L.C;
@@ -145,8 +153,10 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
           store_row<D, GL>(vr, m.v_sum + (size_t)t_ * D, gl);
           if (gl == 0) m.vlen[t_] = vl;
         }
-        refresh_memory_row<D, GL>(L, kr, vr, vl, view.k + (size_t)t_ * D, view.v + (size_t)t_ * D, gl, mine);
+        refresh_memory_row<D, GL>(L, kr, vr, vl, view.k + (size_t)t_ * D, view.v + (size_t)t_ * D, gl, mine,
+                                  WIDE && pool ? m.k_attn + (size_t)t_ * D : nullptr);
       }
+      if constexpr (WIDE) fence_all_proxies();
       if (pool)
         for (int i = tid; i < n0; i += NT) s.cur[i] = i;
       view.pool_next = n0;
@@ -165,7 +175,7 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
       const bool has_next = u + 1 < n_plan;
       src.next_k = has_next ? src.k + (size_t)C * D : nullptr;
       src.next_v = has_next ? v.row(b, h, (long long)(u + 1) * C) : nullptr;
-      memory_update<D, NT, SB, true, WIDE>(L, src, m, view, mem.capacity, pl.state_before, pl.n_append, pk,
+      memory_update<D, NT, SB, true, WIDE != 0>(L, src, m, view, mem.capacity, pl.state_before, pl.n_append, pk,
                                route ? route + ((size_t)row * n_plan + u) * C : nullptr, s, nc, crank);
     }
   }
@@ -177,7 +187,8 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
     for (int c = tid + crank * NT; c < S * CPR; c += NT * nc) {
       const int r = c / CPR, cc = c % CPR;
       const size_t src_off = (size_t)s.cur[r] * D + cc * 8;
-      *reinterpret_cast<uint4*>(m.k_attn + (size_t)r * D + cc * 8) = *reinterpret_cast<const uint4*>(view.k + src_off);
+      if (!WIDE)  // (kept in row order all along)
+        *reinterpret_cast<uint4*>(m.k_attn + (size_t)r * D + cc * 8) = *reinterpret_cast<const uint4*>(view.k + src_off);
       *reinterpret_cast<uint4*>(m.v_attn + (size_t)r * D + cc * 8) = *reinterpret_cast<const uint4*>(view.v + src_off);
     }
   }
@@ -471,11 +482,16 @@ static cudaError_t launch_prefill(const LayerDev& L, int batch, long long T, Ten
     if (e != cudaSuccess) return e;
   } else if (phases & KVM_PREFILL_CHAIN) {
     const bool sb = update_block_fits_smem<D>(L.C, mem.capacity);
-    auto kern = sb ? kvm_chain_kernel<D, NT, true, false> : kvm_chain_kernel<D, NT, false, false>;
-    bool wide = false;
+    auto kern = sb ? kvm_chain_kernel<D, NT, true, 0> : kvm_chain_kernel<D, NT, false, 0>;
+    int wide = 0;
+    CUtensorMap rows_map = {};
     if constexpr (D == 128) {
+      const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)rows * mem.capacity}, strides[1] = {(cuuint64_t)D * 2};
+      const cuuint32_t box[2] = {64, (cuuint32_t)kWideTile};
       wide = update_scan_wide<D>(L.C, mem.capacity);
-      if (wide) kern = kvm_chain_kernel<D, NT, false, true>;
+      if ((long long)rows * mem.capacity >= (1LL << 31) || !encode_bf16_map(&rows_map, mem.k_attn, 2, dims, strides, box)) wide = 0;
+      if (wide == 3) kern = kvm_chain_kernel<D, NT, false, 3>;
+      if (wide == 2) kern = kvm_chain_kernel<D, NT, false, 2>;
     }
     const size_t smem_u = UpdateSmem<D>::bytes(L.C, mem.capacity, sb, wide);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_u);
@@ -518,7 +534,7 @@ static cudaError_t launch_prefill(const LayerDev& L, int batch, long long T, Ten
     attr[0].val.clusterDim.x = nc;
     int* ver_arg = versions ? ver_idx : nullptr;
     e = cudaLaunchKernelEx(&cfg, kern, L, T, k, v, gate, plan_dev, n_plan, mem, pool_k, pool_v, pool_rows, ver_arg, ver_rows,
-                           pk_scr, (const bf16*)pk_all, route, nc, status);
+                           pk_scr, (const bf16*)pk_all, route, nc, status, rows_map);
     if (e != cudaSuccess) return e;
   }
   if (!(phases & KVM_PREFILL_ATTENTION)) return cudaSuccess;

@@ -18,6 +18,8 @@
 // way everywhere).
 #pragma once
 
+#include <cuda.h>
+
 #include "kvm_common.cuh"
 #include "kvm_tc.cuh"
 
@@ -71,7 +73,7 @@ __host__ __device__ constexpr int scan_tile_stride() { return D + 8; }
 // Shared-memory carve-up of the update (sizes depend on C, the memory capacity and SB).
 template <int D>
 struct UpdateSmem {
-  bf16* btile;   // [2][kScanTile][D+8]; wide scan: the token operand [kWideTokens][D] and two tiles [kWideTile][D]
+  bf16* btile;   // [2][kScanTile][D+8]; wide scan: the token operand [kWideTokens][D] and `wide` tiles [kWideTile][D]
   bf16* pk_s;    // [C][D+8]   (SB only)
   bf16* v_s;     // [C][D]     (SB only)
   float* g_s;    // [C] gates
@@ -91,38 +93,43 @@ struct UpdateSmem {
   float* xapp;   // [kMaxCluster][C] partial novelty maxima of the CTAs of a cluster
   float* xbest;  // [kMaxCluster][C] partial best logits
   int* xidx;     // [kMaxCluster][C] partial best rows
-  uint64_t* bars;  // [2] mbarriers of the tcgen05 routing scan, [2] = slot for the tensor-memory base address
+  uint64_t* bars;  // [2] mbarriers of the tcgen05 routing scan, [2] = slot for the tensor-memory base address, wide scan:
+                   // [3..5] a tile has landed, [6], [7] an accumulator buffer has been read
+  int tiles;       // tile buffers of the wide scan
+  const CUtensorMap* rows_map;  // wide scan: the key view of all memories, [kv rows * capacity][D] in row order
+  int rows_at;                  // ... and this kv row's first row in it
   uint32_t tmem;   // tensor-memory base (valid when use_tc)
   bool use_tc;     // the tcgen05 routing scan is available (tensor memory allocated, barriers initialised once)
   uint32_t tc_tiles;  // tiles issued so far by the tcgen05 scan: tile n signals barrier n%2 with phase parity (n/2)%2
   int* status;     // device status word (a bounded wait that ran out is reported here), or null
-  static constexpr int kTokenArrays = 13 + 3 * kMaxCluster;
-  __host__ __device__ static size_t tile_bytes(bool wide) {
-    return wide ? (size_t)(kWideTokens + 2 * kWideTile) * D * sizeof(bf16) : (size_t)2 * kScanTile * scan_tile_stride<D>() * sizeof(bf16);
+  static constexpr int kTokenArrays = 12 + 3 * kMaxCluster;
+  // `wide`: tile buffers of the wide scan, 0 = the other scans
+  __host__ __device__ static size_t tile_bytes(int wide) {
+    return wide ? (size_t)(kWideTokens + wide * kWideTile) * D * sizeof(bf16) : (size_t)2 * kScanTile * scan_tile_stride<D>() * sizeof(bf16);
   }
-  __host__ __device__ static size_t bytes(int C, int capacity, bool sb, bool wide = false) {
+  __host__ __device__ static size_t bytes(int C, int capacity, bool sb, int wide = 0) {
     size_t b = tile_bytes(wide);
     if (sb) b += (size_t)C * (D + 8) * sizeof(bf16) + (size_t)C * D * sizeof(bf16);
     b += (size_t)C * 4 * kTokenArrays;
     b += (size_t)((capacity + 3) / 4 * 4) * 4;
-    b += 36 * 4 + 32;
+    b += 36 * 4 + 64;
     return b;
   }
-  __device__ void carve(unsigned char* base, int C, int capacity, bool sb, bool wide = false) {
+  __device__ void carve(unsigned char* base, int C, int capacity, bool sb, int wide = 0) {
     btile = reinterpret_cast<bf16*>(base);
     base += tile_bytes(wide);
+    tiles = wide;
     pk_s = v_s = nullptr;
     if (sb) {
       pk_s = reinterpret_cast<bf16*>(base); base += (size_t)C * (D + 8) * sizeof(bf16);
       v_s = reinterpret_cast<bf16*>(base); base += (size_t)C * D * sizeof(bf16);
     }
-    int** arr[13] = {reinterpret_cast<int**>(&g_s), reinterpret_cast<int**>(&app), reinterpret_cast<int**>(&best),
-                               &idx, &pos, &flag, &ord, &lead, &tcnt, &tstart, &list, &touched, nullptr};
+    int** arr[12] = {reinterpret_cast<int**>(&g_s), reinterpret_cast<int**>(&app), reinterpret_cast<int**>(&best),
+                               &idx, &pos, &flag, &ord, &lead, &tcnt, &tstart, &list, &touched};
     for (int i = 0; i < 12; ++i) {
       *arr[i] = reinterpret_cast<int*>(base);
       base += (size_t)C * 4;
     }
-    base += (size_t)C * 4;  // spare
     xapp = reinterpret_cast<float*>(base); base += (size_t)kMaxCluster * C * 4;
     xbest = reinterpret_cast<float*>(base); base += (size_t)kMaxCluster * C * 4;
     xidx = reinterpret_cast<int*>(base); base += (size_t)kMaxCluster * C * 4;
@@ -130,6 +137,8 @@ struct UpdateSmem {
     counters = reinterpret_cast<int*>(base); base += 36 * 4;
     bars = reinterpret_cast<uint64_t*>(base);
     tmem = 0;
+    rows_map = nullptr;
+    rows_at = 0;
     use_tc = false;
     tc_tiles = 0;
     status = nullptr;
@@ -144,9 +153,13 @@ __host__ __device__ inline bool update_block_fits_smem(int C, int capacity) {
 }
 // Blocks that are not staged but are whole accumulators of 128 tokens: the routing scan goes to tcgen05 a part of the
 // block at a time (see scan_memory_wide), as long as its operands fit next to the table of the memory rows.
+// Returns its tile buffers: three where they fit (a tile is then fetched two tiles ahead), else two, 0 = no such scan.
 template <int D>
-__host__ __device__ inline bool update_scan_wide(int C, int capacity) {
-  return D == 128 && C % 128 == 0 && !update_block_fits_smem<D>(C, capacity) && UpdateSmem<D>::bytes(C, capacity, false, true) <= kSmemLimit;
+__host__ __device__ inline int update_scan_wide(int C, int capacity) {
+  if (D != 128 || C % 128 || update_block_fits_smem<D>(C, capacity)) return 0;
+  for (int n = 3; n >= 2; --n)
+    if (UpdateSmem<D>::bytes(C, capacity, false, n) <= kSmemLimit) return n;
+  return 0;
 }
 
 // A cluster of up to kMaxCluster CTAs may share one kv row: the memory rows of the routing scan and the
@@ -593,21 +606,23 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
 // The same routing GEMM for blocks that do not fit shared memory (D = 128, C a multiple of 128; prepared keys in global
 // memory).  Same contract as scan_memory_tc.  A pass takes up to 256 tokens and one operand (prepared keys for the novelty,
 // gated keys for the logits) through all memory rows, in tiles of 128 rows: at N = 128 an MMA reads its two operands from
-// shared memory as fast as it multiplies them (64 cycles, N = 64: 48 for half of the work).  Two tiles and two accumulator
-// buffers of 2 x 128 columns: while the tensor core works on one tile, all 16 warps read the other accumulators back (warp
-// w: lanes 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..) and the tile behind it is fetched.  The memory
-// rows are read from L2 once per pass; a block of 512 tokens that only merges takes two passes.
-// Block 512, up to 4096 rows, four CTAs per kv row: an update's scan takes 95 K cycles; as warp-level MMAs, which read their
-// B fragments from shared memory once per 16 tokens, 227 K (262144 tokens, 32 heads: 106.8 -> 64.2 ms).
+// shared memory as fast as it multiplies them (64 cycles, N = 64: 48 for half of the work).  Two accumulator buffers of
+// 2 x 128 columns: while the tensor core works on one tile, 15 warps read the other's accumulators back (warp w: lanes
+// 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..; warp 11 also takes those of warp 15).  One thread of warp
+// 15 only copies and issues: MMAs are issued at the pace of the tensor core, so a warp that also reads back holds up all.
+// The memory rows come from the view in row order, which the update writes next to the pool row of every refreshed row: a
+// tile is two TMA copies.  They are read from L2 once per pass; a block of 512 tokens that only merges takes two passes.
+// FIGURES
+// Rows written by this thread -> other threads' TMA copies behind a barrier, and the other way round.
+__device__ __forceinline__ void fence_all_proxies() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 template <int D, int NT>
-__device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_keys, int C, const bf16* __restrict__ k_attn,
-                                              const int* slots, int n_begin, int n_end, bool want_app, int protected_rows,
-                                              UpdateSmem<D>& s) {
+__device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_keys, int C, int n_begin, int n_end, bool want_app,
+                                              int protected_rows, UpdateSmem<D>& s) {
   static_assert(D == 128 && NT == 512, "wide routing scan: head dimension 128, 16 warps");
   constexpr int TN = kWideTile;
   constexpr uint32_t kWaitLimit = 1u << 16;
@@ -617,69 +632,88 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
   const int n_tiles = (n_end - n_begin + TN - 1) / TN;
   if (n_tiles <= 0) return true;
   unsigned char* A = reinterpret_cast<unsigned char*>(s.btile);  // [2 k-halves][kWideTokens][128 B], swizzled
-  unsigned char* B = A + 2 * kHalfA;                              // two tiles, [2 k-halves][TN][128 B] each
-  const bool issuer = tid == NT - 32;
-  const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64;
+  unsigned char* B = A + 2 * kHalfA;                              // s.tiles tiles, [2 k-halves][TN][128 B] each
+  const bool issuer = tid == NT - 32, reads = warp < NT / 32 - 1;
+  const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64, chunks = warp == NT / 32 - 5 ? 4 : 2;  // of 32 columns
   const uint32_t t_lane = s.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * TN + col0);
+  uint64_t *mma_done = s.bars, *landed = s.bars + 3, *is_read = s.bars + 6;
   bool ok = true;
 
-  auto load_tile = [&](int it) {
-    unsigned char* dst = B + (size_t)(it & 1) * kTileBytes;
-    const int row0 = n_begin + it * TN;
-#pragma unroll
-    for (int i = 0; i < TN * 16 / NT; ++i) {
-      const int c = tid + i * NT, r = c >> 4, cc = c & 15, row = row0 + r;
-      const bool in = row < n_end;
-      const int slot = in ? (slots ? slots[row] : row) : 0;
-      cp_async16(dst + (cc >> 3) * kHalfB + r * 128 + (((cc & 7) ^ (r & 7)) << 4), k_attn + (size_t)slot * D + cc * 8, in ? 16 : 0);
-    }
-    cp_async_commit();
+  // issuing thread: tile n of the kernel, memory rows from `row`, -> its buffer (rows past the end belong to nobody or to the
+  // next memory: masked below)
+  auto load_tile = [&](uint32_t n, int row) {
+    unsigned char* dst = B + (size_t)(n % s.tiles) * kTileBytes;
+    uint64_t* bar = landed + n % s.tiles;
+    tc::mbar_arrive_expect_tx(bar, kTileBytes);
+    tc::tma_load_2d(dst, s.rows_map, 0, s.rows_at + row, bar);
+    tc::tma_load_2d(dst + kHalfB, s.rows_map, 64, s.rows_at + row, bar);
   };
+  // this thread's share of the prepared keys of the tokens from m0, fetched while the pass before runs
+  uint4 u[8];
+  auto fetch = [&](int m0) {
+    const int n = min(kWideTokens, C - m0) * 16 / NT;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i < n) {
+        const int c = tid + i * NT;
+        const bf16* p = blk.pk + (size_t)(m0 + (c >> 4)) * blk.pk_st + (c & 15) * 8;
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u[i].x), "=r"(u[i].y), "=r"(u[i].z), "=r"(u[i].w) : "l"(p));
+      }
+    }
+  };
+  fetch(0);
 
   for (int m0 = 0; m0 < C; m0 += kWideTokens) {
     const int n_mt = min(kWideTokens, C - m0) / 128;
     for (int op = want_app ? 0 : 1; op < 2; ++op) {  // 0: prepared keys (novelty), 1: gated keys (merge logits)
       const uint32_t g0 = s.tc_tiles;
-      for (int it = 0; it < 2 && it < n_tiles; ++it) load_tile(it);
+      if (issuer) {
+        fence_all_proxies();  // (rows that other threads have written since the last scan)
+        for (int it = 0; it < s.tiles && it < n_tiles; ++it) load_tile(g0 + it, n_begin + it * TN);
+      }
       if (op == 0 || !want_app || gate_keys) {  // (without gates both operands are the same)
-        uint4 u[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int c = tid + i * NT;
-          if (i < n_mt * 4) u[i] = *reinterpret_cast<const uint4*>(blk.pk + (size_t)(m0 + (c >> 4)) * blk.pk_st + (c & 15) * 8);
-        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           if (i >= n_mt * 4) break;
           const int c = tid + i * NT, r = c >> 4, cc = c & 15;
+          uint4 w = u[i];
           if (op == 1 && gate_keys) {
             const __nv_bfloat162 g2 = __float2bfloat162_rn(blk.g[m0 + r]);
-            u[i].x = mul_bf16x2(u[i].x, g2);
-            u[i].y = mul_bf16x2(u[i].y, g2);
-            u[i].z = mul_bf16x2(u[i].z, g2);
-            u[i].w = mul_bf16x2(u[i].w, g2);
+            w.x = mul_bf16x2(w.x, g2);
+            w.y = mul_bf16x2(w.y, g2);
+            w.z = mul_bf16x2(w.z, g2);
+            w.w = mul_bf16x2(w.w, g2);
           }
-          *reinterpret_cast<uint4*>(A + (cc >> 3) * kHalfA + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = u[i];
+          *reinterpret_cast<uint4*>(A + (cc >> 3) * kHalfA + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = w;
         }
       }
-      auto issue_mmas = [&](int it) {
-        tc::tc_fence_after_sync();
-        const uint64_t da0 = tc::make_desc(tc::smem_u32(A), 16, 1024);
-        const uint64_t db0 = tc::make_desc(tc::smem_u32(B) + (uint32_t)(it & 1) * kTileBytes, 16, 1024);
-        for (int m = 0; m < n_mt; ++m) {
-#pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks)
-            tc::mma_ss(s.tmem + (uint32_t)((it & 1) * 256 + m * TN),
-                       da0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfA + (uint32_t)m * 128 * 128 + (uint32_t)(ks & 3) * 32u) >> 4),
-                       db0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfB + (uint32_t)(ks & 3) * 32u) >> 4), idesc, ks > 0);
-        }
-        tc::mma_commit_own_cta(&s.bars[(g0 + it) & 1]);
-      };
-      cp_async_wait<0>();
       tc::fence_proxy_async();
       __syncthreads();
-      if (issuer)
-        for (int it = 0; it < 2 && it < n_tiles; ++it) issue_mmas(it);
+      if (issuer) {
+        const uint64_t da0 = tc::make_desc(tc::smem_u32(A), 16, 1024);
+        for (int it = 0; it < n_tiles && ok; ++it) {
+          const uint32_t n = g0 + it;
+          if (it >= 2) ok = tc::mbar_wait_limit(&is_read[n & 1], ((n >> 1) - 1) & 1, kWaitLimit);
+          ok = ok && tc::mbar_wait_limit(&landed[n % s.tiles], (n / s.tiles) & 1, kWaitLimit);
+          if (!ok) break;
+          tc::tc_fence_after_sync();
+          const uint64_t db0 = tc::make_desc(tc::smem_u32(B) + (n % s.tiles) * kTileBytes, 16, 1024);
+          for (int m = 0; m < n_mt; ++m) {
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks)
+              tc::mma_ss(s.tmem + (n & 1) * 256 + (uint32_t)(m * TN),
+                         da0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfA + (uint32_t)m * 128 * 128 + (uint32_t)(ks & 3) * 32u) >> 4),
+                         db0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfB + (uint32_t)(ks & 3) * 32u) >> 4), idesc, ks > 0);
+          }
+          tc::mma_commit_own_cta(&mma_done[n & 1]);
+          if (it >= 1 && it - 1 + s.tiles < n_tiles) {  // the buffer of the tile before is free once its MMAs are done
+            ok = tc::mbar_wait_limit(&mma_done[(n - 1) & 1], ((n - 1) >> 1) & 1, kWaitLimit);
+            if (ok) load_tile(n - 1 + s.tiles, n_begin + (it - 1 + s.tiles) * TN);
+          }
+        }
+      }
+      __syncwarp();
+      if (op == 1 && m0 + kWideTokens < C) fetch(m0 + kWideTokens);
 
       // Running maximum of this thread's columns.  The read-back is bound by the rate of comparisons and selections (half
       // of an add's): eight columns at a time go through three-input maxima, and only the first column of the group that
@@ -689,18 +723,16 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
 #pragma unroll
       for (int j = 0; j < 8; ++j) held[j] = -INFINITY;
       const bool epi = mt < n_mt;
-      for (int it = 0; it < n_tiles; ++it) {
-        ok = ok && tc::mbar_wait_limit(&s.bars[(g0 + it) & 1], ((g0 + it) >> 1) & 1, kWaitLimit);
-        const bool more = it + 2 < n_tiles;
-        if (more) load_tile(it + 2);  // (the MMAs of tile `it` are done with its buffer)
+      for (int it = 0; it < n_tiles && reads; ++it) {
+        const uint32_t n = g0 + it;
+        ok = ok && tc::mbar_wait_limit(&mma_done[n & 1], (n >> 1) & 1, kWaitLimit);
         if (epi) {
           tc::tc_fence_after_sync();
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int n0 = n_begin + it * TN + col0 + half * 32;
-            if (n0 >= n_end) continue;
+          for (int ch = 0; ch < chunks; ++ch) {
+            const int n0 = n_begin + it * TN + col0 + ch * 32;
+            if (n0 >= n_end) break;
             uint32_t r[32];
-            tc::tmem_ld32(t_lane + (uint32_t)((it & 1) * 256 + half * 32), r);
+            tc::tmem_ld32(t_lane + (n & 1) * 256 + (uint32_t)(ch * 32), r);
             tc::tmem_ld_wait();
             const int lo = op == 0 ? 0 : protected_rows;
             if (n0 + 32 > n_end || n0 < lo) {
@@ -726,17 +758,13 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           }
           tc::tc_fence_before_sync();
         }
-        if (more) {
-          cp_async_wait<0>();
-          tc::fence_proxy_async();
-          __syncthreads();  // tile it + 2 is complete, the accumulators of tile `it` have been read
-          if (issuer) issue_mmas(it + 2);
-        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&is_read[n & 1]);
       }
       s.tc_tiles = g0 + (uint32_t)n_tiles;
       if (!__syncthreads_and(ok ? 1 : 0)) return false;
       // the column inside the group, then the two threads of a token (columns 0..63 and 64..127 of every tile), who
-      // exchange through a tile's buffer
+      // exchange through arrays that are not in use yet
       float bv = op == 0 ? bf16_round(best) : best;  // (rounding keeps the order)
       int bi = at;
       if (op == 1 && at >= 0) {
@@ -745,8 +773,8 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           if (held[j] == best) bi = at + j;
       }
       if (op == 1 && at < 0 && col0 == 0 && max(n_begin, protected_rows) < n_end) bi = max(n_begin, protected_rows);  // (no number above -inf)
-      float* xv = reinterpret_cast<float*>(B);
-      int* xi = reinterpret_cast<int*>(B) + kWideTokens;
+      float* xv = reinterpret_cast<float*>(s.ord + m0);
+      int* xi = s.lead + m0;
       const int tok = mt * 128 + (warp & 3) * 32 + lane;
       if (epi && col0 != 0) {
         xv[tok] = bv;
@@ -766,9 +794,9 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           }
         }
       }
-      __syncthreads();  // (the next pass fetches its first tiles over the exchange buffer)
     }
   }
+  __syncthreads();
   return true;
 }
 
@@ -910,7 +938,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
     }
     if constexpr (WIDE) {
       if (s.use_tc) {
-        scanned = scan_memory_wide<D, NT>(blk, L.gate_keys != 0, C, view.k, view.cur, scan_b, scan_e, n_append > 0, protected_rows, s);
+        scanned = scan_memory_wide<D, NT>(blk, L.gate_keys != 0, C, scan_b, scan_e, n_append > 0, protected_rows, s);
         if (!scanned) {
           if (tid == 0 && s.status) atomicExch(s.status, KVM_ERR_DEVICE_TIMEOUT);
           s.use_tc = false;
@@ -1035,8 +1063,10 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
         store_row<D, GL>(vr, mem.v_sum + (size_t)row * D, gl);
         if (gl == 0) mem.vlen[row] = vl;
       }
-      refresh_memory_row<D, GL>(L, kr, vr, vl, view.k + (size_t)slot * D, view.v + (size_t)slot * D, gl, act);
+      refresh_memory_row<D, GL>(L, kr, vr, vl, view.k + (size_t)slot * D, view.v + (size_t)slot * D, gl, act,
+                                WIDE && pool ? mem.k_attn + (size_t)row * D : nullptr);
     }
+    if constexpr (WIDE) fence_all_proxies();
     if (pool) {
       for (int i = tid; i < n_append; i += NT)
         if (S_before + i < capacity) view.cur[S_before + i] = view.pool_next + i;
@@ -1100,7 +1130,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
     // A table over the memory rows (where the scan's tiles were): (first token + 1) << 16 | tokens so far.  Tokens of a warp
     // with the same target are matched, then the warps enter their counts one after the other.  Block 512: 26 K -> 6 K cycles
     // against every token's comparison with every other, which blocks of 256 and less do as fast with their two threads per
-    // token.  (The memory rows fit: they are fewer than kSmemLimit / 4 - tile bytes, the tiles 32768 ints.)
+    // token.  (update_scan_wide admits fewer than 25000 memory rows, the tiles hold 32768 ints.)
     int* tab = reinterpret_cast<int*>(s.btile);
     for (int i = tid; i < S_after; i += NT) tab[i] = 0;
     const int mine = tid < C ? s.idx[tid] : -1;
@@ -1223,6 +1253,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
       if (!is_v) {
         layer_norm_row<D, GL>(sum, L.ln_w, L.ln_b, L.ln_eps, gl);
         if (act) store_row<D, GL>(sum, view.k + (size_t)slot * D, gl);
+        if (WIDE && pool && act) store_row<D, GL>(sum, mem.k_attn + (size_t)row * D, gl);
       } else {
         const float nrm = fmaxf(row_norm<D, GL>(sum), 1e-12f);
         divide_by(sum.x, nrm);
@@ -1232,6 +1263,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
       }
     }
   }
+  if constexpr (WIDE) fence_all_proxies();
   __syncthreads();
   if (pool) {
     for (int i = tid; i < n_touched; i += NT) view.cur[s.idx[s.touched[i]]] = view.pool_next + i;
