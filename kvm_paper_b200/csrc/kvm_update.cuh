@@ -608,8 +608,9 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
 // gated keys for the logits) through all memory rows, in tiles of 128 rows: at N = 128 an MMA reads its two operands from
 // shared memory as fast as it multiplies them (64 cycles, N = 64: 48 for half of the work).  Two accumulator buffers of
 // 2 x 128 columns: while the tensor core works on one tile, 15 warps read the other's accumulators back (warp w: lanes
-// 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..; warp 11 also takes those of warp 15).  One thread of warp
-// 15 only copies and issues: MMAs are issued at the pace of the tensor core, so a warp that also reads back holds up all.
+// 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..; those of warp 15 are split between warps 3 and 7, which
+// reach the same lanes).  One thread of warp 15 only copies and issues: MMAs are issued at the pace of the tensor core, so a
+// warp that also reads back holds up all.
 // The memory rows come from the view in row order, which the update writes next to the pool row of every refreshed row: a
 // tile is two TMA copies.  They are read from L2 once per pass; a block of 512 tokens that only merges takes two passes.
 // FIGURES
@@ -634,7 +635,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
   unsigned char* A = reinterpret_cast<unsigned char*>(s.btile);  // [2 k-halves][kWideTokens][128 B], swizzled
   unsigned char* B = A + 2 * kHalfA;                              // s.tiles tiles, [2 k-halves][TN][128 B] each
   const bool issuer = tid == NT - 32, reads = warp < NT / 32 - 1;
-  const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64, chunks = warp == NT / 32 - 5 ? 4 : 2;  // of 32 columns
+  const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64;
   const uint32_t t_lane = s.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * TN + col0);
   uint64_t *mma_done = s.bars, *landed = s.bars + 3, *is_read = s.bars + 6;
   bool ok = true;
@@ -718,76 +719,94 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
       // Running maximum of this thread's columns.  The read-back is bound by the rate of comparisons and selections (half
       // of an add's): eight columns at a time go through three-input maxima, and only the first column of the group that
       // holds the maximum is noted, with the group's eight values, among which the column is looked up at the end.
-      float best = -INFINITY, held[8];
-      int at = -1;
+      struct Best {
+        float v, held[8];
+        int at;
+      } mine, other;  // this thread's token, and the one of warp 15 that it helps with
+      mine.v = other.v = -INFINITY;
+      mine.at = other.at = -1;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) held[j] = -INFINITY;
-      const bool epi = mt < n_mt;
-      for (int it = 0; it < n_tiles && reads; ++it) {
-        const uint32_t n = g0 + it;
-        ok = ok && tc::mbar_wait_limit(&mma_done[n & 1], (n >> 1) & 1, kWaitLimit);
-        if (epi) {
-          tc::tc_fence_after_sync();
-          for (int ch = 0; ch < chunks; ++ch) {
-            const int n0 = n_begin + it * TN + col0 + ch * 32;
-            if (n0 >= n_end) break;
-            uint32_t r[32];
-            tc::tmem_ld32(t_lane + (n & 1) * 256 + (uint32_t)(ch * 32), r);
-            tc::tmem_ld_wait();
-            const int lo = op == 0 ? 0 : protected_rows;
-            if (n0 + 32 > n_end || n0 < lo) {
+      for (int j = 0; j < 8; ++j) mine.held[j] = other.held[j] = -INFINITY;
+      auto read_columns = [&](Best& b, uint32_t taddr, int n0) {  // 32 of them, the first is memory row n0
+        if (n0 >= n_end) return;
+        uint32_t r[32];
+        tc::tmem_ld32(taddr, r);
+        tc::tmem_ld_wait();
+        const int lo = op == 0 ? 0 : protected_rows;
+        if (n0 + 32 > n_end || n0 < lo) {
 #pragma unroll
-              for (int c = 0; c < 32; ++c)
-                if (n0 + c >= n_end || n0 + c < lo) r[c] = 0xff800000u;  // -inf
-            }
-#pragma unroll
-            for (int c = 0; c < 32; c += 8) {
-              float x[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[c + j]);
-              const float m = fmaxf(max3(max3(x[0], x[1], x[2]), x[6], x[7]), max3(x[3], x[4], x[5]));
-              if (op == 0) {
-                best = fmaxf(best, m);
-              } else if (m > best) {
-                best = m;
-                at = n0 + c;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) held[j] = x[j];
-              }
-            }
-          }
-          tc::tc_fence_before_sync();
+          for (int c = 0; c < 32; ++c)
+            if (n0 + c >= n_end || n0 + c < lo) r[c] = 0xff800000u;  // -inf
         }
+#pragma unroll
+        for (int c = 0; c < 32; c += 8) {
+          float x[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[c + j]);
+          const float m = fmaxf(max3(max3(x[0], x[1], x[2]), x[6], x[7]), max3(x[3], x[4], x[5]));
+          if (op == 0) {
+            b.v = fmaxf(b.v, m);
+          } else if (m > b.v) {
+            b.v = m;
+            b.at = n0 + c;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) b.held[j] = x[j];
+          }
+        }
+      };
+      const bool epi = mt < n_mt, helps = n_mt == 2 && (warp == 3 || warp == 7);
+      const int col1 = 64 + (warp >> 2) * 32;  // of accumulator 1
+      for (int it = 0; it < n_tiles && reads; ++it) {
+        const uint32_t n = g0 + it, buf = (n & 1) * 256;
+        const int row = n_begin + it * TN;
+        ok = ok && tc::mbar_wait_limit(&mma_done[n & 1], (n >> 1) & 1, kWaitLimit);
+        tc::tc_fence_after_sync();
+        if (epi) {
+          read_columns(mine, t_lane + buf, row + col0);
+          read_columns(mine, t_lane + buf + 32, row + col0 + 32);
+        }
+        if (helps) read_columns(other, s.tmem + (96u << 16) + buf + (uint32_t)(TN + col1), row + col1);
+        tc::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&is_read[n & 1]);
       }
       s.tc_tiles = g0 + (uint32_t)n_tiles;
       if (!__syncthreads_and(ok ? 1 : 0)) return false;
-      // the column inside the group, then the two threads of a token (columns 0..63 and 64..127 of every tile), who
-      // exchange through arrays that are not in use yet
-      float bv = op == 0 ? bf16_round(best) : best;  // (rounding keeps the order)
-      int bi = at;
-      if (op == 1 && at >= 0) {
+      // the column inside the group, then the threads of a token (columns 0..63 and 64..127 of every tile), who exchange
+      // through arrays that are not in use yet
+      auto column = [&](const Best& b) {
+        int c = b.at;
 #pragma unroll
         for (int j = 7; j >= 0; --j)
-          if (held[j] == best) bi = at + j;
-      }
-      if (op == 1 && at < 0 && col0 == 0 && max(n_begin, protected_rows) < n_end) bi = max(n_begin, protected_rows);  // (no number above -inf)
-      float* xv = reinterpret_cast<float*>(s.ord + m0);
-      int* xi = s.lead + m0;
-      const int tok = mt * 128 + (warp & 3) * 32 + lane;
-      if (epi && col0 != 0) {
+          if (b.at >= 0 && b.held[j] == b.v) c = b.at + j;
+        return c;
+      };
+      const int tok = mt * 128 + (warp & 3) * 32 + lane, quarter = 128 + 96 + lane;  // the latter: a token of warps 11 and 15
+      float bv = mine.v;
+      int bi = column(mine);
+      float *xv = reinterpret_cast<float*>(s.ord + m0), *xv2 = reinterpret_cast<float*>(s.tcnt + m0);
+      int *xi = s.lead + m0, *xi2 = s.tstart + m0;
+      if (epi && reads && col0 != 0) {
         xv[tok] = bv;
         xi[tok] = bi;
       }
+      if (helps) {
+        (warp == 3 ? xv : xv2)[quarter] = other.v;
+        (warp == 3 ? xi : xi2)[quarter] = column(other);
+      }
       __syncthreads();
       if (epi && col0 == 0) {
-        const float ov = xv[tok];
-        const int oi = xi[tok], row = m0 + tok;
+        const int row = m0 + tok;
+        auto take = [&](float ov, int oi) {
+          if (op == 0) bv = fmaxf(bv, ov);
+          else if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
+        };
+        take(xv[tok], xi[tok]);
+        if (tok == quarter) take(xv2[tok], xi2[tok]);
         if (op == 0) {
-          s.app[row] = fmaxf(bv, ov);
+          s.app[row] = bf16_round(bv);  // (rounding keeps the order)
         } else {
-          if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
+          if (bi < 0 && max(n_begin, protected_rows) < n_end) bi = max(n_begin, protected_rows);  // (no number above -inf)
           if (bi >= 0 && (s.idx[row] < 0 || bv > s.best[row])) {
             s.best[row] = bv;
             s.idx[row] = bi;
