@@ -82,11 +82,11 @@ kvm_chain_kernel(LayerDev L_in, long long T, Tensor4 k, Tensor4 v, Tensor4 gate,
   if constexpr ((SB || WIDE) && D == 128 && NT == 512) {
     if (WIDE || L.C == 128 || L.C == 256) {  // tcgen05 routing scan: its two barriers and tensor memory, once per kernel
       if (threadIdx.x == 0) {
-        tc::mbar_init(&s.bars[0], 1);
-        tc::mbar_init(&s.bars[1], 1);
+        tc::mbar_init(&s.bars[0], WIDE ? 2 : 1);
+        tc::mbar_init(&s.bars[1], WIDE ? 2 : 1);
         if (WIDE) {
           for (int i = 0; i < 3; ++i) tc::mbar_init(&s.bars[3 + i], 1);
-          for (int i = 0; i < 2; ++i) tc::mbar_init(&s.bars[6 + i], NT / 32 - 1);
+          for (int i = 0; i < 2; ++i) tc::mbar_init(&s.bars[6 + i], NT / 32 - 2);
         }
         tc::fence_barrier_init();
       }

@@ -607,13 +607,16 @@ __device__ __noinline__ bool scan_memory_tc(const BlockView& blk, bool gate_keys
 // memory).  Same contract as scan_memory_tc.  A pass takes up to 256 tokens and one operand (prepared keys for the novelty,
 // gated keys for the logits) through all memory rows, in tiles of 128 rows: at N = 128 an MMA reads its two operands from
 // shared memory as fast as it multiplies them (64 cycles, N = 64: 48 for half of the work).  Two accumulator buffers of
-// 2 x 128 columns: while the tensor core works on one tile, 15 warps read the other's accumulators back (warp w: lanes
-// 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..; those of warp 15 are split between warps 3 and 7, which
-// reach the same lanes).  One thread of warp 15 only copies and issues: MMAs are issued at the pace of the tensor core, so a
-// warp that also reads back holds up all.
+// 2 x 128 columns: while the tensor core works on one tile, 14 warps read the other's accumulators back (warp w: lanes
+// 32 * (w % 4).., accumulator w / 8, columns 64 * (w / 4 % 2)..; those of warps 14 and 15 are split between warps 2, 6 and 3,
+// 7, which reach the same lanes).  One thread each of warps 14 and 15 issues the MMAs of one accumulator and does nothing
+// else but copy: issuing takes 170 cycles per MMA, more than the tensor core needs, and a warp that also read back would hold
+// up all.
 // The memory rows come from the view in row order, which the update writes next to the pool row of every refreshed row: a
 // tile is two TMA copies.  They are read from L2 once per pass; a block of 512 tokens that only merges takes two passes.
-// FIGURES
+// Block 512, up to 4096 rows, four CTAs per kv row (262144 tokens, 32 heads): an update's scan takes 80 K cycles (one issuing
+// thread: 91 K; as warp-level MMAs, which read their B fragments from shared memory once per 16 tokens, 227 K), the prefill
+// 60.2 ms (63.7, 106.8).
 // Rows written by this thread -> other threads' TMA copies behind a barrier, and the other way round.
 __device__ __forceinline__ void fence_all_proxies() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -634,7 +637,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
   if (n_tiles <= 0) return true;
   unsigned char* A = reinterpret_cast<unsigned char*>(s.btile);  // [2 k-halves][kWideTokens][128 B], swizzled
   unsigned char* B = A + 2 * kHalfA;                              // s.tiles tiles, [2 k-halves][TN][128 B] each
-  const bool issuer = tid == NT - 32, reads = warp < NT / 32 - 1;
+  const bool copies = tid == NT - 32, issues = warp >= NT / 32 - 2 && lane == 0, reads = warp < NT / 32 - 2;
   const int mt = warp >> 3, col0 = ((warp >> 2) & 1) * 64;
   const uint32_t t_lane = s.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * TN + col0);
   uint64_t *mma_done = s.bars, *landed = s.bars + 3, *is_read = s.bars + 6;
@@ -668,7 +671,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
     const int n_mt = min(kWideTokens, C - m0) / 128;
     for (int op = want_app ? 0 : 1; op < 2; ++op) {  // 0: prepared keys (novelty), 1: gated keys (merge logits)
       const uint32_t g0 = s.tc_tiles;
-      if (issuer) {
+      if (copies) {
         fence_all_proxies();  // (rows that other threads have written since the last scan)
         for (int it = 0; it < s.tiles && it < n_tiles; ++it) load_tile(g0 + it, n_begin + it * TN);
       }
@@ -690,8 +693,9 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
       }
       tc::fence_proxy_async();
       __syncthreads();
-      if (issuer) {
-        const uint64_t da0 = tc::make_desc(tc::smem_u32(A), 16, 1024);
+      if (issues) {
+        const int m = warp & 1;
+        const uint64_t da0 = tc::make_desc(tc::smem_u32(A) + (uint32_t)m * 128 * 128, 16, 1024);
         for (int it = 0; it < n_tiles && ok; ++it) {
           const uint32_t n = g0 + it;
           if (it >= 2) ok = tc::mbar_wait_limit(&is_read[n & 1], ((n >> 1) - 1) & 1, kWaitLimit);
@@ -699,15 +703,15 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           if (!ok) break;
           tc::tc_fence_after_sync();
           const uint64_t db0 = tc::make_desc(tc::smem_u32(B) + (n % s.tiles) * kTileBytes, 16, 1024);
-          for (int m = 0; m < n_mt; ++m) {
+          const uint32_t acc = s.tmem + (n & 1) * 256 + (uint32_t)(m * TN);
+          if (m < n_mt) {
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks)
-              tc::mma_ss(s.tmem + (n & 1) * 256 + (uint32_t)(m * TN),
-                         da0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfA + (uint32_t)m * 128 * 128 + (uint32_t)(ks & 3) * 32u) >> 4),
+              tc::mma_ss(acc, da0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfA + (uint32_t)(ks & 3) * 32u) >> 4),
                          db0 + (uint64_t)(((uint32_t)(ks >> 2) * kHalfB + (uint32_t)(ks & 3) * 32u) >> 4), idesc, ks > 0);
           }
           tc::mma_commit_own_cta(&mma_done[n & 1]);
-          if (it >= 1 && it - 1 + s.tiles < n_tiles) {  // the buffer of the tile before is free once its MMAs are done
+          if (copies && it >= 1 && it - 1 + s.tiles < n_tiles) {  // the buffer of the tile before is free once its MMAs are done
             ok = tc::mbar_wait_limit(&mma_done[(n - 1) & 1], ((n - 1) >> 1) & 1, kWaitLimit);
             if (ok) load_tile(n - 1 + s.tiles, n_begin + (it - 1 + s.tiles) * TN);
           }
@@ -722,7 +726,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
       struct Best {
         float v, held[8];
         int at;
-      } mine, other;  // this thread's token, and the one of warp 15 that it helps with
+      } mine, other;  // this thread's token, and the one of warp 14 or 15 that it helps with
       mine.v = other.v = -INFINITY;
       mine.at = other.at = -1;
 #pragma unroll
@@ -754,7 +758,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           }
         }
       };
-      const bool epi = mt < n_mt, helps = n_mt == 2 && (warp == 3 || warp == 7);
+      const bool epi = mt < n_mt, helps = n_mt == 2 && warp < 8 && (warp & 2);
       const int col1 = 64 + (warp >> 2) * 32;  // of accumulator 1
       for (int it = 0; it < n_tiles && reads; ++it) {
         const uint32_t n = g0 + it, buf = (n & 1) * 256;
@@ -765,7 +769,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           read_columns(mine, t_lane + buf, row + col0);
           read_columns(mine, t_lane + buf + 32, row + col0 + 32);
         }
-        if (helps) read_columns(other, s.tmem + (96u << 16) + buf + (uint32_t)(TN + col1), row + col1);
+        if (helps) read_columns(other, s.tmem + ((uint32_t)((warp & 3) * 32) << 16) + buf + (uint32_t)(TN + col1), row + col1);
         tc::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&is_read[n & 1]);
@@ -781,7 +785,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           if (b.at >= 0 && b.held[j] == b.v) c = b.at + j;
         return c;
       };
-      const int tok = mt * 128 + (warp & 3) * 32 + lane, quarter = 128 + 96 + lane;  // the latter: a token of warps 11 and 15
+      const int tok = mt * 128 + (warp & 3) * 32 + lane, helped = 128 + (warp & 3) * 32 + lane;
       float bv = mine.v;
       int bi = column(mine);
       float *xv = reinterpret_cast<float*>(s.ord + m0), *xv2 = reinterpret_cast<float*>(s.tcnt + m0);
@@ -791,8 +795,8 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
         xi[tok] = bi;
       }
       if (helps) {
-        (warp == 3 ? xv : xv2)[quarter] = other.v;
-        (warp == 3 ? xi : xi2)[quarter] = column(other);
+        (warp < 4 ? xv : xv2)[helped] = other.v;
+        (warp < 4 ? xi : xi2)[helped] = column(other);
       }
       __syncthreads();
       if (epi && col0 == 0) {
@@ -802,7 +806,7 @@ __device__ __noinline__ bool scan_memory_wide(const BlockView& blk, bool gate_ke
           else if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
         };
         take(xv[tok], xi[tok]);
-        if (tok == quarter) take(xv2[tok], xi2[tok]);
+        if (mt == 1 && (warp & 2)) take(xv2[tok], xi2[tok]);
         if (op == 0) {
           s.app[row] = bf16_round(bv);  // (rounding keeps the order)
         } else {
