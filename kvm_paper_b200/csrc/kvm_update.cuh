@@ -362,7 +362,7 @@ __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, i
               const int r = e >> 1;
               const int n = tile_base + (nt + h) * 8 + t * 2 + (e & 1);
               if (n < n_end) {
-                if (want_app) amax[r] = fmaxf(amax[r], cp[h][e]);  // (rounded below: rounding keeps the order)
+                if (want_app) amax[r] = fmaxf(amax[r], bf16_round(cp[h][e]));
                 if (n >= protected_rows && (cg[h][e] > bbest[r] || bidx[r] < 0)) {
                   bbest[r] = cg[h][e];
                   bidx[r] = n;
@@ -390,7 +390,7 @@ __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, i
         }
         if (t == 0) {
           const int row = mt * 16 + g + r * 8;
-          if (want_app) s.app[row] = bf16_round(amax[r]);
+          if (want_app) s.app[row] = amax[r];
           if (bidx[r] >= 0 && (s.idx[row] < 0 || bbest[r] > s.best[row])) {
             s.best[row] = bbest[r];
             s.idx[row] = bidx[r];
