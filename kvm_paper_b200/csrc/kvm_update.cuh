@@ -274,9 +274,11 @@ __device__ __forceinline__ void scan_load_tile(bf16* dst, const bf16* k_attn, co
 // Routing GEMM over memory rows [n_begin, n_end): per token the running maximum of the bf16-rounded
 // pk scores (novelty, only if want_app) and the running fp32 argmax of the gk logits (rows below
 // `protected_rows` excluded).  Results are merged into s.app / s.best / s.idx.
+// first_in_flight: the first tile is already on its way.
 template <int D, int NT>
 __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, int C, const bf16* __restrict__ k_attn, const int* slots,
-                            int n_begin, int n_end, bool want_app, int protected_rows, UpdateSmem<D>& s) {
+                            int n_begin, int n_end, bool want_app, int protected_rows, UpdateSmem<D>& s,
+                            bool first_in_flight = false) {
   constexpr int NW = NT / 32;
   constexpr int KS = D / 16;
   constexpr int STR = scan_tile_stride<D>();
@@ -314,9 +316,11 @@ __device__ __noinline__ void scan_memory(const BlockView& blk, bool gate_keys, i
     float bbest[2] = {-INFINITY, -INFINITY};
     int bidx[2] = {-1, -1};
 
-    __syncthreads();  // previous users of the tile buffers are done
-    scan_load_tile<D, NT>(s.btile, k_attn, slots, n_begin, n_end, tid);
-    cp_async_commit();
+    if (pass0 > 0 || !first_in_flight) {
+      __syncthreads();  // previous users of the tile buffers are done
+      scan_load_tile<D, NT>(s.btile, k_attn, slots, n_begin, n_end, tid);
+      cp_async_commit();
+    }
     for (int it = 0; it < n_tiles; ++it) {
       const int cur = it & 1;
       if (it + 1 < n_tiles) {
@@ -867,6 +871,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
   if constexpr (SB && PKR && D == 128 && NT == 512) use_tc = s.use_tc && (C == 128 || C == 256) && n_merge > 0;
   const bool defer_v = use_tc;
   int tiles_in_flight = 0;
+  bool first_in_flight = false;
   // ---- 0. bring the block in: keys first (needed at once), values behind them
   BlockView blk;
   blk.g = s.g_s;
@@ -893,6 +898,14 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
         cp_async16(s.pk_s + (size_t)r * PST + cc * 8, src.k + (long long)r * src.k_st + cc * 8, 16);
       }
       cp_async_commit();
+      if constexpr (PKR) {
+        // The first tile of the warp-level scan behind them: its gather takes as long as the phases in between (1 x 4096 tokens,
+        // 8 heads x 64: 392.6 -> 389 us).  A decode step's update, which still has its keys to prepare, gains nothing by it
+        // (64 sequences, 32 tokens: 494 us with it, 482 without).
+        first_in_flight = n_merge > 0 && scan_e > scan_b;
+        if (first_in_flight) scan_load_tile<D, NT>(s.btile, view.k, view.cur, scan_b, scan_e, tid);
+        cp_async_commit();
+      }
       for (int c = tid; c < C * CPR; c += NT) {
         const int r = c / CPR, cc = c % CPR;
         cp_async16(s.v_s + (size_t)r * D + cc * 8, src.v + (long long)r * src.v_st + cc * 8, 16);
@@ -920,7 +933,10 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
       asm volatile("prefetch.global.L2 [%0];" ::"l"(src.next_v + (long long)r * src.v_st + l * 64));
     }
   }
-  if constexpr (SB) cp_async_wait<1>();
+  if constexpr (SB) {
+    if (use_tc || !PKR) cp_async_wait<1>();
+    else cp_async_wait<2>();
+  }
   __syncthreads();
 
   // ---- 1. prepared keys (in place in shared memory, or into the global scratch); 8 lanes per token
@@ -969,7 +985,7 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
       }
     }
     if (!scanned)
-      scan_memory<D, NT>(blk, L.gate_keys != 0, C, view.k, view.cur, scan_b, scan_e, n_append > 0, protected_rows, s);
+      scan_memory<D, NT>(blk, L.gate_keys != 0, C, view.k, view.cur, scan_b, scan_e, n_append > 0, protected_rows, s, first_in_flight);
     if constexpr (SB) {
       if (defer_v) {  // the value staging area is free again: fetch the block's values behind the ranking
         for (int c = tid; c < C * CPR; c += NT) {
