@@ -503,7 +503,7 @@ static int decode_step_impl(const kvm_layer* layer, int32_t batch, const kvm_dec
   if (!cache.ring_k || !cache.ring_v || !cache.ring_gate || !cache.total_len || !cache.state_len)
     return fail(KVM_ERR_BAD_ARGUMENT, "decode cache arrays must not be NULL");
   UpdateSet upd;
-  upd.arr = n_append_dev;
+  upd.arr = any_update ? n_append_dev : nullptr;  // (what an earlier token left in a kept array is none of this one's business)
   upd.n = 0;
   if (any_update && n_append_host) {  // the schedule is known here: it travels with the launches as a list, if it fits one
     int n = 0;
