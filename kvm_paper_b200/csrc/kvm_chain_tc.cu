@@ -369,6 +369,7 @@ struct Issuer {
     }
     ++n_p; ++n_g;
     kvm_update_plan pl_next = a.plan[0];  // fetched one update ahead: the table lives in global memory
+    bool g_late = true;                   // the gated keys of the next block are asked for at the head of its update
     for (int u = 0; u < a.n_plan; ++u) {
       const kvm_update_plan pl = pl_next;
       if (u + 1 < a.n_plan) pl_next = a.plan[u + 1];
@@ -377,9 +378,11 @@ struct Issuer {
       if (u > 0) {
         if (!wait_on(&bars->w2i, n_w2i)) return false;  // the resident rows of the previous update are final
         if (!primary) tc::mbar_arrive(&bars->idle);     // (no worker runs two updates ahead of this thread)
-        if (primary && u == 1) load(map_gk, lay.G, &bars->full_g, 1);
+        if (primary && g_late) load(map_gk, lay.G, &bars->full_g, u);
         const bool withhold = (a.test_flags & 1u) && u == 1;
-        if (!wait(&bars->full_g, n_g & 1, a.wait_limit, abort)) return false;
+        // (A block that is appended as a whole asks nothing of the second issuer, so nothing would keep the barrier from
+        // completing the next block's phase before it has looked: it does not look.  The workers do, ahead of their w2i.)
+        if ((primary || nm > 0) && !wait(&bars->full_g, n_g & 1, a.wait_limit, abort)) return false;
         ++n_g;
         // Few appended rows: the logits against the OLD memory do not depend on them, so they go first and the novelty
         // follows behind; many: the novelty first, then the logits against the memory after the appends.
@@ -420,8 +423,11 @@ struct Issuer {
           }
         }
       }
-      // every routing pass was read back before the scatter was asked for: the gated keys of this block are dead
-      if (primary && u > 0 && u + 1 < a.n_plan) load(map_gk, lay.G, &bars->full_g, u + 1);
+      // Every routing pass was read back before the scatter was asked for: the gated keys of this block are dead.  A block
+      // that is appended as a whole has no scatter: the workers may be taking its rows from the buffer until they have
+      // signalled w2i, which is waited for at the head of the next update.
+      g_late = u == 0 || nm == 0;
+      if (primary && !g_late && u + 1 < a.n_plan) load(map_gk, lay.G, &bars->full_g, u + 1);
       if (primary && u + 2 < a.n_plan && crank == (u & (nc - 1))) {  // one CTA of the cluster asks, all profit
         prefetch(map_gk, u + 2);
         if (a.plan[u + 2].n_append > 0) prefetch(map_pk, u + 2);
@@ -852,7 +858,7 @@ struct Workers {
       if (u == 0 || nm == 0) {
         // ---- the block becomes memory rows token by token: the initial memory (model/kvm_mixer.py:434-447), or a block
         // that is appended as a whole
-        ok = ok && wait(&bars->full_p, n_p & 1, a.wait_limit, abort) && (u > 0 || wait(&bars->full_g, 0, a.wait_limit, abort));
+        ok = ok && wait(&bars->full_p, n_p & 1, a.wait_limit, abort) && wait(&bars->full_g, u & 1, a.wait_limit, abort);
         ++n_p;
         if (token) list()[tid] = tid;
         if (!wvote(ok)) return false;

@@ -28,12 +28,23 @@ CASES = {
 
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_tensor_core_chain_equals_the_general_chain(name):
+    _chains_agree(name, gate_appends=0)
+
+
+@pytest.mark.parametrize("name", ["few_rows", "many_rows", "whole_blocks", "whole_blocks_c256"])
+def test_gated_appends_take_the_gated_keys_of_their_own_block(name):
+    """With gated appends the new rows come from the buffer that the next block's gated keys are copied into."""
+    _chains_agree(name, gate_appends=1)
+
+
+def _chains_agree(name, gate_appends):
     C, T, H, B, appends, blocks = CASES[name]
     torch.manual_seed(5)
     gen = torch.Generator(device="cuda").manual_seed(5)
     rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
     sink = C if name == "initial_rows_are_sinks" else 1
     spec = gh.bf16_spec(ko.KvmSpec(H, H, 128, 128, 64, C, 2, blocks, sink, "fixed", state_min_len=C,
+                                   kvm_apply_merge_gate_to_appends=gate_appends,
                                    ln_weight=1.0 + 0.1 * torch.randn(128), ln_bias=0.05 * torch.randn(128)))
     params = gh.layer_params(spec)
     step = iter(appends + [appends[-1]] * 1000)
