@@ -339,13 +339,14 @@ class SequenceMixer(nn.Module):
                 and (self.value_residual_mode != "rwkv" or self.v_gate0.dtype == torch.bfloat16))
 
     @staticmethod
-    def _plain_linear(m, x) -> bool:
-        """A linear layer that ``ops.project`` may stand in for: bf16, no bias, nothing hooked onto it."""
+    def _plain_linear(m, x, width) -> bool:
+        """A linear layer that ``ops.project`` may stand in for on rows of ``width`` values: bf16, no bias, nothing hooked
+        onto it, a weight of the layer's own shape (anything else is the module's to compute or to refuse)."""
         if type(m) is not nn.Linear or m.bias is not None:
             return False
         w = m.weight
-        return (type(w) in (nn.Parameter, torch.Tensor) and w.dtype is torch.bfloat16
-                and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.size(1) % 32 == 0 and w.device == x.device
+        return (type(w) in (nn.Parameter, torch.Tensor) and w.dtype is torch.bfloat16 and w.shape == (m.out_features, width)
+                and w.is_contiguous() and w.data_ptr() % 16 == 0 and width % 32 == 0 and w.device == x.device
                 and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__)
 
     def _few_rows(self, x) -> bool:
@@ -362,7 +363,8 @@ class SequenceMixer(nn.Module):
         gated = self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values
         mixed = self.value_residual_mode == "rwkv"
         lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
-        if not (self._few_rows(x) and all(self._plain_linear(m, x) for m in lins) and (not mixed or self._plain_linear(self.v_gate2, x))):
+        if not (self._few_rows(x) and all(self._plain_linear(m, x, x.size(-1)) for m in lins)
+                and (not mixed or self._plain_linear(self.v_gate2, x, self.v_gate1.out_features))):
             return (self.c_q(x).contiguous(), self.c_k(x).contiguous(), self.c_v(x).contiguous(),
                     self.v_gate2(self.v_gate1(x)) if mixed else None, self.key_weighting(x) if gated else None)
         y = ops.project(x.reshape(B * T, -1), [m.weight for m in lins])
@@ -377,7 +379,7 @@ class SequenceMixer(nn.Module):
     def _output(self, y):
         """``c_proj``."""
         B, T, _ = y.shape
-        if self._few_rows(y) and self._plain_linear(self.c_proj, y) and self.c_proj.out_features % 8 == 0:
+        if self._few_rows(y) and self._plain_linear(self.c_proj, y, y.size(-1)) and self.c_proj.out_features % 8 == 0:
             return ops.project(y.view(B * T, -1), [self.c_proj.weight]).view(B, T, -1)
         return self.c_proj(y)
 
@@ -481,8 +483,10 @@ class SequenceMixer(nn.Module):
         c_proj = self.c_proj
         if (not isinstance(cache, ops.KvmDecodeCache) or cache.owner is not self or cache.batch != B or self.value_residual_mode == "linear"
                 or not (cache.total_len_h == past_key_values.get_seq_length(self.layer_idx)).all()
-                or not all(self._plain_linear(m, x) for m in lins) or not self._plain_linear(c_proj, x) or c_proj.out_features % 8
-                or (mixed and not self._plain_linear(self.v_gate2, x))):
+                or not all(self._plain_linear(m, x, x.size(-1)) for m in lins)
+                or not self._plain_linear(c_proj, x, self.attention_output_size) or c_proj.out_features % 8
+                or (mixed and (not self._plain_linear(self.v_gate2, x, self.v_gate1.out_features)
+                               or self.v_gate2.out_features != self.value_projection_size))):
             return None
         dev = x.device
         call = ops.TokenCall.of(cache, self.layer_params(dev), self._prologue_params_kept(dev))

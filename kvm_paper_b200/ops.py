@@ -383,6 +383,11 @@ def project(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
     """[rows, width] bf16 (at most ``PROJECT_ROWS_MAX`` rows) times the transposed weights, side by side:
     [rows, sum of the weights' rows], in one launch."""
     rows, width = x.shape
+    for w in weights:
+        if w.dim() != 2 or w.size(1) != width or w.dtype is not torch.bfloat16 or not w.is_contiguous() or w.device != x.device:
+            raise ValueError(f"weights must be contiguous bf16 [.., {width}] on {x.device}, got {tuple(w.shape)} {w.dtype} on {w.device}")
+    if x.dtype is not torch.bfloat16 or not x.is_cuda:
+        raise ValueError(f"project expects bf16 rows on a CUDA device, got {x.dtype} on {x.device}")
     if x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < width or x.data_ptr() % 16:
         x = x.clone(memory_format=torch.contiguous_format)
     n = len(weights)

@@ -202,3 +202,20 @@ def test_spans_equal_single_tokens(Hq, Hkv, D, C):
     diff = (got.float() - want.float()).abs()
     assert float(diff.max()) <= 2.0 ** -7 * max(1.0, float(want.float().abs().max())) + 2.0 ** -8 * 6
     assert float(diff.mean()) <= 2.0 ** -8 * float(want.float().abs().mean())
+
+
+@pytest.mark.parametrize("B,T", [(2, 5), (3, 1)])
+def test_hidden_states_of_another_width_are_refused(B, T):
+    """Prompts and tokens, as the layers themselves refuse them; the cache still serves the right width afterwards."""
+    m = _mixer(2, 2, 32, 16, 256)
+    vf = torch.zeros(B, T, 64, device="cuda").bfloat16()
+    past = StatesCache()
+    with torch.no_grad():
+        m.forward_inference(torch.randn(B, T, 256, device="cuda").bfloat16(), vf, _rot(32, 0, T), None, past_key_values=past)
+        for width in (128, 224, 288, 512):
+            for n, cache, at in ((T, StatesCache(), 0), (1, past, T)):
+                with pytest.raises(RuntimeError):
+                    m.forward_inference(torch.randn(B, n, width, device="cuda").bfloat16(), vf[:, :n], _rot(32, at, n), None,
+                                        past_key_values=cache)
+        y = m.forward_inference(torch.randn(B, 1, 256, device="cuda").bfloat16(), vf[:, :1], _rot(32, T, 1), None, past_key_values=past)
+    assert y.shape == (B, 1, 256) and past.get_seq_length(m.layer_idx) == T + 1

@@ -221,3 +221,22 @@ def test_prologue_parameters_are_read_where_they_are():
     a = m._prologue_params_kept(torch.device("cpu"))
     assert not a.shared and not a.ln_bf16 and m._prologue_params_kept(torch.device("cpu")) is not a
     assert not ops.PrologueParams("cpu", ln_q=m.ln_k, ln_k=m.ln_k).ln_bf16  # a caller's own block keeps its copy
+
+
+def test_few_row_layers_are_taken_over_at_their_own_width_only():
+    """The one-launch projection stands in for a layer whose weight has the input's width and the layer's own rows; any other
+    pair is refused, as the module itself refuses it."""
+    lin = torch.nn.Linear(64, 32, bias=False).bfloat16()
+    plain = SequenceMixer._plain_linear
+    x = torch.randn(2, 1, 64).bfloat16()
+    assert plain(lin, x, 64)
+    for width in (32, 96, 128):
+        assert not plain(lin, x, width)
+        with pytest.raises(ValueError):
+            ops.project(torch.randn(2, width).bfloat16(), [lin.weight])
+    with pytest.raises(ValueError):
+        ops.project(x[:, 0], [lin.weight.float()])
+    with pytest.raises(ValueError):
+        ops.project(x[:, 0], [lin.weight])  # (no CUDA tensors)
+    lin.weight = torch.nn.Parameter(lin.weight[:24].detach().clone())  # fewer rows than the layer says
+    assert not plain(lin, x, 64)
