@@ -335,8 +335,25 @@ class SequenceMixer(nn.Module):
         path without the post-shift residual (that variant mixes values after the token shift)."""
         return (x.is_cuda and x.dtype == torch.bfloat16 and self.c_q.weight.dtype == torch.bfloat16
                 and self.d_qk_head in (32, 64, 128) and self.value_projection_size == self.num_key_value_heads * self.d_qk_head
-                and self.value_residual_mode != "rwkv_post_tokenshift"
-                and (self.value_residual_mode != "rwkv" or self.v_gate0.dtype == torch.bfloat16))
+                and self.value_residual_mode != "rwkv_post_tokenshift")
+
+    def _mixes_in_kernel(self) -> bool:
+        """The "rwkv" value residual that the prologue kernel forms itself: the class's own value gate over bf16 parameters."""
+        return (self.value_residual_mode == "rwkv" and self.v_gate0.dtype == torch.bfloat16
+                and self.v_gate0.numel() == self.value_projection_size and "_value_gate" not in self.__dict__
+                and type(self)._value_gate is SequenceMixer._value_gate)
+
+    def _mixed_values(self, x, v, v_first, v_gate):
+        """Values for the prologue kernel: (v, None, None), mixed here, or (v, what the kernel mixes in, room for the last
+        token's mixed value)."""
+        if self.value_residual_mode == "linear":
+            return ((1 - self.lamb) * v + self.lamb * v_first.view_as(v)).contiguous(), None, None
+        if self.value_residual_mode != "rwkv":
+            return v, None, None
+        if v_gate is None:
+            return (v + (v_first.to(v.dtype) - v) * self._value_gate(x).to(v.dtype)).contiguous(), None, None
+        v_last = torch.empty(x.size(0), 1, self.value_projection_size, device=x.device, dtype=x.dtype)
+        return v, (v_first, v_gate, self.v_gate0), v_last
 
     @staticmethod
     def _plain_linear(m, x, width) -> bool:
@@ -358,10 +375,11 @@ class SequenceMixer(nn.Module):
                 and not (_module._global_forward_hooks or _module._global_forward_pre_hooks))
 
     def _project(self, x):
-        """q, k, v projections, output of ``v_gate2`` and merge-gate logits (the last two None where the layer has none)."""
+        """q, k, v projections, output of ``v_gate2`` (None where the kernel forms no residual) and merge-gate logits (None
+        where the layer has none)."""
         B, T, _ = x.shape
         gated = self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values
-        mixed = self.value_residual_mode == "rwkv"
+        mixed = self._mixes_in_kernel()
         lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
         if not (self._few_rows(x) and all(self._plain_linear(m, x, x.size(-1)) for m in lins)
                 and (not mixed or self._plain_linear(self.v_gate2, x, self.v_gate1.out_features))):
@@ -394,12 +412,7 @@ class SequenceMixer(nn.Module):
         if past_len > 0 and T != 1:
             raise AssertionError("cached decode expects single-token inputs.")
         q, k, v, v_gate, gate_lin = self._project(x)
-        residual = v_last = None
-        if self.value_residual_mode == "linear":
-            v = ((1 - self.lamb) * v + self.lamb * v_first.view_as(v)).contiguous()
-        elif self.value_residual_mode == "rwkv":
-            residual = (v_first, v_gate, self.v_gate0)
-            v_last = torch.empty(B, 1, self.value_projection_size, device=x.device, dtype=x.dtype)
+        v, residual, v_last = self._mixed_values(x, v, v_first, v_gate)
         dev = x.device
         prev = None
         if past_key_values is not None:
@@ -434,7 +447,7 @@ class SequenceMixer(nn.Module):
     def _unwatched(self, stage: str) -> bool:
         """Nobody looks at the tensors between the stages of a call (no hook, no override of the stage behind the prefix):
         the stages may run as one library call."""
-        stages = (stage, "forward_prefix_fused", "prefill_raw", "_value_gate")
+        stages = (stage, "forward_prefix_fused", "prefill_raw")
         return not (self.capture_routes or self.check_device_status or torch.is_grad_enabled()
                     or any(n in self.__dict__ or getattr(type(self), n) is not getattr(SequenceMixer, n) for n in stages))
 
@@ -446,12 +459,7 @@ class SequenceMixer(nn.Module):
             raise AssertionError("cached decode expects single-token inputs.")
         dev = x.device
         q, k, v, v_gate, gate_lin = self._project(x)
-        residual = v_last = None
-        if self.value_residual_mode == "linear":
-            v = ((1 - self.lamb) * v + self.lamb * v_first.view_as(v)).contiguous()
-        elif self.value_residual_mode == "rwkv":
-            residual = (v_first, v_gate, self.v_gate0)
-            v_last = torch.empty(B, 1, self.value_projection_size, device=dev, dtype=x.dtype)
+        v, residual, v_last = self._mixed_values(x, v, v_first, v_gate)
         params, pro = self.layer_params(dev), self._prologue_params_kept(dev)
         prev = None
         if past_key_values is not None:
@@ -477,11 +485,12 @@ class SequenceMixer(nn.Module):
         states = past_key_values.get_states(self.layer_idx)
         cache = states.get(self._CACHE_DECODE)
         B = x.size(0)
-        mixed = self.value_residual_mode == "rwkv"
+        mixed = self._mixes_in_kernel()
         gated = bool(self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values)
         lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
         c_proj = self.c_proj
-        if (not isinstance(cache, ops.KvmDecodeCache) or cache.owner is not self or cache.batch != B or self.value_residual_mode == "linear"
+        if (not isinstance(cache, ops.KvmDecodeCache) or cache.owner is not self or cache.batch != B
+                or (self.value_residual_mode != "none" and not mixed)
                 or not (cache.total_len_h == past_key_values.get_seq_length(self.layer_idx)).all()
                 or not all(self._plain_linear(m, x, x.size(-1)) for m in lins)
                 or not self._plain_linear(c_proj, x, self.attention_output_size) or c_proj.out_features % 8

@@ -219,3 +219,34 @@ def test_hidden_states_of_another_width_are_refused(B, T):
                                         past_key_values=cache)
         y = m.forward_inference(torch.randn(B, 1, 256, device="cuda").bfloat16(), vf[:, :1], _rot(32, T, 1), None, past_key_values=past)
     assert y.shape == (B, 1, 256) and past.get_seq_length(m.layer_idx) == T + 1
+
+
+@pytest.mark.parametrize("T", [20, 150])
+@pytest.mark.parametrize("own", ["instance", "subclass", "fp32 parameter"])
+def test_a_value_gate_of_ones_own_is_called(T, own):
+    """Prompts of few and of many rows and cached tokens, staged and as one call, against the prologue in PyTorch."""
+    m = _mixer(4, 2, 64, 32, 256)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(1, T + 8, 256, generator=gen, device="cuda").bfloat16()
+    vf = torch.randn(1, T + 8, 128, generator=gen, device="cuda").bfloat16()
+    stock, _ = _drive(m, x, vf, T, 8, staged=False)
+    calls = []
+
+    def gate(x):
+        calls.append(tuple(x.shape))
+        return 0.25 + 0.0 * m.v_gate2(m.v_gate1(x))
+
+    if own == "instance":
+        m._value_gate = gate
+    elif own == "subclass":
+        m.__class__ = type("Own", (SequenceMixer,), {"_value_gate": lambda self, x: gate(x)})
+    else:
+        m.v_gate0 = torch.nn.Parameter(m.v_gate0.detach().float() * 3.0)
+    ys = [_drive(m, x, vf, T, 8, staged=staged)[0] for staged in (False, True)]
+    assert torch.equal(*ys)
+    assert own == "fp32 parameter" or calls == 2 * ([(1, T, 256)] + 8 * [(1, 1, 256)])
+    m.use_fused_prologue = False
+    want, _ = _drive(m, x, vf, T, 8, staged=False)
+    # (neighbouring bf16 numbers here and there, as above; the stock gate is far off)
+    assert float((ys[0].double() - want.double()).norm() / want.double().norm()) <= 1e-2
+    assert float((stock.double() - want.double()).norm() / want.double().norm()) >= 0.05
