@@ -350,6 +350,7 @@ static int prologue_args(const kvm_layer* layer, int32_t batch, int64_t seq_len,
     (i < 3 ? p.st[i] : p.prev_sb[i - 3]) = st;
   }
   p.gate_st = ext->gate_stride_t ? ext->gate_stride_t : layer->n_kv_heads;
+  if (p.gate_st < layer->n_kv_heads) return fail(KVM_ERR_BAD_ARGUMENT, "kvm_prologue_forward: gate stride %lld below %d", p.gate_st, layer->n_kv_heads);
   p.v_first = static_cast<const bf16*>(ext->v_first);
   p.v_gate = static_cast<const bf16*>(ext->v_gate);
   p.v_gate0 = static_cast<const bf16*>(ext->v_gate0);

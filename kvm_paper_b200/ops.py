@@ -259,7 +259,8 @@ def _token_stride(t: torch.Tensor, B: int, T: int, width: int, name: str) -> int
         raise ValueError(f"{name} projection must be a bf16 CUDA tensor [B,T,{width}], got {tuple(t.shape)} {t.dtype}")
     st = t.stride()
     step = st[1] if T > 1 else (st[0] if B > 1 else (width + 7) // 8 * 8)
-    if (st[2] != 1 and width > 1) or (B > 1 and st[0] != T * step):
+    # (a stride of 0 means "contiguous" to the library: rows that are one and the same row do not pass for that)
+    if (st[2] != 1 and width > 1) or step < width or (B > 1 and st[0] != T * step):
         raise ValueError(f"{name} projection must be contiguous or a column range of contiguous rows, got strides {st}")
     return step
 

@@ -240,3 +240,20 @@ def test_few_row_layers_are_taken_over_at_their_own_width_only():
         ops.project(x[:, 0], [lin.weight])  # (no CUDA tensors)
     lin.weight = torch.nn.Parameter(lin.weight[:24].detach().clone())  # fewer rows than the layer says
     assert not plain(lin, x, 64)
+
+
+def test_projections_that_repeat_one_row_are_refused():
+    """The library takes a stride of 0 as "contiguous": tensors expanded over tokens or sequences must not reach it."""
+    def described(t):  # what _token_stride looks at, of a CPU tensor
+        return types.SimpleNamespace(dtype=t.dtype, is_cuda=True, shape=t.shape, stride=t.stride)
+
+    base = torch.zeros(6, 5, 72).bfloat16()
+    for B, T, rows in ((2, 5, base[:2]), (1, 5, base[:1]), (6, 1, base[:, :1]), (1, 1, base[:1, :1])):
+        assert ops._token_stride(described(rows), B, T, 72, "q") == (360 if T == 1 and B > 1 else 72)
+    assert ops._token_stride(described(base.view(30, 1, 72)[..., :64]), 30, 1, 64, "q") == 72
+    one = base[:1, :1]
+    for B, T in ((1, 5), (2, 5), (2, 1)):
+        with pytest.raises(ValueError):
+            ops._token_stride(described(one.expand(B, T, 72)), B, T, 72, "q")
+    with pytest.raises(ValueError):
+        ops._token_stride(described(base.as_strided((1, 5, 72), (360, 64, 1))), 1, 5, 72, "q")  # overlapping rows
