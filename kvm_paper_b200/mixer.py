@@ -499,7 +499,7 @@ class SequenceMixer(nn.Module):
             return None
         dev = x.device
         call = ops.TokenCall.of(cache, self.layer_params(dev), self._prologue_params_kept(dev))
-        y, lin, v_last = call.run(x, [m.weight for m in lins], self.v_gate2.weight if mixed else None, c_proj.weight, gated,
+        y, lin, v_last = call.run(cache, x, [m.weight for m in lins], self.v_gate2.weight if mixed else None, c_proj.weight, gated,
                                   (v_first, self.v_gate0) if mixed else None, position_embeddings,
                                   (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL)))
         dq, dk = self.q_projection_size, self.k_projection_size

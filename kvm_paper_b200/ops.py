@@ -952,10 +952,11 @@ def prompt_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tensor
 
 
 class TokenCall:
-    """The kept argument block of ``kvm_mixer_token`` for one decode cache: between tokens only a few addresses change."""
+    """The kept argument block of ``kvm_mixer_token`` for one decode cache, which holds it (and is not held by it: a cache that
+    is let go gives its memory back at once): between tokens only a few addresses change."""
 
     def __init__(self, cache: KvmDecodeCache, params: LayerParams, pro: PrologueParams):
-        self.cache, self.params, self.pro, self.decode_src = cache, params, pro, cache._call
+        self.params, self.pro, self.decode_src = params, pro, cache._call
         c = self.c = _lib.KvmTokenCall()
         c.decode = cache._call
         c.scratch_bytes = _lib.load().kvm_token_scratch_bytes(C.byref(params.c), cache.batch)
@@ -976,9 +977,10 @@ class TokenCall:
             t = cache._token = TokenCall(cache, params, pro)
         return t
 
-    def run(self, x, weights, v_gate2, c_proj, gated, residual, position_embeddings, prev):
-        """x [B,1,hidden]; returns (y [B,1,out], projections [B,1,..], last values behind the residual or None)."""
-        cache, cfg = self.cache, self.cache.cfg
+    def run(self, cache: KvmDecodeCache, x, weights, v_gate2, c_proj, gated, residual, position_embeddings, prev):
+        """One token of ``cache``.  x [B,1,hidden]; returns (y [B,1,out], projections [B,1,..], last values behind the residual
+        or None)."""
+        cfg = cache.cfg
         addr, decode, p, w, rows = self._views
         c, B, dev = self.c, cache.batch, cache.device
         keep = []

@@ -257,3 +257,23 @@ def test_projections_that_repeat_one_row_are_refused():
             ops._token_stride(described(one.expand(B, T, 72)), B, T, 72, "q")
     with pytest.raises(ValueError):
         ops._token_stride(described(base.as_strided((1, 5, 72), (360, 64, 1))), 1, 5, 72, "q")  # overlapping rows
+
+
+def test_a_decode_cache_is_freed_with_its_last_reference():
+    """What a cache keeps for its tokens does not hold the cache: its device memory does not wait for the cyclic collector."""
+    import gc
+    import weakref
+
+    cache = ops.KvmDecodeCache.__new__(ops.KvmDecodeCache)
+    params = ops.LayerParams(ops.LayerConfig(2, 2, 32, 16, 2, 16, 1), torch.ones(32), torch.zeros(32), None, None, "cpu")
+    cache.batch, cache.device, cache._call = 1, torch.device("cpu"), _lib.KvmDecodeCall()
+    pro = ops.PrologueParams("cpu")
+    assert ops.TokenCall.of(cache, params, pro) is ops.TokenCall.of(cache, params, pro)
+    ref = weakref.ref(cache)
+    gc.collect()
+    gc.disable()
+    try:
+        del cache
+        assert ref() is None
+    finally:
+        gc.enable()
