@@ -258,10 +258,18 @@ def _token_stride(t: torch.Tensor, B: int, T: int, width: int, name: str) -> int
     if t.dtype is not torch.bfloat16 or not t.is_cuda or t.shape != (B, T, width):
         raise ValueError(f"{name} projection must be a bf16 CUDA tensor [B,T,{width}], got {tuple(t.shape)} {t.dtype}")
     st = t.stride()
+    step = _row_step(st, B, T, width)
+    if step is None:
+        raise ValueError(f"{name} projection must be contiguous or a column range of contiguous rows, got strides {st}")
+    return step
+
+
+def _row_step(st, B: int, T: int, width: int) -> int | None:
+    """Elements from row to row of a [B,T,width] tensor with these strides, None where its rows do not lie one step apart."""
     step = st[1] if T > 1 else (st[0] if B > 1 else (width + 7) // 8 * 8)
     # (a stride of 0 means "contiguous" to the library: rows that are one and the same row do not pass for that)
     if (st[2] != 1 and width > 1) or step < width or (B > 1 and st[0] != T * step):
-        raise ValueError(f"{name} projection must be contiguous or a column range of contiguous rows, got strides {st}")
+        return None
     return step
 
 
@@ -309,7 +317,7 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
     arg.q_stride_t, arg.k_stride_t, arg.v_stride_t = (
         _token_stride(t, B, T, h * D, n) for n, t, h in (("q", q_lin, Hq), ("k", k_lin, Hkv), ("v", v_lin, Hkv)))
     if gate_lin is not None:
-        if gate_lin.dtype is not torch.bfloat16 or gate_lin.shape != (B, T, Hkv):
+        if gate_lin.dtype is not torch.bfloat16 or gate_lin.shape != (B, T, Hkv) or _row_step(gate_lin.stride(), B, T, Hkv) is None:
             gate_lin = gate_lin.to(torch.bfloat16).reshape(B, T, Hkv).contiguous()
             keep.append(gate_lin)
         arg.gate_lin, arg.gate_stride_t = gate_lin.data_ptr(), _token_stride(gate_lin, B, T, Hkv, "gate")

@@ -184,3 +184,18 @@ def test_prologue_kernel_matches_the_oracle_on_random_inputs(D, Hq, Hkv, T, with
     for a, b, what in zip(got, want, ("q", "k", "v", "gate")):
         _assert_bf16_equal_up_to_ties(a, b, f"D{D} T{T} {what}")
     assert torch.equal(got[2].cpu(), want[2])  # token shift alone: the same bits
+
+
+def test_merge_gate_logits_of_any_layout():
+    """Logits stored head by head, expanded over tokens, in fp32 or with four dimensions count like contiguous ones."""
+    B, T, H, D = 2, 21, 4, 64
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()  # noqa: E731
+    params = ops.LayerParams(ops.LayerConfig(H, H, D, 32, 2, 32, 1), torch.ones(D), torch.zeros(D), None, None, "cuda")
+    pro = ops.PrologueParams("cuda")
+    q, k, v = (rnd(B, T, H * D) for _ in range(3))
+    run = lambda g: ops.prologue_forward(params, pro, q, k, v, g, None)[3]  # noqa: E731
+    by_head, one, wide = rnd(B, H, T), rnd(B, 1, H), rnd(B, T, 2 * H)
+    for g in (by_head.transpose(1, 2), one.expand(B, T, H), one[:1].expand(B, T, H), wide[..., 2:2 + H], wide[..., ::2],
+              wide[..., :H].float(), wide[..., :H].unsqueeze(-1), wide[:, :1, :1].expand(B, T, H)):
+        assert torch.equal(run(g), run(g.reshape(B, T, H).bfloat16().contiguous())), g.stride()
