@@ -289,6 +289,12 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
+def _aligned_rows(t: torch.Tensor) -> torch.Tensor:
+    """[B,H,T,D] in bf16 whose rows are contiguous and start on 16-byte boundaries, as a view where that is so already."""
+    t = _as_bf16_view(t)
+    return t if t.data_ptr() % 16 == 0 and not any(s % 8 for s in t.stride()[:-1]) else _aligned(t)
+
+
 def _first_values(v_first: torch.Tensor, B: int, T: int, width: int, dev) -> torch.Tensor:
     """The first layer's values [B,T,width] as the value residual's kernels read them: broadcast, bf16, contiguous, aligned."""
     if v_first.device != dev:
@@ -914,7 +920,7 @@ def decode_cache_from_prefill(params: LayerParams, res: PrefillResult, k: torch.
     S = res.plan.final_state_len
     extra = cfg.chunk_len if extra_capacity is None else extra_capacity
     cache = KvmDecodeCache(params, B, S + extra, desired_state_len, owner, _memory=res.memory if adopt_memory else None)
-    k, v, gate = (_as_bf16_view(t) for t in (k, v, gate))
+    k, v, gate = _aligned_rows(k), _aligned_rows(v), _as_bf16_view(gate.reshape(B, Hkv, T, 1))
     rc = _lib.load().kvm_decode_cache_fill(C.byref(params.c), B, T, _tensor4(k, "k"), _tensor4(v, "v"), _tensor4(gate, "gate"),
                                            res.memory.c(), S, cache._call.cache, cache._ws.data_ptr(), _stream_ptr(cache.device))
     _lib.check(rc)

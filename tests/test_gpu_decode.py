@@ -220,3 +220,31 @@ def test_decode_counters_and_lengths_stay_consistent_when_most_ctas_have_no_work
         assert cache.state_len.cpu().tolist() == [int(cache.state_len_h[0])]
         assert int(head.abs().sum()) == 0, f"step {i - T}: counters {head.cpu().tolist()}"
     cache.check_status()
+
+
+def test_cache_behind_a_prefill_takes_any_layout():
+    """Keys and values off a 16-byte boundary, in fp32 or with strided elements, a gate without its last dimension: the cache
+    is the one that contiguous tensors give."""
+    spec = ko.KvmSpec(4, 2, 64, 64, 32, 32, 2, 4, 1, "power_law", state_growth_factor=4.0, state_min_len=32)
+    B, T = 2, 32 * 5 + 7
+    torch.manual_seed(4)
+    q = torch.randn(B, 4, T, 64).bfloat16()
+    k = torch.nn.functional.layer_norm(torch.randn(B, 2, T, 64), (64,)).bfloat16()
+    v = torch.randn(B, 2, T, 64).bfloat16()
+    g = (1 + torch.nn.functional.elu(torch.randn(B, 2, T, 1))).bfloat16()
+    params, plan, res = gh.device_prefill(spec, q, k, v, g)
+    k, v, g = k.cuda(), v.cuda(), g.cuda()
+    want = ops.decode_cache_from_prefill(params, res, k, v, g, gh.desired_fn(spec))
+
+    def inside(t, pad, at):  # the same numbers as a range of wider rows
+        wide = torch.zeros(*t.shape[:-1], t.size(-1) + pad, device="cuda", dtype=t.dtype)
+        wide[..., at:at + t.size(-1)] = t
+        return wide[..., at:at + t.size(-1)]
+
+    every_second = torch.stack([v, v], -1).flatten(-2)[..., ::2]
+    for kk, vv, gg in ((inside(k, 3, 1), inside(v, 8, 3), g.squeeze(-1)), (k.float(), every_second, g.float()),
+                       (inside(k, 4, 0), v.transpose(1, 2).contiguous().transpose(1, 2), g.transpose(1, 2).contiguous().transpose(1, 2))):
+        assert torch.equal(kk, k) and torch.equal(vv, v)
+        got = ops.decode_cache_from_prefill(params, res, kk, vv, gg, gh.desired_fn(spec))
+        for f in ("ring_k", "ring_v", "ring_gate", "total_len", "state_len"):
+            assert torch.equal(getattr(got, f), getattr(want, f)), f
