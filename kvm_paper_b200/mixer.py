@@ -308,7 +308,10 @@ class SequenceMixer(nn.Module):
             gate = torch.ones((B, self.num_key_value_heads, T, 1), device=x.device, dtype=torch.float)
         return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), gate
 
-    def prologue_params(self, device, share_ln: bool = False) -> ops.PrologueParams:
+    def prologue_params(self, device) -> ops.PrologueParams:
+        return self._prologue_block(device, share_ln=False)
+
+    def _prologue_block(self, device, share_ln: bool) -> ops.PrologueParams:
         ln = isinstance(self.ln_q, nn.LayerNorm)
         shift = self.tokenshift_mode == "rwkv"
         return ops.PrologueParams(device, shift_q=self.x_q if shift else None, shift_k=self.x_k if shift else None,
@@ -317,14 +320,16 @@ class SequenceMixer(nn.Module):
 
     def _prologue_params_kept(self, device) -> ops.PrologueParams:
         """``prologue_params``, kept as long as it consists of views of the parameters (a copy would miss what is written
-        to a parameter behind autograd's back)."""
+        to a parameter behind autograd's back).  A module with a ``prologue_params`` of its own is asked on every call."""
+        if "prologue_params" in self.__dict__ or type(self).prologue_params is not SequenceMixer.prologue_params:
+            return self.prologue_params(device)
         ln = isinstance(self.ln_q, nn.LayerNorm)
         src = [t for m in (self.ln_q, self.ln_k) if isinstance(m, nn.LayerNorm) for t in (m.weight, m.bias)]
         if self.tokenshift_mode == "rwkv":
             src += [self.x_q, self.x_k, self.x_v]
         key = (device, self.ln_q.eps if ln else None, *((t.data_ptr(), t.dtype) for t in src))
         if self._prologue_cache is None or self._prologue_cache[0] != key:
-            pro = self.prologue_params(device, share_ln=True)
+            pro = self._prologue_block(device, share_ln=True)
             if not pro.shared:
                 return pro
             self._prologue_cache = (key, pro)

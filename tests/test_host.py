@@ -277,3 +277,24 @@ def test_a_decode_cache_is_freed_with_its_last_reference():
         assert ref() is None
     finally:
         gc.enable()
+
+
+@pytest.mark.parametrize("on", ["instance", "subclass"])
+def test_prologue_parameters_of_ones_own_are_asked_for(on):
+    """An override of ``prologue_params(device)`` is what the fused prologue reads, as returned on that call."""
+    cfg, m = _mixer_from_fixture(load_fixture("powerlaw_bf16"))
+    stock = m._prologue_params_kept(torch.device("cpu"))
+    made = []
+
+    def own(device):
+        made.append(ops.PrologueParams(device, ln_q=m.ln_q, ln_k=m.ln_q))
+        return made[-1]
+
+    if on == "instance":
+        m.prologue_params = own
+    else:
+        m.__class__ = type("Own", (SequenceMixer,), {"prologue_params": lambda self, device: own(device)})
+    for _ in range(2):
+        pro = m._prologue_params_kept(torch.device("cpu"))
+        assert pro is made[-1] and pro is not stock
+    assert len(made) == 2
