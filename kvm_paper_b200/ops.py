@@ -304,10 +304,15 @@ def _first_values(v_first: torch.Tensor, B: int, T: int, width: int, dev) -> tor
     return _aligned(v_first.to(torch.bfloat16))
 
 
-def _prev_rows(prev, B: int, dev) -> list[torch.Tensor]:
+def _prev_rows(prev, B: int, dev, widths=()) -> list[torch.Tensor]:
     """The cached rows [B,1,width] of the previous token as the prologue kernel reads them."""
-    return [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.stride(2) == 1 and t.stride(0) % 8 == 0
-            and t.stride(0) >= t.size(2) and t.data_ptr() % 16 == 0 else _aligned(t.to(dev, torch.bfloat16).reshape(B, 1, -1)) for t in prev]
+    rows = [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.size(0) == B and t.size(1) == 1 and t.stride(2) == 1
+            and t.stride(0) % 8 == 0 and t.stride(0) >= t.size(2) and t.data_ptr() % 16 == 0
+            else _aligned(t.to(dev, torch.bfloat16).reshape(B, 1, -1)) for t in prev]
+    for t, width in zip(rows, widths):
+        if t.size(2) != width:
+            raise ValueError(f"cached rows must be [{B},1,{width}], got {tuple(t.shape)}")
+    return rows
 
 
 def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin, gate_lin, position_embeddings, prev, value_residual,
@@ -339,7 +344,7 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
     if pro.shift_q is not None:
         arg.shift_q, arg.shift_k, arg.shift_v = pro.shift_ptrs
         if prev is not None and all(t is not None for t in prev):
-            pv = _prev_rows(prev, B, dev)
+            pv = _prev_rows(prev, B, dev, (Hq * D, Hkv * D, Hkv * D))
             keep += pv
             arg.prev_q, arg.prev_k, arg.prev_v = (t.data_ptr() for t in pv)
             if B > 1:
@@ -1019,7 +1024,8 @@ class TokenCall:
             if any(t is None for t in prev):
                 p.prev_q, p.prev_k, p.prev_v = None, None, None
             else:
-                pv = _prev_rows(prev, B, x.device)
+                dk = cfg.n_kv_heads * cfg.head_dim
+                pv = _prev_rows(prev, B, x.device, (cfg.n_q_heads * cfg.head_dim, dk, dk))
                 keep.append(pv)
                 p.prev_q, p.prev_k, p.prev_v = pv[0].data_ptr(), pv[1].data_ptr(), pv[2].data_ptr()
                 if B > 1:

@@ -298,3 +298,15 @@ def test_prologue_parameters_of_ones_own_are_asked_for(on):
         pro = m._prologue_params_kept(torch.device("cpu"))
         assert pro is made[-1] and pro is not stock
     assert len(made) == 2
+
+
+def test_cached_rows_of_another_batch_or_width_are_refused():
+    """The kernel reads one row of the projection's width per sequence."""
+    cpu, widths = torch.device("cpu"), (64, 32, 32)
+    rows = [torch.randn(4, 1, w).bfloat16() for w in widths]
+    assert all(a is b for a, b in zip(ops._prev_rows(rows, 4, cpu, widths), rows))
+    flat = ops._prev_rows([t[:, 0] for t in rows], 4, cpu, widths)
+    assert all(torch.equal(a, b) for a, b in zip(flat, rows))
+    for B, w in ((2, widths), (8, widths), (4, (32, 32, 32)), (4, (64, 32, 64))):
+        with pytest.raises((ValueError, RuntimeError)):
+            ops._prev_rows(rows, B, cpu, w)
