@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import operator
 from dataclasses import dataclass
 from typing import Any, Callable
 
@@ -189,23 +190,41 @@ def _round8(x: int) -> int:
 
 # ----------------------------------------------------------------------------------------- memory
 
+def _array(name: str):
+    """Attribute ``name`` of an object whose arrays' addresses are kept in an argument block: assigning another array counts
+    as a change (``changes``), behind which the block is filled in anew.  (Constructors and code that runs per token use
+    ``_name``.)"""
+    key = "_" + name
+
+    def put(self, value):
+        d = self.__dict__
+        if d.get(key) is not value:
+            d[key] = value
+            d["changes"] = self.changes + 1
+
+    return property(operator.attrgetter(key), put)
+
+
 class MemoryBuffers:
     """The compressed memory of ``n_rows`` kv rows with ``capacity`` rows each (``zero``: rows past the live ones read as
     zeros; the kernels never look at them)."""
 
+    changes = 0
+    k_sum, v_sum, vlen, k_attn, v_attn, capacity = map(_array, ("k_sum", "v_sum", "vlen", "k_attn", "v_attn", "capacity"))
+
     def __init__(self, n_rows: int, capacity: int, head_dim: int, device, zero: bool = True):
-        self.n_rows, self.capacity, self.head_dim = n_rows, int(capacity), head_dim
+        self.n_rows, self._capacity, self.head_dim = n_rows, int(capacity), head_dim
         make = torch.zeros if zero else torch.empty
         kw = dict(device=device, dtype=torch.bfloat16)
-        self.k_sum = make(n_rows, capacity, head_dim, **kw)
-        self.v_sum = make(n_rows, capacity, head_dim, **kw)
-        self.vlen = make(n_rows, capacity, device=device, dtype=torch.float32)
-        self.k_attn = make(n_rows, capacity, head_dim, **kw)
-        self.v_attn = make(n_rows, capacity, head_dim, **kw)
+        self._k_sum = make(n_rows, capacity, head_dim, **kw)
+        self._v_sum = make(n_rows, capacity, head_dim, **kw)
+        self._vlen = make(n_rows, capacity, device=device, dtype=torch.float32)
+        self._k_attn = make(n_rows, capacity, head_dim, **kw)
+        self._v_attn = make(n_rows, capacity, head_dim, **kw)
 
     def c(self) -> KvmMemory:
-        return KvmMemory(self.k_sum.data_ptr(), self.v_sum.data_ptr(), self.vlen.data_ptr(),
-                         self.k_attn.data_ptr(), self.v_attn.data_ptr(), self.capacity)
+        return KvmMemory(self._k_sum.data_ptr(), self._v_sum.data_ptr(), self._vlen.data_ptr(),
+                         self._k_attn.data_ptr(), self._v_attn.data_ptr(), self._capacity)
 
     def grown(self, new_capacity: int) -> "MemoryBuffers":
         out = MemoryBuffers(self.n_rows, new_capacity, self.head_dim, self.k_sum.device)
@@ -610,6 +629,9 @@ class KvmDecodeCache:
     lengths on the device; ``logical_state_dict`` returns the reference's eager cache layout."""
 
     cache_representation = "preallocated memory rows + W*C-token ring, per-sequence lengths on device"
+    changes = 0
+    params, memory, ring_k, ring_v, ring_gate, out = map(_array, ("params", "memory", "ring_k", "ring_v", "ring_gate", "out"))
+    total_len, state_len, total_len_h, state_len_h = map(_array, ("total_len", "state_len", "total_len_h", "state_len_h"))
     _quiet = 0
     _token = None  # the mixer's kept arguments of kvm_mixer_token for this cache
 
@@ -617,24 +639,24 @@ class KvmDecodeCache:
                  desired_state_len: Callable[[int, int, int], int], owner: Any = None, *, _memory: MemoryBuffers | None = None):
         """``_memory``: buffers to live in instead of new ones; the caller fills the cache before it is used (``_fill``)."""
         cfg = params.cfg
-        self.params, self.cfg, self.batch, self.owner = params, cfg, int(batch), owner
+        self._params, self.cfg, self.batch, self.owner = params, cfg, int(batch), owner
         self.desired_state_len = desired_state_len
         dev = params.device
         self.device = dev
         self.kv_rows = batch * cfg.n_kv_heads
         self.ring_capacity = cfg.n_bswa_chunks * cfg.chunk_len
-        self.memory = MemoryBuffers(self.kv_rows, max(int(state_capacity), 1), cfg.head_dim, dev) if _memory is None else _memory
+        self._memory = MemoryBuffers(self.kv_rows, max(int(state_capacity), 1), cfg.head_dim, dev) if _memory is None else _memory
         make = torch.zeros if _memory is None else torch.empty
         kw = dict(device=dev, dtype=torch.bfloat16)
-        self.ring_k = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
-        self.ring_v = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
-        self.ring_gate = make(self.kv_rows, self.ring_capacity, **kw)
+        self._ring_k = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
+        self._ring_v = make(self.kv_rows, self.ring_capacity, cfg.head_dim, **kw)
+        self._ring_gate = make(self.kv_rows, self.ring_capacity, **kw)
         self._lens = make(2, batch, device=dev, dtype=torch.int32)
-        self.total_len, self.state_len = self._lens[0], self._lens[1]
-        self.total_len_h = np.zeros(batch, dtype=np.int64)
-        self.state_len_h = np.zeros(batch, dtype=np.int64)
+        self._total_len, self._state_len = self._lens[0], self._lens[1]
+        self._total_len_h = np.zeros(batch, dtype=np.int64)
+        self._state_len_h = np.zeros(batch, dtype=np.int64)
         self.update_count = 0
-        self.out = torch.empty(batch, 1, cfg.n_q_heads * cfg.head_dim, **kw)
+        self._out = torch.empty(batch, 1, cfg.n_q_heads * cfg.head_dim, **kw)
         self.route = None
         self._last_any_update, self._last_n_append = False, None
         self._quiet = 0  # tokens until the next one that may update a memory or grow one directly (see _plan_step)
@@ -651,20 +673,28 @@ class KvmDecodeCache:
 
     def _alloc_workspace(self, clear: bool = True):
         lib = _lib.load()
-        self._max_rows_bound = self.memory.capacity + self.ring_capacity
-        self._ws_bytes = lib.kvm_decode_workspace_bytes(C.byref(self.params.c), self.batch, self._max_rows_bound)
+        self._max_rows_bound = self._memory.capacity + self.ring_capacity
+        self._ws_bytes = lib.kvm_decode_workspace_bytes(C.byref(self._params.c), self.batch, self._max_rows_bound)
         self._ws = torch.empty(self._ws_bytes, device=self.device, dtype=torch.uint8)
         if clear:  # the counter region at the head of the workspace must start at zero; the kernels leave it zero
             self._ws[:4 * (self.kv_rows + self.batch + 1)].zero_()
         # the kept argument block of kvm_decode_step_call; between tokens only input addresses and launch flags change
         call = self._call = _lib.KvmDecodeCall()
-        call.layer, call.batch = C.addressof(self.params.c), self.batch
-        call.cache = _CCache(self.memory.c(), self.ring_k.data_ptr(), self.ring_v.data_ptr(), self.ring_gate.data_ptr(),
-                             self.total_len.data_ptr(), self.state_len.data_ptr())
+        call.layer, call.batch = C.addressof(self._params.c), self.batch
+        call.cache = _CCache(self._memory.c(), self._ring_k.data_ptr(), self._ring_v.data_ptr(), self._ring_gate.data_ptr(),
+                             self._total_len.data_ptr(), self._state_len.data_ptr())
         call.n_append_dev = _ptr(self._n_append)
-        call.total_len_host, call.state_len_host = self.total_len_h.ctypes.data, self.state_len_h.ctypes.data
-        call.out, call.workspace, call.workspace_bytes = self.out.data_ptr(), self._ws.data_ptr(), self._ws_bytes
+        call.total_len_host, call.state_len_host = self._total_len_h.ctypes.data, self._state_len_h.ctypes.data
+        call.out, call.workspace, call.workspace_bytes = self._out.data_ptr(), self._ws.data_ptr(), self._ws_bytes
         self._call_args = (C.addressof(call), call.q, call.k, call.v, call.gate)
+        self._known = (self.changes, self._memory.changes)  # what the block was filled in from
+
+    def _renew(self):
+        """The argument block anew: an array it names has been replaced since (a batch put in another order, say).  The
+        schedule is walked for the next token."""
+        self._total_len_h, self._state_len_h = (np.ascontiguousarray(t, dtype=np.int64) for t in (self._total_len_h, self._state_len_h))
+        self._alloc_workspace()
+        self._quiet = 0
 
     # -- construction ---------------------------------------------------------------------------
     def load_sequence(self, b: int, *, k_sum, v_sum, vlen, window_k, window_v, window_gate, total_len: int,
@@ -720,12 +750,12 @@ class KvmDecodeCache:
         window.  The walk over the batch is skipped for those tokens (``_quiet`` of them are left)."""
         if self._quiet > 0:
             self._quiet -= 1
-            self.total_len_h += 1
+            self._total_len_h += 1
             self._max_rows += 1
             return None, self._max_rows
         cfg = self.cfg
         Cn, W = cfg.chunk_len, cfg.n_bswa_chunks
-        tl, sl = self.total_len_h, self.state_len_h
+        tl, sl = self._total_len_h, self._state_len_h
         cross = (tl % Cn == 0) & (tl // Cn > W)
         n_app = None
         if cross.any():
@@ -781,16 +811,18 @@ class KvmDecodeCache:
             call.any_update, call.n_append_host, call.route_dev = 0, None, None
         if rc:
             _lib.check(rc)
-        return self.out
+        return self._out
 
     def _begin_step(self):
         """The host side of a token ahead of its launch: schedule, room for the rows it appends.  Returns the append counts
         (None: no sequence updates its memory)."""
+        if self._known != (self.changes, self._memory.changes):
+            self._renew()
         n_app, _ = self._plan_step()
         self._last_any_update, self._last_n_append = n_app is not None, n_app
         if n_app is not None or self._quiet == 0:
-            need = int(self.state_len_h.max())
-            if need > self.memory.capacity:
+            need = int(self._state_len_h.max())
+            if need > self._memory.capacity:
                 self._reserve(need)
             if n_app is not None and int((n_app >= 0).sum()) > _lib.UPDATE_LIST_MAX:
                 self._upload_n_append(n_app)
@@ -829,7 +861,9 @@ class KvmDecodeCache:
         lib, stream = _lib.load(), _stream_ptr(self.device)
         Cn, WC = cfg.chunk_len, self.ring_capacity
         span = max(1, _lib.SPAN_COLUMNS // (cfg.n_q_heads // cfg.n_kv_heads))  # (more query heads: refused by the library)
-        tl, sl = self.total_len_h, self.state_len_h
+        if self._known != (self.changes, self._memory.changes):
+            self._renew()
+        tl, sl = self._total_len_h, self._state_len_h
         self._quiet = 0
         piece = 128  # (a token's place inside a piece fits a byte)
         for lo in range(0, n, piece):

@@ -310,3 +310,44 @@ def test_cached_rows_of_another_batch_or_width_are_refused():
     for B, w in ((2, widths), (8, widths), (4, (32, 32, 32)), (4, (64, 32, 64))):
         with pytest.raises((ValueError, RuntimeError)):
             ops._prev_rows(rows, B, cpu, w)
+
+
+def test_arrays_of_a_decode_cache_may_be_replaced():
+    """The kept argument block names the arrays a cache has now: a batch put in another order, other lengths, other parameters."""
+    import numpy as np
+
+    cfg = ops.LayerConfig(2, 2, 32, 16, 2, 16, 1)
+    make = lambda: ops.LayerParams(cfg, torch.ones(32), torch.zeros(32), None, None, "cpu")  # noqa: E731
+    cache = ops.KvmDecodeCache(make(), 3, 24, lambda ctx, avail, cur: cur)
+
+    def block_names_the_arrays():
+        cache._begin_step()
+        c, m = cache._call, cache.memory
+        assert [c.cache.memory.k_sum, c.cache.memory.v_sum, c.cache.memory.vlen, c.cache.memory.k_attn, c.cache.memory.v_attn] == [
+            t.data_ptr() for t in (m.k_sum, m.v_sum, m.vlen, m.k_attn, m.v_attn)]
+        assert c.cache.memory.capacity == m.capacity
+        assert [c.cache.ring_k, c.cache.ring_v, c.cache.ring_gate, c.cache.total_len, c.cache.state_len, c.out] == [
+            t.data_ptr() for t in (cache.ring_k, cache.ring_v, cache.ring_gate, cache.total_len, cache.state_len, cache.out)]
+        assert [c.total_len_host, c.state_len_host] == [t.ctypes.data for t in (cache.total_len_h, cache.state_len_h)]
+        assert c.layer == ctypes.addressof(cache.params.c) and cache.total_len_h.dtype == np.int64
+        assert c.workspace == cache._ws.data_ptr()
+
+    cache.total_len_h[:], cache.state_len_h[:] = [40, 50, 60], 20
+    block_names_the_arrays()
+    before = cache._call
+    block_names_the_arrays()
+    assert cache._call is before  # (nothing has changed)
+    order = [2, 0, 1]
+    for name in ("ring_k", "ring_v", "ring_gate", "total_len", "state_len", "out"):
+        setattr(cache, name, getattr(cache, name)[order].clone() if name.endswith("len") else getattr(cache, name).clone())
+        block_names_the_arrays()
+    for name in ("k_sum", "v_sum", "vlen", "k_attn", "v_attn"):
+        setattr(cache.memory, name, getattr(cache.memory, name).flip(0))
+        block_names_the_arrays()
+    lens = cache.total_len_h.tolist()
+    cache.total_len_h, cache.state_len_h = np.array(lens, dtype=np.int32)[order], cache.state_len_h[order]
+    block_names_the_arrays()
+    assert cache.total_len_h.tolist() == [lens[i] + 1 for i in order]
+    cache.memory, cache.params = cache.memory.grown(40), make()
+    block_names_the_arrays()
+    assert cache._max_rows_bound == 40 + 32
