@@ -364,11 +364,12 @@ class SequenceMixer(nn.Module):
     def _plain_linear(m, x, width) -> bool:
         """A linear layer that ``ops.project`` may stand in for on rows of ``width`` values: bf16, no bias, nothing hooked
         onto it, a weight of the layer's own shape (anything else is the module's to compute or to refuse)."""
-        if type(m) is not nn.Linear or m.bias is not None:
+        if type(m) is not nn.Linear:
             return False
-        w = m.weight
-        return (type(w) in (nn.Parameter, torch.Tensor) and w.dtype is torch.bfloat16 and w.shape == (m.out_features, width)
-                and w.is_contiguous() and w.data_ptr() % 16 == 0 and width % 32 == 0 and w.device == x.device
+        w = m._parameters.get("weight")
+        return (m._parameters.get("bias") is None and type(w) in (nn.Parameter, torch.Tensor) and w.dtype is torch.bfloat16
+                and w.shape == (m.out_features, width) and w.is_contiguous() and w.data_ptr() % 16 == 0
+                and width % 32 == 0 and w.device == x.device
                 and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__)
 
     def _few_rows(self, x) -> bool:
@@ -382,20 +383,20 @@ class SequenceMixer(nn.Module):
     def _project(self, x):
         """q, k, v projections, output of ``v_gate2`` (None where the kernel forms no residual) and merge-gate logits (None
         where the layer has none)."""
-        B, T, _ = x.shape
+        B, T, width = x.shape
         gated = self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values
         mixed = self._mixes_in_kernel()
         lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
-        if not (self._few_rows(x) and all(self._plain_linear(m, x, x.size(-1)) for m in lins)
+        if not (self._few_rows(x) and all(self._plain_linear(m, x, width) for m in lins)
                 and (not mixed or self._plain_linear(self.v_gate2, x, self.v_gate1.out_features))):
             return (self.c_q(x).contiguous(), self.c_k(x).contiguous(), self.c_v(x).contiguous(),
                     self.v_gate2(self.v_gate1(x)) if mixed else None, self.key_weighting(x) if gated else None)
-        y = ops.project(x.reshape(B * T, -1), [m.weight for m in lins])
+        y = ops.project_checked(x.reshape(B * T, -1), [m.weight for m in lins])
         parts, at = [], 0
         for m in lins:  # (every range but the merge gate's starts on a 16-byte boundary)
             parts.append(y[:, at:at + m.out_features])
             at += m.out_features
-        v_gate = ops.project(parts[3], [self.v_gate2.weight]).view(B, T, -1) if mixed else None
+        v_gate = ops.project_checked(parts[3], [self.v_gate2.weight]).view(B, T, -1) if mixed else None
         q, k, v = (t.view(B, T, -1) for t in parts[:3])
         return q, k, v, v_gate, parts[-1].view(B, T, -1) if gated else None
 
@@ -403,7 +404,7 @@ class SequenceMixer(nn.Module):
         """``c_proj``."""
         B, T, _ = y.shape
         if self._few_rows(y) and self._plain_linear(self.c_proj, y, y.size(-1)) and self.c_proj.out_features % 8 == 0:
-            return ops.project(y.view(B * T, -1), [self.c_proj.weight]).view(B, T, -1)
+            return ops.project_checked(y.view(B * T, -1), [self.c_proj.weight]).view(B, T, -1)
         return self.c_proj(y)
 
     def forward_prefix_fused(self, x, v_first, position_embeddings, past_key_values=None, runner=None):
@@ -489,22 +490,22 @@ class SequenceMixer(nn.Module):
             return None
         states = past_key_values.get_states(self.layer_idx)
         cache = states.get(self._CACHE_DECODE)
-        B = x.size(0)
+        B, _, width = x.shape
         mixed = self._mixes_in_kernel()
         gated = bool(self.config.kvm_use_merge_gate_keys or self.config.kvm_use_merge_gate_values)
         lins = [self.c_q, self.c_k, self.c_v] + ([self.v_gate1] if mixed else []) + ([self.key_weighting] if gated else [])
-        c_proj = self.c_proj
+        c_proj, v_gate2 = self.c_proj, self.v_gate2 if mixed else None
         if (not isinstance(cache, ops.KvmDecodeCache) or cache.owner is not self or cache.batch != B
                 or (self.value_residual_mode != "none" and not mixed)
                 or not (cache.total_len_h == past_key_values.get_seq_length(self.layer_idx)).all()
-                or not all(self._plain_linear(m, x, x.size(-1)) for m in lins)
+                or not all(self._plain_linear(m, x, width) for m in lins)
                 or not self._plain_linear(c_proj, x, self.attention_output_size) or c_proj.out_features % 8
-                or (mixed and (not self._plain_linear(self.v_gate2, x, self.v_gate1.out_features)
-                               or self.v_gate2.out_features != self.value_projection_size))):
+                or (mixed and (not self._plain_linear(v_gate2, x, lins[3].out_features)
+                               or v_gate2.out_features != self.value_projection_size))):
             return None
         dev = x.device
         call = ops.TokenCall.of(cache, self.layer_params(dev), self._prologue_params_kept(dev))
-        y, lin, v_last = call.run(cache, x, [m.weight for m in lins], self.v_gate2.weight if mixed else None, c_proj.weight, gated,
+        y, lin, v_last = call.run(cache, x, [m.weight for m in lins], v_gate2.weight if mixed else None, c_proj.weight, gated,
                                   (v_first, self.v_gate0) if mixed else None, position_embeddings,
                                   (states.get(self._CACHE_Q_FINAL), states.get(self._CACHE_K_FINAL), states.get(self._CACHE_V_FINAL)))
         dq, dk = self.q_projection_size, self.k_projection_size

@@ -323,14 +323,17 @@ def _first_values(v_first: torch.Tensor, B: int, T: int, width: int, dev) -> tor
     return _aligned(v_first.to(torch.bfloat16))
 
 
-def _prev_rows(prev, B: int, dev, widths=()) -> list[torch.Tensor]:
+def _prev_rows(prev, B: int, dev, widths=None) -> list[torch.Tensor]:
     """The cached rows [B,1,width] of the previous token as the prologue kernel reads them."""
-    rows = [t if t.dtype is torch.bfloat16 and t.device == dev and t.dim() == 3 and t.size(0) == B and t.size(1) == 1 and t.stride(2) == 1
-            and t.stride(0) % 8 == 0 and t.stride(0) >= t.size(2) and t.data_ptr() % 16 == 0
-            else _aligned(t.to(dev, torch.bfloat16).reshape(B, 1, -1)) for t in prev]
-    for t, width in zip(rows, widths):
-        if t.size(2) != width:
-            raise ValueError(f"cached rows must be [{B},1,{width}], got {tuple(t.shape)}")
+    rows = []
+    for t, width in zip(prev, widths or [t.size(-1) for t in prev]):
+        st = t.stride()
+        if not (t.shape == (B, 1, width) and t.dtype is torch.bfloat16 and t.device == dev and st[2] == 1 and st[0] % 8 == 0
+                and st[0] >= width and t.data_ptr() % 16 == 0):
+            t = _aligned(t.to(dev, torch.bfloat16).reshape(B, 1, -1))
+            if t.size(2) != width:
+                raise ValueError(f"cached rows must be [{B},1,{width}], got {tuple(t.shape)}")
+        rows.append(t)
     return rows
 
 
@@ -421,16 +424,22 @@ def prologue_forward(params: LayerParams, pro: PrologueParams, q_lin: torch.Tens
 def project(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
     """[rows, width] bf16 (at most ``PROJECT_ROWS_MAX`` rows) times the transposed weights, side by side:
     [rows, sum of the weights' rows], in one launch."""
-    rows, width = x.shape
+    width = x.size(1)
     for w in weights:
         if w.dim() != 2 or w.size(1) != width or w.dtype is not torch.bfloat16 or not w.is_contiguous() or w.device != x.device:
             raise ValueError(f"weights must be contiguous bf16 [.., {width}] on {x.device}, got {tuple(w.shape)} {w.dtype} on {w.device}")
     if x.dtype is not torch.bfloat16 or not x.is_cuda:
         raise ValueError(f"project expects bf16 rows on a CUDA device, got {x.dtype} on {x.device}")
+    return project_checked(x, weights)
+
+
+def project_checked(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
+    """``project`` for a caller that has looked at the weights' types, shapes and devices."""
+    rows, width = x.shape
     if x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < width or x.data_ptr() % 16:
         x = x.clone(memory_format=torch.contiguous_format)
     n = len(weights)
-    sizes = [w.size(0) for w in weights]
+    sizes = [w.shape[0] for w in weights]
     cols = (sum(sizes) + 7) // 8 * 8  # (16-byte aligned rows)
     out = torch.empty(rows, cols, device=x.device, dtype=torch.bfloat16)
     rc = _lib.load().kvm_project(x.data_ptr(), x.stride(0), rows, width, (C.c_void_p * n)(*[w.data_ptr() for w in weights]),
@@ -1066,14 +1075,16 @@ class TokenCall:
                     p.prev_q_stride_b, p.prev_k_stride_b, p.prev_v_stride_b = pv[0].stride(0), pv[1].stride(0), pv[2].stride(0)
         cols = 0
         for i, t in enumerate(weights):
-            w[i], rows[i] = t.data_ptr(), t.size(0)
-            cols += t.size(0)
+            n = t.shape[0]
+            w[i], rows[i] = t.data_ptr(), n
+            cols += n
         cols = (cols + 7) // 8 * 8
         lin = torch.empty(B, 1, cols, device=x.device, dtype=torch.bfloat16)
-        y = torch.empty(B, 1, c_proj.size(0), device=x.device, dtype=torch.bfloat16)
-        c.x, c.x_stride, c.hidden, c.n_weights, c.gated = x.data_ptr(), x.size(2), x.size(2), len(weights), gated
+        hidden, out_features = x.shape[2], c_proj.shape[0]
+        y = torch.empty(B, 1, out_features, device=x.device, dtype=torch.bfloat16)
+        c.x, c.x_stride, c.hidden, c.n_weights, c.gated = x.data_ptr(), hidden, hidden, len(weights), gated
         c.v_gate2 = None if v_gate2 is None else v_gate2.data_ptr()
-        c.c_proj, c.out_features = c_proj.data_ptr(), c_proj.size(0)
+        c.c_proj, c.out_features = c_proj.data_ptr(), out_features
         c.lin, c.lin_stride, c.y = lin.data_ptr(), cols, y.data_ptr()
         n_app = cache._begin_step()
         if self.decode_src is not cache._call:  # (the memory has been moved to larger arrays)
