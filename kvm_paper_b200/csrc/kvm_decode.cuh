@@ -24,19 +24,22 @@ __device__ __forceinline__ void prefetch_2d(const CUtensorMap* m, int x, int y) 
 }
 
 // The new token of one kv row, written by one warp: its ring slot and, while the sequence is still inside its first
-// block, memory row `past` directly (model/kvm_mixer.py:623-638; no gating on this path).
+// block, memory row `past` directly (model/kvm_mixer.py:623-638; no gating on this path).  Returns what this lane wrote to the
+// ring: 16 bytes of the key (the first D / 8 lanes) or of the value (the next D / 8).
 template <int D>
-__device__ __forceinline__ void write_new_token(const LayerDev& L, const DecodeCacheDev& cache, const Tensor4& k, const Tensor4& v,
+__device__ __forceinline__ uint4 write_new_token(const LayerDev& L, const DecodeCacheDev& cache, const Tensor4& k, const Tensor4& v,
                                                 const Tensor4& gate, int b, int h, int past, bool direct, int lane) {
   const int row = b * L.Hkv + h, WC = L.W * L.C, slot = past % WC, cap = cache.mem.capacity;
   const bf16* kp = k.row(b, h, 0);
   const bf16* vp = v.row(b, h, 0);
   constexpr int PPR = D / 8;  // 16-byte pieces per row: keys on the first lanes, values on the next
+  uint4 piece = make_uint4(0, 0, 0, 0);
   if (lane < 2 * PPR) {
     const bool is_v = lane >= PPR;
     const int pc = is_v ? lane - PPR : lane;
     bf16* dst = (is_v ? cache.ring_v : cache.ring_k) + ((size_t)row * WC + slot) * D;
-    *reinterpret_cast<uint4*>(dst + pc * 8) = *reinterpret_cast<const uint4*>((is_v ? vp : kp) + pc * 8);
+    piece = *reinterpret_cast<const uint4*>((is_v ? vp : kp) + pc * 8);
+    *reinterpret_cast<uint4*>(dst + pc * 8) = piece;
   }
   if (lane == 0) cache.ring_g[(size_t)row * WC + slot] = *gate.row(b, h, 0);
   if (direct && past < cap) {
@@ -50,6 +53,7 @@ __device__ __forceinline__ void write_new_token(const LayerDev& L, const DecodeC
     if (lane == 0) cache.mem.vlen[mrow] = vl;
     refresh_memory_row<D>(L, pk, vr, vl, cache.mem.k_attn + mrow * D, cache.mem.v_attn + mrow * D, lane);
   }
+  return piece;
 }
 
 constexpr int kDecConsumers = 8;                           // math warps (16 keys of every chunk each)

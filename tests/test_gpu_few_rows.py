@@ -163,6 +163,17 @@ def test_cache_in_the_prefills_memory(T):
 @pytest.mark.parametrize("Hq,Hkv,D,C", [(2, 2, 32, 16), (3, 3, 128, 64), (6, 2, 64, 32), (16, 2, 128, 64), (16, 1, 128, 32)])
 def test_spans_equal_single_tokens(Hq, Hkv, D, C):
     """Ragged batch: sequences inside their first block, at a boundary, long past the window; spans cut by boundaries."""
+    _spans_against_tokens(Hq, Hkv, D, C, None)
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,C", [(2, 2, 32, 16), (3, 3, 128, 64), (6, 2, 64, 32), (16, 1, 128, 32)])
+@pytest.mark.parametrize("odd", [float("inf"), float("-inf"), float("nan")])
+def test_spans_leave_values_that_are_not_numbers_to_the_tokens_that_see_them(Hq, Hkv, D, C, odd):
+    _spans_against_tokens(Hq, Hkv, D, C, odd)
+
+
+def _spans_against_tokens(Hq, Hkv, D, C, odd):
+    """``odd``: a value that some elements of the last block's tokens have (they stay in the window until the end)."""
     lens, n = [1, C - 1, C, 2 * C, 2 * C + 1, 3 * C, 9 * C - 7, 20 * C + 3], 3 * C + 5
     spec = gh.bf16_spec(ko.KvmSpec(Hq, Hkv, D, D, D // 2, C, 2, 8, 1, "power_law", state_growth_factor=4.0, state_min_len=C))
     params = gh.layer_params(spec)
@@ -184,11 +195,23 @@ def test_spans_equal_single_tokens(Hq, Hkv, D, C):
         c.commit_lengths()
     B = len(lens)
     q, k, v, g = rnd(n, B, Hq, 1, D).bfloat16(), norm(n, B, Hkv, 1, D), rnd(n, B, Hkv, 1, D).bfloat16(), gate(n, B, Hkv, 1, 1)
+    if odd is not None:  # (one element of every head: the memory of a sequence must not take part, so only the last tokens)
+        for i in range(n - 6, n):
+            for s in range(B):
+                v[i, s, :, 0, (7 * i + 5 * s) % D] = odd
     want = torch.stack([caches[0].step(q[i], k[i], v[i], g[i]).view(B, -1).clone() for i in range(n)])
     got = caches[1].run(q, k, v, g)
     for c in caches:
         c.check_status()
     a, b = caches
+    if odd is not None:
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        assert not bool(want.isfinite().all()) and bool(want[:n - 6].isfinite().all())
+        fine = want.isfinite()
+        got, want = got[fine], want[fine]
+        diff = (got.float() - want.float()).abs()
+        assert float(diff.max()) <= 2.0 ** -7 * max(1.0, float(want.float().abs().max())) + 2.0 ** -8 * 6
+        return
     assert torch.equal(a.total_len, b.total_len) and torch.equal(a.state_len, b.state_len) and (a.state_len_h == b.state_len_h).all()
     for f in ("k_sum", "v_sum", "vlen", "k_attn", "v_attn"):
         x, y = getattr(a.memory, f), getattr(b.memory, f)
