@@ -199,3 +199,42 @@ def test_merge_gate_logits_of_any_layout():
     for g in (by_head.transpose(1, 2), one.expand(B, T, H), one[:1].expand(B, T, H), wide[..., 2:2 + H], wide[..., ::2],
               wide[..., :H].float(), wide[..., :H].unsqueeze(-1), wide[:, :1, :1].expand(B, T, H)):
         assert torch.equal(run(g), run(g.reshape(B, T, H).bfloat16().contiguous())), g.stride()
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_kernel_variants_agree(D, mixed):
+    """LayerNorm weights in fp32 and in bf16, projections contiguous and as ranges of wider rows, with and without a value
+    residual: the same numbers give the same bits.  An odd number of rows: the last CTA is not full, warps hold rows of
+    several kinds."""
+    B, T, Hq, Hkv = 2, 13, 3, 1
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()  # noqa: E731
+    params = ops.LayerParams(ops.LayerConfig(Hq, Hkv, D, 32, 2, D // 2, 1), torch.ones(D), torch.zeros(D), None, None, "cuda:0")
+
+    class LN:
+        weight, bias = 1 + 0.1 * rnd(D), 0.1 * rnd(D)
+
+    shift = dict(shift_q=rnd(Hq * D), shift_k=rnd(Hkv * D), shift_v=rnd(Hkv * D))
+    wide = rnd(B, T, (Hq + 2 * Hkv) * D + 16)
+    lins = [wide[..., a * D + 8:b * D + 8] for a, b in ((0, Hq), (Hq, Hq + Hkv), (Hq + Hkv, Hq + 2 * Hkv))]
+    rot, prev = (rnd(1, T, D), rnd(1, T, D)), tuple(rnd(B, 1, h * D) for h in (Hq, Hkv, Hkv))
+    residual = (rnd(B, T, Hkv * D), rnd(B, T, Hkv * D), rnd(Hkv * D)) if mixed else None
+    results = []
+    for share in (False, True):
+        pro = ops.PrologueParams("cuda:0", ln_q=LN, ln_k=LN, share_ln=share, **shift)
+        assert bool(pro.ln_bf16) == share
+        for parts in (False, True):
+            for pv in (None, prev):
+                v_last = torch.zeros(B, 1, Hkv * D, device="cuda").bfloat16() if mixed else None
+                out = ops.prologue_forward(params, pro, *(t if parts else t.contiguous() for t in lins), None, rot, prev=pv,
+                                           value_residual=residual, v_last=v_last)
+                results.append((pv is None, out + ((v_last,) if mixed else ())))
+    for first, out in results:
+        base = next(o for f, o in results if f == first)
+        assert all(torch.equal(a, b) for a, b in zip(out, base))
+    if mixed:  # the first value of a sequence without a cached token is its own predecessor, behind the residual
+        v, (vf, vg, v0) = lins[2], residual
+        want = (v.double() + (vf.double() - v.double()) * torch.sigmoid(v0.double() + vg.double()))[:, -1:]
+        # four roundings to bf16 of terms below 2 x the largest operand
+        assert float((results[0][1][4].double() - want).abs().max()) <= 4 * 2.0 ** -8 * 2 * float(torch.maximum(v.abs().max(), vf.abs().max()))
