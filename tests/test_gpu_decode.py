@@ -175,7 +175,7 @@ def test_decode_adopts_reference_eager_cache():
 
 
 def test_decode_run_equals_step_by_step():
-    """kvm_decode_run (n tokens in one C call) gives the same bits as n calls of kvm_decode_step."""
+    """``KvmDecodeCache.run`` (given tokens, several per launch) gives the bits of ``step`` where both cut the rows alike."""
     torch.manual_seed(9)
     spec = ko.KvmSpec(4, 2, 64, 64, 32, 32, 2, 8, 1, "power_law", state_growth_factor=4.0, state_min_len=32)
     B, T, n = 3, 32 * 4 + 20, 50
@@ -248,3 +248,43 @@ def test_cache_behind_a_prefill_takes_any_layout():
         got = ops.decode_cache_from_prefill(params, res, kk, vv, gg, gh.desired_fn(spec))
         for f in ("ring_k", "ring_v", "ring_gate", "total_len", "state_len"):
             assert torch.equal(getattr(got, f), getattr(want, f)), f
+
+
+def test_decode_run_entry_point_equals_single_tokens():
+    """``kvm_decode_run`` itself (n single-token steps issued by one C call, append counts of every step on the device)."""
+    import ctypes
+
+    from kvm_paper_b200 import _lib
+    from kvm_paper_b200.ops import _CCache, _stream_ptr, _tensor4
+
+    torch.manual_seed(10)
+    spec = ko.KvmSpec(4, 2, 64, 64, 32, 32, 2, 8, 1, "power_law", state_growth_factor=4.0, state_min_len=32)
+    B, T, n = 3, 32 * 4 + 20, 50
+    q = torch.randn(B, 4, T, 64).bfloat16()
+    k = torch.nn.functional.layer_norm(torch.randn(B, 2, T, 64), (64,)).bfloat16()
+    v = torch.randn(B, 2, T, 64).bfloat16()
+    g = (1 + torch.nn.functional.elu(torch.randn(B, 2, T, 1))).bfloat16()
+    params, plan, res = gh.device_prefill(spec, q, k, v, g)
+    mk = lambda: ops.decode_cache_from_prefill(params, res, k.cuda(), v.cuda(), g.cuda(), gh.desired_fn(spec), extra_capacity=64)  # noqa: E731
+    c1, c2 = mk(), mk()
+    dq = torch.randn(n, B, 4, 1, 64).bfloat16().cuda()
+    dk = torch.nn.functional.layer_norm(torch.randn(n, B, 2, 1, 64), (64,)).bfloat16().cuda()
+    dv = torch.randn(n, B, 2, 1, 64).bfloat16().cuda()
+    dg = (1 + torch.nn.functional.elu(torch.randn(n, B, 2, 1, 1))).bfloat16().cuda()
+    want = torch.stack([c1.step(dq[i], dk[i], dv[i], dg[i]).clone().view(B, -1) for i in range(n)])
+    counts, updates, rows = torch.full((n, B), -1, dtype=torch.int32), (ctypes.c_int32 * n)(), (ctypes.c_int32 * n)()
+    for i in range(n):
+        n_app, rows[i] = c2._plan_step()
+        if n_app is not None:
+            counts[i], updates[i] = torch.from_numpy(n_app), int((n_app >= 0).sum())
+    assert int(c2.state_len_h.max()) <= c2.memory.capacity and sum(updates) >= 3
+    counts, got = counts.cuda(), torch.empty(n, B, 4 * 64, device="cuda", dtype=torch.bfloat16)
+    cache = _CCache(c2.memory.c(), c2.ring_k.data_ptr(), c2.ring_v.data_ptr(), c2.ring_gate.data_ptr(), c2.total_len.data_ptr(),
+                    c2.state_len.data_ptr())
+    _lib.check(_lib.load().kvm_decode_run(
+        ctypes.byref(params.c), B, cache, n, _tensor4(dq[0], "q"), _tensor4(dk[0], "k"), _tensor4(dv[0], "v"), _tensor4(dg[0], "gate"),
+        dq.stride(0), dk.stride(0), dg.stride(0), counts.data_ptr(), updates, rows, got.data_ptr(), c2._ws.data_ptr(), c2._ws_bytes,
+        _stream_ptr(c2.device)))
+    c2.check_status()
+    assert torch.equal(got, want)
+    assert torch.equal(c1.memory.k_sum, c2.memory.k_sum) and torch.equal(c1.total_len, c2.total_len) and torch.equal(c1.state_len, c2.state_len)

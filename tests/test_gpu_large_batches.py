@@ -75,3 +75,52 @@ def test_many_sequences_update_at_one_token(B):
         _close(got, want)
     assert int(big.state_len_h[0]) > before and big.update_count == 3 * B
     _same_state(big, small)
+
+
+# sequences of one length, tokens behind the prompt: more at a boundary than one span launch updates (the others wait for the
+# next), more tokens than one piece (a token's place in it is a byte), more sequences than a launch over spans takes
+@pytest.mark.parametrize("B,n", [(_lib.UPDATE_LIST_MAX + 6, 3 * C), (3, 2 * 128 + 9), (_lib.SPAN_BATCH_MAX + 5, C + 3)])
+def test_runs_of_many_sequences_or_tokens(B, n):
+    spec = gh.bf16_spec(SPEC)
+    params = gh.layer_params(spec)
+    gen = torch.Generator(device="cuda").manual_seed(B + n)
+    T, size = 3 * C, 60
+    prompt = tuple(t[:, :, :, 0].transpose(1, 2) for t in _inputs(gen, B, T))
+    (big,), small = _caches(params, spec, prompt, B), _caches(params, spec, prompt, size)
+    x = _inputs(gen, n, B)
+    got = big.run(*x)
+    want = torch.stack([torch.cat([c.step(*(t[j, i * size:(i + 1) * size] for t in x)) for i, c in enumerate(small)]) for j in range(n)])
+    assert got.shape == (n, B, H * D)
+    _close(got, want.view(n, B, -1))
+    assert big.update_count == sum(c.update_count for c in small) > 0
+    _same_state(big, small)
+
+
+def test_captured_token_reads_the_devices_lengths():
+    """A token captured once and replayed goes on from the lengths on the device, like tokens issued one by one."""
+    spec = gh.bf16_spec(SPEC)
+    params = gh.layer_params(spec)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    B, T, n = 5, 3 * C + 2, 9  # (no boundary on the way)
+    prompt = tuple(t[:, :, :, 0].transpose(1, 2) for t in _inputs(gen, B, T))
+    (a,), (b,) = _caches(params, spec, prompt, B), _caches(params, spec, prompt, B)
+    x = _inputs(gen, B)
+    for c in (a, b):  # (also: kernels loaded, attributes set)
+        c.step(*x)
+    fixed = tuple(t.clone() for t in x)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = a.step(*fixed)
+    for i in range(n):
+        x = _inputs(gen, B)
+        for dst, src in zip(fixed, x):
+            dst.copy_(src)
+        graph.replay()
+        _close(y, b.step(*x))
+    a.total_len_h += n - 1  # (the capture itself counted one token on the host)
+    a.commit_lengths()
+    x = _inputs(gen, B)
+    _close(a.step(*x), b.step(*x))
+    _same_state(a, [b])
