@@ -714,41 +714,71 @@ def run_decode(args, dev, rank, world, peaks):
             nbytes += int(rows.sum()) * H * 2 * D * 2
         return nbytes
 
-    nbytes = host_walk()
+    def span_bytes():
+        """The same for tokens given ahead: the rows of a sequence once per span (the tokens up to its next block boundary,
+        at most as many as one launch has columns for)."""
+        from kvm_paper_b200 import _lib
+        total = 0
+        for b in range(n_loc):
+            t, s, left = int(tl[b]), int(sl[b]), steps
+            while left:
+                if t % C == 0 and t > W * C:
+                    want = int(mixer._desired_state_len(t, t - W * C + C, s))
+                    s += min(max(want - s, 0), C)
+                n = min(left, C - t % C, _lib.SPAN_COLUMNS)
+                t, left = t + n, left - n
+                begin = max(0, -(-t // C) * C - W * C)
+                total += ((s if begin else 0) + t - begin) * H * 2 * D * 2
+        return total
 
-    def run_all():
-        out = cache.run(q, k, v, g)       # one C call per 32 tokens: two kernel launches per token
-        return sharding.gather_sequences(out, world, seq_dim=1)  # [steps, all sequences, H*D]
+    nbytes, nbytes_spans = host_walk(), span_bytes()
+    outs = torch.empty(steps, n_loc, H * D, device=dev, dtype=torch.bfloat16) if world > 1 else None
 
-    run_all()  # warm-up pass over the whole trajectory
+    def run_steps():  # one token for every sequence per call, as a server that samples between tokens has to
+        for i in range(steps):
+            y = cache.step(q[i], k[i], v[i], g[i])
+            if outs is not None:
+                outs[i].copy_(y.view(n_loc, -1))
+        return y if outs is None else sharding.gather_sequences(outs, world, seq_dim=1)  # [steps, all sequences, H*D]
+
+    def run_given():  # all tokens given ahead (scoring a continuation)
+        return sharding.gather_sequences(cache.run(q, k, v, g), world, seq_dim=1)
+
+    def timed(fn, nbytes):
+        """(device time of the trajectory, host time, bytes per GPU), behind a warm-up pass over all of it."""
+        fn()
+        restore()
+        if world > 1:
+            dist.barrier()
+        torch.cuda.synchronize()
+        a, b_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0 = time.perf_counter()
+        a.record()
+        fn()
+        b_.record()
+        if world > 1:
+            dist.barrier()
+        torch.cuda.synchronize()
+        wall = time.perf_counter() - t0
+        t = torch.tensor([a.elapsed_time(b_)], device=dev, dtype=torch.float64)
+        nb = torch.tensor([float(nbytes)], device=dev, dtype=torch.float64)
+        if world > 1:
+            dist.all_reduce(t, op=dist.ReduceOp.MAX)
+            dist.all_reduce(nb, op=dist.ReduceOp.SUM)
+        return float(t.item()), wall, float(nb.item()) / world
+
+    given_ms, _, given_nb = timed(run_given, nbytes_spans)
     restore()
-    if world > 1:
-        dist.barrier()
-    torch.cuda.synchronize()
-    a, b_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    t0 = time.perf_counter()
-    a.record()
-    run_all()
-    b_.record()
-    if world > 1:
-        dist.barrier()
-    torch.cuda.synchronize()
-    wall = time.perf_counter() - t0
-    t = torch.tensor([a.elapsed_time(b_)], device=dev, dtype=torch.float64)
-    nb = torch.tensor([float(nbytes)], device=dev, dtype=torch.float64)
-    if world > 1:
-        dist.all_reduce(t, op=dist.ReduceOp.MAX)
-        dist.all_reduce(nb, op=dist.ReduceOp.SUM)
-    ms = float(t.item())
-    gbs = float(nb.item()) / world / (ms * 1e-3) / 1e9  # per GPU
+    updates0 = cache.update_count
+    ms, wall, nb = timed(run_steps, nbytes)
+    n_memory_updates = (cache.update_count - updates0) // 2  # (the warm-up pass ran the same ones)
+    gbs = nb / (ms * 1e-3) / 1e9  # per GPU
     status = "ok"
     try:
         cache.check_status()
     except Exception as exc:
         status = str(exc)
-    n_memory_updates = int(cache.update_count)
-    # the drop-in route: one call of KvmDecodeCache.step per token (what forward_single does), host bookkeeping,
-    # pinned copy and ctypes call included
+    # the same by the host's clock: bookkeeping and ctypes call of every token included
     restore()
     n_api = min(steps, 256)
     torch.cuda.synchronize()
@@ -767,9 +797,13 @@ def run_decode(args, dev, rank, world, peaks):
             "roofline": {"bound": "hbm", "kernel": "kvm_decode_attn_kernel", "achieved": round(gbs, 1),
                          "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": round(gbs / peaks["hbm_gbs"], 4),
                          "peak_source": peaks["source"],
-                         "traffic": _traffic("kvm_decode_attn_kernel", float(nb.item()) / world / steps),
-                         "note": "algorithmic K/V bytes of all steps / whole-step device time (ring write, boundary updates "
-                                 "and combine included); achieved, traffic per token"}}
+                         "traffic": _traffic("kvm_decode_attn_kernel", nb / steps),
+                         "note": "algorithmic K/V bytes of all steps / whole-step device time (new tokens, boundary updates "
+                                 "and combine included); achieved, traffic per token"},
+            "given_tokens": {"api": "KvmDecodeCache.run, all tokens given ahead: rows read once per span of up to 32 tokens",
+                             "tokens_per_s": round(c["n_seq"] * steps / (given_ms * 1e-3), 1), "ms_per_token": round(given_ms / steps, 4),
+                             "achieved": round(given_nb / (given_ms * 1e-3) / 1e9, 1), "unit": "GB/s",
+                             "frac": round(given_nb / (given_ms * 1e-3) / 1e9 / peaks["hbm_gbs"], 4)}}
 
 
 # ------------------------------------------------------------------------------------ CPU oracle
