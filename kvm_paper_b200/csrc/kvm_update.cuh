@@ -900,8 +900,9 @@ __device__ void memory_update(const LayerDev& L, const TokenSrc& src, const Memo
       cp_async_commit();
       if constexpr (PKR) {
         // The first tile of the warp-level scan behind them: its gather takes as long as the phases in between (1 x 4096 tokens,
-        // 8 heads x 64: 392.6 -> 389 us).  A decode step's update, which still has its keys to prepare, gains nothing by it
-        // (64 sequences, 32 tokens: 494 us with it, 482 without).
+        // 8 heads x 64, twelve processes of either kind in turn: 388.0 .. 392.7 us, mean 390.2; without 391.9 .. 395.0, mean
+        // 392.6).  A decode step's update, which still has its keys to prepare, gains nothing by it (64 sequences, 32 tokens:
+        // 494 us with it, 482 without).
         first_in_flight = n_merge > 0 && scan_e > scan_b;
         if (first_in_flight) scan_load_tile<D, NT>(s.btile, view.k, view.cur, scan_b, scan_e, tid);
         cp_async_commit();

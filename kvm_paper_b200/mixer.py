@@ -6,9 +6,13 @@ has the constructor, config fields, parameter names, ``forward`` / ``forward_inf
 ``forward_prefill`` / ``forward_single`` signatures and carried-state layout of
 ``model.kvm_mixer.SequenceMixer`` and ``model.kvm_triton_mixer.SequenceMixer`` of the reference.
 
-Host code (this file) = the projections, token shift, value residual, q/k LayerNorm, RoPE and merge
-gate in PyTorch (reference: model/value_residual_mixin.py:173-237, model/kvm_mixer.py:367-401);
-everything between the post-QKV tensors and the input of ``c_proj`` runs in the CUDA library.
+What runs where: everything between the post-QKV tensors and the input of ``c_proj`` is the CUDA
+library's, always.  The prefix (reference: model/value_residual_mixin.py:173-237,
+model/kvm_mixer.py:367-401) of bf16 modules is one library kernel behind the projections (value
+residual, token shift, q/k LayerNorm, rotary embedding, merge gate); a prompt, and a cached token with
+its projections and ``c_proj``, are one library call where nothing looks between the stages.  Linear
+layers over up to 128 rows run in the library, over more in PyTorch.  Other modules (fp32, the
+post-shift residual, ``use_fused_prologue = False``) run the prefix in PyTorch.
 There is no CPU or eager fallback: without a CUDA device or without the built library the
 attention entry points raise.
 """
