@@ -325,7 +325,8 @@ class SequenceMixer(nn.Module):
     def _prologue_params_kept(self, device) -> ops.PrologueParams:
         """``prologue_params``, kept as long as it consists of views of the parameters (a copy would miss what is written
         to a parameter behind autograd's back).  A module with a ``prologue_params`` of its own is asked on every call."""
-        if "prologue_params" in self.__dict__ or type(self).prologue_params is not SequenceMixer.prologue_params:
+        own = type(self)
+        if "prologue_params" in self.__dict__ or (own is not SequenceMixer and own.prologue_params is not SequenceMixer.prologue_params):
             return self.prologue_params(device)
         ln = isinstance(self.ln_q, nn.LayerNorm)
         src = [t for m in (self.ln_q, self.ln_k) if isinstance(m, nn.LayerNorm) for t in (m.weight, m.bias)]
@@ -348,9 +349,11 @@ class SequenceMixer(nn.Module):
 
     def _mixes_in_kernel(self) -> bool:
         """The "rwkv" value residual that the prologue kernel forms itself: the class's own value gate over bf16 parameters."""
-        return (self.value_residual_mode == "rwkv" and self.v_gate0.dtype == torch.bfloat16
-                and self.v_gate0.numel() == self.value_projection_size and "_value_gate" not in self.__dict__
-                and type(self)._value_gate is SequenceMixer._value_gate)
+        if self.value_residual_mode != "rwkv":
+            return False
+        own, v_gate0 = type(self), self.v_gate0
+        return (v_gate0.dtype is torch.bfloat16 and v_gate0.numel() == self.value_projection_size and "_value_gate" not in self.__dict__
+                and (own is SequenceMixer or own._value_gate is SequenceMixer._value_gate))
 
     def _mixed_values(self, x, v, v_first, v_gate):
         """Values for the prologue kernel: (v, None, None), mixed here, or (v, what the kernel mixes in, room for the last
@@ -380,7 +383,8 @@ class SequenceMixer(nn.Module):
         """Up to 128 rows (tokens x sequences) the linear layers are bound by reading the weights and by launches: the
         library's kernel takes all layers of one input at once.  More rows are left to the library GEMMs, and so is
         whatever else looks at the modules' calls (autocast, hooks on all modules)."""
-        return (0 < x.size(0) * x.size(1) <= _lib.PROJECT_ROWS_MAX and x.is_cuda and x.dtype is torch.bfloat16
+        B, T = x.shape[:2]
+        return (0 < B * T <= _lib.PROJECT_ROWS_MAX and x.is_cuda and x.dtype is torch.bfloat16
                 and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
                 and not (_module._global_forward_hooks or _module._global_forward_pre_hooks))
 
@@ -457,9 +461,11 @@ class SequenceMixer(nn.Module):
     def _unwatched(self, stage: str) -> bool:
         """Nobody looks at the tensors between the stages of a call (no hook, no override of the stage behind the prefix):
         the stages may run as one library call."""
-        stages = (stage, "forward_prefix_fused", "prefill_raw")
-        return not (self.capture_routes or self.check_device_status or torch.is_grad_enabled()
-                    or any(n in self.__dict__ or getattr(type(self), n) is not getattr(SequenceMixer, n) for n in stages))
+        d, own = self.__dict__, type(self)
+        if (self.capture_routes or self.check_device_status or torch.is_grad_enabled() or stage in d or "forward_prefix_fused" in d
+                or "prefill_raw" in d):
+            return False
+        return own is SequenceMixer or all(getattr(own, n) is getattr(SequenceMixer, n) for n in (stage, "forward_prefix_fused", "prefill_raw"))
 
     def _prompt(self, x, v_first, position_embeddings, past_key_values):
         """``forward_prefix_fused`` and ``forward_prefill`` of a prompt in one library call between the linear layers; the

@@ -350,10 +350,13 @@ def _prologue_arg(params: LayerParams, pro: PrologueParams, q_lin, k_lin, v_lin,
     arg.q_stride_t, arg.k_stride_t, arg.v_stride_t = (
         _token_stride(t, B, T, h * D, n) for n, t, h in (("q", q_lin, Hq), ("k", k_lin, Hkv), ("v", v_lin, Hkv)))
     if gate_lin is not None:
-        if gate_lin.dtype is not torch.bfloat16 or gate_lin.shape != (B, T, Hkv) or _row_step(gate_lin.stride(), B, T, Hkv) is None:
+        fits = gate_lin.dtype is torch.bfloat16 and gate_lin.is_cuda and gate_lin.shape == (B, T, Hkv)
+        step = _row_step(gate_lin.stride(), B, T, Hkv) if fits else None
+        if step is None:
             gate_lin = gate_lin.to(torch.bfloat16).reshape(B, T, Hkv).contiguous()
             keep.append(gate_lin)
-        arg.gate_lin, arg.gate_stride_t = gate_lin.data_ptr(), _token_stride(gate_lin, B, T, Hkv, "gate")
+            step = _token_stride(gate_lin, B, T, Hkv, "gate")
+        arg.gate_lin, arg.gate_stride_t = gate_lin.data_ptr(), step
     if value_residual is not None:
         v_first = _first_values(value_residual[0], B, T, Hkv * D, dev)
         v_gate, v_gate0 = (_aligned(t.to(dev, torch.bfloat16)) for t in value_residual[1:])
@@ -436,13 +439,15 @@ def project(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
 def project_checked(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
     """``project`` for a caller that has looked at the weights' types, shapes and devices."""
     rows, width = x.shape
-    if x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < width or x.data_ptr() % 16:
+    step, inner = x.stride()
+    if inner != 1 or step % 8 or step < width or x.data_ptr() % 16:
         x = x.clone(memory_format=torch.contiguous_format)
+        step = x.stride(0)
     n = len(weights)
     sizes = [w.shape[0] for w in weights]
     cols = (sum(sizes) + 7) // 8 * 8  # (16-byte aligned rows)
     out = torch.empty(rows, cols, device=x.device, dtype=torch.bfloat16)
-    rc = _lib.load().kvm_project(x.data_ptr(), x.stride(0), rows, width, (C.c_void_p * n)(*[w.data_ptr() for w in weights]),
+    rc = _lib.load().kvm_project(x.data_ptr(), step, rows, width, (C.c_void_p * n)(*[w.data_ptr() for w in weights]),
                                  (C.c_int32 * n)(*sizes), n, out.data_ptr(), cols, _stream_ptr(x.device))
     if rc:
         _lib.check(rc)
