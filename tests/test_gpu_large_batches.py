@@ -16,10 +16,10 @@ SPEC = ko.KvmSpec(H, H, D, D, D // 2, C, 2, 8, 1, "power_law", state_growth_fact
 FIELDS = ("k_sum", "v_sum", "vlen", "k_attn", "v_attn")
 
 
-def _inputs(gen, *lead):
+def _inputs(gen, *lead, h=H):
     rnd = lambda *s: torch.randn(*lead, *s, generator=gen, device="cuda")  # noqa: E731
     norm = lambda t: torch.nn.functional.layer_norm(t, (D,)).bfloat16()  # noqa: E731
-    return norm(rnd(H, 1, D)), norm(rnd(H, 1, D)), rnd(H, 1, D).bfloat16(), (1 + torch.nn.functional.elu(rnd(H, 1, 1))).bfloat16()
+    return norm(rnd(h, 1, D)), norm(rnd(h, 1, D)), rnd(h, 1, D).bfloat16(), (1 + torch.nn.functional.elu(rnd(h, 1, 1))).bfloat16()
 
 
 def _caches(params, spec, prompt, size):
@@ -34,7 +34,7 @@ def _caches(params, spec, prompt, size):
     return out
 
 
-def _same_state(big, small):
+def _same_state(big, small, h=H):
     """The batch `big` and the caches `small` of its sequences in order: lengths, live memory rows, rings."""
     for c in (big, *small):
         c.check_status()
@@ -45,7 +45,7 @@ def _same_state(big, small):
     for f in FIELDS:
         parts = torch.cat([getattr(c.memory, f)[:, :S] for c in small])
         for s, rows in enumerate(big.state_len_h.tolist()):
-            assert torch.equal(getattr(big.memory, f)[s * H:(s + 1) * H, :rows], parts[s * H:(s + 1) * H, :rows]), f
+            assert torch.equal(getattr(big.memory, f)[s * h:(s + 1) * h, :rows], parts[s * h:(s + 1) * h, :rows]), f
     for f in ("ring_k", "ring_v", "ring_gate"):
         assert torch.equal(getattr(big, f), torch.cat([getattr(c, f) for c in small])), f
 
@@ -124,3 +124,22 @@ def test_captured_token_reads_the_devices_lengths():
     x = _inputs(gen, B)
     _close(a.step(*x), b.step(*x))
     _same_state(a, [b])
+
+
+@pytest.mark.parametrize("B,h", [(255, 5), (255, 12), (290, 9)])
+def test_many_rows_end_in_one_cta(B, h):
+    """About eight, twenty and seventeen kv rows per CTA: the new tokens of the first eight are waited for by themselves, those
+    of all others together; lengths from the host and from the device."""
+    import dataclasses
+
+    spec = gh.bf16_spec(dataclasses.replace(SPEC, num_attention_heads=h, num_key_value_heads=h))
+    params = gh.layer_params(spec)
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    T, n, size = C + 5, 2 * C, 16
+    prompt = tuple(t[:, :, :, 0].transpose(1, 2) for t in _inputs(gen, B, T, h=h))
+    (big,), small = _caches(params, spec, prompt, B), _caches(params, spec, prompt, size)
+    for _ in range(n):
+        x = _inputs(gen, B, h=h)
+        got = big.step(*x)
+        _close(got, torch.cat([c.step(*(t[i * size:(i + 1) * size] for t in x)) for i, c in enumerate(small)]))
+    _same_state(big, small, h)
